@@ -180,6 +180,12 @@ class StepGraphs {
 public:
     StepGraphs(cudaStream_t st, int steps) : st_(st), steps_(steps)
     {
+        // a stream that the caller is capturing takes the launches themselves
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (steps_ > 0 && (cudaStreamIsCapturing(st_, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) {
+            cudaGetLastError();
+            steps_ = 0;
+        }
         if (steps_ > 0) SWEEP_CUDA(cudaStreamCreateWithFlags(&cs_, cudaStreamNonBlocking));
     }
     StepGraphs(const StepGraphs&) = delete;
