@@ -20,524 +20,193 @@
 //     of u(it) every step, the last two states at the end; the reverse
 //     reconstructs the box minus the strips, restores the strips, takes the
 //     source back out of a strip cell, images, re-injects.
-// One thread per cell on 32 x 8 tiles (x, z in 2-D; x, y per z plane in
-// 3-D), shots on the grid's last axis, stencils through the read-only path.
+//
+// One launch per step and pass carries the stencils, the strips and the
+// image (`fwd`, `rev`), a second one the sources and receivers.  Four x cells
+// per thread (vec4.cuh) on pitched rows; a warp covers 32 x 4 (x, y) cells in
+// 3-D and 32 x 4 (x, z) in 2-D, shots fastest in the grid so that the cells of
+// one model tile meet in L2.  An axis's CPML runs, and its memories are read
+// and written, only where its profile reaches.
+//
+// Measured, order 4: the 16-shot 256 x 768 survey's steps 24 us forward and
+// 52 us reverse (31 and 66 + 31 + 14 us in nine launches with one cell per
+// thread; 8.5 and 26 us of field traffic at the copy rate), a 101 x 119 x 141
+// grid's with two shots 70 and 124 us (123 and 296 us; 20 and 50 us).  Bound
+// by latency at 64 registers a thread and, in the layers, by the memories'
+// taps.
 // Memory: boundary saving with fp32 strips in device memory (SWEEP_MEM_BOUNDARY).
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <vector>
 
 #include "common.cuh"
 #include "acoustic_orders.cuh"
+#include "acoustic_vec.cuh"
 
 namespace sweep {
 namespace aord {
 
-constexpr int MAXM = 7;
+using namespace avec;
 
-struct Geo {
-    int nd, B, nz, ny, nx, nt;      // ny = 1 in 2-D
-    long long S;                    // cells per shot
-    int pad[6];                     // z_lo, z_hi, y_lo, y_hi, x_lo, x_hi
-    int z0, z1, y0, y1, x0, x1;     // physical box
-    int rz0, rz1, ry0, ry1, rx0, rx1;   // reconstruction box (physical box minus the strips)
-    float dt, dz, dy, dx;
-    float lc[MAXM + 1], gc[MAXM + 1];
-    const float *az, *bz, *dbz, *ay, *by, *dby, *ax, *bx, *dbx;
-    const float* vp;
-    long long vps;                  // model stride between shots (0 or S)
-    int nsrc, nrec;
-    const int *src, *rec;           // (B, n, nd): x[, y], z
-    const float* wavelet;           // (B, nsrc, nt)
-    const int* cells;               // strip cells of a shot grid
-    int ns;
-};
+constexpr int kThreads = 256;
+// blocks per SM the step kernels are compiled for: what the taps' registers
+// leave (at order 4, no bound / 3 / 4 / 5 / 6 blocks took 27.3 / 24.8 / 22.0 / 26.5
+// / 30.0 ms on the 2-D survey's gradient, 43 / 36.7 / 33.8 / 44.8 / 58.7 ms on a
+// 101 x 119 x 141 grid's)
+constexpr int blocks_for(int m) { return m <= 2 ? 4 : m <= 4 ? 3 : 2; }
 
-__device__ __forceinline__ float ld(const float* p) { return __ldg(p); }
-__device__ __forceinline__ float tap(float uk, float u0) { return __fsub_rn(uk, u0); }
-
-// forward / reconstruction Laplacian along one axis (stride s, spacing h)
-template <int M>
-__device__ __forceinline__ float lap_f(const float* __restrict__ u, long long i, long long s, const Geo& G, float h)
+// the forward step on the core, and the strips of u
+template <int M, int ND>
+__global__ void __launch_bounds__(kThreads, blocks_for(M)) fwd(const Geo G, const Step A)
 {
-    const float u0 = ld(u + i);
-    if (M == 2)
-        return ((G.lc[1] * (ld(u + i - s) + ld(u + i + s)) + G.lc[2] * (ld(u + i - 2 * s) + ld(u + i + 2 * s))) -
-                2.5f * u0) /
-               (h * h);
-    float acc = G.lc[1] * (tap(ld(u + i - s), u0) + tap(ld(u + i + s), u0));
+    const Cell<ND> q(G);
+    if (!q.core) return;
+    const long long k = q.b * G.S + q.i;
+    F4 u0;
+    const F4 un = step_cells<M, ND>(G, q, A, k, u0);
+    store_core(G, q, A.unx + k, un);
+    if (!A.slot) return;
+    bool phys[4], rec[4], any;
+    lanes<ND>(G, q, phys, rec, any);
+    if (!any) return;
+    float* slot = A.slot + (long long)q.b * G.ns;
 #pragma unroll
-    for (int k = 2; k <= M; ++k) acc = acc + G.lc[k] * (tap(ld(u + i - k * s), u0) + tap(ld(u + i + k * s), u0));
-    return acc / (h * h);
+    for (int l = 0; l < 4; ++l)
+        if (phys[l] && !rec[l]) slot[strip_index<ND>(G, q.c[2], q.c[1], q.c[0] + l)] = u0.v[l];
 }
 
-// centred first derivative sum_k g_k (u_k - u_-k) / h
-template <int M>
-__device__ __forceinline__ float grad_c(const float* __restrict__ u, long long i, long long s, const Geo& G, float h)
+// lambda(it) on the core; u(it-1) on the physical box -- rebuilt in the
+// reconstruction box, the saved strips around it -- and its image with
+// lambda(it), before the step's residuals and source (`rev_events` adds what
+// these change).
+template <int M, int ND>
+__global__ void __launch_bounds__(kThreads, blocks_for(M)) rev(const Geo G, const Rev A)
 {
-    float acc = G.gc[1] * (ld(u + i + s) - ld(u + i - s));
+    const Cell<ND> q(G);
+    if (!q.core) return;
+    const long long k = q.b * G.S + q.i, mi = q.b * G.ms + q.i;
+    const F4 lx = adj_cells<M, ND>(G, q, A, k, mi);
+    store_core(G, q, A.lx + k, lx);
+    if (!A.rx) return;
+    bool phys[4], rec[4], any;
+    lanes<ND>(G, q, phys, rec, any);
+    if (!any) return;
+    const F4 u0 = v4::ldg(A.rn + k), up = v4::ldg(A.rp + k);
+    F4 un = u0;
+    if (rec[0] || rec[1] || rec[2] || rec[3]) un = recon_cells<M, ND>(G, A.rn, k, mi, u0, up);
+    const float* slot = A.slot + (long long)q.b * G.ns;
+    F4 g = v4::ld(A.g + k);
+    bool all = true;
 #pragma unroll
-    for (int k = 2; k <= M; ++k) acc = acc + G.gc[k] * (ld(u + i + k * s) - ld(u + i - k * s));
-    return acc / h;
-}
-
-// the fused d(a psi) / dx tap form of the 2-D forward
-template <int M>
-__device__ __forceinline__ float grad_apsi(const float* __restrict__ a, int ia, const float* __restrict__ psi,
-                                           long long i, long long s, const Geo& G, float h)
-{
-    float acc = G.gc[1] * (ld(a + ia + 1) * ld(psi + i + s) - ld(a + ia - 1) * ld(psi + i - s));
-#pragma unroll
-    for (int k = 2; k <= M; ++k)
-        acc = acc + G.gc[k] * (ld(a + ia + k) * ld(psi + i + k * s) - ld(a + ia - k) * ld(psi + i - k * s));
-    return acc / h;
-}
-
-// ------------------------------------------------------------------- 2-D
-struct Step2 {
-    const float *un, *up;
-    float* unx;
-    const float *psx, *psz;         // CPML psi (read)
-    float *psxn, *pszn;             // (written)
-    float *zx, *zz;                 // zeta, in place
-};
-
-// u_next = (2 u - u_prev) + v^2 dt^2 w on [M, n - M)^2 (reference
-// acoustic2d/forward_split.cu:86-168)
-template <int M>
-__global__ void __launch_bounds__(256) fwd2(const Geo G, Step2 A)
-{
-    const int ix = blockIdx.x * 32 + threadIdx.x, iz = blockIdx.y * 8 + threadIdx.y, b = blockIdx.z;
-    if (ix < M || ix >= G.nx - M || iz < M || iz >= G.nz - M) return;
-    const long long o = b * G.S, i = (long long)iz * G.nx + ix;
-    const float* un = A.un + o;
-    const float* vp = G.vp + b * G.vps;
-    const float lx = lap_f<M>(un, i, 1, G, G.dx), lz = lap_f<M>(un, i, G.nx, G, G.dz);
-    const float v = ld(vp + i);
-    const float v2dt2 = ((v * v) * G.dt) * G.dt;
-    const int pml_x0 = G.pad[4] + M, pml_x1 = G.nx - (G.pad[5] + M);
-    const int pml_z0 = G.pad[0] + M, pml_z1 = G.nz - (G.pad[1] + M);
-    const bool cx = ix < pml_x0 + M || ix >= pml_x1 - M;
-    const bool cz = iz < pml_z0 + M || iz >= pml_z1 - M;
-    float w;
-    if (!cx && !cz) {
-        w = lx + lz;
+    for (int l = 0; l < 4; ++l) {
+        all &= phys[l];
+        if (!phys[l]) continue;
+        if (!rec[l]) un.v[l] = __ldg(slot + strip_index<ND>(G, q.c[2], q.c[1], q.c[0] + l));
+        g.v[l] += ((un.v[l] - 2.f * u0.v[l]) + up.v[l]) * lx.v[l];
+    }
+    v4::st(A.g + k, g);
+    if (all) {
+        v4::st(A.rx + k, un);
     } else {
-        w = 0.f;
-        if (cx) {
-            const float* ps = A.psx + o;
-            float* zt = A.zx + o;
-            const float a = G.ax[ix], bb = G.bx[ix], db = G.dbx[ix];
-            const float du = grad_c<M>(un, i, 1, G, G.dx);
-            const float dap = grad_apsi<M>(G.ax, ix, ps, i, 1, G, G.dx);
-            const float tmp = ((1.f + bb) * lx + db * du) + dap;
-            const float z = zt[i];
-            w = w + ((1.f + bb) * tmp + a * z);
-            A.psxn[o + i] = bb * du + a * ps[i];
-            zt[i] = bb * tmp + a * z;
-        } else {
-            w = w + lx;
-        }
-        if (cz) {
-            const float* ps = A.psz + o;
-            float* zt = A.zz + o;
-            const float a = G.az[iz], bb = G.bz[iz], db = G.dbz[iz];
-            const float du = grad_c<M>(un, i, G.nx, G, G.dz);
-            const float dap = grad_apsi<M>(G.az, iz, ps, i, G.nx, G, G.dz);
-            const float tmp = ((1.f + bb) * lz + db * du) + dap;
-            const float z = zt[i];
-            w = w + ((1.f + bb) * tmp + a * z);
-            A.pszn[o + i] = bb * du + a * ps[i];
-            zt[i] = bb * tmp + a * z;
-        } else {
-            w = w + lz;
-        }
+#pragma unroll
+        for (int l = 0; l < 4; ++l)
+            if (phys[l]) A.rx[k + l] = un.v[l];
     }
-    A.unx[o + i] = (2.f * un[i] - ld(A.up + o + i)) + v2dt2 * w;
 }
 
-struct Adj2 {
-    const float *ln, *lp;
-    float* lnx;
-    const float *psx, *psz, *zx, *zz;       // adjoint CPML memories (read)
-    float *psxo, *pszo, *zxo, *zzo;         // (written)
+// ---------------------------------------------------- sources and receivers
+// cell of location l (x[, y], z) as z, y, x, or false off the grid
+__device__ __forceinline__ bool cell_at(const Geo& G, const int* l, int& z, int& y, int& x)
+{
+    x = l[0];
+    y = G.nd == 3 ? l[1] : 0;
+    z = l[G.nd - 1];
+    return x >= 0 && x < G.nx && y >= 0 && y < G.ny && z >= 0 && z < G.nz;
+}
+__device__ __forceinline__ long long offset(const Geo& G, int b, int z, int y, int x)
+{
+    return b * G.S + ((long long)z * G.SZ + y * G.SY + x);
+}
+__device__ __forceinline__ bool in_box_nd(const Geo& G, const int* lo, const int* hi, int z, int y, int x)
+{
+    return G.nd == 3 ? in_box<3>(lo, hi, z, y, x) : in_box<2>(lo, hi, z, y, x);
+}
+
+// Forward: u(cell) += wavelet[b, s, it] at the shot's sources, then (after a
+// block barrier when `part` asks for both) record[b, it, r] = u(cell) at its
+// receivers; records start zeroed, off-grid receivers stay 0.  One block per
+// shot and part 3, or blocks over part 1 / part 2.
+enum { PART_SRC = 1, PART_REC = 2 };
+
+__global__ void fwd_events(const Geo G, float* u, float* record, int it, int part)
+{
+    const int b = blockIdx.y;
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    int z, y, x;
+    if (part & PART_SRC)
+        for (int s = t0; s < G.nsrc; s += step) {
+            const long long e = (long long)b * G.nsrc + s;
+            if (cell_at(G, G.src + e * G.nd, z, y, x)) atomicAdd(u + offset(G, b, z, y, x), G.wavelet[e * G.nt + it]);
+        }
+    if (part == (PART_SRC | PART_REC)) __syncthreads();
+    if (part & PART_REC)
+        for (int r = t0; r < G.nrec; r += step)
+            if (cell_at(G, G.rec + ((long long)b * G.nrec + r) * G.nd, z, y, x))
+                record[((long long)b * G.nt + it) * G.nrec + r] = __ldcg(u + offset(G, b, z, y, x));
+}
+
+// Reverse, after `rev`: the residuals into lambda(it) and what they add to the
+// image; then the wavelet gradient, and the source put back: into u(it-1) in
+// the reconstruction box; a strip cell was restored with it, so there its
+// share leaves the image.
+struct RevEv {
+    float *lx, *rx;                 // rx null at it = 0
+    const float *rn, *rp, *adj;
+    float *g, *gwav;                // gwav null: no wavelet gradient
+    int add_src;
 };
 
-// exact adjoint step (reference acoustic2d/adjoint_split.cu:27-196): the pure
-// interior in difference form around gw = ((v v) dt^2) lambda; elsewhere the
-// transposed CPML terms along both axes
-template <int M>
-__global__ void __launch_bounds__(256) adj2(const Geo G, Adj2 A)
+__global__ void rev_events(const Geo G, const RevEv A, int it, int part)
 {
-    const int ix = blockIdx.x * 32 + threadIdx.x, iz = blockIdx.y * 8 + threadIdx.y, b = blockIdx.z;
-    if (ix < M || ix >= G.nx - M || iz < M || iz >= G.nz - M) return;
-    const long long o = b * G.S, i = (long long)iz * G.nx + ix;
-    const int nx = G.nx;
-    const float* vp = G.vp + b * G.vps;
-    const float* ln = A.ln + o;
-    const float dt2 = G.dt * G.dt;
-    const float invdx2 = 1.f / (G.dx * G.dx), invdz2 = 1.f / (G.dz * G.dz);
-    const float invdx = 1.f / G.dx, invdz = 1.f / G.dz;
-    const int ix_in0 = G.pad[4] + 2 * M + 1, ix_in1 = nx - (G.pad[5] + 2 * M + 1);
-    const int iz_in0 = G.pad[0] + 2 * M + 1, iz_in1 = G.nz - (G.pad[1] + 2 * M + 1);
-    auto gwat = [&](long long n) { const float v = ld(vp + n); return ((v * v) * dt2) * ld(ln + n); };
-    const float gun = ld(ln + i);
-    float c0c = ld(vp + i);
-    c0c = (c0c * c0c) * dt2;
-    const float gw = c0c * gun;
-    const bool pure = ix >= ix_in0 && ix < ix_in1 && iz >= iz_in0 && iz < iz_in1;
-    if (pure) {
-        float lx = 0.f, lz = 0.f;
-#pragma unroll
-        for (int k = 1; k <= M; ++k) {
-            lx = lx + G.lc[k] * (tap(gwat(i + k), gw) + tap(gwat(i - k), gw));
-            lz = lz + G.lc[k] * (tap(gwat(i + (long long)k * nx), gw) + tap(gwat(i - (long long)k * nx), gw));
+    const int b = blockIdx.y;
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    int z, y, x;
+    if (part & PART_REC)
+        for (int r = t0; r < G.nrec; r += step) {
+            if (!cell_at(G, G.rec + ((long long)b * G.nrec + r) * G.nd, z, y, x)) continue;
+            const long long o = offset(G, b, z, y, x);
+            const float res = __ldg(A.adj + ((long long)b * G.nt + it) * G.nrec + r);
+            atomicAdd(A.lx + o, res);
+            if (A.rx && in_box_nd(G, G.lo, G.hi, z, y, x))
+                atomicAdd(A.g + o, ((A.rx[o] - 2.f * A.rn[o]) + A.rp[o]) * res);
         }
-        A.lnx[o + i] = ((2.f * gun - ld(A.lp + o + i)) + lx * invdx2) + lz * invdz2;
-        return;
-    }
-    const float *psx = A.psx + o, *psz = A.psz + o, *zx = A.zx + o, *zz = A.zz + o;
-    const float ax_ = G.ax[ix], az_ = G.az[iz], bx_ = G.bx[ix], bz_ = G.bz[iz];
-    const float gtx0 = bx_ * zx[i] + (1.f + bx_) * gw;
-    const float gtz0 = bz_ * zz[i] + (1.f + bz_) * gw;
-    auto gtx = [&](long long n, int c) {
-        const float v = ld(vp + n);
-        return G.bx[c] * zx[n] + ((1.f + G.bx[c]) * ((v * v) * dt2)) * ld(ln + n);
-    };
-    auto gtz = [&](long long n, int c) {
-        const float v = ld(vp + n);
-        return G.bz[c] * zz[n] + ((1.f + G.bz[c]) * ((v * v) * dt2)) * ld(ln + n);
-    };
-    const float lx0 = (1.f + bx_) * gtx0;
-    float Lx = 0.f, Dgx = 0.f, Dqx = 0.f;
-#pragma unroll
-    for (int k = 1; k <= M; ++k) {
-        const long long np = i + k, nm = i - k;
-        const int cp = ix + k, cm = ix - k;
-        const float tp = gtx(np, cp), tm = gtx(nm, cm);
-        const float bp = G.bx[cp], bm = G.bx[cm];
-        Lx = Lx + G.lc[k] * (tap((1.f + bp) * tp, lx0) + tap((1.f + bm) * tm, lx0));
-        Dgx = Dgx + G.gc[k] * ((bp * psx[np] + G.dbx[cp] * tp) - (bm * psx[nm] + G.dbx[cm] * tm));
-        Dqx = Dqx + G.gc[k] * (tp - tm);
-    }
-    Lx = Lx * invdx2; Dgx = Dgx * invdx; Dqx = Dqx * invdx;
-    const float lz0 = (1.f + bz_) * gtz0;
-    float Lz = 0.f, Dgz = 0.f, Dqz = 0.f;
-#pragma unroll
-    for (int k = 1; k <= M; ++k) {
-        const long long np = i + (long long)k * nx, nm = i - (long long)k * nx;
-        const int cp = iz + k, cm = iz - k;
-        const float tp = gtz(np, cp), tm = gtz(nm, cm);
-        const float bp = G.bz[cp], bm = G.bz[cm];
-        Lz = Lz + G.lc[k] * (tap((1.f + bp) * tp, lz0) + tap((1.f + bm) * tm, lz0));
-        Dgz = Dgz + G.gc[k] * ((bp * psz[np] + G.dbz[cp] * tp) - (bm * psz[nm] + G.dbz[cm] * tm));
-        Dqz = Dqz + G.gc[k] * (tp - tm);
-    }
-    Lz = Lz * invdz2; Dgz = Dgz * invdz; Dqz = Dqz * invdz;
-    A.lnx[o + i] = (2.f * gun - ld(A.lp + o + i)) + (((Lx + Lz) - Dgx) - Dgz);
-    A.psxo[o + i] = ax_ * (psx[i] - Dqx);
-    A.pszo[o + i] = az_ * (psz[i] - Dqz);
-    A.zxo[o + i] = ax_ * (zx[i] + gw);
-    A.zzo[o + i] = az_ * (zz[i] + gw);
-}
-
-// ------------------------------------------------------------------- 3-D
-struct Step3 {
-    const float *un, *up;
-    float* unx;
-    const float* ps[3];             // CPML psi per axis (x, y, z), read
-    float* psn[3];                  // written
-    float* zt[3];                   // zeta per axis, in place
-};
-
-__device__ __forceinline__ bool cell3(const Geo& G, int M, int& b, int& iz, int& iy, int& ix)
-{
-    ix = blockIdx.x * 32 + threadIdx.x;
-    iy = blockIdx.y * 8 + threadIdx.y;
-    b = blockIdx.z / G.nz;
-    iz = blockIdx.z - b * G.nz;
-    return ix >= M && ix < G.nx - M && iy >= M && iy < G.ny - M && iz >= M && iz < G.nz - M;
-}
-
-// one axis of the 3-D forward's CPML shell: tmp = (((1 + b) lap + db du) +
-// a d(psi)) + d(a) psi; w += (1 + b) tmp + a zeta; psi' = b du + a psi;
-// zeta = b tmp + a zeta (reference acoustic3d/forward_split.cu:120-215)
-template <int M>
-__device__ __forceinline__ float shell3(const Geo& G, const float* __restrict__ un, long long i, long long s, int c,
-                                        const float* __restrict__ A_, const float* __restrict__ B_,
-                                        const float* __restrict__ DB_, const float* __restrict__ ps, float* psn,
-                                        float* zt, float l, float h)
-{
-    const float du = grad_c<M>(un, i, s, G, h);
-    const float dps = grad_c<M>(ps, i, s, G, h);
-    const float a = A_[c], bb = B_[c], db = DB_[c];
-    const float da = grad_c<M>(A_, c, 1, G, h);
-    const float p = ps[i];
-    const float tmp = ((((1.f + bb) * l + db * du) + a * dps) + da * p);
-    const float z = zt[i];
-    psn[i] = bb * du + a * p;
-    zt[i] = bb * tmp + a * z;
-    return (1.f + bb) * tmp + a * z;
-}
-
-template <int M>
-__global__ void __launch_bounds__(256) fwd3(const Geo G, Step3 A)
-{
-    int b, iz, iy, ix;
-    if (!cell3(G, M, b, iz, iy, ix)) return;
-    const long long sy = G.nx, sz = (long long)G.nx * G.ny;
-    const long long o = b * G.S, i = iz * sz + iy * sy + ix;
-    const float* un = A.un + o;
-    const float lx = lap_f<M>(un, i, 1, G, G.dx), ly = lap_f<M>(un, i, sy, G, G.dy),
-                lz = lap_f<M>(un, i, sz, G, G.dz);
-    const int px0 = G.pad[4] + M, px1 = G.nx - G.pad[5] - M;
-    const int py0 = G.pad[2] + M, py1 = G.ny - G.pad[3] - M;
-    const int pz0 = G.pad[0] + M, pz1 = G.nz - G.pad[1] - M;
-    const bool inx = ix < px0 + 1 || ix >= px1 - 1;
-    const bool iny = iy < py0 + 1 || iy >= py1 - 1;
-    const bool inz = iz < pz0 + 1 || iz >= pz1 - 1;
-    float w;
-    if (!inx && !iny && !inz) {
-        w = (lx + ly) + lz;
-    } else {
-        w = 0.f;
-        w = w + (inx ? shell3<M>(G, un, i, 1, ix, G.ax, G.bx, G.dbx, A.ps[0] + o, A.psn[0] + o, A.zt[0] + o, lx, G.dx)
-                     : lx);
-        w = w + (iny ? shell3<M>(G, un, i, sy, iy, G.ay, G.by, G.dby, A.ps[1] + o, A.psn[1] + o, A.zt[1] + o, ly, G.dy)
-                     : ly);
-        w = w + (inz ? shell3<M>(G, un, i, sz, iz, G.az, G.bz, G.dbz, A.ps[2] + o, A.psn[2] + o, A.zt[2] + o, lz, G.dz)
-                     : lz);
-    }
-    const float v = ld(G.vp + b * G.vps + i);
-    A.unx[o + i] = (2.f * un[i] - ld(A.up + o + i)) + (((v * v) * G.dt) * G.dt) * w;
-}
-
-// gw = ((v v) dt^2) lambda on every cell (the 3-D adjoint's taps read it)
-__global__ void gw3(const Geo G, const float* __restrict__ ln, float* __restrict__ gw)
-{
-    const long long n = (long long)G.B * G.S;
-    const float dt2 = G.dt * G.dt;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const long long b = k / G.S;
-        const float v = ld(G.vp + b * G.vps + (k - b * G.S));
-        gw[k] = ((v * v) * dt2) * ln[k];
-    }
-}
-
-struct Adj3 {
-    const float *ln, *lp, *gw;
-    float* lnx;
-    const float *ps[3], *zt[3];     // adjoint CPML memories (read)
-    float *pso[3], *zto[3];         // (written)
-};
-
-// exact 3-D adjoint step (reference acoustic3d/adjoint_split.cu:14-320)
-template <int M>
-__global__ void __launch_bounds__(256) adj3(const Geo G, Adj3 A)
-{
-    int b, iz, iy, ix;
-    if (!cell3(G, M, b, iz, iy, ix)) return;
-    const long long sy = G.nx, sz = (long long)G.nx * G.ny;
-    const long long o = b * G.S, i = iz * sz + iy * sy + ix;
-    const float* vp = G.vp + b * G.vps;
-    const float* ln = A.ln + o;
-    const float* gwb = A.gw + o;
-    const float dt2 = G.dt * G.dt;
-    const int c[3] = {ix, iy, iz};
-    const long long st[3] = {1, sy, sz};
-    const float h[3] = {G.dx, G.dy, G.dz};
-    const int lo[3] = {G.pad[4] + 2 * M + 1, G.pad[2] + 2 * M + 1, G.pad[0] + 2 * M + 1};
-    const int hi[3] = {G.nx - (G.pad[5] + 2 * M + 1), G.ny - (G.pad[3] + 2 * M + 1), G.nz - (G.pad[1] + 2 * M + 1)};
-    const float gun = ld(ln + i);
-    float c0c = ld(vp + i);
-    c0c = (c0c * c0c) * dt2;
-    const float gw = c0c * gun;
-    bool in[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) in[a] = c[a] < lo[a] || c[a] >= hi[a];
-    float L[3], Dg[3] = {0.f, 0.f, 0.f};
-    if (!in[0] && !in[1] && !in[2]) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            float acc = 0.f;
-#pragma unroll
-            for (int k = 1; k <= M; ++k)
-                acc = acc + G.lc[k] * (tap(ld(gwb + i + k * st[a]), gw) + tap(ld(gwb + i - k * st[a]), gw));
-            L[a] = acc;
+    if (part == (PART_SRC | PART_REC)) __syncthreads();
+    if (part & PART_SRC)
+        for (int s = t0; s < G.nsrc; s += step) {
+            const long long e = (long long)b * G.nsrc + s;
+            if (!cell_at(G, G.src + e * G.nd, z, y, x)) continue;
+            const long long o = offset(G, b, z, y, x);
+            const float l = __ldcg(A.lx + o);
+            if (A.gwav) A.gwav[e * G.nt + it] = l;
+            if (!A.rx) continue;
+            const float w = G.wavelet[e * G.nt + it];
+            const bool strip = in_box_nd(G, G.lo, G.hi, z, y, x) && !in_box_nd(G, G.rlo, G.rhi, z, y, x);
+            if (strip) atomicAdd(A.g + o, -w * l);
+            else if (A.add_src) atomicAdd(A.rx + o, w);
         }
-        A.lnx[o + i] = (((2.f * gun - ld(A.lp + o + i)) + L[0] * (1.f / (h[0] * h[0]))) + L[1] * (1.f / (h[1] * h[1]))) +
-                       L[2] * (1.f / (h[2] * h[2]));
-        return;
-    }
-    const float* av[3] = {G.ax, G.ay, G.az};
-    const float* bv[3] = {G.bx, G.by, G.bz};
-    const float* dbv[3] = {G.dbx, G.dby, G.dbz};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const float invh2 = 1.f / (h[a] * h[a]), invh = 1.f / h[a];
-        if (in[a]) {
-            const float *Av = av[a], *Bv = bv[a], *DB = dbv[a];
-            const float* Z = A.zt[a] + o;
-            const float* PS = A.ps[a] + o;
-            const float a_ = Av[c[a]], b_ = Bv[c[a]];
-            const float da = grad_c<M>(Av, c[a], 1, G, h[a]);
-            const float gt0 = b_ * Z[i] + (1.f + b_) * gw;
-            const float l0 = (1.f + b_) * gt0;
-            float Lq = 0.f, Dq = 0.f, Dgg = 0.f;
-#pragma unroll
-            for (int k = 1; k <= M; ++k) {
-                const long long np = i + k * st[a], nm = i - k * st[a];
-                const int cp = c[a] + k, cm = c[a] - k;
-                const float vpp = ld(vp + np), vpm = ld(vp + nm);
-                const float tp = Bv[cp] * Z[np] + ((1.f + Bv[cp]) * ((vpp * vpp) * dt2)) * ld(ln + np);
-                const float tm = Bv[cm] * Z[nm] + ((1.f + Bv[cm]) * ((vpm * vpm) * dt2)) * ld(ln + nm);
-                Lq = Lq + G.lc[k] * (tap((1.f + Bv[cp]) * tp, l0) + tap((1.f + Bv[cm]) * tm, l0));
-                Dgg = Dgg + G.gc[k] * ((Bv[cp] * PS[np] + DB[cp] * tp) - (Bv[cm] * PS[nm] + DB[cm] * tm));
-                Dq = Dq + G.gc[k] * (Av[cp] * tp - Av[cm] * tm);
-            }
-            L[a] = Lq * invh2;
-            Dg[a] = Dgg * invh;
-            Dq = Dq * invh;
-            A.pso[a][o + i] = (a_ * PS[i] + da * gt0) - Dq;
-            A.zto[a][o + i] = a_ * (Z[i] + gw);
-        } else {
-            float acc = 0.f;
-#pragma unroll
-            for (int k = 1; k <= M; ++k)
-                acc = acc + G.lc[k] * (tap(ld(gwb + i + k * st[a]), gw) + tap(ld(gwb + i - k * st[a]), gw));
-            L[a] = acc * invh2;
-        }
-    }
-    A.lnx[o + i] = (2.f * gun - ld(A.lp + o + i)) + (((((L[0] + L[1]) + L[2]) - Dg[0]) - Dg[1]) - Dg[2]);
 }
 
-// ------------------------------------------------------- per-step helpers
-// grid offset of location l (x[, y], z) of shot b, or -1 off the grid
-__device__ __forceinline__ long long loc_cell(const Geo& G, const int* l)
-{
-    const int x = l[0], y = G.nd == 3 ? l[1] : 0, z = l[G.nd - 1];
-    if (x < 0 || x >= G.nx || y < 0 || y >= G.ny || z < 0 || z >= G.nz) return -1;
-    return ((long long)z * G.ny + y) * G.nx + x;
-}
-
-__device__ __forceinline__ bool in_phys(const Geo& G, long long c)
-{
-    const int x = (int)(c % G.nx), r = (int)(c / G.nx), y = r % G.ny, z = r / G.ny;
-    return x >= G.x0 && x < G.x1 && y >= G.y0 && y < G.y1 && z >= G.z0 && z < G.z1;
-}
-
-__device__ __forceinline__ bool in_recon(const Geo& G, long long c)
-{
-    const int x = (int)(c % G.nx), r = (int)(c / G.nx), y = r % G.ny, z = r / G.ny;
-    return x >= G.rx0 && x < G.rx1 && y >= G.ry0 && y < G.ry1 && z >= G.rz0 && z < G.rz1;
-}
-
-// u(cell) += sign * wavelet[b, s, it] at every source (one thread per (shot, source))
-__global__ void inject_src(const Geo G, float* u, int it, float sign, int only_strip)
+// u(cell) += sign * wavelet[b, s, it] at every source in a strip (strip) or
+// outside the strips
+__global__ void add_src(const Geo G, float* u, int it, float sign, int strip)
 {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= G.B * G.nsrc) return;
     const int b = e / G.nsrc;
-    const long long c = loc_cell(G, G.src + (long long)e * G.nd);
-    if (c < 0) return;
-    if (only_strip && !(in_phys(G, c) && !in_recon(G, c))) return;
-    atomicAdd(u + b * G.S + c, sign * G.wavelet[(long long)e * G.nt + it]);
-}
-
-// lambda(cell) += adj[b, it, r] at every receiver
-__global__ void inject_res(const Geo G, float* l, const float* __restrict__ adj, int it)
-{
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= G.B * G.nrec) return;
-    const int b = e / G.nrec, r = e - b * G.nrec;
-    const long long c = loc_cell(G, G.rec + (long long)e * G.nd);
-    if (c < 0) return;
-    atomicAdd(l + b * G.S + c, adj[((long long)b * G.nt + it) * G.nrec + r]);
-}
-
-// record[b, it, r] = u(cell) (records start zeroed: off-grid receivers stay 0)
-__global__ void gather_rec(const Geo G, const float* __restrict__ u, float* record, int it)
-{
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= G.B * G.nrec) return;
-    const int b = e / G.nrec, r = e - b * G.nrec;
-    const long long c = loc_cell(G, G.rec + (long long)e * G.nd);
-    if (c < 0) return;
-    record[((long long)b * G.nt + it) * G.nrec + r] = u[b * G.S + c];
-}
-
-// grad_wavelet[b, s, it] = lambda(cell) at every source
-__global__ void gather_src(const Geo G, const float* __restrict__ l, float* gwav, int it)
-{
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= G.B * G.nsrc) return;
-    const int b = e / G.nsrc;
-    const long long c = loc_cell(G, G.src + (long long)e * G.nd);
-    if (c < 0) return;
-    gwav[(long long)e * G.nt + it] = l[b * G.S + c];
-}
-
-// strip save (restore = 0) of u into one step slot (B, ns), or restore
-__global__ void strips(const Geo G, float* u, float* slot, int restore)
-{
-    const long long n = (long long)G.B * G.ns;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const long long b = e / G.ns;
-        const long long i = b * G.S + G.cells[e - b * G.ns];
-        if (restore) u[i] = slot[e];
-        else slot[e] = u[i];
-    }
-}
-
-// image 2 dt^2 u_tt lambda / v, u_tt = ((u(it-1) - 2 u(it)) + u(it+1)) / dt^2
-__device__ __forceinline__ void image(const Geo& G, long long b, long long c, const float* rx, const float* rn,
-                                      const float* rp, const float* ln, float* g)
-{
-    const long long i = b * G.S + c;
-    const float dt2 = G.dt * G.dt;
-    const float utt = ((rx[i] - 2.f * rn[i]) + rp[i]) / dt2;
-    g[i] = g[i] + ((((2.f * G.dt) * G.dt) * utt) * ln[i]) / ld(G.vp + b * G.vps + c);
-}
-
-__global__ void strip_image(const Geo G, const float* rx, const float* rn, const float* rp, const float* ln,
-                            float* g)
-{
-    const long long n = (long long)G.B * G.ns;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const long long b = e / G.ns;
-        image(G, b, G.cells[e - b * G.ns], rx, rn, rp, ln, g);
-    }
-}
-
-// u(it-1) = (2 u(it) - u(it+1)) + v^2 dt^2 Lap u(it) on the reconstruction box,
-// with the fused image (reference acoustic2d/kernels.cuh:474-528,
-// acoustic3d/forward_split.cu:292-372)
-template <int M>
-__global__ void __launch_bounds__(256) recon(const Geo G, const float* rn, const float* rp, float* rx,
-                                             const float* ln, float* g)
-{
-    int ix, iy, iz, b;
-    if (G.nd == 2) {
-        ix = blockIdx.x * 32 + threadIdx.x; iz = blockIdx.y * 8 + threadIdx.y; iy = 0; b = blockIdx.z;
-    } else {
-        ix = blockIdx.x * 32 + threadIdx.x; iy = blockIdx.y * 8 + threadIdx.y;
-        b = blockIdx.z / G.nz; iz = blockIdx.z - b * G.nz;
-    }
-    if (ix < G.rx0 || ix >= G.rx1 || iz < G.rz0 || iz >= G.rz1 || (G.nd == 3 && (iy < G.ry0 || iy >= G.ry1))) return;
-    const long long sy = G.nx, sz = (long long)G.nx * G.ny;
-    const long long o = (long long)b * G.S, c = iz * sz + iy * sy + ix;
-    const float* u = rn + o;
-    float w;
-    if (G.nd == 2) w = lap_f<M>(u, c, 1, G, G.dx) + lap_f<M>(u, c, sz, G, G.dz);
-    else w = (lap_f<M>(u, c, 1, G, G.dx) + lap_f<M>(u, c, sy, G, G.dy)) + lap_f<M>(u, c, sz, G, G.dz);
-    const float v = ld(G.vp + b * G.vps + c);
-    const float u0 = u[c], up = rp[o + c];
-    const float un = (2.f * u0 - up) + (((v * v) * G.dt) * G.dt) * w;
-    rx[o + c] = un;
-    const float dt2 = G.dt * G.dt;
-    const float utt = ((un - 2.f * u0) + up) / dt2;
-    g[o + c] = g[o + c] + ((((2.f * G.dt) * G.dt) * utt) * ln[o + c]) / v;
+    int z, y, x;
+    if (!cell_at(G, G.src + (long long)e * G.nd, z, y, x)) return;
+    const bool s = in_box_nd(G, G.lo, G.hi, z, y, x) && !in_box_nd(G, G.rlo, G.rhi, z, y, x);
+    if (s == (strip != 0)) atomicAdd(u + offset(G, b, z, y, x), sign * G.wavelet[(long long)e * G.nt + it]);
 }
 
 // illumination on the physical box: ir += lambda^2; is += u_tt^2 (is null:
@@ -548,8 +217,8 @@ __global__ void illum(const Geo G, const float* rx, const float* rn, const float
     const long long n = (long long)G.B * G.S;
     const float dt2 = G.dt * G.dt;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const long long c = k % G.S;
-        if (!in_phys(G, c)) continue;
+        const int c = (int)(k % G.S), x = c % G.P, r = c / G.P;
+        if (!in_box_nd(G, G.lo, G.hi, r / G.ny, r % G.ny, x)) continue;
         ir[k] += ln[k] * ln[k];
         if (is) {
             const float utt = ((rx[k] - 2.f * rn[k]) + rp[k]) / dt2;
@@ -558,23 +227,40 @@ __global__ void illum(const Geo G, const float* rx, const float* rn, const float
     }
 }
 
-// per-shot slots (B, S) -> out: (B, S) for per-shot models, else the sum over
-// shots in shot order
-__global__ void finalize(const Geo G, const float* __restrict__ slots, int per_shot, float* out)
+// per-shot slots (B, S) -> out, unpitched: (B, cells) for per-shot models, else
+// the sum over shots in shot order; image: times 2 / v (the factor 2 dt^2 / v
+// of the reference's image and the 1 / dt^2 of its u_tt)
+__global__ void finalize(const Geo G, const float* __restrict__ slots, int image, float* out)
 {
-    const long long n = per_shot ? (long long)G.B * G.S : G.S;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+    const long long cells = (long long)G.nz * G.ny * G.nx;
+    const bool per_shot = G.ms != 0;
+    const long long n = per_shot ? G.B * cells : cells;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+        const long long row = e / G.nx, k = row * G.P + (e - row * G.nx);
         float v = slots[k];
         if (!per_shot)
-            for (int b = 1; b < G.B; ++b) v += slots[(long long)b * G.S + k];
-        out[k] = v;
+            for (int b = 1; b < G.B; ++b) v += slots[b * G.S + k];
+        out[e] = image ? 2.f * v / G.vp[e] : v;
+    }
+}
+
+// model fields of the steps, pitched
+__global__ void prep(const Geo G, long long rows, float* __restrict__ cf, float* __restrict__ ca)
+{
+    const long long n = rows * G.P;
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+        const long long row = k / G.P;
+        const int x = (int)(k - row * G.P);
+        const float v = x < G.nx ? G.vp[row * G.nx + x] : 0.f;
+        cf[k] = ((v * v) * G.dt) * G.dt;
+        ca[k] = (v * v) * (G.dt * G.dt);
     }
 }
 
 // ------------------------------------------------------------------- host
 struct Plan {
     Geo G;
-    std::vector<int> cells;
+    int nm;                         // model copies
 };
 
 static Plan make_plan(const sweep_acoustic_desc* d, int mem_mode)
@@ -589,71 +275,61 @@ static Plan make_plan(const sweep_acoustic_desc* d, int mem_mode)
                   2 * d->M, mem_mode);
     SWEEP_REQUIRE(d->B >= 1 && d->nt >= 1, "acoustic: B and nt must be >= 1");
     SWEEP_REQUIRE(d->nsrc >= 0 && d->nrec >= 0, "acoustic: negative source/receiver count");
-    const int nf = d->ndim == 2 ? 4 : 6;
     for (int f = 0; f < 6; ++f)
         SWEEP_REQUIRE(d->pad[f] >= 0, "acoustic: negative PML pad on face %d", f);
-    (void)nf;
     Plan pl{};
     Geo& G = pl.G;
     const int M = d->M;
-    G.nd = d->ndim; G.B = d->B; G.nz = d->nz; G.nx = d->nx; G.nt = d->nt;
+    G.nd = d->ndim; G.B = d->B; G.nz = d->nz; G.nx = d->nx; G.nt = d->nt; G.M = M;
     G.ny = d->ndim == 3 ? d->ny : 1;
-    G.S = (long long)G.nz * G.ny * G.nx;
-    SWEEP_REQUIRE(G.S < (1LL << 31), "acoustic: one shot's grid must hold < 2^31 cells");
+    G.P = (G.nx + 7) / 8 * 8;
+    G.SY = G.P; G.SZ = G.ny * G.P;
+    G.S = (long long)G.nz * G.ny * G.P;
+    const long long cells = (long long)G.nz * G.ny * G.nx;
+    SWEEP_REQUIRE(cells < (1LL << 31) && G.S < (1LL << 31), "acoustic: one shot's grid must hold < 2^31 cells");
     SWEEP_REQUIRE(d->ndim == 2 || (long long)G.nz * G.B <= 65535, "acoustic: nz x shots must be <= 65535");
     SWEEP_REQUIRE(d->ndim == 3 || G.B <= 65535, "acoustic: at most 65535 shots per call");
-    for (int f = 0; f < 6; ++f) G.pad[f] = d->pad[f];
-    if (d->ndim == 2) { G.pad[2] = G.pad[3] = 0; }
-    G.z0 = G.pad[0] + M; G.z1 = G.nz - G.pad[1] - M;
-    G.x0 = G.pad[4] + M; G.x1 = G.nx - G.pad[5] - M;
-    if (d->ndim == 3) { G.y0 = G.pad[2] + M; G.y1 = G.ny - G.pad[3] - M; }
-    else { G.y0 = 0; G.y1 = 1; }
-    SWEEP_REQUIRE(G.z1 > G.z0 && G.x1 > G.x0 && G.y1 > G.y0, "acoustic: the physical box is empty");
-    G.rz0 = G.pad[0] + 2 * M + 1; G.rz1 = G.nz - (G.pad[1] + 2 * M + 1);
-    G.rx0 = G.pad[4] + 2 * M + 1; G.rx1 = G.nx - (G.pad[5] + 2 * M + 1);
-    if (d->ndim == 3) { G.ry0 = G.pad[2] + 2 * M + 1; G.ry1 = G.ny - (G.pad[3] + 2 * M + 1); }
-    else { G.ry0 = 0; G.ry1 = 1; }
-    G.dt = d->dt; G.dz = d->dz; G.dy = d->dy; G.dx = d->dx;
-    for (int k = 0; k <= MAXM; ++k) { G.lc[k] = k <= M ? d->lap[k] : 0.f; G.gc[k] = k <= M ? d->grad[k] : 0.f; }
-    G.az = d->az; G.bz = d->bz; G.dbz = d->dbz;
-    G.ay = d->ay; G.by = d->by; G.dby = d->dby;
-    G.ax = d->ax; G.bx = d->bx; G.dbx = d->dbx;
-    G.vp = d->vp;
-    SWEEP_REQUIRE(d->vp_stride == 0 || d->vp_stride == G.S, "acoustic: vp_stride must be 0 or the cells per shot");
-    G.vps = d->vp_stride;
-    G.nsrc = d->nsrc; G.nrec = d->nrec;
-    G.src = d->src_loc; G.rec = d->rec_loc; G.wavelet = d->wavelet;
+    const int n[3] = {G.nx, G.ny, G.nz};
+    const int plo[3] = {d->pad[4], d->pad[2], d->pad[0]}, phi[3] = {d->pad[5], d->pad[3], d->pad[1]};
+    const float h[3] = {d->dx, d->dy, d->dz};
     // strip cells: the physical box within M + 1 of its faces (widths clipped
     // on a thin box: boundary/strip.cuh:63-67)
-    const int w = M + 1;
-    auto widths = [&](int e, int& lo, int& hi) {
-        lo = std::min(w, std::max(e, 0));
-        hi = std::min(w, std::max(e - lo, 0));
-    };
-    int wzl, wzh, wyl, wyh, wxl, wxh;
-    widths(G.z1 - G.z0, wzl, wzh);
-    widths(G.y1 - G.y0, wyl, wyh);
-    widths(G.x1 - G.x0, wxl, wxh);
-    if (d->ndim == 2) { wyl = wyh = 0; }
-    for (int iz = G.z0; iz < G.z1; ++iz)
-        for (int iy = G.y0; iy < G.y1; ++iy)
-            for (int ix = G.x0; ix < G.x1; ++ix) {
-                const bool zs = iz < G.z0 + wzl || iz >= G.z1 - wzh;
-                const bool ys = iy < G.y0 + wyl || iy >= G.y1 - wyh;
-                const bool xs = ix < G.x0 + wxl || ix >= G.x1 - wxh;
-                if (zs || ys || xs) pl.cells.push_back((int)(((long long)iz * G.ny + iy) * G.nx + ix));
-            }
-    G.ns = (int)pl.cells.size();
+    for (int a = 0; a < 3; ++a) {
+        if (G.nd == 2 && a == 1) { G.lo[a] = G.rlo[a] = 0; G.hi[a] = G.rhi[a] = 1; continue; }
+        G.lo[a] = plo[a] + M; G.hi[a] = n[a] - phi[a] - M;
+        G.rlo[a] = G.lo[a] + M + 1; G.rhi[a] = G.hi[a] - (M + 1);
+        G.wl[a] = std::min(M + 1, std::max(G.hi[a] - G.lo[a], 0));
+        G.wh[a] = std::min(M + 1, std::max(G.hi[a] - G.lo[a] - G.wl[a], 0));
+        G.ih2[a] = 1.f / (h[a] * h[a]);
+        G.ih[a] = 1.f / h[a];
+    }
+    SWEEP_REQUIRE(G.hi[2] > G.lo[2] && G.hi[0] > G.lo[0] && G.hi[1] > G.lo[1], "acoustic: the physical box is empty");
+    const long long bx = G.hi[0] - G.lo[0], by = G.hi[1] - G.lo[1], bz = G.hi[2] - G.lo[2];
+    const long long byi = std::max(0LL, by - G.wl[1] - G.wh[1]), bzi = std::max(0LL, bz - G.wl[2] - G.wh[2]);
+    G.n_top = (int)(G.wl[2] * by * bx);
+    G.n_bot = (int)(G.wh[2] * by * bx);
+    G.nring = (int)((G.wl[1] + G.wh[1]) * bx + byi * (G.wl[0] + G.wh[0]));
+    G.ns = (int)(G.n_top + G.n_bot + bzi * G.nring);
+    G.dt = d->dt;
+    for (int k = 0; k <= MAXM; ++k) { G.lc[k] = k <= M ? d->lap[k] : 0.f; G.gc[k] = k <= M ? d->grad[k] : 0.f; }
+    G.vp = d->vp;
+    SWEEP_REQUIRE(d->vp_stride == 0 || d->vp_stride == cells, "acoustic: vp_stride must be 0 or the cells per shot");
+    G.ms = d->vp_stride ? G.S : 0;
+    pl.nm = d->vp_stride ? G.B : 1;
+    G.nsrc = d->nsrc; G.nrec = d->nrec;
+    G.src = d->src_loc; G.rec = d->rec_loc; G.wavelet = d->wavelet;
+    G.nbx = (G.nx + 31) / 32;
     return pl;
 }
 
 struct Ws {
-    int* cells;
+    float *cf, *ca;
+    float* prof[3];
     float* u[3];                    // forward: u_prev, u, u_next; backward: reconstruction
     float* l[3];                    // backward: adjoint
     float* ps[2][3];                // CPML psi (forward) / adjoint psi, double-buffered
     float* zt[2][3];                // zeta (forward: [0] only) / adjoint zeta, double-buffered
-    float *g, *gw, *is, *ir;        // backward: per-shot image, gw buffer, illumination slots
+    float *g, *is, *ir;             // backward: per-shot image, illumination slots
     char *zero0, *zero1;
 };
 
@@ -662,14 +338,19 @@ static void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
     const Geo& G = pl.G;
     const long long n = (long long)G.B * G.S;
     w = Ws{};
-    w.cells = c.take<int>(std::max(G.ns, 1));
+    w.cf = c.take<float>(pl.nm * G.S);
+    w.ca = c.take<float>(pl.nm * G.S);
+    const int len[3] = {G.P + 2 * kGuard, G.ny + 2 * kGuard, G.nz + 2 * kGuard};
+    for (int a = 0; a < 3; ++a) w.prof[a] = c.take<float>(4LL * len[a]);
     c.take<char>(0);
     w.zero0 = c.base ? c.base + c.off : nullptr;
     for (int k = 0; k < 3; ++k) w.u[k] = c.take<float>(n);
     for (int s = 0; s < 2; ++s)
-        for (int a = 0; a < G.nd; ++a) w.ps[s][a] = c.take<float>(n);
+        for (int a = 0; a < 3; ++a)
+            if (a != 1 || G.nd == 3) w.ps[s][a] = c.take<float>(n);
     for (int s = 0; s < (rev ? 2 : 1); ++s)
-        for (int a = 0; a < G.nd; ++a) w.zt[s][a] = c.take<float>(n);
+        for (int a = 0; a < 3; ++a)
+            if (a != 1 || G.nd == 3) w.zt[s][a] = c.take<float>(n);
     if (rev) {
         for (int k = 0; k < 3; ++k) w.l[k] = c.take<float>(n);
         w.g = c.take<float>(n);
@@ -678,10 +359,18 @@ static void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
     }
     c.take<char>(0);
     w.zero1 = c.base ? c.base + c.off : nullptr;
-    if (rev && G.nd == 3) w.gw = c.take<float>(n);
 }
 
 static long long slot_floats(const Plan& pl) { return (long long)pl.G.B * pl.G.ns; }
+
+// The tape's states hold the grid's cells alone, without the rows' pitch.
+static long long state_floats(const Geo& G) { return (long long)G.B * G.nz * G.ny * G.nx; }
+
+static void copy_state(const Geo& G, float* dst, int dst_pitch, const float* src, int src_pitch, cudaStream_t st)
+{
+    SWEEP_CUDA(cudaMemcpy2DAsync(dst, (size_t)dst_pitch * 4, src, (size_t)src_pitch * 4, (size_t)G.nx * 4,
+                                 (size_t)G.B * G.nz * G.ny, cudaMemcpyDeviceToDevice, st));
+}
 
 void sizes(const sweep_acoustic_desc* d, int mem_mode, int, int64_t* ws_bytes, int64_t* tape_bytes)
 {
@@ -691,92 +380,107 @@ void sizes(const sweep_acoustic_desc* d, int mem_mode, int, int64_t* ws_bytes, i
     carve(f, pl, false, w);
     carve(r, pl, true, w);
     *ws_bytes = std::max(f.off, r.off);
-    *tape_bytes = ((long long)pl.G.nt * slot_floats(pl) + 2LL * pl.G.B * pl.G.S) * 4;
+    *tape_bytes = ((long long)pl.G.nt * slot_floats(pl) + 2 * state_floats(pl.G)) * 4;
+}
+
+// Rows of a 2-D block: 32, or 8 where that leaves the GPU with less than a
+// block per SM (a small grid's step is one round of memory latency, and lasts
+// as long as its fullest SM).
+static int rows_of(const Geo& G)
+{
+    return (long long)G.nbx * G.B * ((G.nz + 31) / 32) >= 2 * 148 ? 32 : 8;
 }
 
 static dim3 cell_grid(const Geo& G)
 {
-    if (G.nd == 2) return dim3((G.nx + 31) / 32, (G.nz + 7) / 8, (unsigned)G.B);
-    return dim3((G.nx + 31) / 32, (G.ny + 7) / 8, (unsigned)(G.nz * G.B));
+    if (G.nd == 2) return dim3((unsigned)(G.nbx * G.B), (unsigned)((G.nz + rows_of(G) - 1) / rows_of(G)));
+    return dim3((unsigned)(G.nbx * G.B), (G.ny + kBY - 1) / kBY, (G.nz + kBZ - 1) / kBZ);
 }
 
-static unsigned blocks_of(long long n, int per) { return (unsigned)std::max<long long>(std::min<long long>((n + per - 1) / per, 8192), 1); }
+static dim3 cell_block(const Geo& G) { return G.nd == 2 ? dim3(8, (unsigned)rows_of(G)) : dim3(8, kBY, kBZ); }
 
-template <int M>
-static void fwd_step(const Geo& G, const Ws& w, float* un, float* up, float* unx, int cur, cudaStream_t st)
+static unsigned blocks_of(long long n, int per)
 {
-    const dim3 grid = cell_grid(G), block(32, 8);
-    if (G.nd == 2) {
-        Step2 A{un, up, unx, w.ps[cur][0], w.ps[cur][1], w.ps[cur ^ 1][0], w.ps[cur ^ 1][1], w.zt[0][0], w.zt[0][1]};
-        fwd2<M><<<grid, block, 0, st>>>(G, A);
-    } else {
-        Step3 A{};
-        A.un = un; A.up = up; A.unx = unx;
-        for (int a = 0; a < 3; ++a) { A.ps[a] = w.ps[cur][a]; A.psn[a] = w.ps[cur ^ 1][a]; A.zt[a] = w.zt[0][a]; }
-        fwd3<M><<<grid, block, 0, st>>>(G, A);
-    }
+    return (unsigned)std::max<long long>(std::min<long long>((n + per - 1) / per, 8192), 1);
 }
 
-template <int M>
-static void adj_step(const Geo& G, const Ws& w, float* ln, float* lp, float* lnx, int cur, cudaStream_t st)
+static void setup(const sweep_acoustic_desc* d, Plan& pl, const Ws& w, cudaStream_t st)
 {
-    const dim3 grid = cell_grid(G), block(32, 8);
-    if (G.nd == 2) {
-        // the 2-D axes are x (slot 0) and z (slot 1)
-        Adj2 A{ln, lp, lnx, w.ps[cur][0], w.ps[cur][1], w.zt[cur][0], w.zt[cur][1],
-               w.ps[cur ^ 1][0], w.ps[cur ^ 1][1], w.zt[cur ^ 1][0], w.zt[cur ^ 1][1]};
-        adj2<M><<<grid, block, 0, st>>>(G, A);
-    } else {
-        gw3<<<blocks_of((long long)G.B * G.S, 256), 256, 0, st>>>(G, ln, w.gw);
-        Adj3 A{};
-        A.ln = ln; A.lp = lp; A.gw = w.gw; A.lnx = lnx;
-        for (int a = 0; a < 3; ++a) {
-            A.ps[a] = w.ps[cur][a]; A.zt[a] = w.zt[cur][a];
-            A.pso[a] = w.ps[cur ^ 1][a]; A.zto[a] = w.zt[cur ^ 1][a];
-        }
-        adj3<M><<<grid, block, 0, st>>>(G, A);
+    Geo& G = pl.G;
+    G.cf = w.cf; G.ca = w.ca;
+    const long long rows = (long long)pl.nm * G.nz * G.ny;
+    prep<<<blocks_of(rows * G.P, 256), 256, 0, st>>>(G, rows, w.cf, w.ca);
+    const float* in[3][3] = {{d->ax, d->bx, d->dbx}, {d->ay, d->by, d->dby}, {d->az, d->bz, d->dbz}};
+    const int n[3] = {G.nx, G.ny, G.nz};
+    for (int a = 0; a < 3; ++a) {
+        if (a == 1 && G.nd == 2) continue;
+        const int len = (a == 0 ? G.P : n[a]) + 2 * kGuard;
+        prep_profiles<<<blocks_of(len, 256), 256, 0, st>>>(in[a][0], in[a][1], in[a][2], n[a], G, G.ih[a], kGuard, len,
+                                                           w.prof[a]);
+        G.a[a] = w.prof[a] + kGuard; G.b[a] = G.a[a] + len; G.db[a] = G.b[a] + len; G.da[a] = G.db[a] + len;
     }
+    SWEEP_LAUNCH_CHECK();
+    SWEEP_CUDA(cudaMemsetAsync(w.zero0, 0, w.zero1 - w.zero0, st));
 }
 
-template <int M>
-static void forward_m(Plan& pl, float* record, void* tape, void* ws, int64_t ws_bytes, cudaStream_t st)
+// Sources and receivers of a step: one launch with a block per shot while a
+// block walks the receivers in a few rounds, else one launch per kind.
+constexpr int kEventBlock = 512;
+static bool one_launch(const Geo& G) { return G.nrec <= 4 * kEventBlock && G.nsrc <= 4 * kEventBlock; }
+static dim3 event_grid(const Geo& G, int n)
+{
+    return dim3((unsigned)std::max(1, (n + kEventBlock - 1) / kEventBlock), (unsigned)G.B);
+}
+
+template <int M, int ND>
+static void forward_m(const sweep_acoustic_desc* d, Plan& pl, float* record, void* tape, void* ws, int64_t ws_bytes,
+                      cudaStream_t st)
 {
     Carve c(ws);
     Ws w;
     carve(c, pl, false, w);
     SWEEP_REQUIRE(ws != nullptr && c.off <= ws_bytes, "acoustic forward: workspace too small (%lld < %lld bytes)",
                   (long long)ws_bytes, (long long)c.off);
-    Geo& G = pl.G;
-    G.cells = w.cells;
-    if (G.ns > 0)
-        SWEEP_CUDA(cudaMemcpyAsync(w.cells, pl.cells.data(), sizeof(int) * G.ns, cudaMemcpyHostToDevice, st));
-    SWEEP_CUDA(cudaMemsetAsync(w.zero0, 0, w.zero1 - w.zero0, st));
-    if (record && G.nrec > 0)
-        SWEEP_CUDA(cudaMemsetAsync(record, 0, sizeof(float) * (size_t)G.B * G.nt * G.nrec, st));
+    setup(d, pl, w, st);
+    const Geo& G = pl.G;
+    if (G.nrec == 0) record = nullptr;
+    if (record) SWEEP_CUDA(cudaMemsetAsync(record, 0, sizeof(float) * (size_t)G.B * G.nt * G.nrec, st));
     float* tp = static_cast<float*>(tape);
-    const long long n = (long long)G.B * G.S;
     float *up = w.u[0], *un = w.u[1], *unx = w.u[2];
     int cur = 0;
-    const unsigned sb = blocks_of(slot_floats(pl), 256);
+    const dim3 grid = cell_grid(G), block = cell_block(G);
+    const int parts = (G.nsrc > 0 ? PART_SRC : 0) | (record ? PART_REC : 0);
+    StepGraphs sg(st, resolve_graph_steps(-1));
     for (int it = 0; it < G.nt; ++it) {
-        fwd_step<M>(G, w, un, up, unx, cur, st);
-        if (tp && G.ns > 0) strips<<<sb, 256, 0, st>>>(G, un, tp + (long long)it * slot_floats(pl), 0);
-        if (G.nsrc > 0) inject_src<<<(G.B * G.nsrc + 127) / 128, 128, 0, st>>>(G, unx, it, 1.f, 0);
-        if (record && G.nrec > 0) gather_rec<<<(G.B * G.nrec + 127) / 128, 128, 0, st>>>(G, unx, record, it);
+        cudaStream_t s = sg.stream();
+        Step A{};
+        A.un = un; A.up = up; A.unx = unx;
+        for (int a = 0; a < 3; ++a) { A.ps[a] = w.ps[cur][a]; A.psn[a] = w.ps[cur ^ 1][a]; A.zt[a] = w.zt[0][a]; }
+        A.slot = tp ? tp + (long long)it * slot_floats(pl) : nullptr;
+        fwd<M, ND><<<grid, block, 0, s>>>(G, A);
+        if (parts && one_launch(G)) {
+            fwd_events<<<dim3(1, G.B), kEventBlock, 0, s>>>(G, unx, record, it, parts);
+        } else {
+            if (parts & PART_SRC) fwd_events<<<event_grid(G, G.nsrc), kEventBlock, 0, s>>>(G, unx, record, it, PART_SRC);
+            if (parts & PART_REC) fwd_events<<<event_grid(G, G.nrec), kEventBlock, 0, s>>>(G, unx, record, it, PART_REC);
+        }
         SWEEP_LAUNCH_CHECK();
+        sg.step_done();
         float* t = up; up = un; un = unx; unx = t;
         cur ^= 1;
     }
+    sg.flush();
     if (tp) {
         float* tail = tp + (long long)G.nt * slot_floats(pl);
-        SWEEP_CUDA(cudaMemcpyAsync(tail, up, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
-        SWEEP_CUDA(cudaMemcpyAsync(tail + n, un, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+        copy_state(G, tail, G.nx, up, G.P, st);
+        copy_state(G, tail + state_floats(G), G.nx, un, G.P, st);
     }
 }
 
-template <int M>
-static void backward_m(Plan& pl, const float* adj, const void* tape, float* grad_vp, float* grad_wavelet,
-                       float* illum_src, float* illum_rec, void* ws, int64_t ws_bytes, cudaStream_t st)
+template <int M, int ND>
+static void backward_m(const sweep_acoustic_desc* d, Plan& pl, const float* adj, const void* tape, float* grad_vp,
+                       float* grad_wavelet, float* illum_src, float* illum_rec, void* ws, int64_t ws_bytes,
+                       cudaStream_t st)
 {
     Carve c(ws);
     Ws w;
@@ -784,49 +488,64 @@ static void backward_m(Plan& pl, const float* adj, const void* tape, float* grad
     SWEEP_REQUIRE(ws != nullptr && c.off <= ws_bytes, "acoustic backward: workspace too small (%lld < %lld bytes)",
                   (long long)ws_bytes, (long long)c.off);
     SWEEP_REQUIRE(tape != nullptr, "acoustic backward: the forward's tape is required");
-    Geo& G = pl.G;
-    G.cells = w.cells;
-    if (G.ns > 0)
-        SWEEP_CUDA(cudaMemcpyAsync(w.cells, pl.cells.data(), sizeof(int) * G.ns, cudaMemcpyHostToDevice, st));
-    SWEEP_CUDA(cudaMemsetAsync(w.zero0, 0, w.zero1 - w.zero0, st));
-    if (grad_wavelet && G.nsrc > 0)
+    setup(d, pl, w, st);
+    const Geo& G = pl.G;
+    if (G.nsrc == 0) grad_wavelet = nullptr;
+    if (grad_wavelet)
         SWEEP_CUDA(cudaMemsetAsync(grad_wavelet, 0, sizeof(float) * (size_t)G.B * G.nsrc * G.nt, st));
     const float* tp = static_cast<const float*>(tape);
     const long long n = (long long)G.B * G.S;
     const bool il = illum_src || illum_rec;
     float *rp = w.u[0], *rn = w.u[1], *rx = w.u[2];
     const float* tail = tp + (long long)G.nt * slot_floats(pl);
-    SWEEP_CUDA(cudaMemcpyAsync(rp, tail + n, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
-    SWEEP_CUDA(cudaMemcpyAsync(rn, tail, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+    copy_state(G, rp, G.P, tail + state_floats(G), G.nx, st);
+    copy_state(G, rn, G.P, tail, G.nx, st);
     float *lp = w.l[0], *ln = w.l[1], *lx = w.l[2];
     int cur = 0;
-    const dim3 grid = cell_grid(G), block(32, 8);
-    const unsigned sb = blocks_of(slot_floats(pl), 256), cb = blocks_of(n, 256);
-    const unsigned srcb = (unsigned)(G.B * G.nsrc + 127) / 128, recb = (unsigned)(G.B * G.nrec + 127) / 128;
+    const dim3 grid = cell_grid(G), block = cell_block(G);
+    const unsigned cb = blocks_of(n, 256), srcb = (unsigned)(G.B * G.nsrc + 127) / 128;
+    const int parts = (G.nsrc > 0 ? PART_SRC : 0) | (G.nrec > 0 ? PART_REC : 0);
+    StepGraphs sg(st, resolve_graph_steps(-1));
     for (int it = G.nt - 1; it >= 0; --it) {
-        adj_step<M>(G, w, ln, lp, lx, cur, st);
-        if (G.nrec > 0) inject_res<<<recb, 128, 0, st>>>(G, lx, adj, it);
-        { float* t = lp; lp = ln; ln = lx; lx = t; }
-        cur ^= 1;
-        if (grad_wavelet && G.nsrc > 0) gather_src<<<srcb, 128, 0, st>>>(G, ln, grad_wavelet, it);
-        if (it == 0) {
-            if (il) illum<<<cb, 256, 0, st>>>(G, rx, rn, rp, ln, nullptr, w.ir);
-            SWEEP_LAUNCH_CHECK();
-            break;
+        cudaStream_t s = sg.stream();
+        const bool recon = it > 0;
+        Rev A{};
+        A.ln = ln; A.lp = lp; A.lx = lx;
+        for (int a = 0; a < 3; ++a) {
+            A.ps[a] = w.ps[cur][a]; A.zt[a] = w.zt[cur][a];
+            A.pso[a] = w.ps[cur ^ 1][a]; A.zto[a] = w.zt[cur ^ 1][a];
         }
-        recon<M><<<grid, block, 0, st>>>(G, rn, rp, rx, ln, w.g);
-        if (G.ns > 0) strips<<<sb, 256, 0, st>>>(G, rx, const_cast<float*>(tp) + (long long)(it - 1) * slot_floats(pl), 1);
-        if (G.nsrc > 0) inject_src<<<srcb, 128, 0, st>>>(G, rx, it, -1.f, 1);
-        if (G.ns > 0) strip_image<<<sb, 256, 0, st>>>(G, rx, rn, rp, ln, w.g);
-        if (il) illum<<<cb, 256, 0, st>>>(G, rx, rn, rp, ln, w.is, w.ir);
-        if (G.nsrc > 0) inject_src<<<srcb, 128, 0, st>>>(G, rx, it, 1.f, 0);
+        A.rn = rn; A.rp = rp; A.rx = recon ? rx : nullptr;
+        A.slot = recon ? tp + (long long)(it - 1) * slot_floats(pl) : nullptr;
+        A.g = w.g;
+        rev<M, ND><<<grid, block, 0, s>>>(G, A);
+        const RevEv E{lx, recon ? rx : nullptr, rn, rp, adj, w.g, grad_wavelet, il ? 0 : 1};
+        if (parts && one_launch(G)) {
+            rev_events<<<dim3(1, G.B), kEventBlock, 0, s>>>(G, E, it, parts);
+        } else {
+            if (parts & PART_REC) rev_events<<<event_grid(G, G.nrec), kEventBlock, 0, s>>>(G, E, it, PART_REC);
+            if (parts & PART_SRC) rev_events<<<event_grid(G, G.nsrc), kEventBlock, 0, s>>>(G, E, it, PART_SRC);
+        }
+        if (il) {
+            // u_tt without the source: out of the restored strips for the
+            // illumination's read, then back everywhere
+            if (recon && G.nsrc > 0) add_src<<<srcb, 128, 0, s>>>(G, rx, it, -1.f, 1);
+            illum<<<cb, 256, 0, s>>>(G, rx, rn, rp, lx, recon ? w.is : nullptr, w.ir);
+            if (recon && G.nsrc > 0) {
+                add_src<<<srcb, 128, 0, s>>>(G, rx, it, 1.f, 1);
+                add_src<<<srcb, 128, 0, s>>>(G, rx, it, 1.f, 0);
+            }
+        }
         SWEEP_LAUNCH_CHECK();
+        sg.step_done();
+        { float* t = lp; lp = ln; ln = lx; lx = t; }
         { float* t = rp; rp = rn; rn = rx; rx = t; }
+        cur ^= 1;
     }
-    const int per_shot = G.vps != 0;
-    finalize<<<cb, 256, 0, st>>>(G, w.g, per_shot, grad_vp);
-    if (illum_src) finalize<<<cb, 256, 0, st>>>(G, w.is, per_shot, illum_src);
-    if (illum_rec) finalize<<<cb, 256, 0, st>>>(G, w.ir, per_shot, illum_rec);
+    sg.flush();
+    finalize<<<cb, 256, 0, st>>>(G, w.g, 1, grad_vp);
+    if (illum_src) finalize<<<cb, 256, 0, st>>>(G, w.is, 0, illum_src);
+    if (illum_rec) finalize<<<cb, 256, 0, st>>>(G, w.ir, 0, illum_rec);
     SWEEP_LAUNCH_CHECK();
 }
 
@@ -845,7 +564,9 @@ void forward(const sweep_acoustic_desc* d, int mem_mode, int, float* record, voi
              cudaStream_t st)
 {
     Plan pl = make_plan(d, mem_mode);
-#define SWEEP_AORD_FWD(m) forward_m<m>(pl, record, tape, ws, ws_bytes, st)
+#define SWEEP_AORD_FWD(m)                                                                        \
+    (d->ndim == 2 ? forward_m<m, 2>(d, pl, record, tape, ws, ws_bytes, st)                       \
+                  : forward_m<m, 3>(d, pl, record, tape, ws, ws_bytes, st))
     SWEEP_AORD_DISPATCH(d->M, SWEEP_AORD_FWD)
 #undef SWEEP_AORD_FWD
 }
@@ -854,7 +575,9 @@ void backward(const sweep_acoustic_desc* d, int mem_mode, int, const float* adj,
               float* grad_wavelet, float* illum_src, float* illum_rec, void* ws, int64_t ws_bytes, cudaStream_t st)
 {
     Plan pl = make_plan(d, mem_mode);
-#define SWEEP_AORD_BWD(m) backward_m<m>(pl, adj, tape, grad_vp, grad_wavelet, illum_src, illum_rec, ws, ws_bytes, st)
+#define SWEEP_AORD_BWD(m)                                                                                        \
+    (d->ndim == 2 ? backward_m<m, 2>(d, pl, adj, tape, grad_vp, grad_wavelet, illum_src, illum_rec, ws, ws_bytes, st) \
+                  : backward_m<m, 3>(d, pl, adj, tape, grad_vp, grad_wavelet, illum_src, illum_rec, ws, ws_bytes, st))
     SWEEP_AORD_DISPATCH(d->M, SWEEP_AORD_BWD)
 #undef SWEEP_AORD_BWD
 }
