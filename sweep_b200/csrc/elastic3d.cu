@@ -14,33 +14,28 @@
 //     src3 / strips3 / rec3   source injection per source field, the nine
 //               fields' boundary strips, the receiver gather  driver_traits.cuh:265-300
 //   reverse, per step (driver_traits.cuh:680-905):
-//     vsrc3     body-force rho correction (before the residuals)
 //     res3      signed residual injection (stress -1, velocity +1); src3 with
 //               -w takes the forward source back out
-//     srev3     stress reconstruction on the box minus one cell   kernels.cuh:653-768
+//     stress_rev   stress reconstruction on the box minus one cell
+//               (kernels.cuh:653-768) and the vp / vs imaging of the
+//               stress-adjoint prepare                        kernels.cuh:1367-1615
 //     strips3   stress strips of step it - 1 restored
-//     sprep3    stress-adjoint prepare (q and the adjoint memories of the
-//               velocity derivatives) with the fused vp / vs / rho imaging
-//                                                             kernels.cuh:1367-1615
-//     rrho3     receiver rho correction                       common/common.cu:77-116
-//     sapp3     stress-adjoint apply (adjoint velocities)     kernels.cuh:1683-1780
-//     vprep3 / vapp3   velocity-adjoint prepare / apply       kernels.cuh:959-1236
-//     cap3, vrev3, strips3   v(it) carriers, velocity reconstruction,
-//               velocity strips of step it - 1                kernels.cuh:536-652
+//     adj_vel   the stress step's transpose (adjoint velocities)
+//                                                             kernels.cuh:1367-1780
+//     adj_str   the velocity step's transpose (adjoint stresses)
+//                                                             kernels.cuh:959-1236
+//     vel_rev   velocity reconstruction (kernels.cuh:536-652) with the rho
+//               image of the step it takes back; the reference images v(it) -
+//               v(it + 1) and corrects it at the receivers and body-force
+//               sources (common/common.cu:40-116)
+//     restore_velocity   velocity strips of step it - 1
 //
-// One thread per cell on 32 x 4 x 2 (x, y, z) blocks, two z planes of a shot
-// per grid row (against 32 x 8 tiles of one plane: 4.47 against 4.2 Gcell/s);
-// the stencils read global memory through the read-only path.  (A z-marching
-// variant with shared-memory planes and register z-queues, run at two CTAs
-// per SM without a load pipeline, measured 2.8x slower in the forward; four
-// cells of a column per thread with the z taps in a register window, at
-// three CTAs per SM, 1.23x slower; the kernels that beat this layout need the
-// 3-D acoustic kernels' TMA plane rings.)
-// Layout: fields (B, nz, ny, nx), x fastest; CPML memories in per-axis slabs
-// covering the cells outside the box shrunk by one cell along their axis
-// (x: (B, nz, ny, WX), y: (B, nz, WY, nx), z: (B, WZ, ny, nx)).  Cells in the
-// CPML branch because of another axis have zero coefficients on this one and
-// keep no memory (as the reference's stored() gating).
+// Four x cells per thread on pitched rows (vec4.cuh).  Layout: fields
+// (B, nz, ny, P), x fastest, P = nx rounded up to 8; CPML memories in per-axis
+// slabs covering the cells outside the box shrunk by one cell along their
+// axis.  Cells in the CPML branch because of another axis have zero
+// coefficients on this one and keep no memory (as the reference's stored()
+// gating).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>

@@ -10,11 +10,15 @@
 #error "define EL3D_NS (the namespace of this order) before including elastic3d_impl.cuh"
 #endif
 
+#include "bands.cuh"
+#include "vec4.cuh"
+
 namespace sweep {
 namespace EL3D_NS {
 
 constexpr int M = EL3D_M;
-constexpr int NTHX = 32, NTHY = 4, NTHZ = 2;
+constexpr int kGuard = 16;          // zero floats before and after a packed x profile
+constexpr int kMaxGroup = 4;        // shots of an imaging thread, at most
 
 // Staggered first-derivative weight k of order 2M (reference
 // operators/staggered.cuh:146-147 order 4, 248-250 order 6, 351-354 order 8;
@@ -34,6 +38,8 @@ enum { MX_VX, MX_VY, MX_VZ, MX_SXX, MX_SXY, MX_SXZ };
 enum { MY_VX, MY_VY, MY_VZ, MY_SXY, MY_SYY, MY_SYZ };
 enum { MZ_VX, MZ_VY, MZ_VZ, MZ_SXZ, MZ_SYZ, MZ_SZZ };
 
+// CPML memories of the band of each axis: x (B, nz, ny, WX), y (B, nz, WY, P),
+// z (B, WZ, ny, P); the x slab holds whole groups of four cells.
 struct Slabs {
     float *x[6], *y[6], *z[6];
 };
@@ -64,11 +70,15 @@ struct StripStore {
 
 struct Geo {
     int B, nz, ny, nx, nt;
-    long long S;                    // cells per shot
+    int P, SZ;                      // row pitch (y stride), z stride
+    long long S;                    // shot stride
+    int nbx, group, nslot;          // x blocks; shots per imaging thread, gradient slots
     int z0, z1, y0, y1, x0, x1;     // physical box
-    int SXL, SXH, SYL, SYH, SZL, SZH;   // slab sides (box edge + one cell)
+    int XL, XH, SYL, SYH, SZL, SZH;     // slab sides: x below XL or from XH on (multiples of 4); box edge + one cell
     int WX, WY, WZ;
     float dt, idx, idy, idz;
+    // profiles a, b at integer and at half positions; the x ones are padded
+    // with zeros (kGuard floats before their start and past their end)
     const float *az, *bz, *azh, *bzh, *ay, *by, *ayh, *byh, *ax, *bx, *axh, *bxh;
     int nsrc, nrec, nsf, nrf;
     int sf[9], rf[9];
@@ -83,44 +93,51 @@ struct Geo {
 };
 
 struct Models {
-    const float *lam, *mu, *kv;     // kv = dt * (1 / rho)
-    const float *vp, *vs, *rho;     // the caller's models (imaging)
+    const float *lam, *mu, *kv;     // kv = dt * (1 / rho), pitched
 };
 
-#if EL3D_M == 4
-// order 8 as one expression of the four taps: the form the order-8 kernels
-// were tuned in (a loop over wt(k) changes their register allocation and runs
-// the step 10 % slower)
-__device__ __forceinline__ float dp(const float* __restrict__ u, long long i, long long s, float inv)
-{
-    return (wt(1) * (__ldg(u + i + s) - __ldg(u + i)) + wt(2) * (__ldg(u + i + 2 * s) - __ldg(u + i - s)) +
-            wt(3) * (__ldg(u + i + 3 * s) - __ldg(u + i - 2 * s)) +
-            wt(4) * (__ldg(u + i + 4 * s) - __ldg(u + i - 3 * s))) *
-           inv;
-}
-__device__ __forceinline__ float dm(const float* __restrict__ u, long long i, long long s, float inv)
-{
-    return (wt(1) * (__ldg(u + i) - __ldg(u + i - s)) + wt(2) * (__ldg(u + i + s) - __ldg(u + i - 2 * s)) +
-            wt(3) * (__ldg(u + i + 2 * s) - __ldg(u + i - 3 * s)) +
-            wt(4) * (__ldg(u + i + 3 * s) - __ldg(u + i - 4 * s))) *
-           inv;
-}
-#else
-__device__ __forceinline__ float dp(const float* __restrict__ u, long long i, long long s, float inv)
-{
-    float g = wt(1) * (__ldg(u + i + s) - __ldg(u + i));
+using v4::F4;
+
+// Rows and planes of a block of 8 x 4 x 4 threads, compiled for eight blocks
+// per SM (64 registers).  The gradient of the 2-shot 128^3 survey at order 8:
+// 8 x 8 x 4 blocks at 3 / 4 per SM 81.8 / 79.3 ms, 8 x 4 x 4 ones at
+// 6 / 8 per SM 79.6 / 78.1 ms.
+constexpr int kBY = 4, kBZ = 4;
+constexpr int kThreads = 8 * kBY * kBZ, kBlocks = 8;
+
+// the thread's four cells x .. x + 3 of one row
+struct Cell {
+    int b, z, y, x, i;              // shot (group), coordinates of lane 0, offset in a shot
+    bool grid, core;                // inside the grid; some lane is updated by the steps
+    __device__ __forceinline__ explicit Cell(const Geo& G)
+    {
+        const int xb = blockIdx.x % G.nbx;
+        b = blockIdx.x / G.nbx;
+        x = 4 * (xb * 8 + threadIdx.x);
+        y = blockIdx.y * kBY + threadIdx.y;
+        z = blockIdx.z * kBZ + threadIdx.z;
+        i = z * G.SZ + y * G.P + x;
+        grid = x < G.nx && y < G.ny && z < G.nz;
+        core = grid && x + 3 >= M && x < G.nx - M && y >= M && y < G.ny - M && z >= M && z < G.nz - M;
+    }
+    __device__ __forceinline__ bool lane(const Geo& G, int l) const { return x + l >= M && x + l < G.nx - M; }
+};
+
+// Staggered differences of the group at p (v4::diff with this order's
+// weights): dp to the half cell above, dm to the half cell below.
+struct Weights {
+    float c[M + 1];
+    __device__ __forceinline__ Weights()
+    {
+        c[0] = 0.f;
 #pragma unroll
-    for (int k = 2; k <= M; ++k) g = g + wt(k) * (__ldg(u + i + k * s) - __ldg(u + i - (k - 1) * s));
-    return g * inv;
-}
-__device__ __forceinline__ float dm(const float* __restrict__ u, long long i, long long s, float inv)
-{
-    float g = wt(1) * (__ldg(u + i) - __ldg(u + i - s));
-#pragma unroll
-    for (int k = 2; k <= M; ++k) g = g + wt(k) * (__ldg(u + i + (k - 1) * s) - __ldg(u + i - k * s));
-    return g * inv;
-}
-#endif
+        for (int k = 1; k <= M; ++k) c[k] = wt(k);
+    }
+};
+__device__ __forceinline__ F4 dp(const float* p, int s, float inv) { return v4::diff_col<M, true>(p, s, Weights().c, inv); }
+__device__ __forceinline__ F4 dm(const float* p, int s, float inv) { return v4::diff_col<M, false>(p, s, Weights().c, inv); }
+__device__ __forceinline__ F4 dpx(const float* p, float inv) { return v4::diff_row<M, true>(p, Weights().c, inv); }
+__device__ __forceinline__ F4 dmx(const float* p, float inv) { return v4::diff_row<M, false>(p, Weights().c, inv); }
 
 // ------------------------------------------------ traction-free top face
 // The reference's 3-D image method (common/elastic_free_surface.cuh:723-952,
@@ -133,57 +150,49 @@ __device__ __forceinline__ float dm(const float* __restrict__ u, long long i, lo
 // the surface down.  The surface row's sxx and syy take the Robertsson
 // correction and its szz is zeroed.
 template <bool FS, bool FWD>
-__device__ __forceinline__ float dz_fs(const Geo& G, const float* __restrict__ u, long long i, int iz, bool odd,
-                                       bool half)
+__device__ __forceinline__ F4 dz_fs(const Geo& G, const float* p, int iz, bool odd, bool half)
 {
-    const long long sz = (long long)G.nx * G.ny;
-    if (!FS || iz >= G.z0 + M) return FWD ? dp(u, i, sz, G.idz) : dm(u, i, sz, G.idz);
+    if (!FS || iz >= G.z0 + M) return FWD ? dp(p, G.SZ, G.idz) : dm(p, G.SZ, G.idz);
     auto at = [&](int k) {
-        if (k >= G.z0) return __ldg(u + i + (long long)(k - iz) * sz);
+        if (k >= G.z0) return v4::ldg(p + (k - iz) * G.SZ);
         const int m = half ? 2 * G.z0 - 1 - k : 2 * G.z0 - k;
-        const float v = __ldg(u + i + (long long)(m - iz) * sz);
-        return odd ? -v : v;
+        F4 v = v4::ldg(p + (m - iz) * G.SZ);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) v.v[l] = odd ? -v.v[l] : v.v[l];
+        return v;
     };
-    float w[M];
-#pragma unroll
-    for (int m = 0; m < M; ++m) w[m] = wt(m + 1);
-    float g = 0.f;
-#pragma unroll
-    for (int m = 0; m < M; ++m)
-        g += w[m] * (FWD ? at(iz + m + 1) - at(iz - m) : at(iz + m) - at(iz - m - 1));
-    return g * G.idz;
+    return v4::diff<M, FWD>([&](int k) { return at(iz + k); }, Weights().c, G.idz);
 }
-// negated transpose of dz_fs (the plain one: D- for a D+ forward)
-template <bool FS, bool FWD>
-__device__ __forceinline__ float adz_fs(const Geo& G, const float* __restrict__ q, long long i, int iz, bool odd,
-                                        bool half)
+// negated transpose of dz_fs (the plain one: D- for a D+ forward) of the rows
+// row(k), k planes away
+template <bool FS, bool FWD, class R>
+__device__ __forceinline__ F4 adz_fs(const Geo& G, const R& row, int iz, bool odd, bool half)
 {
-    const long long sz = (long long)G.nx * G.ny;
-    if (!FS || iz > G.z0 + M) return FWD ? dm(q, i, sz, G.idz) : dp(q, i, sz, G.idz);
+    if (!FS || iz > G.z0 + M) return v4::diff<M, !FWD>(row, Weights().c, G.idz);
     const int top = G.z0, lo = half ? top - 1 : top;
     const float par = odd ? -1.f : 1.f;
-    auto at = [&](int k) { return __ldg(q + i + (long long)(k - iz) * sz); };
-    float w[M];
+    F4 g = v4::splat(0.f);
+    auto add = [&](float w, int j) {
+        const F4 r = row(j - iz);
 #pragma unroll
-    for (int m = 0; m < M; ++m) w[m] = wt(m + 1);
-    float g = 0.f;
-#pragma unroll
+        for (int l = 0; l < 4; ++l) g.v[l] += w * r.v[l];
+    };
+#pragma unroll 1
     for (int m = 0; m < M; ++m) {
+        const float w = wt(m + 1);
         const int jp = FWD ? iz + m : iz + m + 1;
         const int jm = FWD ? iz - m - 1 : iz - m;
         const int jg = FWD ? (half ? 2 * top - 1 + m - iz : 2 * top + m - iz)
                            : (half ? 2 * top + m - iz : 2 * top + m + 1 - iz);
-        if (jp >= top) g += w[m] * at(jp);
-        if (jm >= top) g -= w[m] * at(jm);
-        if (iz > lo && jg >= top) g += w[m] * par * at(jg);
+        if (jp >= top) add(w, jp);
+        if (jm >= top) add(-w, jm);
+        if (iz > lo && jg >= top) add(w * par, jg);
     }
-    return g * G.idz;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) g.v[l] *= G.idz;
+    return g;
 }
 
-__device__ __forceinline__ bool interior(const Geo& G, int ix, int iy, int iz)
-{
-    return ix >= G.x0 + 1 && ix < G.x1 - 1 && iy >= G.y0 + 1 && iy < G.y1 - 1 && iz >= G.z0 + 1 && iz < G.z1 - 1;
-}
 __device__ __forceinline__ bool in_core(const Geo& G, int ix, int iy, int iz)
 {
     return ix >= M && ix < G.nx - M && iy >= M && iy < G.ny - M && iz >= M && iz < G.nz - M;
@@ -192,43 +201,46 @@ __device__ __forceinline__ bool in_box(const Geo& G, int ix, int iy, int iz)
 {
     return ix >= G.x0 && ix < G.x1 && iy >= G.y0 && iy < G.y1 && iz >= G.z0 && iz < G.z1;
 }
-// slab offsets of a cell (-1: no memory along that axis)
-__device__ __forceinline__ long long xsl(const Geo& G, int b, int iz, int iy, int ix)
+// slab offsets of a group (-1: no memory along that axis).  A profile is zero
+// off its slab, and every cell with a nonzero one lies outside the box shrunk
+// by one cell, where the reference's steps run their CPML branch.
+__device__ __forceinline__ int xslab(const Geo& G, int x) { return x < G.XL ? x : x >= G.XH ? G.XL + x - G.XH : -1; }
+__device__ __forceinline__ int yslab(const Geo& G, int y)
 {
-    const int s = ix < G.SXL ? ix : (ix >= G.nx - G.SXH ? G.SXL + ix - (G.nx - G.SXH) : -1);
-    return s < 0 ? -1 : (((long long)b * G.nz + iz) * G.ny + iy) * G.WX + s;
+    return y < G.SYL ? y : y >= G.ny - G.SYH ? G.SYL + y - (G.ny - G.SYH) : -1;
 }
-__device__ __forceinline__ long long ysl(const Geo& G, int b, int iz, int iy, int ix)
+__device__ __forceinline__ int zslab(const Geo& G, int z)
 {
-    const int s = iy < G.SYL ? iy : (iy >= G.ny - G.SYH ? G.SYL + iy - (G.ny - G.SYH) : -1);
-    return s < 0 ? -1 : (((long long)b * G.nz + iz) * G.WY + s) * G.nx + ix;
+    return z < G.SZL ? z : z >= G.nz - G.SZH ? G.SZL + z - (G.nz - G.SZH) : -1;
 }
-__device__ __forceinline__ long long zsl(const Geo& G, int b, int iz, int iy, int ix)
+__device__ __forceinline__ long long xsl(const Geo& G, int b, int z, int y, int x)
 {
-    const int s = iz < G.SZL ? iz : (iz >= G.nz - G.SZH ? G.SZL + iz - (G.nz - G.SZH) : -1);
-    return s < 0 ? -1 : (((long long)b * G.WZ + s) * G.ny + iy) * G.nx + ix;
+    const int s = xslab(G, x);
+    return s < 0 ? -1 : (((long long)b * G.nz + z) * G.ny + y) * G.WX + s;
 }
-
-// thread -> (b, iz, iy, ix) on NTHX x NTHY x NTHZ blocks (NTHZ z planes of a
-// shot per grid row); false past the grid
-__device__ __forceinline__ bool cell_of(const Geo& G, int& b, int& iz, int& iy, int& ix)
+__device__ __forceinline__ long long ysl(const Geo& G, int b, int z, int y, int x)
 {
-    const int zb = (G.nz + NTHZ - 1) / NTHZ;
-    ix = blockIdx.x * NTHX + threadIdx.x;
-    iy = blockIdx.y * NTHY + threadIdx.y;
-    b = blockIdx.z / zb;
-    iz = (blockIdx.z - b * zb) * NTHZ + threadIdx.z;
-    return ix < G.nx && iy < G.ny && iz < G.nz;
+    const int s = yslab(G, y);
+    return s < 0 ? -1 : (((long long)b * G.nz + z) * G.WY + s) * G.P + x;
+}
+__device__ __forceinline__ long long zsl(const Geo& G, int b, int z, int y, int x)
+{
+    const int s = zslab(G, z);
+    return s < 0 ? -1 : (((long long)b * G.WZ + s) * G.ny + y) * G.P + x;
 }
 
 // forward CPML memory update of derivative d along an axis: m = a m + b d,
-// d += m (at == -1: no memory, the coefficients are zero there)
-__device__ __forceinline__ void mem(float* __restrict__ m, long long at, float a, float b, float& d)
+// d += m, on the core's lanes
+__device__ __forceinline__ void mem(float* m, const F4& a, const F4& b, F4& d, const bool (&on)[4])
 {
-    if (at < 0) return;
-    const float v = a * m[at] + b * d;
-    m[at] = v;
-    d += v;
+    const F4 old = v4::ld(m);
+    F4 v;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        v.v[l] = on[l] ? a.v[l] * old.v[l] + b.v[l] * d.v[l] : 0.f;
+        d.v[l] += v.v[l];
+    }
+    v4::st(m, v);
 }
 
 // ------------------------------------------------------------------ forward
@@ -239,87 +251,153 @@ struct Fwd {
     Slabs mem;
 };
 
+// Nine derivatives of a staggered step by field and axis, through their
+// memories; U names the field, X / Y / Z the derivative.
+struct Nine {
+    F4 xx, xy, xz, yx, yy, yz, zx, zy, zz;
+};
+
 template <bool FS>
-__global__ void __launch_bounds__(NTHX * NTHY * NTHZ) vel3(Fwd A)
+__device__ __forceinline__ Nine stress_diffs(const Geo& G, float* const* f, long long k, int iz)
+{
+    Nine d;
+    d.xx = dpx(f[SXX] + k, G.idx);
+    d.xy = dm(f[SXY] + k, G.P, G.idy);
+    d.xz = dz_fs<FS, false>(G, f[SXZ] + k, iz, true, true);
+    d.yx = dmx(f[SXY] + k, G.idx);
+    d.yy = dp(f[SYY] + k, G.P, G.idy);
+    d.yz = dz_fs<FS, false>(G, f[SYZ] + k, iz, true, true);
+    d.zx = dmx(f[SXZ] + k, G.idx);
+    d.zy = dm(f[SYZ] + k, G.P, G.idy);
+    d.zz = dz_fs<FS, true>(G, f[SZZ] + k, iz, true, false);
+    return d;
+}
+// d(v_i) / d(j): xx = dvx/dx, xy = dvx/dy, ..., zz = dvz/dz
+template <bool FS>
+__device__ __forceinline__ Nine velocity_diffs(const Geo& G, float* const* f, long long k, int iz)
+{
+    Nine d;
+    d.xx = dmx(f[VX] + k, G.idx);
+    d.xy = dp(f[VX] + k, G.P, G.idy);
+    d.xz = dz_fs<FS, true>(G, f[VX] + k, iz, false, false);
+    d.yx = dpx(f[VY] + k, G.idx);
+    d.yy = dm(f[VY] + k, G.P, G.idy);
+    d.yz = dz_fs<FS, true>(G, f[VY] + k, iz, false, false);
+    d.zx = dpx(f[VZ] + k, G.idx);
+    d.zy = dp(f[VZ] + k, G.P, G.idy);
+    d.zz = dz_fs<FS, false>(G, f[VZ] + k, iz, true, true);
+    return d;
+}
+
+// Velocity and stress steps.  2-shot 128^3 survey at order 8 (9.5 M cells):
+// 208 and 245 us, 350 and 428 us with one cell per thread; their field and
+// memory traffic takes 100 and 117 us at the copy rate, the rest is the taps'
+// L1 and L2 traffic.
+template <bool FS>
+__global__ void __launch_bounds__(kThreads, kBlocks) vel3(const Fwd A)
 {
     const Geo& G = A.G;
-    int b, iz, iy, ix;
-    if (!cell_of(G, b, iz, iy, ix) || !in_core(G, ix, iy, iz)) return;
-    const long long sy = G.nx;
-    const long long c = (iz * (long long)G.ny + iy) * G.nx + ix, i = b * G.S + c;
-    float* const* f = A.f;
-    float dsxx_dx = dp(f[SXX], i, 1, G.idx);
-    float dsxy_dy = dm(f[SXY], i, sy, G.idy);
-    float dsxz_dz = dz_fs<FS, false>(G, f[SXZ], i, iz, true, true);
-    float dsxy_dx = dm(f[SXY], i, 1, G.idx);
-    float dsyy_dy = dp(f[SYY], i, sy, G.idy);
-    float dsyz_dz = dz_fs<FS, false>(G, f[SYZ], i, iz, true, true);
-    float dsxz_dx = dm(f[SXZ], i, 1, G.idx);
-    float dsyz_dy = dm(f[SYZ], i, sy, G.idy);
-    float dszz_dz = dz_fs<FS, true>(G, f[SZZ], i, iz, true, false);
-    if (!interior(G, ix, iy, iz)) {
-        const long long xo = xsl(G, b, iz, iy, ix), yo = ysl(G, b, iz, iy, ix), zo = zsl(G, b, iz, iy, ix);
-        mem(A.mem.z[MZ_SZZ], zo, G.azh[iz], G.bzh[iz], dszz_dz);
-        mem(A.mem.x[MX_SXZ], xo, G.ax[ix], G.bx[ix], dsxz_dx);
-        mem(A.mem.z[MZ_SXZ], zo, G.az[iz], G.bz[iz], dsxz_dz);
-        mem(A.mem.x[MX_SXX], xo, G.axh[ix], G.bxh[ix], dsxx_dx);
-        mem(A.mem.y[MY_SXY], yo, G.ay[iy], G.by[iy], dsxy_dy);
-        mem(A.mem.x[MX_SXY], xo, G.ax[ix], G.bx[ix], dsxy_dx);
-        mem(A.mem.y[MY_SYY], yo, G.ayh[iy], G.byh[iy], dsyy_dy);
-        mem(A.mem.z[MZ_SYZ], zo, G.az[iz], G.bz[iz], dsyz_dz);
-        mem(A.mem.y[MY_SYZ], yo, G.ay[iy], G.by[iy], dsyz_dy);
+    const Cell q(G);
+    if (!q.core) return;
+    const long long k = q.b * G.S + q.i;
+    Nine d = stress_diffs<FS>(G, A.f, k, q.z);
+    bool on[4];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) on[l] = q.lane(G, l);
+    if (const long long o = xsl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::ldg(G.ax + q.x), b = v4::ldg(G.bx + q.x);
+        mem(A.mem.x[MX_SXX] + o, v4::ldg(G.axh + q.x), v4::ldg(G.bxh + q.x), d.xx, on);
+        mem(A.mem.x[MX_SXY] + o, a, b, d.yx, on);
+        mem(A.mem.x[MX_SXZ] + o, a, b, d.zx, on);
     }
-    const float k = A.m.kv[b * G.ms + c];
-    f[VX][i] += k * (dsxx_dx + dsxy_dy + dsxz_dz);
-    f[VY][i] += k * (dsxy_dx + dsyy_dy + dsyz_dz);
-    f[VZ][i] += k * (dsxz_dx + dsyz_dy + dszz_dz);
+    if (const long long o = ysl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::splat(__ldg(G.ay + q.y)), b = v4::splat(__ldg(G.by + q.y));
+        mem(A.mem.y[MY_SXY] + o, a, b, d.xy, on);
+        mem(A.mem.y[MY_SYY] + o, v4::splat(__ldg(G.ayh + q.y)), v4::splat(__ldg(G.byh + q.y)), d.yy, on);
+        mem(A.mem.y[MY_SYZ] + o, a, b, d.zy, on);
+    }
+    if (const long long o = zsl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::splat(__ldg(G.az + q.z)), b = v4::splat(__ldg(G.bz + q.z));
+        mem(A.mem.z[MZ_SXZ] + o, a, b, d.xz, on);
+        mem(A.mem.z[MZ_SYZ] + o, a, b, d.yz, on);
+        mem(A.mem.z[MZ_SZZ] + o, v4::splat(__ldg(G.azh + q.z)), v4::splat(__ldg(G.bzh + q.z)), d.zz, on);
+    }
+    const F4 kv = v4::ldg(A.m.kv + q.b * G.ms + q.i);
+    F4 vx = v4::ld(A.f[VX] + k), vy = v4::ld(A.f[VY] + k), vz = v4::ld(A.f[VZ] + k);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        if (!on[l]) continue;
+        vx.v[l] += kv.v[l] * (d.xx.v[l] + d.xy.v[l] + d.xz.v[l]);
+        vy.v[l] += kv.v[l] * (d.yx.v[l] + d.yy.v[l] + d.yz.v[l]);
+        vz.v[l] += kv.v[l] * (d.zx.v[l] + d.zy.v[l] + d.zz.v[l]);
+    }
+    v4::st(A.f[VX] + k, vx);
+    v4::st(A.f[VY] + k, vy);
+    v4::st(A.f[VZ] + k, vz);
+}
+
+// the six stresses of the group at k: s += sgn dt C : d on the lanes `on`
+__device__ __forceinline__ void stress_update(const Geo& G, float* const* f, long long k, const Nine& d, const F4& lam,
+                                              const F4& mu, float sdt, const bool (&on)[4], bool surf)
+{
+    auto update = [&](int fl, auto value) {
+        F4 s = v4::ld(f[fl] + k);
+#pragma unroll
+        for (int l = 0; l < 4; ++l)
+            if (on[l]) s.v[l] = value(l, s.v[l]);
+        v4::st(f[fl] + k, s);
+    };
+    auto div = [&](int l) { return d.xx.v[l] + d.yy.v[l] + d.zz.v[l]; };
+    // surface row: Robertsson sxx / syy (forward only), then szz = 0
+    auto rob = [&](int l) {
+        return -G.dt * lam.v[l] * (lam.v[l] / (lam.v[l] + 2.f * mu.v[l]) * (d.xx.v[l] + d.yy.v[l]) + d.zz.v[l]);
+    };
+    update(SXX, [&](int l, float s) {
+        s += sdt * (lam.v[l] * div(l) + 2.f * mu.v[l] * d.xx.v[l]);
+        return surf ? s + rob(l) : s;
+    });
+    update(SYY, [&](int l, float s) {
+        s += sdt * (lam.v[l] * div(l) + 2.f * mu.v[l] * d.yy.v[l]);
+        return surf ? s + rob(l) : s;
+    });
+    update(SZZ, [&](int l, float s) {
+        return surf ? 0.f : s + sdt * (lam.v[l] * div(l) + 2.f * mu.v[l] * d.zz.v[l]);
+    });
+    update(SXY, [&](int l, float s) { return s + sdt * mu.v[l] * (d.xy.v[l] + d.yx.v[l]); });
+    update(SXZ, [&](int l, float s) { return s + sdt * mu.v[l] * (d.xz.v[l] + d.zx.v[l]); });
+    update(SYZ, [&](int l, float s) { return s + sdt * mu.v[l] * (d.yz.v[l] + d.zy.v[l]); });
 }
 
 template <bool FS>
-__global__ void __launch_bounds__(NTHX * NTHY * NTHZ) str3(Fwd A)
+__global__ void __launch_bounds__(kThreads, kBlocks) str3(const Fwd A)
 {
     const Geo& G = A.G;
-    int b, iz, iy, ix;
-    if (!cell_of(G, b, iz, iy, ix) || !in_core(G, ix, iy, iz)) return;
-    const long long sy = G.nx;
-    const long long c = (iz * (long long)G.ny + iy) * G.nx + ix, i = b * G.S + c;
-    float* const* f = A.f;
-    float dvx_dx = dm(f[VX], i, 1, G.idx);
-    float dvx_dy = dp(f[VX], i, sy, G.idy);
-    float dvx_dz = dz_fs<FS, true>(G, f[VX], i, iz, false, false);
-    float dvy_dx = dp(f[VY], i, 1, G.idx);
-    float dvy_dy = dm(f[VY], i, sy, G.idy);
-    float dvy_dz = dz_fs<FS, true>(G, f[VY], i, iz, false, false);
-    float dvz_dx = dp(f[VZ], i, 1, G.idx);
-    float dvz_dy = dp(f[VZ], i, sy, G.idy);
-    float dvz_dz = dz_fs<FS, false>(G, f[VZ], i, iz, true, true);
-    if (!interior(G, ix, iy, iz)) {
-        const long long xo = xsl(G, b, iz, iy, ix), yo = ysl(G, b, iz, iy, ix), zo = zsl(G, b, iz, iy, ix);
-        mem(A.mem.z[MZ_VZ], zo, G.az[iz], G.bz[iz], dvz_dz);
-        mem(A.mem.y[MY_VY], yo, G.ay[iy], G.by[iy], dvy_dy);
-        mem(A.mem.x[MX_VX], xo, G.ax[ix], G.bx[ix], dvx_dx);
-        mem(A.mem.z[MZ_VX], zo, G.azh[iz], G.bzh[iz], dvx_dz);
-        mem(A.mem.x[MX_VZ], xo, G.axh[ix], G.bxh[ix], dvz_dx);
-        mem(A.mem.y[MY_VX], yo, G.ayh[iy], G.byh[iy], dvx_dy);
-        mem(A.mem.x[MX_VY], xo, G.axh[ix], G.bxh[ix], dvy_dx);
-        mem(A.mem.z[MZ_VY], zo, G.azh[iz], G.bzh[iz], dvy_dz);
-        mem(A.mem.y[MY_VZ], yo, G.ayh[iy], G.byh[iy], dvz_dy);
+    const Cell q(G);
+    if (!q.core) return;
+    const long long k = q.b * G.S + q.i, mi = q.b * G.ms + q.i;
+    Nine d = velocity_diffs<FS>(G, A.f, k, q.z);
+    bool on[4];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) on[l] = q.lane(G, l);
+    if (const long long o = xsl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::ldg(G.axh + q.x), b = v4::ldg(G.bxh + q.x);
+        mem(A.mem.x[MX_VX] + o, v4::ldg(G.ax + q.x), v4::ldg(G.bx + q.x), d.xx, on);
+        mem(A.mem.x[MX_VY] + o, a, b, d.yx, on);
+        mem(A.mem.x[MX_VZ] + o, a, b, d.zx, on);
     }
-    const long long mi = b * G.ms + c;
-    const float lam = A.m.lam[mi], mu = A.m.mu[mi];
-    const float div = dvx_dx + dvy_dy + dvz_dz;
-    f[SXX][i] += G.dt * (lam * div + 2.f * mu * dvx_dx);
-    f[SYY][i] += G.dt * (lam * div + 2.f * mu * dvy_dy);
-    f[SZZ][i] += G.dt * (lam * div + 2.f * mu * dvz_dz);
-    f[SXY][i] += G.dt * mu * (dvx_dy + dvy_dx);
-    f[SXZ][i] += G.dt * mu * (dvx_dz + dvz_dx);
-    f[SYZ][i] += G.dt * mu * (dvy_dz + dvz_dy);
-    if (FS && iz == G.z0) {   // surface row: Robertsson sxx / syy, then szz = 0
-        const float rob = -G.dt * lam * (lam / (lam + 2.f * mu) * (dvx_dx + dvy_dy) + dvz_dz);
-        f[SXX][i] += rob;
-        f[SYY][i] += rob;
-        f[SZZ][i] = 0.f;
+    if (const long long o = ysl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::splat(__ldg(G.ayh + q.y)), b = v4::splat(__ldg(G.byh + q.y));
+        mem(A.mem.y[MY_VX] + o, a, b, d.xy, on);
+        mem(A.mem.y[MY_VY] + o, v4::splat(__ldg(G.ay + q.y)), v4::splat(__ldg(G.by + q.y)), d.yy, on);
+        mem(A.mem.y[MY_VZ] + o, a, b, d.zy, on);
     }
+    if (const long long o = zsl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::splat(__ldg(G.azh + q.z)), b = v4::splat(__ldg(G.bzh + q.z));
+        mem(A.mem.z[MZ_VX] + o, a, b, d.xz, on);
+        mem(A.mem.z[MZ_VY] + o, a, b, d.yz, on);
+        mem(A.mem.z[MZ_VZ] + o, v4::splat(__ldg(G.az + q.z)), v4::splat(__ldg(G.bz + q.z)), d.zz, on);
+    }
+    stress_update(G, A.f, k, d, v4::ldg(A.m.lam + mi), v4::ldg(A.m.mu + mi), G.dt, on, FS && q.z == G.z0);
 }
 
 // Source injection of step it with sign (+1 forward, -1 taking the forward
@@ -331,7 +409,7 @@ __global__ void src3(const Geo G, const Fields F, int it, float sign)
     for (int s = threadIdx.x; s < G.nsrc; s += blockDim.x) {
         const int* l = G.src_loc + ((long long)b * G.nsrc + s) * 3;
         if (l[0] < 0 || l[0] >= G.nx || l[1] < 0 || l[1] >= G.ny || l[2] < 0 || l[2] >= G.nz) continue;
-        const long long i = b * G.S + ((long long)l[2] * G.ny + l[1]) * G.nx + l[0];
+        const long long i = b * G.S + (long long)l[2] * G.SZ + l[1] * G.P + l[0];
         const float w = sign * G.wavelet[((long long)b * G.nsrc + s) * G.nt + it];
         for (int k = 0; k < G.nsf; ++k) atomicAdd(f[G.sf[k]] + i, w);
     }
@@ -345,7 +423,7 @@ __global__ void rec3(const Geo G, const Fields F, float* record, int it)
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < G.nrec; r += gridDim.x * blockDim.x) {
         const int* l = G.rec_loc + ((long long)b * G.nrec + r) * 3;
         if (l[0] < 0 || l[0] >= G.nx || l[1] < 0 || l[1] >= G.ny || l[2] < 0 || l[2] >= G.nz) continue;
-        const long long i = b * G.S + ((long long)l[2] * G.ny + l[1]) * G.nx + l[0];
+        const long long i = b * G.S + (long long)l[2] * G.SZ + l[1] * G.P + l[0];
         float* out = record + (((long long)b * G.nt + it) * G.nrec + r) * G.nrf;
         for (int k = 0; k < G.nrf; ++k) out[k] = f[G.rf[k]][i];
     }
@@ -404,7 +482,7 @@ __device__ __forceinline__ T pick6(const T (&a)[6], int f)
 // (code - 128) x scale / 127).
 __device__ __forceinline__ float face_val(const Geo& G, const void* slot, int fl, int b, int c)
 {
-    const int ix = c % G.nx, r = c / G.nx, iy = r % G.ny, iz = r / G.ny;
+    const int ix = c % G.P, r = c / G.P, iy = r % G.ny, iz = r / G.ny;
     int f;
     const int i = face_index(G, iz, iy, ix, f);
     const StripStore& S = G.st;
@@ -468,7 +546,7 @@ __global__ void __launch_bounds__(kQB) quant3(const Geo G, const Fields F, void*
     if (in) {
         int iz, iy, ix;
         face_cell(G, f, idx, iz, iy, ix);
-        v = F.f[fl][b * G.S + ((long long)iz * G.ny + iy) * G.nx + ix];
+        v = F.f[fl][b * G.S + (long long)iz * G.SZ + iy * G.P + ix];
     }
     float m = fabsf(v);
 #pragma unroll
@@ -496,33 +574,49 @@ __global__ void __launch_bounds__(kQB) quant3(const Geo G, const Fields F, void*
 }
 
 // ------------------------------------------------------------------ reverse
+//
+// Per step: residuals and source, `stress_rev` (stress reconstruction and the
+// vp / vs image), the stress strips, `adj_vel` (the stress step's transpose
+// into the adjoint velocities), `adj_str` (the velocity step's transpose into
+// the adjoint stresses), `vel_rev` (velocity reconstruction and the rho
+// image), the velocity strips.  `adj_str` leaves q = dt C lambda_s beside the
+// adjoint stresses it writes (six fields; the reference's nine differ by the
+// CPML memory alone) and `adj_vel` p = kv lambda_v beside the velocities, so
+// no pass of its own prepares them and the stencils read one field per tap; a
+// band's taps add the adjoint memory, which is therefore double-buffered.
+// (q and p formed at every tap from lambda, the stiffness and 1 / rho instead:
+// 666 + 556 us a step against 366 + 301 on the 2-shot 128^3 survey at order 8.)  The rho image of step `it` is
+// lambda_v . (v(it - 1) - v(it)): inside, minus kv lambda_v . div s (what the
+// reconstruction takes back), on the box's outermost layer the difference of
+// the restored strips (`restore_velocity`).  The image of the update of step
+// 1 is left out, as by the reference's staggered reverse.
 struct Rev {
     Geo G;
     Models m;
     float* f[NFLD];      // reconstructed forward fields
     float* a[NFLD];      // adjoint fields
-    float* cv[3];        // v(it + 1) carriers on the box
-    float* q[9];         // prepare -> apply scratch (q, then p)
-    Slabs am;            // adjoint memories
-    float *gvp, *gvs, *grho;   // per-shot gradient slots (B, S)
+    float* q[6];         // dt C lambda_s: xx, yy, zz, xy, xz, yz
+    float* p[3];         // kv lambda_v
+    Slabs ai, ao;        // adjoint memories: read, written
+    float* g[3];         // slots of a shot group: gl, gm - 2 gl and the rho image (times rho)
     const float* adj;    // (B, nt, nrec, nrf)
     int it;
 };
 
-__global__ void vsrc3(Rev A)
+// dt C s of the diagonal; on a surface row the transposes of the corrected
+// updates, with szz counting as zero
+__device__ __forceinline__ void stiff(float dt, float lam, float mu, float x, float y, float z, bool surf, float (&q)[3])
 {
-    const Geo& G = A.G;
-    const int b = blockIdx.x;
-    for (int s = threadIdx.x; s < G.nsrc; s += blockDim.x) {
-        const int* l = G.src_loc + ((long long)b * G.nsrc + s) * 3;
-        if (l[0] < 0 || l[0] >= G.nx || l[1] < 0 || l[1] >= G.ny || l[2] < 0 || l[2] >= G.nz) continue;
-        const long long c = ((long long)l[2] * G.ny + l[1]) * G.nx + l[0];
-        const float w = G.wavelet[((long long)b * G.nsrc + s) * G.nt + A.it];
-        for (int k = 0; k < G.nsf; ++k) {
-            const int fl = G.sf[k];
-            if (fl > VZ) continue;
-            atomicAdd(A.grho + b * G.S + c, (A.a[fl][b * G.S + c] * w) / A.m.rho[b * G.ms + c]);
-        }
+    const float l2m = lam + 2.f * mu;
+    if (surf) {
+        const float c1 = 4.f * mu * (lam + mu) / l2m, c2 = 2.f * lam * mu / l2m;
+        q[0] = dt * (c1 * x + c2 * y);
+        q[1] = dt * (c2 * x + c1 * y);
+        q[2] = 0.f;
+    } else {
+        q[0] = dt * (l2m * x + lam * y + lam * z);
+        q[1] = dt * (lam * x + l2m * y + lam * z);
+        q[2] = dt * (lam * x + lam * y + l2m * z);
     }
 }
 
@@ -533,259 +627,405 @@ __global__ void res3(Rev A)
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < G.nrec; r += gridDim.x * blockDim.x) {
         const int* l = G.rec_loc + ((long long)b * G.nrec + r) * 3;
         if (l[0] < 0 || l[0] >= G.nx || l[1] < 0 || l[1] >= G.ny || l[2] < 0 || l[2] >= G.nz) continue;
-        const long long i = b * G.S + ((long long)l[2] * G.ny + l[1]) * G.nx + l[0];
+        const long long i = b * G.S + (long long)l[2] * G.SZ + l[1] * G.P + l[0];
         const float* res = A.adj + (((long long)b * G.nt + A.it) * G.nrec + r) * G.nrf;
         for (int k = 0; k < G.nrf; ++k) {
             const int fl = G.rf[k];
-            atomicAdd(A.a[fl] + i, fl >= SXX ? -res[k] : res[k]);
+            const float v = fl >= SXX ? -res[k] : res[k];
+            atomicAdd(A.a[fl] + i, v);
+            if (fl < SXX) continue;
+            // and what it adds to q
+            const float lam = A.m.lam[b * G.ms + i - b * G.S], mu = A.m.mu[b * G.ms + i - b * G.S];
+            if (fl >= SXY) { atomicAdd(A.q[fl - SXX] + i, G.dt * mu * v); continue; }
+            const float x = fl == SXX ? v : 0.f, y = fl == SYY ? v : 0.f, z = fl == SZZ ? v : 0.f;
+            float q3[3];
+            stiff(G.dt, lam, mu, x, y, z, G.fst && l[2] == G.z0, q3);
+            for (int j = 0; j < 3; ++j)
+                if (q3[j] != 0.f) atomicAdd(A.q[j] + i, q3[j]);
         }
     }
 }
 
-// Receiver rho correction after the image (velocity receivers in the core).
-__global__ void rrho3(Rev A)
+__device__ __forceinline__ void add4(float* p, const F4& a)
+{
+    F4 t = v4::ld(p);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) t.v[l] += a.v[l];
+    v4::st(p, t);
+}
+
+// Stress reconstruction on the box minus one cell, and on the box the image:
+// with gl, gm the derivatives of the misfit by lambda and mu (up to -dt),
+// grad vp = -2 rho vp dt gl, grad vs = -2 rho vs dt (gm - 2 gl), and the
+// stiffness part of rho times grad rho, -dt (gl (lam + 2 mu) + (gm - 2 gl) mu).
+template <bool FS>
+__global__ void __launch_bounds__(kThreads, kBlocks) stress_rev(const Rev A)
 {
     const Geo& G = A.G;
-    const int b = blockIdx.y;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < G.nrec; r += gridDim.x * blockDim.x) {
-        const int* l = G.rec_loc + ((long long)b * G.nrec + r) * 3;
-        if (!in_core(G, l[0], l[1], l[2])) continue;
-        const long long c = ((long long)l[2] * G.ny + l[1]) * G.nx + l[0];
-        const float* res = A.adj + (((long long)b * G.nt + A.it) * G.nrec + r) * G.nrf;
-        for (int k = 0; k < G.nrf; ++k) {
-            const int fl = G.rf[k];
-            if (fl > VZ) continue;
-            const float now = A.f[fl][b * G.S + c], nxt = A.cv[fl][b * G.S + c];
-            atomicAdd(A.grho + b * G.S + c, -res[k] * (now - nxt) / A.m.rho[b * G.ms + c]);
+    const Cell q(G);
+    if (!q.core || q.x + 3 < G.x0 || q.x >= G.x1 || q.y < G.y0 || q.y >= G.y1 || q.z < G.z0 || q.z >= G.z1) return;
+    const bool inner = q.y > G.y0 && q.y < G.y1 - 1 && q.z > G.z0 && q.z < G.z1 - 1, surf = FS && q.z == G.z0;
+    bool box[4], on[4];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        box[l] = q.x + l >= G.x0 && q.x + l < G.x1;
+        on[l] = inner && q.x + l > G.x0 && q.x + l < G.x1 - 1;
+    }
+    F4 sl = v4::splat(0.f), sm = sl, sr = sl;
+    const int b1 = min((q.b + 1) * G.group, G.B);
+    for (int b = q.b * G.group; b < b1; ++b) {
+        const long long k = b * G.S + q.i, mi = b * G.ms + q.i;
+        const Nine d = velocity_diffs<FS>(G, A.f, k, q.z);
+        const F4 lam = v4::ldg(A.m.lam + mi), mu = v4::ldg(A.m.mu + mi);
+        const F4 bxx = v4::ldg(A.a[SXX] + k), byy = v4::ldg(A.a[SYY] + k), bzz = v4::ldg(A.a[SZZ] + k);
+        const F4 bxy = v4::ldg(A.a[SXY] + k), bxz = v4::ldg(A.a[SXZ] + k), byz = v4::ldg(A.a[SYZ] + k);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            if (!box[l]) continue;
+            const float shear = bxz.v[l] * (d.xz.v[l] + d.zx.v[l]) + bxy.v[l] * (d.xy.v[l] + d.yx.v[l]) +
+                                byz.v[l] * (d.yz.v[l] + d.zy.v[l]);
+            const float l2m = lam.v[l] + 2.f * mu.v[l];
+            float gl, gm;
+            if (surf) {
+                // the surface row's corrected sxx / syy updates (kernels.cuh:1440-1452)
+                const float r = mu.v[l] / l2m, w = lam.v[l] / l2m;
+                const float dcl = 4.f * r * r, dcm = 4.f * (1.f - 2.f * r + 2.f * r * r), dc2m = 2.f * w * w;
+                gl = dcl * (bxx.v[l] + byy.v[l]) * (d.xx.v[l] + d.yy.v[l]);
+                gm = bxx.v[l] * (dcm * d.xx.v[l] + dc2m * d.yy.v[l]) +
+                     byy.v[l] * (dc2m * d.xx.v[l] + dcm * d.yy.v[l]) + shear;
+            } else {
+                gl = (bxx.v[l] + byy.v[l] + bzz.v[l]) * (d.xx.v[l] + d.yy.v[l] + d.zz.v[l]);
+                gm = 2.f * (bxx.v[l] * d.xx.v[l] + byy.v[l] * d.yy.v[l] + bzz.v[l] * d.zz.v[l]) + shear;
+            }
+            const float gm2 = gm - 2.f * gl;
+            sl.v[l] += gl;
+            sm.v[l] += gm2;
+            sr.v[l] -= G.dt * (gl * l2m + gm2 * mu.v[l]);
+        }
+        if (inner) stress_update(G, A.f, k, d, lam, mu, -G.dt, on, false);
+    }
+    const long long o = q.b * G.S + q.i;
+    add4(A.g[0] + o, sl);
+    add4(A.g[1] + o, sm);
+    add4(A.g[2] + o, sr);
+}
+
+// Velocity reconstruction on the box minus one cell with its rho image.
+template <bool FS>
+__global__ void __launch_bounds__(kThreads, kBlocks) vel_rev(const Rev A)
+{
+    const Geo& G = A.G;
+    const Cell q(G);
+    if (!q.core || q.x + 3 <= G.x0 || q.x >= G.x1 - 1 || q.y <= G.y0 || q.y >= G.y1 - 1 || q.z <= G.z0 || q.z >= G.z1 - 1)
+        return;
+    F4 sr = v4::splat(0.f);
+    const int b1 = min((q.b + 1) * G.group, G.B);
+    for (int b = q.b * G.group; b < b1; ++b) {
+        const long long k = b * G.S + q.i;
+        const Nine d = stress_diffs<FS>(G, A.f, k, q.z);
+        const F4 kv = v4::ldg(A.m.kv + b * G.ms + q.i);
+        const F4 lx = v4::ldg(A.a[VX] + k), ly = v4::ldg(A.a[VY] + k), lz = v4::ldg(A.a[VZ] + k);
+        F4 vx = v4::ld(A.f[VX] + k), vy = v4::ld(A.f[VY] + k), vz = v4::ld(A.f[VZ] + k);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            if (!(q.x + l > G.x0 && q.x + l < G.x1 - 1)) continue;
+            const float ux = kv.v[l] * (d.xx.v[l] + d.xy.v[l] + d.xz.v[l]);
+            const float uy = kv.v[l] * (d.yx.v[l] + d.yy.v[l] + d.yz.v[l]);
+            const float uz = kv.v[l] * (d.zx.v[l] + d.zy.v[l] + d.zz.v[l]);
+            vx.v[l] -= ux;
+            vy.v[l] -= uy;
+            vz.v[l] -= uz;
+            sr.v[l] -= lx.v[l] * ux + ly.v[l] * uy + lz.v[l] * uz;
+        }
+        v4::st(A.f[VX] + k, vx);
+        v4::st(A.f[VY] + k, vy);
+        v4::st(A.f[VZ] + k, vz);
+    }
+    if (A.it > 1) add4(A.g[2] + q.b * G.S + q.i, sr);
+}
+
+// Velocity strips from a step slot; the rho image of the box's outermost
+// layer is the difference this makes.
+__global__ void restore_velocity(const Rev A, const void* slot, int fmt)
+{
+    const Geo& G = A.G;
+    const long long n = (long long)G.B * G.ns;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+        const int b = (int)(e / G.ns), k = (int)(e - (long long)b * G.ns);
+        const int c = G.cells[k];
+        const int ix = c % G.P, r = c / G.P;
+        const bool img = A.it > 1 && in_box(G, ix, r % G.ny, r / G.ny);
+        float s = 0.f;
+        for (int fl = VX; fl <= VZ; ++fl) {
+            const long long t = ((long long)b * NFLD + fl) * G.ns + k, i = b * G.S + c;
+            const float v = fmt == SF_F32    ? static_cast<const float*>(slot)[t]
+                            : fmt == SF_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(slot)[t])
+                                             : face_val(G, slot, fl, b, c);
+            if (img) s += A.a[fl][i] * (v - A.f[fl][i]);
+            A.f[fl][i] = v;
+        }
+        if (img) atomicAdd(A.g[2] + b / G.group * G.S + c, s);
+    }
+}
+
+// a q / p entry through its adjoint CPML memory w: bar + b (w + bar); the
+// owner's next memory is a (w + bar)
+__device__ __forceinline__ F4 through(const F4& bar, const F4& b, const F4& w)
+{
+    F4 t;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) t.v[l] = bar.v[l] + b.v[l] * (w.v[l] + bar.v[l]);
+    return t;
+}
+__device__ __forceinline__ void keep(const float* wi, float* wo, const F4& a, const F4& bar)
+{
+    const F4 w = v4::ldg(wi);
+    F4 t;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) t.v[l] = a.v[l] * (w.v[l] + bar.v[l]);
+    v4::st(wo, t);
+}
+// A transpose's stencil along an axis of field u with the adjoint memory m of
+// its taps in the band (profile prof).  Off the band's reach it is the plain
+// one; within it every tap takes its memory, those off the slab at a clamped
+// place and with the profile's zero, so that a thread's loads leave together
+// (a test per tap serialised them: 709 + 438 us a step in the two transposes
+// of the 2-shot 128^3 survey at order 8, 377 + 345 us this way).
+template <bool PLUS>
+__device__ __forceinline__ F4 adj_x(const Geo& G, const Cell& q, const float* u, const float* m, const float* prof)
+{
+    using S = v4::Span<M, PLUS>;
+    float w[S::N];
+    v4::window<S::LO, S::HI>(u, w);
+    const int lo = q.x - 4 * S::LO, hi = min(q.x + 4 * S::HI, (G.nx - 1) / 4 * 4);
+    if (lo < G.XL || hi >= G.XH) {
+        const float* row = m + (((long long)q.b * G.nz + q.z) * G.ny + q.y) * G.WX;
+#pragma unroll
+        for (int j = -S::LO; j <= S::HI; ++j) {
+            const int x = min(max(q.x + 4 * j, 0), hi), s = max(xslab(G, x), 0);
+            const F4 b = v4::ldg(prof + q.x + 4 * j), t = v4::ldg(row + s);
+#pragma unroll
+            for (int l = 0; l < 4; ++l) {
+                float& e = w[4 * (j + S::LO) + l];
+                e = e + b.v[l] * (t.v[l] + e);
+            }
         }
     }
+    return v4::diff_x<M, PLUS, S::O>(w, Weights().c, G.idx);
+}
+template <bool PLUS>
+__device__ __forceinline__ F4 adj_y(const Geo& G, const Cell& q, const float* u, const float* m, const float* prof)
+{
+    if (yslab(G, q.y - M) < 0 && yslab(G, q.y + M) < 0) return v4::diff_col<M, PLUS>(u, G.P, Weights().c, G.idy);
+    const float* col = m + ((long long)q.b * G.nz + q.z) * G.WY * G.P + q.x;
+    return v4::diff<M, PLUS>(
+        [&](int j) {
+            return through(v4::ldg(u + j * G.P), v4::splat(__ldg(prof + q.y + j)),
+                           v4::ldg(col + (long long)max(yslab(G, q.y + j), 0) * G.P));
+        },
+        Weights().c, G.idy);
+}
+template <bool FS, bool FWD>
+__device__ __forceinline__ F4 adj_z(const Geo& G, const Cell& q, const float* u, const float* m, const float* prof,
+                                    bool odd, bool half)
+{
+    const bool surf = FS && q.z <= G.z0 + M;
+    if (!surf && zslab(G, q.z - M) < 0 && zslab(G, q.z + M) < 0)
+        return v4::diff_col<M, !FWD>(u, G.SZ, Weights().c, G.idz);
+    const float* col = m + ((long long)q.b * G.WZ * G.ny + q.y) * G.P + q.x;
+    return adz_fs<FS, FWD>(
+        G,
+        [&](int j) {
+            return through(v4::ldg(u + j * G.SZ), v4::splat(__ldg(prof + q.z + j)),
+                           v4::ldg(col + (long long)max(zslab(G, q.z + j), 0) * G.ny * G.P));
+        },
+        q.z, odd, half);
 }
 
+// The stress step's transpose: lambda_v += D(q) on the core, q through the
+// memories of the velocities' derivatives; then p = kv lambda_v.
 template <bool FS>
-__global__ void __launch_bounds__(NTHX * NTHY * NTHZ) srev3(Rev A)
+__global__ void __launch_bounds__(kThreads, kBlocks) adj_vel(const Rev A)
 {
     const Geo& G = A.G;
-    int b, iz, iy, ix;
-    if (!cell_of(G, b, iz, iy, ix) || !interior(G, ix, iy, iz)) return;
-    const long long sy = G.nx;
-    const long long c = (iz * (long long)G.ny + iy) * G.nx + ix, i = b * G.S + c;
-    float* const* f = A.f;
-    const float dvx_dx = dm(f[VX], i, 1, G.idx), dvx_dy = dp(f[VX], i, sy, G.idy);
-    const float dvx_dz = dz_fs<FS, true>(G, f[VX], i, iz, false, false);
-    const float dvy_dx = dp(f[VY], i, 1, G.idx), dvy_dy = dm(f[VY], i, sy, G.idy);
-    const float dvy_dz = dz_fs<FS, true>(G, f[VY], i, iz, false, false);
-    const float dvz_dx = dp(f[VZ], i, 1, G.idx), dvz_dy = dp(f[VZ], i, sy, G.idy);
-    const float dvz_dz = dz_fs<FS, false>(G, f[VZ], i, iz, true, true);
-    const long long mi = b * G.ms + c;
-    const float lam = A.m.lam[mi], mu = A.m.mu[mi];
-    const float div = dvx_dx + dvy_dy + dvz_dz;
-    f[SXX][i] -= G.dt * (lam * div + 2.f * mu * dvx_dx);
-    f[SYY][i] -= G.dt * (lam * div + 2.f * mu * dvy_dy);
-    f[SZZ][i] -= G.dt * (lam * div + 2.f * mu * dvz_dz);
-    f[SXY][i] -= G.dt * mu * (dvx_dy + dvy_dx);
-    f[SXZ][i] -= G.dt * mu * (dvx_dz + dvz_dx);
-    f[SYZ][i] -= G.dt * mu * (dvy_dz + dvz_dy);
-}
-
-template <bool FS>
-__global__ void __launch_bounds__(NTHX * NTHY * NTHZ) vrev3(Rev A)
-{
-    const Geo& G = A.G;
-    int b, iz, iy, ix;
-    if (!cell_of(G, b, iz, iy, ix) || !interior(G, ix, iy, iz)) return;
-    const long long sy = G.nx;
-    const long long c = (iz * (long long)G.ny + iy) * G.nx + ix, i = b * G.S + c;
-    float* const* f = A.f;
-    const float dsxx_dx = dp(f[SXX], i, 1, G.idx), dsxy_dy = dm(f[SXY], i, sy, G.idy);
-    const float dsxz_dz = dz_fs<FS, false>(G, f[SXZ], i, iz, true, true), dsxy_dx = dm(f[SXY], i, 1, G.idx);
-    const float dsyy_dy = dp(f[SYY], i, sy, G.idy), dsyz_dz = dz_fs<FS, false>(G, f[SYZ], i, iz, true, true);
-    const float dsxz_dx = dm(f[SXZ], i, 1, G.idx), dsyz_dy = dm(f[SYZ], i, sy, G.idy);
-    const float dszz_dz = dz_fs<FS, true>(G, f[SZZ], i, iz, true, false);
-    const float k = A.m.kv[b * G.ms + c];
-    f[VX][i] -= k * (dsxx_dx + dsxy_dy + dsxz_dz);
-    f[VY][i] -= k * (dsxy_dx + dsyy_dy + dsyz_dz);
-    f[VZ][i] -= k * (dsxz_dx + dsyz_dy + dszz_dz);
-}
-
-// adjoint CPML memory of one q / p entry: t = m + bar; q = bar + b t; m' = a t
-__device__ __forceinline__ float amem(float* __restrict__ m, long long at, float a, float b, float bar)
-{
-    if (at < 0) return bar;
-    const float t = m[at] + bar;
-    m[at] = a * t;
-    return bar + b * t;
-}
-
-template <bool FS>
-__global__ void __launch_bounds__(NTHX * NTHY * NTHZ) sprep3(Rev A)
-{
-    const Geo& G = A.G;
-    int b, iz, iy, ix;
-    if (!cell_of(G, b, iz, iy, ix)) return;
-    const long long sy = G.nx;
-    const long long c = (iz * (long long)G.ny + iy) * G.nx + ix, i = b * G.S + c, mi = b * G.ms + c;
-    const float lam = A.m.lam[mi], mu = A.m.mu[mi], l2m = lam + 2.f * mu;
-    const bool surf = FS && iz == G.z0;
-    if (surf) A.a[SZZ][i] = 0.f;   // the surface row's adjoint szz (its forward value is zeroed)
-    const float bsxx = A.a[SXX][i], bsyy = A.a[SYY][i], bszz = surf ? 0.f : A.a[SZZ][i];
-    const float bsxy = A.a[SXY][i], bsxz = A.a[SXZ][i], bsyz = A.a[SYZ][i];
-    if (in_box(G, ix, iy, iz)) {
-        float* const* f = A.f;
-        const float fvx_x = dm(f[VX], i, 1, G.idx), fvx_y = dp(f[VX], i, sy, G.idy);
-        const float fvx_z = dz_fs<FS, true>(G, f[VX], i, iz, false, false);
-        const float fvy_x = dp(f[VY], i, 1, G.idx), fvy_y = dm(f[VY], i, sy, G.idy);
-        const float fvy_z = dz_fs<FS, true>(G, f[VY], i, iz, false, false);
-        const float fvz_x = dp(f[VZ], i, 1, G.idx), fvz_y = dp(f[VZ], i, sy, G.idy);
-        const float fvz_z = dz_fs<FS, false>(G, f[VZ], i, iz, true, true);
-        const float rho = A.m.rho[mi], vp = A.m.vp[mi], vs = A.m.vs[mi];
-        float gl, gm;
-        if (surf) {
-            // the surface row's corrected sxx / syy updates (kernels.cuh:1440-1452)
-            const float vp2 = vp * vp, vs2 = vs * vs, vp4 = vp2 * vp2;
-            const float dcl = 4.f * vs2 * vs2 / vp4;
-            const float dcm = 4.f * (vp4 - 2.f * vp2 * vs2 + 2.f * vs2 * vs2) / vp4;
-            const float dc2m = 2.f * (vp2 - 2.f * vs2) * (vp2 - 2.f * vs2) / vp4;
-            gl = dcl * (bsxx + bsyy) * (fvx_x + fvy_y);
-            gm = bsxx * (dcm * fvx_x + dc2m * fvy_y) + bsyy * (dc2m * fvx_x + dcm * fvy_y) + bsxz * (fvx_z + fvz_x) +
-                 bsxy * (fvx_y + fvy_x) + bsyz * (fvy_z + fvz_y);
-        } else {
-            gl = (bsxx + bsyy + bszz) * (fvx_x + fvy_y + fvz_z);
-            gm = 2.f * (bsxx * fvx_x + bsyy * fvy_y + bszz * fvz_z) + bsxz * (fvx_z + fvz_x) +
-                 bsxy * (fvx_y + fvy_x) + bsyz * (fvy_z + fvz_y);
+    const Cell q(G);
+    if (!q.grid) return;
+    const long long k = q.b * G.S + q.i;
+    const float *qxx = A.q[0] + k, *qyy = A.q[1] + k, *qzz = A.q[2] + k, *qxy = A.q[3] + k, *qxz = A.q[4] + k,
+                *qyz = A.q[5] + k;
+    // the next memories of this group
+    if (const long long o = xsl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::ldg(G.axh + q.x);
+        keep(A.ai.x[MX_VX] + o, A.ao.x[MX_VX] + o, v4::ldg(G.ax + q.x), v4::ldg(qxx));
+        keep(A.ai.x[MX_VY] + o, A.ao.x[MX_VY] + o, a, v4::ldg(qxy));
+        keep(A.ai.x[MX_VZ] + o, A.ao.x[MX_VZ] + o, a, v4::ldg(qxz));
+    }
+    if (const long long o = ysl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::splat(__ldg(G.ayh + q.y));
+        keep(A.ai.y[MY_VX] + o, A.ao.y[MY_VX] + o, a, v4::ldg(qxy));
+        keep(A.ai.y[MY_VY] + o, A.ao.y[MY_VY] + o, v4::splat(__ldg(G.ay + q.y)), v4::ldg(qyy));
+        keep(A.ai.y[MY_VZ] + o, A.ao.y[MY_VZ] + o, a, v4::ldg(qyz));
+    }
+    if (const long long o = zsl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::splat(__ldg(G.azh + q.z));
+        keep(A.ai.z[MZ_VX] + o, A.ao.z[MZ_VX] + o, a, v4::ldg(qxz));
+        keep(A.ai.z[MZ_VY] + o, A.ao.z[MZ_VY] + o, a, v4::ldg(qyz));
+        keep(A.ai.z[MZ_VZ] + o, A.ao.z[MZ_VZ] + o, v4::splat(__ldg(G.az + q.z)), v4::ldg(qzz));
+    }
+    const F4 kv = v4::ldg(A.m.kv + q.b * G.ms + q.i);
+    auto put = [&](int fl, const F4& a, const F4& b, const F4& c) {
+        F4 v = v4::ld(A.a[fl] + k), p;
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            if (q.core && q.lane(G, l)) v.v[l] += a.v[l] + b.v[l] + c.v[l];
+            p.v[l] = kv.v[l] * v.v[l];
         }
-        A.gvp[i] += -2.f * rho * vp * gl * G.dt;
-        A.gvs[i] += -(-4.f * rho * vs * gl + 2.f * rho * vs * gm) * G.dt;
-        float gr = (A.a[VX][i] * (f[VX][i] - A.cv[0][i]) + A.a[VY][i] * (f[VY][i] - A.cv[1][i]) +
-                    A.a[VZ][i] * (f[VZ][i] - A.cv[2][i])) / rho;
-        gr -= gl * (vp * vp - 2.f * vs * vs) * G.dt + gm * (vs * vs) * G.dt;
-        A.grho[i] += gr;
+        v4::st(A.a[fl] + k, v);
+        v4::st(A.p[fl] + k, p);
+    };
+    if (!q.core) {
+        const F4 z = v4::splat(0.f);
+        for (int fl = VX; fl <= VZ; ++fl) put(fl, z, z, z);
+        return;
     }
-    float qxx, qyy, qzz;
-    if (surf) {   // transposes of the corrected surface updates
-        const float coef = 4.f * mu * (lam + mu) / l2m, coef2 = 2.f * lam * mu / l2m;
-        qxx = G.dt * (coef * bsxx + coef2 * bsyy);
-        qyy = G.dt * (coef2 * bsxx + coef * bsyy);
-        qzz = 0.f;
-    } else {
-        qxx = G.dt * (l2m * bsxx + lam * bsyy + lam * bszz);
-        qyy = G.dt * (lam * bsxx + l2m * bsyy + lam * bszz);
-        qzz = G.dt * (lam * bsxx + lam * bsyy + l2m * bszz);
-    }
-    float qxy = G.dt * mu * bsxy, qxz = G.dt * mu * bsxz;
-    float qyx = G.dt * mu * bsxy, qyz = G.dt * mu * bsyz;
-    float qzx = G.dt * mu * bsxz, qzy = G.dt * mu * bsyz;
-    if (!interior(G, ix, iy, iz)) {
-        const long long xo = xsl(G, b, iz, iy, ix), yo = ysl(G, b, iz, iy, ix), zo = zsl(G, b, iz, iy, ix);
-        qxx = amem(A.am.x[MX_VX], xo, G.ax[ix], G.bx[ix], qxx);
-        qyx = amem(A.am.x[MX_VY], xo, G.axh[ix], G.bxh[ix], qyx);
-        qzx = amem(A.am.x[MX_VZ], xo, G.axh[ix], G.bxh[ix], qzx);
-        qxy = amem(A.am.y[MY_VX], yo, G.ayh[iy], G.byh[iy], qxy);
-        qyy = amem(A.am.y[MY_VY], yo, G.ay[iy], G.by[iy], qyy);
-        qzy = amem(A.am.y[MY_VZ], yo, G.ayh[iy], G.byh[iy], qzy);
-        qxz = amem(A.am.z[MZ_VX], zo, G.azh[iz], G.bzh[iz], qxz);
-        qyz = amem(A.am.z[MZ_VY], zo, G.azh[iz], G.bzh[iz], qyz);
-        qzz = amem(A.am.z[MZ_VZ], zo, G.az[iz], G.bz[iz], qzz);
-    }
-    A.q[0][i] = qxx; A.q[1][i] = qxy; A.q[2][i] = qxz;
-    A.q[3][i] = qyx; A.q[4][i] = qyy; A.q[5][i] = qyz;
-    A.q[6][i] = qzx; A.q[7][i] = qzy; A.q[8][i] = qzz;
+    put(VX, adj_x<true>(G, q, qxx, A.ai.x[MX_VX], G.bx), adj_y<false>(G, q, qxy, A.ai.y[MY_VX], G.byh),
+        adj_z<FS, true>(G, q, qxz, A.ai.z[MZ_VX], G.bzh, false, false));
+    put(VY, adj_x<false>(G, q, qxy, A.ai.x[MX_VY], G.bxh), adj_y<true>(G, q, qyy, A.ai.y[MY_VY], G.by),
+        adj_z<FS, true>(G, q, qyz, A.ai.z[MZ_VY], G.bzh, false, false));
+    put(VZ, adj_x<false>(G, q, qxz, A.ai.x[MX_VZ], G.bxh), adj_y<false>(G, q, qyz, A.ai.y[MY_VZ], G.byh),
+        adj_z<FS, false>(G, q, qzz, A.ai.z[MZ_VZ], G.bz, true, true));
 }
 
+// The velocity step's transpose: lambda_s += D(p) on the core, p through the
+// memories of the stresses' derivatives; then q = dt C lambda_s.
 template <bool FS>
-__global__ void __launch_bounds__(NTHX * NTHY * NTHZ) sapp3(Rev A)
+__global__ void __launch_bounds__(kThreads, kBlocks) adj_str(const Rev A)
 {
     const Geo& G = A.G;
-    int b, iz, iy, ix;
-    if (!cell_of(G, b, iz, iy, ix) || !in_core(G, ix, iy, iz)) return;
-    const long long sy = G.nx;
-    const long long i = b * G.S + (iz * (long long)G.ny + iy) * G.nx + ix;
-    float* const* q = A.q;
-    A.a[VX][i] += dp(q[0], i, 1, G.idx) + dm(q[1], i, sy, G.idy) + adz_fs<FS, true>(G, q[2], i, iz, false, false);
-    A.a[VY][i] += dm(q[3], i, 1, G.idx) + dp(q[4], i, sy, G.idy) + adz_fs<FS, true>(G, q[5], i, iz, false, false);
-    A.a[VZ][i] += dm(q[6], i, 1, G.idx) + dm(q[7], i, sy, G.idy) + adz_fs<FS, false>(G, q[8], i, iz, true, true);
-}
-
-__global__ void __launch_bounds__(NTHX * NTHY * NTHZ) vprep3(Rev A)
-{
-    const Geo& G = A.G;
-    int b, iz, iy, ix;
-    if (!cell_of(G, b, iz, iy, ix)) return;
-    const long long c = (iz * (long long)G.ny + iy) * G.nx + ix, i = b * G.S + c;
-    const float k = A.m.kv[b * G.ms + c];
-    const float bx_ = k * A.a[VX][i], by_ = k * A.a[VY][i], bz_ = k * A.a[VZ][i];
-    float pxx = bx_, pxy = bx_, pxz = bx_, pyx = by_, pyy = by_, pyz = by_, pzx = bz_, pzy = bz_, pzz = bz_;
-    if (!interior(G, ix, iy, iz)) {
-        const long long xo = xsl(G, b, iz, iy, ix), yo = ysl(G, b, iz, iy, ix), zo = zsl(G, b, iz, iy, ix);
-        pxx = amem(A.am.x[MX_SXX], xo, G.axh[ix], G.bxh[ix], pxx);
-        pyx = amem(A.am.x[MX_SXY], xo, G.ax[ix], G.bx[ix], pyx);
-        pzx = amem(A.am.x[MX_SXZ], xo, G.ax[ix], G.bx[ix], pzx);
-        pxy = amem(A.am.y[MY_SXY], yo, G.ay[iy], G.by[iy], pxy);
-        pyy = amem(A.am.y[MY_SYY], yo, G.ayh[iy], G.byh[iy], pyy);
-        pzy = amem(A.am.y[MY_SYZ], yo, G.ay[iy], G.by[iy], pzy);
-        pxz = amem(A.am.z[MZ_SXZ], zo, G.az[iz], G.bz[iz], pxz);
-        pyz = amem(A.am.z[MZ_SYZ], zo, G.az[iz], G.bz[iz], pyz);
-        pzz = amem(A.am.z[MZ_SZZ], zo, G.azh[iz], G.bzh[iz], pzz);
+    const Cell q(G);
+    if (!q.grid) return;
+    const long long k = q.b * G.S + q.i, mi = q.b * G.ms + q.i;
+    const float *px = A.p[0] + k, *py = A.p[1] + k, *pz = A.p[2] + k;
+    if (const long long o = xsl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::ldg(G.ax + q.x);
+        keep(A.ai.x[MX_SXX] + o, A.ao.x[MX_SXX] + o, v4::ldg(G.axh + q.x), v4::ldg(px));
+        keep(A.ai.x[MX_SXY] + o, A.ao.x[MX_SXY] + o, a, v4::ldg(py));
+        keep(A.ai.x[MX_SXZ] + o, A.ao.x[MX_SXZ] + o, a, v4::ldg(pz));
     }
-    A.q[0][i] = pxx; A.q[1][i] = pxy; A.q[2][i] = pxz;
-    A.q[3][i] = pyx; A.q[4][i] = pyy; A.q[5][i] = pyz;
-    A.q[6][i] = pzx; A.q[7][i] = pzy; A.q[8][i] = pzz;
-}
-
-template <bool FS>
-__global__ void __launch_bounds__(NTHX * NTHY * NTHZ) vapp3(Rev A)
-{
-    const Geo& G = A.G;
-    int b, iz, iy, ix;
-    if (!cell_of(G, b, iz, iy, ix) || !in_core(G, ix, iy, iz)) return;
-    const long long sy = G.nx;
-    const long long i = b * G.S + (iz * (long long)G.ny + iy) * G.nx + ix;
-    float* const* p = A.q;
-    A.a[SXX][i] += dm(p[0], i, 1, G.idx);
-    A.a[SXY][i] += dp(p[1], i, sy, G.idy) + dp(p[3], i, 1, G.idx);
-    A.a[SXZ][i] += adz_fs<FS, false>(G, p[2], i, iz, true, true) + dp(p[6], i, 1, G.idx);
-    A.a[SYY][i] += dm(p[4], i, sy, G.idy);
-    A.a[SYZ][i] += adz_fs<FS, false>(G, p[5], i, iz, true, true) + dp(p[7], i, sy, G.idy);
-    A.a[SZZ][i] += adz_fs<FS, true>(G, p[8], i, iz, true, false);
-}
-
-// v(it) carriers on the box (they hold v(it + 1) for the next reverse step)
-__global__ void __launch_bounds__(NTHX * NTHY * NTHZ) cap3(Rev A)
-{
-    const Geo& G = A.G;
-    int b, iz, iy, ix;
-    if (!cell_of(G, b, iz, iy, ix) || !in_box(G, ix, iy, iz)) return;
-    const long long i = b * G.S + (iz * (long long)G.ny + iy) * G.nx + ix;
-    for (int k = 0; k < 3; ++k) A.cv[k][i] = A.f[k][i];
+    if (const long long o = ysl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::splat(__ldg(G.ay + q.y));
+        keep(A.ai.y[MY_SXY] + o, A.ao.y[MY_SXY] + o, a, v4::ldg(px));
+        keep(A.ai.y[MY_SYY] + o, A.ao.y[MY_SYY] + o, v4::splat(__ldg(G.ayh + q.y)), v4::ldg(py));
+        keep(A.ai.y[MY_SYZ] + o, A.ao.y[MY_SYZ] + o, a, v4::ldg(pz));
+    }
+    if (const long long o = zsl(G, q.b, q.z, q.y, q.x); o >= 0) {
+        const F4 a = v4::splat(__ldg(G.az + q.z));
+        keep(A.ai.z[MZ_SXZ] + o, A.ao.z[MZ_SXZ] + o, a, v4::ldg(px));
+        keep(A.ai.z[MZ_SYZ] + o, A.ao.z[MZ_SYZ] + o, a, v4::ldg(py));
+        keep(A.ai.z[MZ_SZZ] + o, A.ao.z[MZ_SZZ] + o, v4::splat(__ldg(G.azh + q.z)), v4::ldg(pz));
+    }
+    const F4 mu = v4::ldg(A.m.mu + mi);
+    const F4 zero = v4::splat(0.f);
+    auto sum = [](const F4& a, const F4& b) {
+        F4 t;
+#pragma unroll
+        for (int l = 0; l < 4; ++l) t.v[l] = a.v[l] + b.v[l];
+        return t;
+    };
+    auto put = [&](int fl, const F4& d, bool clear) {
+        F4 v = v4::ld(A.a[fl] + k);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            if (clear) v.v[l] = 0.f;
+            if (q.core && q.lane(G, l)) v.v[l] += d.v[l];
+        }
+        v4::st(A.a[fl] + k, v);
+        return v;
+    };
+    auto shear = [&](int fl, const F4& d) {
+        F4 v = put(fl, d, false);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) v.v[l] = G.dt * mu.v[l] * v.v[l];
+        v4::st(A.q[fl - SXX] + k, v);
+    };
+    const bool c = q.core;
+    shear(SXY, c ? sum(adj_y<true>(G, q, px, A.ai.y[MY_SXY], G.by), adj_x<true>(G, q, py, A.ai.x[MX_SXY], G.bx)) : zero);
+    shear(SXZ, c ? sum(adj_z<FS, false>(G, q, px, A.ai.z[MZ_SXZ], G.bz, true, true),
+                       adj_x<true>(G, q, pz, A.ai.x[MX_SXZ], G.bx)) : zero);
+    shear(SYZ, c ? sum(adj_z<FS, false>(G, q, py, A.ai.z[MZ_SYZ], G.bz, true, true),
+                       adj_y<true>(G, q, pz, A.ai.y[MY_SYZ], G.by)) : zero);
+    const bool surf = FS && q.z == G.z0;
+    const F4 sxx = put(SXX, c ? adj_x<false>(G, q, px, A.ai.x[MX_SXX], G.bxh) : zero, false);
+    const F4 syy = put(SYY, c ? adj_y<false>(G, q, py, A.ai.y[MY_SYY], G.byh) : zero, false);
+    const F4 szz = put(SZZ, c ? adj_z<FS, true>(G, q, pz, A.ai.z[MZ_SZZ], G.bzh, true, false) : zero, surf);
+    const F4 lam = v4::ldg(A.m.lam + mi);
+    F4 qd[3];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        float t[3];
+        stiff(G.dt, lam.v[l], mu.v[l], sxx.v[l], syy.v[l], szz.v[l], surf, t);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) qd[j].v[l] = t[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) v4::st(A.q[j] + k, qd[j]);
 }
 
 __global__ void prep3(const float* __restrict__ vp, const float* __restrict__ vs, const float* __restrict__ rho,
-                      long long n, float dt, float* olam, float* omu, float* okv)
+                      long long rows, int nx, int P, float dt, float* olam, float* omu, float* okv)
 {
+    const long long n = rows * P;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const float v = vp[k], s = vs[k], r = rho[k];
+        const long long row = k / P;
+        const int x = (int)(k - row * P);
+        if (x >= nx) { olam[k] = omu[k] = okv[k] = 0.f; continue; }
+        const long long i = row * nx + x;
+        const float v = vp[i], s = vs[i], r = rho[i];
         omu[k] = __fmul_rn(__fmul_rn(r, s), s);
         olam[k] = __fmul_rn(r, __fsub_rn(__fmul_rn(v, v), __fmul_rn(__fmul_rn(2.0f, s), s)));
         okv[k] = dt * (1.f / r);
     }
 }
 
-// Gradient output: the shots' slots summed in shot order (shared model) or
-// copied (per-shot models) on the physical box, zero elsewhere.
-__global__ void finalize3(const float* __restrict__ slots, int B, int per_shot, Geo G, float* out)
+// the x profiles, zero past their ends
+__global__ void prep_profiles3(const float* a, const float* b, const float* ah, const float* bh, int nx, int len,
+                               float* out)
 {
-    const int nout = per_shot ? B : 1;
-    const long long n = (long long)nout * G.S;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const long long b = k / G.S, c = k - b * G.S;
-        const int iz = (int)(c / ((long long)G.ny * G.nx));
-        const int iy = (int)((c / G.nx) % G.ny), ix = (int)(c % G.nx);
-        float v = 0.f;
+    const float* in[4] = {a, b, ah, bh};
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 4 * len; e += gridDim.x * blockDim.x) {
+        const int f = e / len, c = e - f * len - kGuard;
+        out[e] = c >= 0 && c < nx ? in[f][c] : 0.f;
+    }
+}
+
+// Gradients on the physical box, zero elsewhere, unpitched: per shot for
+// per-shot models, else the slots summed in order.
+struct Out {
+    const float *vp, *vs, *rho;     // the caller's models
+    float* g[3];                    // vp, vs, rho
+};
+
+__global__ void finalize3(const Rev A, const Out o)
+{
+    const Geo& G = A.G;
+    const long long cells = (long long)G.nz * G.ny * G.nx, n = (G.ms ? G.B : 1) * cells;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+        const long long b = e / cells;
+        const int c = (int)(e - b * cells);
+        const int ix = c % G.nx, r = c / G.nx, iy = r % G.ny, iz = r / G.ny;
+        float t[3] = {0.f, 0.f, 0.f};
         if (in_box(G, ix, iy, iz)) {
-            if (per_shot) v = slots[k];
-            else
-                for (int s = 0; s < B; ++s) v += slots[s * G.S + c];
+            const long long i = (long long)iz * G.SZ + iy * G.P + ix;
+            for (int j = 0; j < 3; ++j) {
+                t[j] = A.g[j][b * G.S + i];
+                for (int s = 1; !G.ms && s < G.nslot; ++s) t[j] += A.g[j][s * G.S + i];
+            }
+            const float rho = o.rho[e];
+            t[0] = -2.f * rho * o.vp[e] * t[0] * G.dt;
+            t[1] = -2.f * rho * o.vs[e] * t[1] * G.dt;
+            t[2] = t[2] / rho;
         }
-        out[k] = v;
+        for (int j = 0; j < 3; ++j) o.g[j][e] = t[j];
     }
 }
 
@@ -794,7 +1034,7 @@ struct Plan {
     Geo G;
     int nm;                      // model copies
     bool host_tape;              // boundary-saving tape in pinned host memory (SWEEP_MEM_HOST_TAPE)
-    std::vector<int> cells;      // strip cells
+    bands::Bands bands;          // strip cells
 };
 
 static void check_mode(int mem_mode, int ckpt_every)
@@ -843,8 +1083,11 @@ static Plan make_plan(const sweep_elastic3d_desc* d)
     Geo& G = pl.G;
     G.fst = d->free_surface ? 1 : 0;
     G.B = d->B; G.nz = d->nz; G.ny = d->ny; G.nx = d->nx; G.nt = d->nt;
-    G.S = (long long)d->nz * d->ny * d->nx;
-    SWEEP_REQUIRE(G.S < (1LL << 31), "elastic3d: one shot's grid must hold < 2^31 cells");
+    const long long cells = (long long)d->nz * d->ny * d->nx;
+    G.P = (d->nx + 7) / 8 * 8;
+    G.SZ = d->ny * G.P;
+    G.S = (long long)d->nz * d->ny * G.P;
+    SWEEP_REQUIRE(cells < (1LL << 31) && G.S < (1LL << 31), "elastic3d: one shot's grid must hold < 2^31 cells");
     G.z0 = d->pad[0] + M; G.z1 = d->nz - d->pad[1] - M;
     G.y0 = d->pad[2] + M; G.y1 = d->ny - d->pad[3] - M;
     G.x0 = d->pad[4] + M; G.x1 = d->nx - d->pad[5] - M;
@@ -852,36 +1095,29 @@ static Plan make_plan(const sweep_elastic3d_desc* d)
                   "elastic3d: the physical box must be at least 2 cells along every axis");
     G.SZL = std::min(G.z0 + 1, d->nz); G.SZH = std::min(d->nz - (G.z1 - 1), d->nz - G.SZL);
     G.SYL = std::min(G.y0 + 1, d->ny); G.SYH = std::min(d->ny - (G.y1 - 1), d->ny - G.SYL);
-    G.SXL = std::min(G.x0 + 1, d->nx); G.SXH = std::min(d->nx - (G.x1 - 1), d->nx - G.SXL);
-    G.WX = G.SXL + G.SXH; G.WY = G.SYL + G.SYH; G.WZ = G.SZL + G.SZH;
+    G.XL = (G.x0 + 1 + 3) / 4 * 4; G.XH = std::max(G.XL, (G.x1 - 1) / 4 * 4);
+    G.WX = G.XL + std::max(0, (d->nx + 3) / 4 * 4 - G.XH); G.WY = G.SYL + G.SYH; G.WZ = G.SZL + G.SZH;
     G.dt = d->dt; G.idx = 1.f / d->dx; G.idy = 1.f / d->dy; G.idz = 1.f / d->dz;
     G.az = d->az; G.bz = d->bz; G.azh = d->azh; G.bzh = d->bzh;
     G.ay = d->ay; G.by = d->by; G.ayh = d->ayh; G.byh = d->byh;
-    G.ax = d->ax; G.bx = d->bx; G.axh = d->axh; G.bxh = d->bxh;
     G.nsrc = d->nsrc; G.nrec = d->nrec;
     G.nsf = d->nsrc_fields; G.nrf = d->nrec_fields;
     for (int k = 0; k < 9; ++k) { G.sf[k] = d->src_fields[k]; G.rf[k] = d->rec_fields[k]; }
     G.src_loc = d->src_loc; G.rec_loc = d->rec_loc; G.wavelet = d->wavelet;
     const bool per_shot = d->model_stride != 0;
-    SWEEP_REQUIRE(!per_shot || d->model_stride == G.S, "elastic3d: model_stride must be 0 or nz * ny * nx");
+    SWEEP_REQUIRE(!per_shot || d->model_stride == cells, "elastic3d: model_stride must be 0 or nz * ny * nx");
     G.ms = per_shot ? G.S : 0;
     pl.nm = per_shot ? d->B : 1;
-    // strip cells: per face a band M + 1 wide from M cells outside the box,
-    // spanning the box along the other two axes (each cell once)
-    std::vector<char> mark((size_t)G.S, 0);
-    auto put = [&](int z, int y, int x) { mark[((size_t)z * G.ny + y) * G.nx + x] = 1; };
-    for (int z = G.z0 - M; z <= G.z0; ++z)
-        for (int y = G.y0; y < G.y1; ++y)
-            for (int x = G.x0; x < G.x1; ++x) { put(z, y, x); put(G.z1 - 1 + (G.z0 - z), y, x); }
-    for (int z = G.z0; z < G.z1; ++z) {
-        for (int y = G.y0 - M; y <= G.y0; ++y)
-            for (int x = G.x0; x < G.x1; ++x) { put(z, y, x); put(z, G.y1 - 1 + (G.y0 - y), x); }
-        for (int y = G.y0; y < G.y1; ++y)
-            for (int x = G.x0 - M; x <= G.x0; ++x) { put(z, y, x); put(z, y, G.x1 - 1 + (G.x0 - x)); }
-    }
-    for (size_t c = 0; c < mark.size(); ++c)
-        if (mark[c]) pl.cells.push_back((int)c);
-    G.ns = (int)pl.cells.size();
+    G.nbx = (G.nx + 31) / 32;
+    // shots per imaging thread: as many as still leave four blocks per SM; one
+    // for per-shot models
+    const long long blocks = (long long)G.nbx * ((G.ny + 7) / 8) * ((G.nz + 3) / 4);
+    G.group = 1;
+    if (!per_shot)
+        while (G.group < kMaxGroup && G.group < G.B && blocks * ((G.B + G.group) / (G.group + 1)) >= 4LL * 148) ++G.group;
+    G.nslot = (G.B + G.group - 1) / G.group;
+    pl.bands = bands::make<3>(M, G.z0, G.z1, G.y0, G.y1, G.x0, G.x1);
+    G.ns = pl.bands.count;
     return pl;
 }
 
@@ -930,20 +1166,24 @@ static unsigned quant_blocks(const Geo& G)
 
 struct Common {
     float *lam, *mu, *kv;
+    float* xprof;                // a, b, a_half, b_half along x, padded
     int* cells;
 };
+
+static int xprof_len(const Geo& G) { return G.P + 2 * kGuard; }
 
 static void carve_common(Carve& c, const Plan& pl, Common& w)
 {
     const long long mc = (long long)pl.nm * pl.G.S;
     w.lam = c.take<float>(mc); w.mu = c.take<float>(mc); w.kv = c.take<float>(mc);
+    w.xprof = c.take<float>(4LL * xprof_len(pl.G));
     w.cells = c.take<int>(std::max(pl.G.ns, 1));
 }
 
 static long long slab_count(const Geo& G, int axis)
 {
     return axis == 0 ? (long long)G.B * G.nz * G.ny * G.WX
-         : axis == 1 ? (long long)G.B * G.nz * G.WY * G.nx : (long long)G.B * G.WZ * G.ny * G.nx;
+         : axis == 1 ? (long long)G.B * G.nz * G.WY * G.P : (long long)G.B * G.WZ * G.ny * G.P;
 }
 
 static void carve_slabs(Carve& c, const Geo& G, Slabs& s)
@@ -979,10 +1219,10 @@ struct RevWs {
     Common cm;
     float* f[NFLD];
     float* a[NFLD];
-    float* cv[3];
-    float* q[9];
-    Slabs am;
-    float *gvp, *gvs, *grho;
+    float* q[6];
+    float* p[3];
+    Slabs am[2];                 // adjoint memories, double-buffered
+    float* g[3];
     char *zero0, *zero1;
     char* ring;                  // host tape: HostRing::R device strip slots
     Slabs fmem;                  // checkpoint modes: forward CPML memories of the replay
@@ -995,13 +1235,13 @@ static void carve_rev(Carve& c, const Plan& pl, RevWs& w)
     const Geo& G = pl.G;
     const long long n = (long long)G.B * G.S;
     for (int k = 0; k < NFLD; ++k) w.f[k] = c.take<float>(n);
-    for (int k = 0; k < 9; ++k) w.q[k] = c.take<float>(n);
     c.take<char>(0);
     w.zero0 = c.base ? c.base + c.off : nullptr;
     for (int k = 0; k < NFLD; ++k) w.a[k] = c.take<float>(n);
-    for (int k = 0; k < 3; ++k) w.cv[k] = c.take<float>(n);
-    carve_slabs(c, G, w.am);
-    w.gvp = c.take<float>(n); w.gvs = c.take<float>(n); w.grho = c.take<float>(n);
+    for (float*& p : w.q) p = c.take<float>(n);
+    for (float*& p : w.p) p = c.take<float>(n);
+    for (Slabs& s : w.am) carve_slabs(c, G, s);
+    for (float*& p : w.g) p = c.take<float>(G.nslot * G.S);
     c.take<char>(0);
     w.zero1 = c.base ? c.base + c.off : nullptr;
     if (pl.host_tape) w.ring = c.take<char>((long long)HostRing::R * G.st.step);
@@ -1115,28 +1355,30 @@ void sizes(const sweep_elastic3d_desc* d, int mem_mode, int ckpt_every, int64_t*
     *ws_bytes = std::max(f.off, r.off);
 }
 
-static void setup_common(const sweep_elastic3d_desc* d, const Plan& pl, const Common& w, cudaStream_t st)
+static void setup_common(const sweep_elastic3d_desc* d, Plan& pl, const Common& w, cudaStream_t st)
 {
-    const long long n = (long long)pl.nm * pl.G.S;
-    prep3<<<592, 256, 0, st>>>(d->vp, d->vs, d->rho, n, d->dt, w.lam, w.mu, w.kv);
+    Geo& G = pl.G;
+    G.cells = w.cells;
+    prep3<<<1184, 256, 0, st>>>(d->vp, d->vs, d->rho, (long long)pl.nm * G.nz * G.ny, G.nx, G.P, d->dt, w.lam, w.mu,
+                                w.kv);
+    const int len = xprof_len(G);
+    prep_profiles3<<<8, 256, 0, st>>>(d->ax, d->bx, d->axh, d->bxh, G.nx, len, w.xprof);
+    G.ax = w.xprof + kGuard; G.bx = G.ax + len; G.axh = G.bx + len; G.bxh = G.axh + len;
+    bands::band_table<3><<<592, 256, 0, st>>>(pl.bands, G.P, G.SZ, w.cells);
     SWEEP_LAUNCH_CHECK();
-    if (pl.G.ns > 0)
-        SWEEP_CUDA(cudaMemcpyAsync(w.cells, pl.cells.data(), sizeof(int) * pl.G.ns, cudaMemcpyHostToDevice, st));
 }
 
-static Models models_of(const sweep_elastic3d_desc* d, const Common& w)
-{
-    return Models{w.lam, w.mu, w.kv, d->vp, d->vs, d->rho};
-}
+static Models models_of(const Common& w) { return Models{w.lam, w.mu, w.kv}; }
 
 static dim3 rec_grid(const Geo& G)
 {
     return dim3((unsigned)std::min((G.nrec + 127) / 128, 64), (unsigned)G.B);
 }
 
-static dim3 cell_grid(const Geo& G)
+// n: shots, or shot groups
+static dim3 cell_grid(const Geo& G, int n)
 {
-    return dim3((G.nx + NTHX - 1) / NTHX, (G.ny + NTHY - 1) / NTHY, (unsigned)((G.nz + NTHZ - 1) / NTHZ * G.B));
+    return dim3((unsigned)(G.nbx * n), (G.ny + kBY - 1) / kBY, (G.nz + kBZ - 1) / kBZ);
 }
 
 static unsigned strip_blocks(const Geo& G)
@@ -1153,7 +1395,7 @@ static void forward_steps(const Fwd& A, int it0, int it1, StripsOf strips_of, in
     const Geo& G = A.G;
     Fields F{};
     for (int k = 0; k < NFLD; ++k) F.f[k] = A.f[k];
-    const dim3 grid = cell_grid(G), block(NTHX, NTHY, NTHZ);
+    const dim3 grid = cell_grid(G, G.B), block(8, kBY, kBZ);
     const bool scaled = fmt == SF_F16 || fmt == SF_I8;
     for (int it = it0; it < it1; ++it) {
         if (G.fst) {
@@ -1188,14 +1430,13 @@ void forward(const sweep_elastic3d_desc* d, int mem_mode, int ckpt_every, float*
     SWEEP_REQUIRE(ws != nullptr && c.off <= ws_bytes, "elastic3d forward: workspace too small (%lld < %lld bytes)",
                   (long long)ws_bytes, (long long)c.off);
     Geo& G = pl.G;
-    G.cells = w.cm.cells;
     setup_common(d, pl, w.cm, st);
     SWEEP_CUDA(cudaMemsetAsync(w.zero0, 0, w.zero1 - w.zero0, st));
     if (record && G.nrec > 0)
         SWEEP_CUDA(cudaMemsetAsync(record, 0, sizeof(float) * (size_t)G.B * G.nt * G.nrec * G.nrf, st));
     Fwd A{};
     A.G = G;
-    A.m = models_of(d, w.cm);
+    A.m = models_of(w.cm);
     for (int k = 0; k < NFLD; ++k) A.f[k] = w.f[k];
     A.mem = w.mem;
     const long long n = (long long)G.B * G.S;
@@ -1253,24 +1494,20 @@ void backward(const sweep_elastic3d_desc* d, int mem_mode, int ckpt_every, const
     SWEEP_REQUIRE(ws != nullptr && c.off <= ws_bytes, "elastic3d backward: workspace too small (%lld < %lld bytes)",
                   (long long)ws_bytes, (long long)c.off);
     Geo& G = pl.G;
-    G.cells = w.cm.cells;
     setup_common(d, pl, w.cm, st);
     SWEEP_CUDA(cudaMemsetAsync(w.zero0, 0, w.zero1 - w.zero0, st));
     const long long n = (long long)G.B * G.S;
     Rev A{};
     A.G = G;
-    A.m = models_of(d, w.cm);
+    A.m = models_of(w.cm);
     for (int k = 0; k < NFLD; ++k) { A.f[k] = w.f[k]; A.a[k] = w.a[k]; }
-    for (int k = 0; k < 3; ++k) A.cv[k] = w.cv[k];
-    for (int k = 0; k < 9; ++k) A.q[k] = w.q[k];
-    A.am = w.am;
-    A.gvp = w.gvp; A.gvs = w.gvs; A.grho = w.grho;
+    for (int k = 0; k < 6; ++k) A.q[k] = w.q[k];
+    for (int k = 0; k < 3; ++k) { A.p[k] = w.p[k]; A.g[k] = w.g[k]; }
     A.adj = adj;
     Fields F{};
     for (int k = 0; k < NFLD; ++k) F.f[k] = w.f[k];
-    const dim3 grid = cell_grid(G), block(NTHX, NTHY, NTHZ);
-    bool vsrc = false;
-    for (int k = 0; k < G.nsf; ++k) vsrc |= G.sf[k] <= VZ;
+    const dim3 grid = cell_grid(G, G.B), ggrid = cell_grid(G, G.nslot), block(8, kBY, kBZ);
+    int cur = 0;                 // adjoint memories read by the next reverse step
     HostRing hr;
     const bool host = pl.host_tape && !ckpt && !recursive;
     // Reverse steps it1 - 1 .. max(it0, 1) (the staggered reverse has no
@@ -1281,24 +1518,24 @@ void backward(const sweep_elastic3d_desc* d, int mem_mode, int ckpt_every, const
             A.it = it;
             void* prev = strips_of(it - 1);
             if (host) hr.before_read(it - 1);
-            if (vsrc && G.nsrc > 0) vsrc3<<<G.B, 128, 0, st>>>(A);
+            A.ai = w.am[cur];
+            A.ao = w.am[cur ^ 1];
+            cur ^= 1;
             if (G.nrec > 0) res3<<<rec_grid(G), 128, 0, st>>>(A);
             if (G.nsrc > 0) src3<<<G.B, 128, 0, st>>>(G, F, it, -1.f);
-            if (G.fst) srev3<true><<<grid, block, 0, st>>>(A);
-            else srev3<false><<<grid, block, 0, st>>>(A);
+            if (G.fst) stress_rev<true><<<ggrid, block, 0, st>>>(A);
+            else stress_rev<false><<<ggrid, block, 0, st>>>(A);
             if (G.ns > 0) strips3<<<strip_blocks(G), 256, 0, st>>>(G, F, prev, fmt, SXX, NFLD, 1);
-            if (G.fst) sprep3<true><<<grid, block, 0, st>>>(A);
-            else sprep3<false><<<grid, block, 0, st>>>(A);
-            if (G.nrec > 0) rrho3<<<rec_grid(G), 128, 0, st>>>(A);
-            if (G.fst) sapp3<true><<<grid, block, 0, st>>>(A);
-            else sapp3<false><<<grid, block, 0, st>>>(A);
-            vprep3<<<grid, block, 0, st>>>(A);
-            if (G.fst) vapp3<true><<<grid, block, 0, st>>>(A);
-            else vapp3<false><<<grid, block, 0, st>>>(A);
-            cap3<<<grid, block, 0, st>>>(A);
-            if (G.fst) vrev3<true><<<grid, block, 0, st>>>(A);
-            else vrev3<false><<<grid, block, 0, st>>>(A);
-            if (G.ns > 0) strips3<<<strip_blocks(G), 256, 0, st>>>(G, F, prev, fmt, VX, SXX, 1);
+            if (G.fst) {
+                adj_vel<true><<<grid, block, 0, st>>>(A);
+                adj_str<true><<<grid, block, 0, st>>>(A);
+                vel_rev<true><<<ggrid, block, 0, st>>>(A);
+            } else {
+                adj_vel<false><<<grid, block, 0, st>>>(A);
+                adj_str<false><<<grid, block, 0, st>>>(A);
+                vel_rev<false><<<ggrid, block, 0, st>>>(A);
+            }
+            if (G.ns > 0) restore_velocity<<<strip_blocks(G), 256, 0, st>>>(A, prev, fmt);
             if (host) {
                 hr.after_read(it - 1);
                 if (it - 1 - HostRing::R >= std::max(it0 - 1, 0)) hr.fetch(it - 1 - HostRing::R, true);
@@ -1407,10 +1644,7 @@ void backward(const sweep_elastic3d_desc* d, int mem_mode, int ckpt_every, const
             reverse(it0, it1, [&](int t) { return chunk_slot(t - (it0 - 1)); }, SF_F32);
         }
     }
-    const int per_shot = d->model_stride != 0;
-    finalize3<<<592, 256, 0, st>>>(w.gvp, G.B, per_shot, G, grad_vp);
-    finalize3<<<592, 256, 0, st>>>(w.gvs, G.B, per_shot, G, grad_vs);
-    finalize3<<<592, 256, 0, st>>>(w.grho, G.B, per_shot, G, grad_rho);
+    finalize3<<<1184, 256, 0, st>>>(A, Out{d->vp, d->vs, d->rho, {grad_vp, grad_vs, grad_rho}});
     SWEEP_LAUNCH_CHECK();
 }
 
