@@ -36,6 +36,7 @@
 #include <functional>
 
 #include "acoustic2d.cuh"
+#include "acoustic_vec.cuh"
 #include "tma.cuh"
 
 namespace sweep {
@@ -50,6 +51,7 @@ constexpr int SN = SW * SH;          // staged halo tile, floats
 constexpr int TN = TX * TZ;          // centre tile, floats
 constexpr int CPT = TN / NTH;        // cells per thread (8)
 constexpr int kMaxG = 16;            // shots per CTA, at most
+constexpr int SX = 32, SZ = 8;       // tile of the small-grid kernels: 8 threads of four cells x 8 rows
 
 enum ErrCode { ERR_TMA_WAIT_FWD = 1, ERR_TMA_WAIT_REV = 2 };
 
@@ -73,7 +75,7 @@ struct StripStore {
 struct Params {
     int B, nz, nx, nt, nsrc, nrec;
     int P;                           // row pitch (floats)
-    int ntx, ntz, G, per_shot;
+    int tx, tz, ntx, ntz, G, per_shot;   // tile (of the events), tiles, shots per CTA
     long long S;                     // shot stride (nz * P)
     long long ms;                    // model stride: 0 (shared) or S
     float dt, dz, dx;
@@ -914,6 +916,178 @@ __global__ void __launch_bounds__(NTH, 2) rev_kernel(const __grid_constant__ Rev
     }
 }
 
+// ------------------------------------------------------- small grids
+// The same steps on grids that fill no GPU with 64 x 32 tiles: one group of
+// four cells per thread (acoustic_vec.cuh), 32 x 8 cells per CTA of 64
+// threads, every load of a step issued at once instead of stage by stage.
+// Such a step is latency, not bandwidth: 96 x 128, one shot, forward 3.9 us
+// and reverse 6.5 us a step (12.3 and 18.5 us on the tiled kernels).
+constexpr int SNTH = SX / 4 * SZ;
+
+__device__ __forceinline__ avec::Cell<2> small_cell(const avec::Geo& G, const Params& P, int tile, int b)
+{
+    avec::Cell<2> q;
+    q.b = b;
+    q.c[0] = (tile % P.ntx) * SX + 4 * (threadIdx.x & 7);
+    q.c[1] = 0;
+    q.c[2] = (tile / P.ntx) * SZ + (threadIdx.x >> 3);
+    q.finish(G);
+    return q;
+}
+
+// grid (shot, tile)
+__global__ void __launch_bounds__(SNTH) fwd_small(const __grid_constant__ avec::Geo G, const __grid_constant__ Params P,
+                                                  const __grid_constant__ FwdPtrs F, const float* now,
+                                                  const float* prev, const int it)
+{
+    __shared__ __align__(16) float out[SX * SZ];
+    const int tile = P.order[blockIdx.y], b = blockIdx.x, key = b * P.ntx * P.ntz + tile;
+    const int s_beg = P.src.off[key], s_end = P.src.off[key + 1], r_beg = P.rec.off[key], r_end = P.rec.off[key + 1];
+    const avec::Cell<2> q = small_cell(G, P, tile, b);
+    const long long k = b * P.S + q.i;
+    avec::F4 un = v4::splat(0.f), u0;
+    if (q.core) {
+        avec::Step A{};
+        A.un = now; A.up = prev;
+        A.ps[0] = F.psix; A.ps[2] = F.psiz; A.psn[0] = F.psixn; A.psn[2] = F.psizn;
+        A.zt[0] = F.zetax; A.zt[2] = F.zetaz;
+        un = avec::step_cells<M, 2>(G, q, A, k, u0);
+        if (F.strips) {
+            const int z = q.c[2];
+            const bool row = z >= P.z0 && z < P.z1;
+            if (row && q.c[0] + 3 >= P.x0 && q.c[0] < P.x1 &&
+                !(z >= P.rz0 && z < P.rz1 && q.c[0] >= P.rx0 && q.c[0] + 3 < P.rx1)) {
+#pragma unroll
+                for (int l = 0; l < 4; ++l) {
+                    const int e = strip_index(P, z, q.c[0] + l);
+                    if (e < 0) continue;
+                    const long long o = (long long)b * P.nstrip + e;
+                    if (F.sbf16) static_cast<__nv_bfloat16*>(F.strips)[o] = __float2bfloat16(u0.v[l]);
+                    else static_cast<float*>(F.strips)[o] = u0.v[l];
+                }
+            }
+        }
+    }
+    if (s_beg != s_end || r_beg != r_end) {
+        v4::st(out + 4 * threadIdx.x, un);
+        __syncthreads();
+        for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
+            const int2 ev = P.src.ev[e];
+            atomicAdd(out + ev.x, __ldg(P.wavelet + (long long)ev.y * P.nt + it));
+        }
+        __syncthreads();
+        for (int e = r_beg + threadIdx.x; F.record && e < r_end; e += SNTH) {
+            const int2 ev = P.rec.ev[e];
+            const int rb = ev.y / P.nrec, rr = ev.y - rb * P.nrec;
+            F.record[((long long)rb * P.nt + it) * P.nrec + rr] = out[ev.x];
+        }
+        un = v4::ld(out + 4 * threadIdx.x);
+    }
+    if (q.core) avec::store_core(G, q, F.u_next + k, un);
+}
+
+// grid (shot, tile); the step of rev_kernel
+__global__ void __launch_bounds__(SNTH) rev_small(const __grid_constant__ avec::Geo G, const __grid_constant__ Params P,
+                                                  const __grid_constant__ RevPtrs R, const float* lnow,
+                                                  const float* lprev, const float* rnow, const float* rprev,
+                                                  const int it, const int do_recon)
+{
+    __shared__ __align__(16) float lo[SX * SZ], ro[SX * SZ];
+    const int tile = P.order[blockIdx.y], b = blockIdx.x, key = b * P.ntx * P.ntz + tile;
+    const int s_beg = P.src.off[key], s_end = P.src.off[key + 1], r_beg = P.rec.off[key], r_end = P.rec.off[key + 1];
+    const avec::Cell<2> q = small_cell(G, P, tile, b);
+    const long long k = b * P.S + q.i, mi = b * P.ms + q.i;
+    const int z = q.c[2], x = q.c[0];
+    avec::F4 lx = v4::splat(0.f), un = lx, u0 = lx, up = lx;
+    bool phys[4] = {false, false, false, false};
+    if (q.core) {
+        avec::Rev A{};
+        A.ln = lnow; A.lp = lprev;
+        A.ps[0] = R.apx; A.ps[2] = R.apz; A.zt[0] = R.azx; A.zt[2] = R.azz;
+        A.pso[0] = R.apx_o; A.pso[2] = R.apz_o; A.zto[0] = R.azx_o; A.zto[2] = R.azz_o;
+        lx = avec::adj_cells<M, 2>(G, q, A, k, mi);
+        const bool row = z >= P.z0 && z < P.z1;
+#pragma unroll
+        for (int l = 0; l < 4; ++l) phys[l] = row && x + l >= P.x0 && x + l < P.x1;
+        if (do_recon && (phys[0] || phys[3] || phys[1] || phys[2])) {
+            u0 = v4::ldg(rnow + k);
+            up = v4::ldg(rprev + k);
+            const bool rrow = z >= P.rz0 && z < P.rz1;
+            if (rrow && x + 3 >= P.rx0 && x < P.rx1) un = avec::recon_cells<M, 2>(G, rnow, k, mi, u0, up);
+#pragma unroll
+            for (int l = 0; l < 4; ++l)
+                if (phys[l] && !(rrow && x + l >= P.rx0 && x + l < P.rx1))
+                    un.v[l] = strip_value(P, R.strips, b, z, x + l);
+        }
+    }
+    const bool events = s_beg != s_end || r_beg != r_end;
+    if (events) {
+        v4::st(lo + 4 * threadIdx.x, lx);
+        v4::st(ro + 4 * threadIdx.x, un);
+        __syncthreads();
+        for (int e = r_beg + threadIdx.x; e < r_end; e += SNTH) {
+            const int2 ev = P.rec.ev[e];
+            const int rb = ev.y / P.nrec, rr = ev.y - rb * P.nrec;
+            atomicAdd(lo + ev.x, __ldg(R.adj + ((long long)rb * P.nt + it) * P.nrec + rr));
+        }
+        if (do_recon) {
+            for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
+                const int2 ev = P.src.ev[e];
+                if (strip_index(P, (tile / P.ntx) * SZ + ev.x / SX, (tile % P.ntx) * SX + ev.x % SX) >= 0)
+                    atomicAdd(ro + ev.x, -__ldg(P.wavelet + (long long)ev.y * P.nt + it));
+            }
+        }
+        __syncthreads();
+        if (R.grad_w)
+            for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
+                const int2 ev = P.src.ev[e];
+                R.grad_w[(long long)ev.y * P.nt + it] = lo[ev.x];
+            }
+        lx = v4::ld(lo + 4 * threadIdx.x);
+        un = v4::ld(ro + 4 * threadIdx.x);
+    }
+    if (q.core) {
+        avec::store_core(G, q, R.l_next + k, lx);
+        const float dt2 = P.dt * P.dt;
+        const avec::F4 v = v4::ldg(P.vv + mi);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            if (!phys[l]) continue;
+            const long long o = k + l;               // the shot's slot
+            float utt = 0.f;
+            if (do_recon) {
+                utt = (un.v[l] - 2.f * u0.v[l] + up.v[l]) / dt2;
+                const float g = 2.f * P.dt * P.dt * utt * lx.v[l] / v.v[l];
+                const float y = g - R.gcomp[o];
+                const float t = R.gacc[o] + y;
+                R.gcomp[o] = (t - R.gacc[o]) - y;
+                R.gacc[o] = t;
+            }
+            if (R.illum_s) {
+                R.illum_s[o] += utt * utt;
+                R.illum_r[o] += lx.v[l] * lx.v[l];
+            }
+        }
+    }
+    if (!do_recon) return;
+    if (events) {
+        __syncthreads();
+        for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
+            const int2 ev = P.src.ev[e];
+            atomicAdd(ro + ev.x, __ldg(P.wavelet + (long long)ev.y * P.nt + it));
+        }
+        __syncthreads();
+        un = v4::ld(ro + 4 * threadIdx.x);
+    }
+    if (phys[0] && phys[3]) {
+        v4::st(R.r_next + k, un);
+    } else {
+#pragma unroll
+        for (int l = 0; l < 4; ++l)
+            if (phys[l]) R.r_next[k + l] = un.v[l];
+    }
+}
+
 // One step's strips (fp32 strip set, `strips`) into the scaled faces of a step
 // slot: one CTA per (shot, face, block of kQB cells) -- max |value| of the
 // block, its scale, the codes (reference boundarysaver.cu:957-990, 1050-1080:
@@ -1015,8 +1189,12 @@ __global__ void pitch_copy_kernel(const float* __restrict__ src, float* __restri
 }
 
 // ------------------------------------------------------------------- host
+constexpr long long kSmallTiles = 2960;
+
 struct Plan {
     Params P;
+    bool small;                      // the small-grid kernels run this shape
+    avec::Geo geo;                   // their view of it
     bool host_tape = false;          // boundary-saving tape in pinned host memory (SWEEP_MEM_HOST_TAPE)
     int nslot;                       // gradient accumulator slots (backward)
     int nm;                          // model copies (1 shared, B per-shot)
@@ -1037,7 +1215,7 @@ static int build_events(const Params& P, const int32_t* loc, int n, int32_t* off
         const int ix = loc[2 * e], iz = loc[2 * e + 1];
         // cells of the outer stencil halo are never updated: treated as off-grid
         if (ix < M || ix >= P.nx - M || iz < M || iz >= P.nz - M) return -1;
-        return (e / n) * ntiles + (iz / TZ) * P.ntx + ix / TX;
+        return (e / n) * ntiles + (iz / P.tz) * P.ntx + ix / P.tx;
     };
     for (int e = 0; e < P.B * n; ++e) {
         const int k = key_of(e);
@@ -1049,7 +1227,7 @@ static int build_events(const Params& P, const int32_t* loc, int n, int32_t* off
         const int k = key_of(e);
         if (k < 0) continue;
         const int ix = loc[2 * e], iz = loc[2 * e + 1];
-        ev[fill[k]++] = make_int2((iz % TZ) * TX + ix % TX, e);
+        ev[fill[k]++] = make_int2((iz % P.tz) * P.tx + ix % P.tx, e);
     }
     return off[nkey];
 }
@@ -1117,9 +1295,10 @@ static Plan make_plan(const sweep_acoustic_desc* d)
     P.ms = P.per_shot ? P.S : 0;
     pl.nm = P.per_shot ? d->B : 1;
     P.wavelet = d->wavelet;
+    P.tx = TX; P.tz = TZ;
     P.ntx = (d->nx + TX - 1) / TX;
     P.ntz = (d->nz + TZ - 1) / TZ;
-    const int ntiles = P.ntx * P.ntz;
+    int ntiles = P.ntx * P.ntz;
     const sweep_b200_schedule sc = recorded_schedule(d);
     pl.Gf = P.per_shot ? 1 : choose_group(ntiles, P.B, "SWEEP_B200_SHOTS_PER_CTA_FWD", 2, sc.shots_fwd);
     pl.Gr = P.per_shot ? 1 : choose_group(ntiles, P.B, "SWEEP_B200_SHOTS_PER_CTA_REV", 8, sc.shots_rev);
@@ -1129,6 +1308,23 @@ static Plan make_plan(const sweep_acoustic_desc* d)
     pl.gridr = dim3((P.B + pl.Gr - 1) / pl.Gr, ntiles);
     pl.nslot = P.per_shot ? P.B : (int)pl.gridr.x;
     P.G = pl.Gr;
+    // Few tiles: a step of the tiled kernels lasts as long as one CTA, which
+    // walks its shots' tiles through its stages eight cells per thread, so
+    // these grids run four cells per thread on 32 x 8 tiles, one shot per CTA
+    // (the schedule's shots per CTA do not apply).  The line is where the
+    // fields of a step leave the L2, which the tiled kernels' reuse over shots
+    // then saves: gradients of 200 steps, small / tiled, 96 x 128 one shot
+    // (15 tiles) 2.7 / 6.8 ms, 200 x 400 x 8 shots (512) 8.3 / 11.2,
+    // 256 x 768 x 8 (1232) 14.1 / 29.5, x 12 (1848) 22.7 / 34.6, x 16 (2464)
+    // 31.0 / 37.3, x 32 (4928) 63 / 51.6, 400 x 1200 x 8 (2480) 33.1 / 36.6.
+    pl.small = (long long)ntiles * P.B <= kSmallTiles;
+    if (pl.small) {
+        P.tx = SX; P.tz = SZ;
+        P.ntx = (d->nx + SX - 1) / SX;
+        P.ntz = (d->nz + SZ - 1) / SZ;
+        pl.gridf = pl.gridr = dim3((unsigned)P.B, (unsigned)(P.ntx * P.ntz));
+        pl.nslot = P.B;
+    }
     return pl;
 }
 
@@ -1138,6 +1334,7 @@ struct Common {
     int2 *src_ev, *rec_ev;
     int* order;
     int* err;
+    float *profx, *profz;            // small grids: a, b, d b, d a, zero past their ends
 };
 
 struct FwdWork {
@@ -1171,6 +1368,10 @@ static Common carve_common(Carve& c, const Plan& pl)
     w.rec_ev = c.take<int2>((long long)pl.P.B * std::max(pl.P.nrec, 1));
     w.order = c.take<int>((long long)pl.P.ntx * pl.P.ntz);
     w.err = c.take<int>(1);
+    if (pl.small) {
+        w.profx = c.take<float>(4LL * (pl.P.P + 2 * avec::kGuard));
+        w.profz = c.take<float>(4LL * (pl.P.nz + 2 * avec::kGuard));
+    }
     return w;
 }
 
@@ -1322,13 +1523,40 @@ static void tile_order(const Params& P, int32_t* order)
     int n = 0;
     for (int want = 2; want >= 0; --want)
         for (int t = 0; t < ntiles; ++t) {
-            const int tx0 = (t % P.ntx) * TX, tz0 = (t / P.ntx) * TZ;
-            const bool rx = tx0 < P.px0 || tx0 + TX > P.px1, rz = tz0 < P.pz0 || tz0 + TZ > P.pz1;
+            const int tx0 = (t % P.ntx) * P.tx, tz0 = (t / P.ntx) * P.tz;
+            const bool rx = tx0 < P.px0 || tx0 + P.tx > P.px1, rz = tz0 < P.pz0 || tz0 + P.tz > P.pz1;
             if ((rx ? 1 : 0) + (rz ? 1 : 0) == want) order[n++] = t;
         }
 }
 
 // Per-call set-up shared by both passes: model fields, event tables, error flag.
+static void small_setup(Plan& pl, const Common& w, cudaStream_t st)
+{
+    const Params& P = pl.P;
+    avec::Geo& G = pl.geo;
+    G = avec::Geo{};
+    G.nd = 2; G.B = P.B; G.nz = P.nz; G.ny = 1; G.nx = P.nx; G.nt = P.nt; G.M = M;
+    G.P = G.SY = G.SZ = P.P;
+    G.S = P.S;
+    G.lo[0] = P.x0; G.hi[0] = P.x1; G.lo[2] = P.z0; G.hi[2] = P.z1;
+    G.hi[1] = 1;
+    G.nbx = P.ntx;
+    G.dt = P.dt;
+    G.ih2[0] = 1.0f / (P.dx * P.dx); G.ih2[2] = 1.0f / (P.dz * P.dz);
+    G.ih[0] = 1.0f / P.dx; G.ih[2] = 1.0f / P.dz;
+    for (int k = 0; k <= M; ++k) { G.lc[k] = P.lc[k]; G.gc[k] = P.gc[k]; }
+    G.cf = w.cf; G.ca = w.ca; G.ms = P.ms;
+    const int lx = P.P + 2 * avec::kGuard, lz = P.nz + 2 * avec::kGuard;
+    avec::prep_profiles<<<8, 256, 0, st>>>(P.ax, P.bx, P.dbx, P.nx, G, G.ih[0], avec::kGuard, lx, w.profx);
+    avec::prep_profiles<<<8, 256, 0, st>>>(P.az, P.bz, P.dbz, P.nz, G, G.ih[2], avec::kGuard, lz, w.profz);
+    SWEEP_LAUNCH_CHECK();
+    auto axis = [&](int a, const float* p, int len) {
+        G.a[a] = p + avec::kGuard; G.b[a] = G.a[a] + len; G.db[a] = G.b[a] + len; G.da[a] = G.db[a] + len;
+    };
+    axis(0, w.profx, lx);
+    axis(2, w.profz, lz);
+}
+
 static void setup_common(const sweep_acoustic_desc* d, Plan& pl, const Common& w, cudaStream_t st,
                          const HostStage& h)
 {
@@ -1336,6 +1564,7 @@ static void setup_common(const sweep_acoustic_desc* d, Plan& pl, const Common& w
     prep_kernel<<<592, 256, 0, st>>>(d->vp, pl.nm, d->nz, d->nx, P.P, d->dt, w.cf, w.ca, w.vv);
     SWEEP_LAUNCH_CHECK();
     P.cf = w.cf; P.vv = w.vv;
+    if (pl.small) small_setup(pl, w, st);
     const size_t ns = (size_t)d->B * d->nsrc * 2, nr = (size_t)d->B * d->nrec * 2;
     if (ns) SWEEP_CUDA(cudaMemcpyAsync(h.loc_src, d->src_loc, ns * 4, cudaMemcpyDeviceToHost, st));
     if (nr) SWEEP_CUDA(cudaMemcpyAsync(h.loc_rec, d->rec_loc, nr * 4, cudaMemcpyDeviceToHost, st));
@@ -1522,7 +1751,8 @@ static void forward_steps(const Plan& pl, const FwdMaps& maps, const FwdWork& w,
         F.strips = (slot && scaled) ? static_cast<void*>(w.scratch) : slot;
         F.sbf16 = PF.st.fmt == SF_BF16;
         const cudaStream_t ls = gs.stream();
-        fwd_kernel<<<pl.gridf, NTH, fwd_smem(), ls>>>(maps, PF, F, it);
+        if (pl.small) fwd_small<<<pl.gridf, SNTH, 0, ls>>>(pl.geo, PF, F, w.u[S.in], w.u[S.ip], it);
+        else fwd_kernel<<<pl.gridf, NTH, fwd_smem(), ls>>>(maps, PF, F, it);
         SWEEP_LAUNCH_CHECK();
         if (slot && scaled) {
             quantize_strips<<<qblocks, kQB, 0, ls>>>(PF, w.scratch, slot);
@@ -1815,7 +2045,11 @@ void backward_with(const sweep_acoustic_desc* d, int mem_mode, int ckpt_every, c
             R.rprev = rp; R.rnow = rn; R.r_next = w.r[rx];
             R.strips = do_recon ? strips_of(it - 1) : nullptr;
             if (host && do_recon) hr.before_read(it - 1);
-            rev_kernel<<<pl.gridr, NTH, rev_smem(), gs.stream()>>>(maps, P, R, it, do_recon);
+            if (pl.small)
+                rev_small<<<pl.gridr, SNTH, 0, gs.stream()>>>(pl.geo, P, R, w.l[ln], w.l[lp], w.r[rn], w.r[rp], it,
+                                                              do_recon);
+            else
+                rev_kernel<<<pl.gridr, NTH, rev_smem(), gs.stream()>>>(maps, P, R, it, do_recon);
             SWEEP_LAUNCH_CHECK();
             if (host && do_recon) {
                 hr.after_read(it - 1);
