@@ -11,29 +11,19 @@
 //               + source injection, the 5-field boundary-strip save and the
 //               receiver gather of the same step, done by the CTA that owns
 //               the cell                                   sg_driver.cuh:291-340
-//   reverse, per step (reference: 8-13 launches, sg_driver.cuh:786-806):
-//     rev_str   stress reconstruction (NOPML) + strip restore, the residual
-//               injection, the vp/vs/rho imaging and the receiver rho fix,
-//               sharing the velocity derivatives between reconstruction and
-//               imaging                                    kernels.cuh:455-535,
-//                                                          601-663; common.cu:77-117
-//     rev_sadj  stress-adjoint apply; the four q fields (stress-adjoint
-//               prepare, kernels.cuh:548-750) are built in shared memory for
-//               the tile and its halo instead of a global round trip
-//     rev_vadj  velocity-adjoint apply with p built the same way
-//               (kernels.cuh:873-1019) + carrier capture, velocity
-//               reconstruction (NOPML) and strip restore  kernels.cuh:365-450,
-//                                                          driver_traits.cuh:758-826
-//
-// Building q / p in shared memory lets every CTA recompute them for its halo,
-// so the adjoint CPML memories are double-buffered (read the old set, write
-// the new one) and neighbouring CTAs never race on them.
+//   reverse, per step (reference: 8-13 launches, sg_driver.cuh:786-806): the
+//     four-cells-per-thread kernels of elastic_vec.cuh between two restores of
+//     the strips -- `events` (residuals in, sources out), `rev_a` (transpose
+//     into the adjoint velocities beside the stress reconstruction with its
+//     image), stress strips, `rev_b` (transpose into the adjoint stresses
+//     beside the velocity reconstruction with its rho image), velocity strips.
 //
 // Layout: fields are pitched (B, nz, P), P = nx rounded up to 32 floats.
 // CPML memories live in per-axis slabs (x: (B, nz, WX), z: (B, WZ, P)) that
 // cover the PML band plus one cell (the half-cell profile reaches one cell
 // further inward on the high side; reference context.h:359-400 keeps wider
-// slabs for the same reason).  Tiles are 32 x 32 cells, 256 threads, 4 rows
+// slabs for the same reason); the adjoint memories are laid out by
+// elastic_vec.cuh.  The forward's tiles are 32 x 32 cells, 256 threads, 4 rows
 // per thread.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -46,6 +36,7 @@
 
 #include "common.cuh"
 #include "elastic2d.cuh"
+#include "elastic_vec.cuh"
 #include "tma.cuh"
 
 namespace sweep {
@@ -104,12 +95,12 @@ struct Geo {
     int fs;                         // bit f: traction-free face f (z_lo, z_hi, x_lo, x_hi), pad 0
 };
 
-enum { ERR_WAIT_FWD = 1, ERR_WAIT_REV = 2 };
+enum { ERR_WAIT_FWD = 1 };
 constexpr int CN = TX * TZ;         // floats of a centre tile
 
 // Models on the pitched grid, one copy (shared) or B copies (per shot).
 struct Models {
-    const float *rho, *lam, *mu, *bv, *vp, *vs;   // bv = dt * (1 / rho)
+    const float *lam, *mu, *bv;                   // bv = dt * (1 / rho)
 };
 
 // Memory-variable slabs of one wavefield set: x slab m_x[k] (B, nz, WX) and
@@ -134,12 +125,6 @@ __device__ __forceinline__ bool in_pml(const Geo& G, int ix, int iz)
 __device__ __forceinline__ bool in_core(const Geo& G, int ix, int iz)
 {
     return ix >= M && ix < G.nx - M && iz >= M && iz < G.nz - M;
-}
-// Reverse (NOPML) reconstruction region: the box minus one cell per face
-// (reference kernels.cuh:430-440, band abcn + M + 1).
-__device__ __forceinline__ bool in_recon(const Geo& G, int ix, int iz)
-{
-    return ix > G.x0 && ix < G.x1 - 1 && iz > G.z0 && iz < G.z1 - 1;
 }
 __device__ __forceinline__ bool in_box(const Geo& G, int ix, int iz)
 {
@@ -280,15 +265,6 @@ __device__ __forceinline__ bool fs_band(const FsAx& a, int j)
 {
     return (a.lo_on && j >= a.lo && j < a.lo + M) || (a.hi_on && j > a.hi - M && j <= a.hi);
 }
-__device__ __forceinline__ bool fs_air(const FsAx& a, int j)
-{
-    return (a.lo_on && j < a.lo) || (a.hi_on && j > a.hi);
-}
-// a cell whose adjoint stencil reaches a band or an image
-__device__ __forceinline__ bool fs_near(const FsAx& a, int j)
-{
-    return (a.lo_on && j < a.lo + 2 * M) || (a.hi_on && j > a.hi - 2 * M);
-}
 __device__ __forceinline__ bool fs_zrow(const Geo& G, int iz)
 {
     return ((G.fs & 1) && iz == G.z0) || ((G.fs & 2) && iz == G.z1 - 1);
@@ -336,92 +312,6 @@ __device__ __forceinline__ float d_fs(const FsAx& a, const float* t, int c, int 
     if (!FS || !fs_band(a, j)) return d_plain<S, FWD>(t, c, inv);
     return (FWD ? fs_val<S>(a, t, c, j, j + 1, odd, half) - fs_val<S>(a, t, c, j, j, odd, half)
                 : fs_val<S>(a, t, c, j, j, odd, half) - fs_val<S>(a, t, c, j, j - 1, odd, half)) * inv;
-}
-
-// Transposed reduced stencil at index m, read from the tile line through
-// cell c (index j0): output cells in a band contribute with weight 1, the
-// others with the full weight; air cells hold no adjoint (sources and
-// receivers beyond a free surface are off the grid).  Every cell it reads
-// lies within M of j0; the range test only guards the tile.
-template <int S, bool FWD>
-__device__ __forceinline__ float adj_red(const FsAx& a, const float* q, int c, int j0, int m, int n)
-{
-    auto live = [&](int j) { return j >= 0 && j < n && !fs_band(a, j) && !fs_air(a, j) && j - j0 >= -M && j - j0 <= M; };
-    auto at = [&](int j) { return (j - j0 >= -M && j - j0 <= M) ? q[c + (j - j0) * S] : 0.f; };
-    const float w[M] = {C1, C2, C3, C4};
-    float acc = 0.f;
-#pragma unroll
-    for (int k = 1; k <= M; ++k) {
-        const int jp = FWD ? m + k - 1 : m + k;
-        const int jm = FWD ? m - k : m - k + 1;
-        if (live(jp)) acc += w[k - 1] * at(jp);
-        if (live(jm)) acc -= w[k - 1] * at(jm);
-    }
-    if (FWD) {
-        if (fs_band(a, m)) acc += at(m);
-        if (fs_band(a, m - 1)) acc -= at(m - 1);
-    } else {
-        if (fs_band(a, m + 1)) acc += at(m + 1);
-        if (fs_band(a, m)) acc -= at(m);
-    }
-    return acc;
-}
-
-// Adjoint of d_fs (negated transpose; the plain one is D- for a D+ forward
-// and D+ for a D- forward): the reduced transpose plus, for each free face
-// whose image of this cell lies in the air, the transpose there folded back
-// with the field's parity.
-template <bool FS, int S, bool FWD>
-__device__ __forceinline__ float adj_fs(const FsAx& a, const float* q, int c, int j, int n, bool odd, bool half,
-                                        float inv)
-{
-    if (!FS || !fs_near(a, j)) return d_plain<S, !FWD>(q, c, inv);
-    if (fs_air(a, j)) return 0.f;
-    float g = adj_red<S, FWD>(a, q, c, j, j, n);
-    const float par = odd ? -1.f : 1.f;
-    if (a.lo_on) {
-        const int mj = half ? 2 * a.lo - 1 - j : 2 * a.lo - j;
-        if (mj < a.lo) g += par * adj_red<S, FWD>(a, q, c, j, mj, n);
-    }
-    if (a.hi_on) {
-        const int mj = half ? 2 * a.hi - 1 - j : 2 * a.hi - j;
-        if (mj >= (half ? a.hi : a.hi + 1)) g += par * adj_red<S, FWD>(a, q, c, j, mj, n);
-    }
-    return g * inv;
-}
-
-// Cooperative load of NF fields' tiles plus an M-cell halo (zero outside the
-// grid) into shared memory: every thread issues all its global loads before
-// its first shared store, so the loads of a CTA are in flight together.
-constexpr int NLD = (HN + NTH - 1) / NTH;   // loads per thread per field
-
-template <int NF>
-__device__ __forceinline__ void load_tiles(float* const (&t)[NF], const float* const (&g)[NF], const Geo& G,
-                                           int tz0, int tx0)
-{
-    const int tid = threadIdx.x + threadIdx.y * TX;
-    float v[NF][NLD];
-    long long off[NLD];
-    bool ok[NLD];
-#pragma unroll
-    for (int j = 0; j < NLD; ++j) {
-        const int k = tid + j * NTH;
-        const int lz = k / HX, lx = k - lz * HX;
-        const int iz = tz0 - M + lz, ix = tx0 - M + lx;
-        ok[j] = k < HN && (unsigned)iz < (unsigned)G.nz && (unsigned)ix < (unsigned)G.nx;
-        off[j] = (long long)iz * G.P + ix;
-    }
-#pragma unroll
-    for (int f = 0; f < NF; ++f)
-#pragma unroll
-        for (int j = 0; j < NLD; ++j) v[f][j] = ok[j] ? __ldg(g[f] + off[j]) : 0.f;
-#pragma unroll
-    for (int f = 0; f < NF; ++f)
-#pragma unroll
-        for (int j = 0; j < NLD; ++j) {
-            const int k = tid + j * NTH;
-            if (k < HN) t[f][k] = v[f][j];
-        }
 }
 
 // Add w to the stress field `fld` (one of SXX, SZZ, SXZ) held in registers.
@@ -825,443 +715,56 @@ __global__ void vsrc_forward(const Geo G, float* vx, float* vz, void* strips, fl
     }
 }
 
-// Body-force sources, reverse step it (reference fix_rho_grad_at_sources,
-// common.cu:40-75, then uninject_forward_source; elastic2d/driver_traits.cuh
-// 380-410): before this step's residuals enter the adjoint, add
-// (adjoint v * w) / rho to the rho-gradient slot of the shot at each source
-// cell, and take the wavelet back out of the reconstructed vx / vz there.
-__global__ void vsrc_reverse(const Geo G, const float* avx, const float* avz, float* vx, float* vz,
-                             float* grho, const float* rho, int g_shots, int it)
-{
-    const int b = blockIdx.x;
-    const long long so = (long long)b * G.S;
-    const float* const av[2] = {avx, avz};
-    float* const vf[2] = {vx, vz};
-    float* const gslot = grho + (long long)(b / g_shots) * G.S;
-    for (int s = threadIdx.x; s < G.nsrc; s += blockDim.x) {
-        const int ix = G.src_loc[2 * ((long long)b * G.nsrc + s)], iz = G.src_loc[2 * ((long long)b * G.nsrc + s) + 1];
-        if (ix < 0 || ix >= G.nx || iz < 0 || iz >= G.nz) continue;
-        const long long c = (long long)iz * G.P + ix;
-        const float w = G.wavelet[((long long)b * G.nsrc + s) * G.nt + it];
-        for (int k = 0; k < G.nvf; ++k) {
-            const int fld = G.vf[k];
-            atomicAdd(gslot + c, (av[fld][so + c] * w) / rho[(long long)b * G.ms + c]);
-            atomicAdd(vf[fld] + so + c, -w);
-        }
-    }
-}
-
 // ------------------------------------------------------------------ reverse
-struct RevArgs {
-    Geo G;
-    Models m;
-    float* f[5];          // reconstructed forward fields
-    float* cvx;           // carriers: v of the next step (box cells)
-    float* cvz;
-    float* a[5];          // adjoint fields (stress ones hold the negated adjoint)
-    Slabs mo, mn;         // adjoint memories: read set (old), write set (new)
-    const void* strips;   // step slot holding the strips of step it - 1 (format G.st)
-    const float* adj;     // (B, nt, nrec, nrf) residuals
-    float* gvp;           // gradient slots (nslot, S)
-    float* gvs;
-    float* grho;
-    int G_shots;          // shots per CTA of rev_str (shared models)
-    int it;
-};
-// adjoint memory slots: x {vxx, vzx, sxxx, sxzx}, z {vzz, vxz, szzz, sxzz}
-
-// Reverse stress half for shots [g*G_shots, ...): residual injection
-// (reference inject_residuals, signs: stress -1, velocity +1), stress
-// reconstruction on the NOPML region with the forward source removed
-// (kernels.cuh:455-493 after uninject_forward_source) or strip restore, the
-// fused vp / vs / rho imaging on the physical box (kernels.cuh:601-663) and
-// the receiver rho correction (common.cu:77-117).  The gradient contributions
-// of the CTA's shots are summed in registers and added to slot blockIdx.y.
-template <bool FS>
-__global__ void __launch_bounds__(NTH, 4) rev_str(RevArgs A)
+// Grid cell of strip index si (the inverse of strip_index).
+__device__ __forceinline__ void strip_cell(const Geo& G, int si, int& iz, int& ix)
 {
-    extern __shared__ float sm[];
-    float *tvx = sm, *tvz = sm + HN;
-    const Geo& G = A.G;
-    const int tile = blockIdx.x, grp = blockIdx.y;
-    int tz0, tx0;
-    tile_origin(G, tile, tz0, tx0);
-    const int lx = threadIdx.x, ix = tx0 + lx;
-    const int b_lo = grp * A.G_shots, b_hi = min(G.B, b_lo + A.G_shots);
-    float gvp[RPT], gvs[RPT], grho[RPT];
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) gvp[r] = gvs[r] = grho[r] = 0.f;
-    const int tid = threadIdx.x + threadIdx.y * TX;
-
-    for (int b = b_lo; b < b_hi; ++b) {
-        const long long so = (long long)b * G.S;
-        const int key = b * G.ntx * G.ntz + tile;
-        const int r0 = G.rec.off[key], r1 = G.rec.off[key + 1];
-        const int s0 = G.src.off[key], s1 = G.src.off[key + 1];
-        __syncthreads();                       // previous shot's tiles consumed
-        {
-            float* const t[2] = {tvx, tvz};
-            const float* const g[2] = {A.f[VX] + so, A.f[VZ] + so};
-            load_tiles<2>(t, g, G, tz0, tx0);
-        }
-        // residuals of step it into the adjoint fields of this tile's receivers
-        for (int e = r0 + tid; e < r1; e += NTH) {
-            const int2 ev = G.rec.ev[e];
-            const long long i = so + (long long)(tz0 + ev.x / TX) * G.P + tx0 + ev.x % TX;
-            const float* res = A.adj + ((long long)(b * G.nt + A.it) * G.nrec + (ev.y - b * G.nrec)) * G.nrf;
-            for (int k = 0; k < G.nrf; ++k) {
-                const int fld = G.rf[k];
-                atomicAdd(A.a[fld] + i, fld >= SXX ? -res[k] : res[k]);
-            }
-        }
-        __syncthreads();
-        const float* __restrict__ lam_ = A.m.lam + (long long)b * G.ms;
-        const float* __restrict__ mu_ = A.m.mu + (long long)b * G.ms;
-        const float* __restrict__ rho_ = A.m.rho + (long long)b * G.ms;
-        const float* __restrict__ vp_ = A.m.vp + (long long)b * G.ms;
-        const float* __restrict__ vs_ = A.m.vs + (long long)b * G.ms;
-#pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-            const int lz = threadIdx.y + 8 * r, iz = tz0 + lz;
-            if (iz >= G.nz || ix >= G.nx) continue;
-            const long long i = (long long)iz * G.P + ix;
-            if (!in_core(G, ix, iz)) {
-                const int si = strip_index(G, iz, ix);
-                if (si >= 0) {
-                    A.f[SXX][so + i] = strip_val(G, A.strips, b, SXX, iz, ix, si);
-                    A.f[SZZ][so + i] = strip_val(G, A.strips, b, SZZ, iz, ix, si);
-                    A.f[SXZ][so + i] = strip_val(G, A.strips, b, SXZ, iz, ix, si);
-                }
-                continue;
-            }
-            const int c = (lz + M) * HX + lx + M;
-            const FsAx az = fs_zax(G), ax = fs_xax(G);
-            const float dvx_dx = d_fs<FS, 1, false>(ax, tvx, c, ix, true, true, G.idx);
-            const float dvz_dz = d_fs<FS, HX, false>(az, tvz, c, iz, true, true, G.idz);
-            const float dvx_dz = d_fs<FS, HX, true>(az, tvx, c, iz, false, false, G.idz);
-            const float dvz_dx = d_fs<FS, 1, true>(ax, tvz, c, ix, false, false, G.idx);
-            if (in_recon(G, ix, iz)) {
-                float sxx = A.f[SXX][so + i], szz = A.f[SZZ][so + i], sxz = A.f[SXZ][so + i];
-                const int cell = lz * TX + lx;
-                for (int e = s0; e < s1; ++e) {
-                    const int2 ev = G.src.ev[e];
-                    if (ev.x != cell) continue;
-                    const float w = G.wavelet[(long long)ev.y * G.nt + A.it];
-                    for (int k = 0; k < G.nsf; ++k) add_to(G.sf[k], -w, sxx, szz, sxz);
-                }
-                const float lam = lam_[i], mu = mu_[i];
-                A.f[SXX][so + i] = sxx - G.dt * ((lam + 2.f * mu) * dvx_dx + lam * dvz_dz);
-                A.f[SZZ][so + i] = szz - G.dt * ((lam + 2.f * mu) * dvz_dz + lam * dvx_dx);
-                A.f[SXZ][so + i] = sxz - G.dt * mu * (dvx_dz + dvz_dx);
-            } else {
-                const int si = strip_index(G, iz, ix);
-                if (si >= 0) {
-                    A.f[SXX][so + i] = strip_val(G, A.strips, b, SXX, iz, ix, si);
-                    A.f[SZZ][so + i] = strip_val(G, A.strips, b, SZZ, iz, ix, si);
-                    A.f[SXZ][so + i] = strip_val(G, A.strips, b, SXZ, iz, ix, si);
-                }
-            }
-            if (in_box(G, ix, iz)) {
-                // the stresses a surface zeroes carry no adjoint there
-                const bool zs = FS && fs_zrow(G, iz), xs = FS && fs_xcol(G, ix);
-                const float bsxx = xs ? 0.f : A.a[SXX][so + i];
-                const float bszz = zs ? 0.f : A.a[SZZ][so + i];
-                const float bsxz = FS && fs_zero_shear(G, ix, iz) ? 0.f : A.a[SXZ][so + i];
-                const float rho = rho_[i], vp = vp_[i], vs = vs_[i];
-                float gl, gm;
-                if (zs && xs) {
-                    gl = gm = 0.f;           // a corner: every stress is zeroed
-                } else if (zs || xs) {
-                    // d / d(lam, mu) of the corrected surface update dt C d(v
-                    // along the surface), C = 4 mu (lam + mu) / (lam + 2 mu)
-                    // (kernels.cuh:633-646)
-                    const float vp2 = vp * vp, vs2 = vs * vs, vp4 = vp2 * vp2;
-                    const float a = zs ? bsxx * dvx_dx : bszz * dvz_dz;
-                    gl = a * 4.f * vs2 * vs2 / vp4;
-                    gm = a * 4.f * (vp4 - 2.f * vp2 * vs2 + 2.f * vs2 * vs2) / vp4;
-                } else {
-                    gl = (bsxx + bszz) * (dvx_dx + dvz_dz);
-                    gm = 2.f * (bsxx * dvx_dx + bszz * dvz_dz);
-                }
-                gm += bsxz * (dvx_dz + dvz_dx);
-                gvp[r] += -2.f * rho * vp * gl * G.dt;
-                gvs[r] += -(-4.f * rho * vs * gl + 2.f * rho * vs * gm) * G.dt;
-                float gr = (A.a[VX][so + i] * (tvx[c] - A.cvx[so + i]) + A.a[VZ][so + i] * (tvz[c] - A.cvz[so + i])) / rho;
-                gr -= gl * (vp * vp - 2.f * vs * vs) * G.dt + gm * (vs * vs) * G.dt;
-                grho[r] += gr;
-            }
-        }
-    }
-    // add the group's image to its slot
-    const long long slot = (long long)grp * G.S;
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        const int iz = tz0 + threadIdx.y + 8 * r;
-        if (!in_box(G, ix, iz)) continue;
-        const long long i = slot + (long long)iz * G.P + ix;
-        A.gvp[i] += gvp[r];
-        A.gvs[i] += gvs[r];
-        A.grho[i] += grho[r];
-    }
-    // receiver rho correction after the image (velocity receivers in the box)
-    bool any = false;
-    for (int b = b_lo; b < b_hi; ++b) {
-        const int key = b * G.ntx * G.ntz + tile;
-        any |= G.rec.off[key + 1] > G.rec.off[key];
-    }
-    if (!any) return;
-    __syncthreads();
-    for (int b = b_lo; b < b_hi; ++b) {
-        const long long so = (long long)b * G.S;
-        const int key = b * G.ntx * G.ntz + tile;
-        const float* __restrict__ rho_ = A.m.rho + (long long)b * G.ms;
-        for (int e = G.rec.off[key] + tid; e < G.rec.off[key + 1]; e += NTH) {
-            const int2 ev = G.rec.ev[e];
-            const int iz = tz0 + ev.x / TX, jx = tx0 + ev.x % TX;
-            if (!in_box(G, jx, iz)) continue;
-            const long long i = (long long)iz * G.P + jx;
-            const float* res = A.adj + ((long long)(b * G.nt + A.it) * G.nrec + (ev.y - b * G.nrec)) * G.nrf;
-            for (int k = 0; k < G.nrf; ++k) {
-                const int fld = G.rf[k];
-                if (fld > VZ) continue;
-                const float now = A.f[fld][so + i];
-                const float nxt = (fld == VX ? A.cvx : A.cvz)[so + i];
-                atomicAdd(A.grho + slot + i, -res[k] * (now - nxt) / rho_[i]);
-            }
-        }
+    constexpr int W = M + 1;
+    const int row = G.bw + 2 * M, base = 2 * M * G.bw;
+    if (si < base) {
+        const int r = si / G.bw;
+        iz = r < M ? G.z0 - M + r : G.z1 + r - M;
+        ix = G.x0 + si - r * G.bw;
+    } else if (si < base + 2 * row) {
+        const int r = (si - base) / row;
+        iz = r ? G.z1 - 1 : G.z0;
+        ix = G.x0 - M + si - base - r * row;
+    } else {
+        const int r = (si - base - 2 * row) / (2 * W), j = si - base - 2 * row - r * 2 * W;
+        iz = G.z0 + 1 + r;
+        ix = j < W ? G.x0 - M + j : G.x1 - 1 + j - W;
     }
 }
 
-__device__ __forceinline__ bool owns(int lz, int lx)
+// Field f0 + blockIdx.y of the strips from a step slot.  Velocities add the rho
+// image of the box cells outside the reverse box: the difference this makes in
+// the two of them.
+__global__ void restore(const Geo G, const evec::Geo E, const evec::Rev R, const void* __restrict__ slot, int f0)
 {
-    return lz >= M && lz < M + TZ && lx >= M && lx < M + TX;
-}
-
-// Stress-adjoint apply (reference kernels.cuh:807-837) with q = (qxx, qzz,
-// qxz, qzx) of the stress-adjoint prepare (kernels.cuh:676-750) built in
-// shared memory for the tile and its halo.  The owner of a cell writes its new
-// adjoint CPML memories.
-template <bool FS>
-__global__ void __launch_bounds__(NTH, 4) rev_sadj(RevArgs A)
-{
-    extern __shared__ float sm[];
-    float* tq[4] = {sm, sm + HN, sm + 2 * HN, sm + 3 * HN};
-    const Geo& G = A.G;
-    const int b = blockIdx.y;
-    int tz0, tx0;
-    tile_origin(G, blockIdx.x, tz0, tx0);
-    const long long so = (long long)b * G.S;
-    const float* __restrict__ lam_ = A.m.lam + (long long)b * G.ms;
-    const float* __restrict__ mu_ = A.m.mu + (long long)b * G.ms;
-    const int tid = threadIdx.x + threadIdx.y * TX;
-    const float* __restrict__ mo_vxx = A.mo.x[XM_VXX];
-    const float* __restrict__ mo_vzx = A.mo.x[XM_VZX];
-    const float* __restrict__ mo_vzz = A.mo.z[ZM_VZZ];
-    const float* __restrict__ mo_vxz = A.mo.z[ZM_VXZ];
-    float* __restrict__ mn_vxx = A.mn.x[XM_VXX];
-    float* __restrict__ mn_vzx = A.mn.x[XM_VZX];
-    float* __restrict__ mn_vzz = A.mn.z[ZM_VZZ];
-    float* __restrict__ mn_vxz = A.mn.z[ZM_VXZ];
-    float rs[NLD][5];
-#pragma unroll
-    for (int j = 0; j < NLD; ++j) {
-        const int k = tid + j * NTH;
-        const int lz = k / HX, lx = k - lz * HX;
-        const int iz = tz0 - M + lz, ix = tx0 - M + lx;
-        const bool ok = k < HN && (unsigned)iz < (unsigned)G.nz && (unsigned)ix < (unsigned)G.nx;
-        const long long i = (long long)iz * G.P + ix;
-        rs[j][0] = ok ? A.a[SXX][so + i] : 0.f;
-        rs[j][1] = ok ? A.a[SZZ][so + i] : 0.f;
-        rs[j][2] = ok ? A.a[SXZ][so + i] : 0.f;
-        rs[j][3] = ok ? lam_[i] : 0.f;
-        rs[j][4] = ok ? mu_[i] : 0.f;
+    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e >= (long long)G.B * G.nstrip) return;
+    const int b0 = (int)(e / G.nstrip), si = (int)(e - (long long)b0 * G.nstrip);
+    int iz, ix;
+    strip_cell(G, si, iz, ix);
+    const long long c = (long long)iz * G.P + ix;
+    const bool img = f0 == VX && R.it > 1 && in_box(G, ix, iz) &&
+                     !(iz >= E.rz0 && iz < E.rz1 && ix >= E.rx0 && ix < E.rx1);
+    if (!img) {
+        const int f = f0 + blockIdx.y;
+        R.f.f[f][b0 * G.S + c] = strip_val(G, slot, b0, f, iz, ix, si);
+        return;
     }
-#pragma unroll
-    for (int j = 0; j < NLD; ++j) {
-        const int k = tid + j * NTH;
-        if (k >= HN) continue;
-        const int lz = k / HX, lx = k - lz * HX;
-        const int iz = tz0 - M + lz, ix = tx0 - M + lx;
-        const bool ing = (unsigned)iz < (unsigned)G.nz && (unsigned)ix < (unsigned)G.nx;
-        const bool zs = FS && ing && fs_zrow(G, iz), xs = FS && ing && fs_xcol(G, ix);
-        const float bsxx = xs ? 0.f : rs[j][0], bszz = zs ? 0.f : rs[j][1];
-        const float bsxz = FS && ing && fs_zero_shear(G, ix, iz) ? 0.f : rs[j][2];
-        const float lam = rs[j][3], mu = rs[j][4];
-        float q0, q1;
-        if (zs || xs) {
-            // transposes of the corrected surface updates (a corner: none)
-            const float cs = zs && xs ? 0.f : G.dt * (4.f * mu * (lam + mu) / (lam + 2.f * mu));
-            q0 = zs ? cs * bsxx : 0.f;
-            q1 = xs ? cs * bszz : 0.f;
-        } else {
-            q0 = G.dt * ((lam + 2.f * mu) * bsxx + lam * bszz);
-            q1 = G.dt * ((lam + 2.f * mu) * bszz + lam * bsxx);
-        }
-        float q2 = G.dt * mu * bsxz;
-        float q3 = G.dt * mu * bsxz;
-        if ((unsigned)iz < (unsigned)G.nz && (unsigned)ix < (unsigned)G.nx && in_pml(G, ix, iz)) {
-            const bool own = owns(lz, lx);
-            const int xs = xslab(G, ix), zs = zslab(G, iz);
-            if (xs >= 0) {
-                const long long xi = ((long long)b * G.nz + iz) * G.WX + xs;
-                const float t0 = mo_vxx[xi] + q0, t3 = mo_vzx[xi] + q3;
-                if (own) {
-                    mn_vxx[xi] = G.ax[ix] * t0;
-                    mn_vzx[xi] = G.axh[ix] * t3;
-                }
-                q0 = q0 + G.bx[ix] * t0;
-                q3 = q3 + G.bxh[ix] * t3;
-            }
-            if (zs >= 0) {
-                const long long zi = ((long long)b * G.WZ + zs) * G.P + ix;
-                const float t1 = mo_vzz[zi] + q1, t2 = mo_vxz[zi] + q2;
-                if (own) {
-                    mn_vzz[zi] = G.az[iz] * t1;
-                    mn_vxz[zi] = G.azh[iz] * t2;
-                }
-                q1 = q1 + G.bz[iz] * t1;
-                q2 = q2 + G.bzh[iz] * t2;
-            }
-        }
-        tq[0][k] = q0; tq[1][k] = q1; tq[2][k] = q2; tq[3][k] = q3;
-    }
-    __syncthreads();
-    const int lx = threadIdx.x, ix = tx0 + lx;
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        const int lz = threadIdx.y + 8 * r, iz = tz0 + lz;
-        if (!in_core(G, ix, iz)) continue;
-        const int c = (lz + M) * HX + lx + M;
-        const long long i = so + (long long)iz * G.P + ix;
-        const FsAx az = fs_zax(G), ax = fs_xax(G);
-        A.a[VX][i] += adj_fs<FS, 1, false>(ax, tq[0], c, ix, G.nx, true, true, G.idx) +
-                      adj_fs<FS, HX, true>(az, tq[2], c, iz, G.nz, false, false, G.idz);
-        A.a[VZ][i] += adj_fs<FS, 1, true>(ax, tq[3], c, ix, G.nx, false, false, G.idx) +
-                      adj_fs<FS, HX, false>(az, tq[1], c, iz, G.nz, true, true, G.idz);
-    }
-}
-
-// Velocity-adjoint apply (reference kernels.cuh:989-1019) with p = (pxx,
-// pzz, pxz, pzx) of the velocity-adjoint prepare (kernels.cuh:873-958) built
-// in shared memory, then the reverse velocity half of the forward
-// reconstruction: carrier capture of v(it) on the box, the NOPML velocity
-// step (kernels.cuh:365-401) and the velocity strip restore of step it - 1.
-template <bool FS>
-__global__ void __launch_bounds__(NTH, 4) rev_vadj(RevArgs A)
-{
-    extern __shared__ float sm[];
-    float* tp[4] = {sm, sm + HN, sm + 2 * HN, sm + 3 * HN};
-    float *tsxx = sm + 4 * HN, *tszz = sm + 5 * HN, *tsxz = sm + 6 * HN;
-    const Geo& G = A.G;
-    const int b = blockIdx.y;
-    int tz0, tx0;
-    tile_origin(G, blockIdx.x, tz0, tx0);
-    const long long so = (long long)b * G.S;
-    const float* __restrict__ bv_ = A.m.bv + (long long)b * G.ms;
-    const int tid = threadIdx.x + threadIdx.y * TX;
-    const float* __restrict__ mo_sxxx = A.mo.x[XM_SXXX];
-    const float* __restrict__ mo_sxzx = A.mo.x[XM_SXZX];
-    const float* __restrict__ mo_sxzz = A.mo.z[ZM_SXZZ];
-    const float* __restrict__ mo_szzz = A.mo.z[ZM_SZZZ];
-    float* __restrict__ mn_sxxx = A.mn.x[XM_SXXX];
-    float* __restrict__ mn_sxzx = A.mn.x[XM_SXZX];
-    float* __restrict__ mn_sxzz = A.mn.z[ZM_SXZZ];
-    float* __restrict__ mn_szzz = A.mn.z[ZM_SZZZ];
-    float rv[NLD][3];
-#pragma unroll
-    for (int j = 0; j < NLD; ++j) {
-        const int k = tid + j * NTH;
-        const int lz = k / HX, lx = k - lz * HX;
-        const int iz = tz0 - M + lz, ix = tx0 - M + lx;
-        const bool ok = k < HN && (unsigned)iz < (unsigned)G.nz && (unsigned)ix < (unsigned)G.nx;
-        const long long i = (long long)iz * G.P + ix;
-        rv[j][0] = ok ? A.a[VX][so + i] : 0.f;
-        rv[j][1] = ok ? A.a[VZ][so + i] : 0.f;
-        rv[j][2] = ok ? bv_[i] : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < NLD; ++j) {
-        const int k = tid + j * NTH;
-        if (k >= HN) continue;
-        const int lz = k / HX, lx = k - lz * HX;
-        const int iz = tz0 - M + lz, ix = tx0 - M + lx;
-        const float avx = rv[j][0], avz = rv[j][1], k_ = rv[j][2];
-        float p0 = k_ * avx;      // pxx
-        float p2 = k_ * avx;      // pxz
-        float p3 = k_ * avz;      // pzx
-        float p1 = k_ * avz;      // pzz
-        if ((unsigned)iz < (unsigned)G.nz && (unsigned)ix < (unsigned)G.nx && in_pml(G, ix, iz)) {
-            const bool own = owns(lz, lx);
-            const int xs = xslab(G, ix), zs = zslab(G, iz);
-            if (xs >= 0) {
-                const long long xi = ((long long)b * G.nz + iz) * G.WX + xs;
-                const float t0 = mo_sxxx[xi] + p0, t3 = mo_sxzx[xi] + p3;
-                if (own) {
-                    mn_sxxx[xi] = G.axh[ix] * t0;
-                    mn_sxzx[xi] = G.ax[ix] * t3;
-                }
-                p0 = p0 + G.bxh[ix] * t0;
-                p3 = p3 + G.bx[ix] * t3;
-            }
-            if (zs >= 0) {
-                const long long zi = ((long long)b * G.WZ + zs) * G.P + ix;
-                const float t2 = mo_sxzz[zi] + p2, t1 = mo_szzz[zi] + p1;
-                if (own) {
-                    mn_sxzz[zi] = G.az[iz] * t2;
-                    mn_szzz[zi] = G.azh[iz] * t1;
-                }
-                p2 = p2 + G.bz[iz] * t2;
-                p1 = p1 + G.bzh[iz] * t1;
-            }
-        }
-        tp[0][k] = p0; tp[1][k] = p1; tp[2][k] = p2; tp[3][k] = p3;
-    }
-    {
-        float* const t[3] = {tsxx, tszz, tsxz};
-        const float* const g[3] = {A.f[SXX] + so, A.f[SZZ] + so, A.f[SXZ] + so};
-        load_tiles<3>(t, g, G, tz0, tx0);
-    }
-    __syncthreads();
-    const int lx = threadIdx.x, ix = tx0 + lx;
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        const int lz = threadIdx.y + 8 * r, iz = tz0 + lz;
-        if (!in_core(G, ix, iz)) continue;
-        const int c = (lz + M) * HX + lx + M;
-        const long long i = (long long)iz * G.P + ix;
-        // the stresses a surface zeroes had their adjoint zeroed by this
-        // step's stress half
-        const FsAx az = fs_zax(G), ax = fs_xax(G);
-        const float sxx0 = FS && fs_xcol(G, ix) ? 0.f : A.a[SXX][so + i];
-        const float szz0 = FS && fs_zrow(G, iz) ? 0.f : A.a[SZZ][so + i];
-        const float sxz0 = FS && fs_zero_shear(G, ix, iz) ? 0.f : A.a[SXZ][so + i];
-        A.a[SXX][so + i] = sxx0 + adj_fs<FS, 1, true>(ax, tp[0], c, ix, G.nx, true, false, G.idx);
-        A.a[SZZ][so + i] = szz0 + adj_fs<FS, HX, true>(az, tp[1], c, iz, G.nz, true, false, G.idz);
-        A.a[SXZ][so + i] = sxz0 + (adj_fs<FS, HX, false>(az, tp[2], c, iz, G.nz, true, true, G.idz) +
-                                   adj_fs<FS, 1, false>(ax, tp[3], c, ix, G.nx, true, true, G.idx));
-        if (!in_box(G, ix, iz)) continue;
-        const float vx = A.f[VX][so + i], vz = A.f[VZ][so + i];
-        A.cvx[so + i] = vx;
-        A.cvz[so + i] = vz;
-        if (in_recon(G, ix, iz)) {
-            const float k_ = bv_[i];
-            A.f[VX][so + i] = vx - k_ * (d_fs<FS, 1, true>(ax, tsxx, c, ix, true, false, G.idx) +
-                                         d_fs<FS, HX, false>(az, tsxz, c, iz, true, true, G.idz));
-            A.f[VZ][so + i] = vz - k_ * (d_fs<FS, 1, false>(ax, tsxz, c, ix, true, true, G.idx) +
-                                         d_fs<FS, HX, true>(az, tszz, c, iz, true, false, G.idz));
+    const int nb = evec::image_shots(E, b0, blockIdx.y);
+    float sum = 0.f;
+    for (int b = b0; b < b0 + nb; ++b) {
+        const long long i = b * G.S + c;
+        for (int f = VX; f <= VZ; ++f) {
+            const float v = strip_val(G, slot, b, f, iz, ix, si);
+            sum += R.a.f[f][i] * (v - R.f.f[f][i]);
+            R.f.f[f][i] = v;
         }
     }
-    // strips (box ring and the M cells outside it) of step it - 1
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        const int lz = threadIdx.y + 8 * r, iz = tz0 + lz;
-        if (iz >= G.nz || ix >= G.nx || in_recon(G, ix, iz)) continue;
-        const int si = strip_index(G, iz, ix);
-        if (si < 0) continue;
-        const long long i = so + (long long)iz * G.P + ix;
-        A.f[VX][i] = strip_val(G, A.strips, b, VX, iz, ix, si);
-        A.f[VZ][i] = strip_val(G, A.strips, b, VZ, iz, ix, si);
-    }
+    if (nb) R.g[2][b0 / E.group * G.S + c] += sum;
 }
 
 // One step's strips (fp32 strip set (B, 5, nstrip) in `scratch`) into the
@@ -1308,47 +811,23 @@ __global__ void __launch_bounds__(kQB) quantize_strips(const Geo G, const float*
     }
 }
 
-// Models onto the pitched grid: rho, Lame parameters (reference
-// derived_models.cu:27-37, same rounding), bv = dt * (1 / rho) (the velocity
-// kernels' dt * inv_rho, kernels.cuh:73, 389, 901), vp and vs for the imaging.
+// Models onto the pitched grid (zero past a row's end): Lame parameters
+// (reference derived_models.cu:27-37, same rounding), bv = dt * (1 / rho) (the
+// velocity kernels' dt * inv_rho, kernels.cuh:73, 389, 901).
 __global__ void prep_kernel(const float* __restrict__ vp, const float* __restrict__ vs,
                             const float* __restrict__ rho, int nm, int nz, int nx, int P, float dt,
-                            float* orho, float* olam, float* omu, float* obv, float* ovp, float* ovs)
+                            float* olam, float* omu, float* obv)
 {
-    const long long n = (long long)nm * nz * nx;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const long long b = k / ((long long)nz * nx), rem = k - b * nz * nx;
-        const int iz = (int)(rem / nx), ix = (int)(rem - (long long)iz * nx);
-        const long long o = (b * nz + iz) * P + ix;
+    const long long n = (long long)nm * nz * P;
+    for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < n; o += (long long)gridDim.x * blockDim.x) {
+        const long long row = o / P;
+        const int ix = (int)(o - row * P);
+        if (ix >= nx) { olam[o] = omu[o] = obv[o] = 0.f; continue; }
+        const long long k = row * nx + ix;
         const float v = vp[k], s = vs[k], r = rho[k];
-        orho[o] = r;
         omu[o] = __fmul_rn(__fmul_rn(r, s), s);
         olam[o] = __fmul_rn(r, __fsub_rn(__fmul_rn(v, v), __fmul_rn(__fmul_rn(2.0f, s), s)));
         obv[o] = dt * (1.f / r);
-        ovp[o] = v;
-        ovs[o] = s;
-    }
-}
-
-// Gradient output: sum of the slots in slot order on the physical box, zero
-// elsewhere, unpitched (nout, nz, nx); slot s of a per-shot model is shot s.
-__global__ void finalize_kernel(const float* __restrict__ slots, int nslot, int per_shot, Geo G, float* out)
-{
-    const int nout = per_shot ? nslot : 1;
-    const long long n = (long long)nout * G.nz * G.nx;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const long long b = k / ((long long)G.nz * G.nx), rem = k - b * G.nz * G.nx;
-        const int iz = (int)(rem / G.nx), ix = (int)(rem - (long long)iz * G.nx);
-        float v = 0.f;
-        if (in_box(G, ix, iz)) {
-            const long long o = (long long)iz * G.P + ix;
-            if (per_shot) {
-                v = slots[b * G.S + o];
-            } else {
-                for (int s = 0; s < nslot; ++s) v += slots[s * G.S + o];
-            }
-        }
-        out[k] = v;
     }
 }
 
@@ -1356,9 +835,9 @@ __global__ void finalize_kernel(const float* __restrict__ slots, int nslot, int 
 struct Plan {
     Geo G;
     int nm;          // model copies
-    int gshots;      // shots per rev_str CTA
+    int gshots;      // shots per thread of the reverse's imaging
+    evec::Geo E;     // the reverse kernels' view of G
     int graph_steps; // time steps per captured CUDA graph (0: stream launches)
-    int nslot;       // gradient slots
     bool host_tape;  // boundary-saving tape in pinned host memory (SWEEP_MEM_HOST_TAPE)
 };
 
@@ -1432,24 +911,36 @@ static Plan make_plan(const sweep_elastic_desc* d)
     G.ms = per_shot ? G.S : 0;
     G.wavelet = d->wavelet;
     pl.nm = per_shot ? d->B : 1;
-    // shots per CTA: the shape's recorded schedule value if any, else the
+    // shots per CTA or thread: the shape's recorded schedule value if any, else the
     // environment, else the measured default (the forward's capped to keep at
     // least two waves of CTAs)
     const sweep_b200_schedule sc = recorded_schedule(d);
-    pl.gshots = per_shot ? 1
-                         : std::min(sc.shots_rev >= 1 ? sc.shots_rev : env_int("SWEEP_B200_EL_SHOTS_PER_CTA", 4), d->B);
+    evec::Geo& E = pl.E;
+    E.B = G.B; E.nz = G.nz; E.nx = G.nx; E.nt = G.nt; E.M = M;
+    E.P = G.P; E.S = G.S; E.ms = G.ms; E.fs = G.fs;
+    E.z0 = G.z0; E.z1 = G.z1; E.x0 = G.x0; E.x1 = G.x1;
+    E.dt = G.dt; E.ihz = G.idz; E.ihx = G.idx;
+    const float wt[M + 1] = {0.f, C1, C2, C3, C4};
+    for (int k = 0; k <= M; ++k) E.c[k] = wt[k];
+    E.az = G.az; E.bz = G.bz; E.azh = G.azh; E.bzh = G.bzh;
+    E.nsrc = G.nsrc; E.nrec = G.nrec; E.nrf = G.nrf; E.nsf = d->nsrc_fields;
+    for (int k = 0; k < E.nsf; ++k) E.sf[k] = d->src_fields[k];
+    for (int k = 0; k < 5; ++k) E.rf[k] = G.rf[k];
+    E.src = d->src_loc; E.rec = d->rec_loc; E.wavelet = d->wavelet;
+    evec::layout(E, per_shot ? 1 : std::min(env_int("SWEEP_B200_EL_SHOTS_PER_CTA", 4), d->B));
+    if (!per_shot && sc.shots_rev >= 1) evec::set_group(E, sc.shots_rev);
+    pl.gshots = E.group;
     const long long ntl = (long long)G.ntx * G.ntz;
     int gf = per_shot ? 1 : std::min(env_int("SWEEP_B200_EL_SHOTS_PER_CTA_FWD", 4), d->B);
     while (gf > 1 && ntl * ((d->B + gf - 1) / gf) < 2LL * 148 * 4) --gf;
     if (!per_shot && sc.shots_fwd >= 1) gf = std::min(sc.shots_fwd, d->B);
     G.gf = gf;
     pl.graph_steps = resolve_graph_steps(sc.graph_steps);
-    pl.nslot = (d->B + pl.gshots - 1) / pl.gshots;
     return pl;
 }
 
 struct Common {
-    float *rho, *lam, *mu, *bv, *vp, *vs;
+    float *lam, *mu, *bv;
     int32_t *src_off, *rec_off;
     int2 *src_ev, *rec_ev;
     int* err;
@@ -1459,8 +950,7 @@ static void carve_common(Carve& c, const Plan& pl, Common& w)
 {
     const Geo& G = pl.G;
     const long long mc = (long long)pl.nm * G.S;
-    w.rho = c.take<float>(mc); w.lam = c.take<float>(mc); w.mu = c.take<float>(mc);
-    w.bv = c.take<float>(mc); w.vp = c.take<float>(mc); w.vs = c.take<float>(mc);
+    w.lam = c.take<float>(mc); w.mu = c.take<float>(mc); w.bv = c.take<float>(mc);
     const long long nkey = (long long)G.B * G.ntx * G.ntz + 1;
     w.src_off = c.take<int32_t>(nkey);
     w.rec_off = c.take<int32_t>(nkey);
@@ -1501,10 +991,12 @@ static void carve_fwd(Carve& c, const Plan& pl, FwdWs& w)
 struct RevWs {
     Common cm;
     float* f[5];
-    float *cvx, *cvz;
+    float* xprof;
     float* a[5];
-    Slabs m[2];
-    float *gvp, *gvs, *grho;
+    float* q[3];
+    float* p[2];
+    float* m[2][evec::NMEM];
+    float* g[3];
     char* zero0;
     char* zero1;
     Slabs fmem;           // checkpoint mode: forward CPML memories of the replay
@@ -1519,16 +1011,15 @@ static void carve_rev(Carve& c, const Plan& pl, RevWs& w)
     for (int k = 0; k < 5; ++k) w.f[k] = c.take<float>((long long)G.B * G.S);
     c.take<char>(0);
     w.zero0 = c.base ? c.base + c.off : nullptr;
-    w.cvx = c.take<float>((long long)G.B * G.S);
-    w.cvz = c.take<float>((long long)G.B * G.S);
-    for (int k = 0; k < 5; ++k) w.a[k] = c.take<float>((long long)G.B * G.S);
-    carve_slabs(c, G, w.m[0]);
-    carve_slabs(c, G, w.m[1]);
-    w.gvp = c.take<float>((long long)pl.nslot * G.S);
-    w.gvs = c.take<float>((long long)pl.nslot * G.S);
-    w.grho = c.take<float>((long long)pl.nslot * G.S);
+    for (float*& p : w.a) p = c.take<float>((long long)G.B * G.S);
+    for (float*& p : w.q) p = c.take<float>((long long)G.B * G.S);
+    for (auto& m : w.m)
+        for (int k = 0; k < evec::NMEM; ++k) m[k] = c.take<float>(evec::mem_floats(pl.E, k));
+    for (float*& p : w.g) p = c.take<float>((long long)pl.E.nslot * G.S);
     c.take<char>(0);
     w.zero1 = c.base ? c.base + c.off : nullptr;
+    for (float*& p : w.p) p = c.take<float>((long long)G.B * G.S);
+    w.xprof = c.take<float>(4LL * evec::xprof_len(pl.E));
     if (pl.host_tape) w.ring = c.take<char>((long long)HostRing::R * G.st.step);
 }
 
@@ -1677,7 +1168,7 @@ static void setup_common(const sweep_elastic_desc* d, Plan& pl, const Common& w,
     Geo& G = pl.G;
     SWEEP_REQUIRE(d->vp && d->vs && d->rho, "elastic2d: null model pointer");
     prep_kernel<<<592, 256, 0, st>>>(d->vp, d->vs, d->rho, pl.nm, d->nz, d->nx, G.P, d->dt,
-                                     w.rho, w.lam, w.mu, w.bv, w.vp, w.vs);
+                                     w.lam, w.mu, w.bv);
     SWEEP_LAUNCH_CHECK();
     std::vector<int32_t> ls((size_t)d->B * d->nsrc * 2 + 1), lr((size_t)d->B * d->nrec * 2 + 1);
     const size_t ns = (size_t)d->B * d->nsrc * 2, nr = (size_t)d->B * d->nrec * 2;
@@ -1728,7 +1219,7 @@ static FwdMaps fwd_maps(float* const* f, const Geo& G)
 
 static Models models_of(const Common& w)
 {
-    return Models{w.rho, w.lam, w.mu, w.bv, w.vp, w.vs};
+    return Models{w.lam, w.mu, w.bv};
 }
 
 constexpr size_t SM_FWD_VEL = sizeof(VelSmem);
@@ -1744,9 +1235,6 @@ static void set_attrs()
     SWEEP_CUDA(cudaFuncSetAttribute(fwd_str<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_FWD_STR));
     done = true;
 }
-constexpr size_t SM_REV_STR = 2 * HN * sizeof(float);
-constexpr size_t SM_REV_SADJ = 4 * HN * sizeof(float);
-constexpr size_t SM_REV_VADJ = 7 * HN * sizeof(float);
 
 static void check_mode(int mem_mode, int ckpt_every)
 {
@@ -1930,16 +1418,19 @@ static void backward_with(const sweep_elastic_desc* d, int mem_mode, int ckpt_ev
     setup_common(d, pl, w.cm, st);
     const Geo& G = pl.G;
     const long long n = (long long)G.B * G.S;
-    RevArgs A{};
-    A.G = G;
-    A.m = models_of(w.cm);
-    for (int k = 0; k < 5; ++k) { A.f[k] = w.f[k]; A.a[k] = w.a[k]; }
-    A.cvx = w.cvx; A.cvz = w.cvz;
-    A.adj = adj;
-    A.gvp = w.gvp; A.gvs = w.gvs; A.grho = w.grho;
-    A.G_shots = pl.gshots;
-    const dim3 block(TX, 8);
-    const dim3 grid_s(G.ntx * G.ntz, pl.nslot), grid_b(G.ntx * G.ntz, G.B);
+    evec::Geo& E = pl.E;
+    E.lam = w.cm.lam; E.mu = w.cm.mu; E.kv = w.cm.bv;
+    const int plen = evec::xprof_len(E);
+    evec::prep_profiles<<<8, 256, 0, st>>>(G.ax, G.bx, G.axh, G.bxh, G.nx, plen, w.xprof);
+    SWEEP_LAUNCH_CHECK();
+    E.ax = w.xprof + evec::kGuard; E.bx = E.ax + plen; E.axh = E.bx + plen; E.bxh = E.axh + plen;
+    evec::Rev R{};
+    for (int k = 0; k < 5; ++k) { R.f.f[k] = w.f[k]; R.a.f[k] = w.a[k]; }
+    for (int k = 0; k < 3; ++k) { R.q[k] = w.q[k]; R.g[k] = w.g[k]; }
+    for (int k = 0; k < 2; ++k) R.p[k] = w.p[k];
+    R.adj = adj;
+    const long long ne = (long long)G.B * G.nsrc + (long long)G.B * G.nrec;
+    const unsigned rblocks = (unsigned)(((long long)G.B * G.nstrip + 255) / 256);
     int cur = stepped && !first ? seg->idx[0] : 0;
     // Reverse steps it1 - 1 .. max(it0, 1) (the staggered reverse has no
     // it = 0 step) on the reconstruction state after step it1 - 1;
@@ -1949,23 +1440,18 @@ static void backward_with(const sweep_elastic_desc* d, int mem_mode, int ckpt_ev
     auto reverse = [&](int it0, int it1, auto strips_of) {
         StepGraphs gs(st, host ? 0 : pl.graph_steps);
         for (int it = it1 - 1; it >= std::max(it0, 1); --it) {
-            A.it = it;
-            A.strips = strips_of(it - 1);
-            A.mo = w.m[cur];
-            A.mn = w.m[cur ^ 1];
+            R.it = it;
+            const void* strips = strips_of(it - 1);
+            for (int k = 0; k < evec::NMEM; ++k) { R.ai.m[k] = w.m[cur][k]; R.ao.m[k] = w.m[cur ^ 1][k]; }
             if (host) hr.before_read(it - 1);
             const cudaStream_t ls = gs.stream();
-            if (G.nvf)
-                vsrc_reverse<<<G.B, 128, 0, ls>>>(G, A.a[VX], A.a[VZ], A.f[VX], A.f[VZ], A.grho, A.m.rho, A.G_shots, it);
-            if (G.fs) {
-                rev_str<true><<<grid_s, block, SM_REV_STR, ls>>>(A);
-                rev_sadj<true><<<grid_b, block, SM_REV_SADJ, ls>>>(A);
-                rev_vadj<true><<<grid_b, block, SM_REV_VADJ, ls>>>(A);
-            } else {
-                rev_str<false><<<grid_s, block, SM_REV_STR, ls>>>(A);
-                rev_sadj<false><<<grid_b, block, SM_REV_SADJ, ls>>>(A);
-                rev_vadj<false><<<grid_b, block, SM_REV_VADJ, ls>>>(A);
-            }
+            if (ne > 0) evec::events<<<(unsigned)((ne + 127) / 128), 128, 0, ls>>>(E, R);
+            if (G.fs) evec::launch_a<M, true>(E, R, ls);
+            else evec::launch_a<M, false>(E, R, ls);
+            restore<<<dim3(rblocks, 3), 256, 0, ls>>>(G, E, R, strips, SXX);
+            if (G.fs) evec::launch_b<M, true>(E, R, ls);
+            else evec::launch_b<M, false>(E, R, ls);
+            restore<<<dim3(rblocks, 2), 256, 0, ls>>>(G, E, R, strips, VX);
             if (host) {
                 hr.after_read(it - 1);
                 if (it - 1 - HostRing::R >= std::max(it0 - 1, 0)) hr.fetch(it - 1 - HostRing::R, true);
@@ -1986,7 +1472,7 @@ static void backward_with(const sweep_elastic_desc* d, int mem_mode, int ckpt_ev
         const long long cs = (long long)G.B * 5 * G.nstrip;
         FwdArgs F{};
         F.G = G;
-        F.m = A.m;
+        F.m = models_of(w.cm);
         for (int f = 0; f < 5; ++f) F.f[f] = w.f[f];
         F.mem = w.fmem;
         F.record = nullptr;
@@ -2069,7 +1555,7 @@ static void backward_with(const sweep_elastic_desc* d, int mem_mode, int ckpt_ev
         const long long cs = (long long)G.B * 5 * G.nstrip;
         FwdArgs F{};
         F.G = G;
-        F.m = A.m;
+        F.m = models_of(w.cm);
         for (int f = 0; f < 5; ++f) F.f[f] = w.f[f];     // replay straight into the reconstruction fields
         F.mem = w.fmem;
         F.record = nullptr;
@@ -2095,10 +1581,8 @@ static void backward_with(const sweep_elastic_desc* d, int mem_mode, int ckpt_ev
         }
     }
     if (stepped) seg->idx[0] = cur;
-    const int per_shot = G.ms != 0;
-    finalize_kernel<<<592, 256, 0, st>>>(w.gvp, pl.nslot, per_shot, G, grad_vp);
-    finalize_kernel<<<592, 256, 0, st>>>(w.gvs, pl.nslot, per_shot, G, grad_vs);
-    finalize_kernel<<<592, 256, 0, st>>>(w.grho, pl.nslot, per_shot, G, grad_rho);
+    const evec::Out out{d->vp, d->vs, d->rho, {grad_vp, grad_vs, grad_rho}};
+    evec::finalize<<<592, 256, 0, st>>>(E, R, out);
     SWEEP_LAUNCH_CHECK();
     check_err(w.cm, st, "backward");
 }

@@ -114,3 +114,11 @@ def test_acoustic2d_small_and_tiled(shape, B):
     which order 8 leaves its small-grid kernels (6 tiles per shot)."""
     from sweep_b200 import Acoustic
     _check(Acoustic, O.Acoustic2D, ("vp",), shape, B, 8)
+
+
+@pytest.mark.parametrize("shape,B,free", [
+    ((11, 13), 1, False), ((33, 32), 3, True), ((41, 58), 6, False), ((64, 129), 5, True), ((130, 350), 21, False)])
+def test_elastic2d_order8(shape, B, free):
+    """The last one sums the images of several shots per thread."""
+    from sweep_b200 import Elastic
+    _check(Elastic, O.Elastic2D, ("vp", "vs", "rho"), shape, B, 8, free)
