@@ -372,6 +372,18 @@ SWEEP_B200_API int sweep_b200_conv3x3_wgrad(const void* x, const void* dy, float
                                             int32_t w, int32_t c, int32_t co, void* stream, char* err,
                                             int32_t err_cap);
 
+/* The whole backward from the output gradient gout (n, h, w, co) float32, taken
+ * in bf16 for the products: dx (n, h, w, c) bf16 (rounded to nearest even from
+ * the FP32 sums) from the weights wb (co, 3, 3, c) bf16, dw (co, 3, 3, c)
+ * float32 from x (n, h, w, c) bf16, db (co) float32 the column sums of gout; a
+ * null dx, dw or db is left out.  scratch holds backward_bytes bytes, 256-byte
+ * aligned. */
+SWEEP_B200_API int64_t sweep_b200_conv3x3_backward_bytes(int32_t n, int32_t h, int32_t w, int32_t c, int32_t co);
+SWEEP_B200_API int sweep_b200_conv3x3_backward(const float* gout, const void* x, const void* wb, void* dx, float* dw,
+                                               float* db, void* scratch, int64_t scratch_bytes, int32_t n, int32_t h,
+                                               int32_t w, int32_t c, int32_t co, void* stream, char* err,
+                                               int32_t err_cap);
+
 /* Waits for `stream` and reports (then clears) a timed-out tensor-core wait
  * in any convolution launched since the last call: the convolution entries
  * return at launch, so their device-side failures surface here. */

@@ -42,6 +42,8 @@ SYMBOLS = (
     "sweep_b200_vti3d_forward",
     "sweep_b200_vti3d_backward",
     "sweep_b200_conv3x3_gemm",
+    "sweep_b200_conv3x3_backward_bytes",
+    "sweep_b200_conv3x3_backward",
     "sweep_b200_conv3x3_wgrad",
     "sweep_b200_conv3x3_status",
     "sweep_b200_schedule_set",
@@ -215,6 +217,10 @@ def load():
                                               ctypes.c_char_p, c_i32]
     lib.sweep_b200_conv3x3_gemm.argtypes = [c_p, c_p, c_p, c_p, c_i32, c_i32, c_i32, c_i32, c_i32, c_i32, c_p,
                                             ctypes.c_char_p, c_i32]
+    lib.sweep_b200_conv3x3_backward_bytes.argtypes = [c_i32, c_i32, c_i32, c_i32, c_i32]
+    lib.sweep_b200_conv3x3_backward_bytes.restype = c_i64
+    lib.sweep_b200_conv3x3_backward.argtypes = [c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_i32, c_i32, c_i32, c_i32,
+                                                c_i32, c_p, ctypes.c_char_p, c_i32]
     lib.sweep_b200_conv3x3_wgrad.argtypes = [c_p, c_p, c_p, c_i32, c_i32, c_i32, c_i32, c_i32, c_p,
                                              ctypes.c_char_p, c_i32]
     lib.sweep_b200_conv3x3_status.argtypes = [c_p, ctypes.c_char_p, c_i32]

@@ -51,20 +51,20 @@ class _Conv3x3(torch.autograd.Function):
         x, wb = ctx.saved_tensors
         n, h, wd, c = x.shape
         co = wb.shape[0]
-        g = gout.to(torch.bfloat16).contiguous()
-        gx = gw = gb = None
-        if ctx.needs_input_grad[0]:
-            wt = wb.permute(3, 1, 2, 0).contiguous()            # (C, 3, 3, Co): per-tap transpose
-            gx32 = torch.empty((n, h, wd, c), dtype=torch.float32, device=x.device)
-            _lib.call("sweep_b200_conv3x3_gemm", g.data_ptr(), wt.data_ptr(), None, gx32.data_ptr(),
-                      n, h, wd, co, c, -1, _stream(x))
-            gx = gx32.to(torch.bfloat16)
+        gout = gout.contiguous()
+        if gout.data_ptr() % 16:
+            gout = gout.clone()
+        gx = torch.empty_like(x) if ctx.needs_input_grad[0] else None
+        gw = gb = None
         if ctx.needs_input_grad[1]:
             gw = torch.empty((co, 3, 3, c), dtype=torch.float32, device=x.device)
-            _lib.call("sweep_b200_conv3x3_wgrad", x.data_ptr(), g.data_ptr(), gw.data_ptr(), n, h, wd, c, co,
-                      _stream(x))
         if ctx.needs_input_grad[2]:
-            gb = gout.sum(dim=(0, 1, 2))
+            gb = torch.empty(co, dtype=torch.float32, device=x.device)
+        size = _lib.load().sweep_b200_conv3x3_backward_bytes(n, h, wd, c, co)
+        scratch = torch.empty(size, dtype=torch.uint8, device=x.device)
+        _lib.call("sweep_b200_conv3x3_backward", gout.data_ptr(), x.data_ptr(), wb.data_ptr(),
+                  *(None if t is None else t.data_ptr() for t in (gx, gw, gb)), scratch.data_ptr(), size,
+                  n, h, wd, c, co, _stream(x))
         return gx, gw, gb
 
 

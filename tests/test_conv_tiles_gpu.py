@@ -1,0 +1,38 @@
+"""The 3x3 convolution and its three gradients where the tiles of 8 x 16
+pixels, the steps of 64 channels and the 64 outputs of a CTA end: against
+float64 on the same bf16 operands.
+
+Tolerances: FP32 sums of at most 9 * 264 (weights: 1200) products, relative to the result's
+norm well under 1e-5 for random operands; a bf16 result (8 bits) rounds by at
+most 2**-8."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from tests._util import rel
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+@pytest.mark.parametrize("n,h,w,c,co", [
+    (1, 1, 1, 8, 8), (2, 16, 8, 64, 64), (1, 17, 9, 72, 80), (3, 5, 50, 136, 72), (2, 33, 24, 24, 8),
+    (1, 16, 64, 128, 200), (5, 20, 12, 264, 16), (2, 9, 23, 56, 136)])
+def test_conv3x3_matches_float64(n, h, w, c, co):
+    from sweep_b200 import unet
+    gen = torch.Generator().manual_seed(n + 3 * h + 7 * w + c + co)
+    x = torch.randn((n, h, w, c), generator=gen).to(torch.bfloat16)
+    wt = (torch.randn((co, 3, 3, c), generator=gen) * 0.1).to(torch.bfloat16).float()
+    b = torch.randn(co, generator=gen)
+    g = torch.randn((n, h, w, co), generator=gen).to(torch.bfloat16).float()
+    leaves = [t.to(DEV).requires_grad_(True) for t in (x, wt, b)]
+    y = unet.conv3x3(*leaves)
+    y.backward(g.to(DEV))
+    unet.check()
+    ref = [t.double().requires_grad_(True) for t in (x, wt, b)]
+    yr = F.conv2d(ref[0].permute(0, 3, 1, 2), ref[1].permute(0, 3, 1, 2), ref[2], padding=1).permute(0, 2, 3, 1)
+    yr.backward(g.double())
+    errs = [rel(y.detach().cpu(), yr.detach())] + [rel(a.grad.float().cpu(), r.grad) for a, r in zip(leaves, ref)]
+    print(f"{(n, h, w, c, co)}: y {errs[0]:.1e}, dx {errs[1]:.1e}, dw {errs[2]:.1e}, db {errs[3]:.1e}")
+    assert errs[0] < 1e-5 and errs[2] < 1e-5 and errs[3] < 1e-5
+    assert errs[1] < 2.0 ** -8 + 1e-5
