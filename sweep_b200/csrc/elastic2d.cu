@@ -927,8 +927,9 @@ static Plan make_plan(const sweep_elastic_desc* d)
     for (int k = 0; k < E.nsf; ++k) E.sf[k] = d->src_fields[k];
     for (int k = 0; k < 5; ++k) E.rf[k] = G.rf[k];
     E.src = d->src_loc; E.rec = d->rec_loc; E.wavelet = d->wavelet;
-    evec::layout(E, per_shot ? 1 : std::min(env_int("SWEEP_B200_EL_SHOTS_PER_CTA", 4), d->B));
-    if (!per_shot && sc.shots_rev >= 1) evec::set_group(E, sc.shots_rev);
+    evec::layout(E, per_shot ? 1 : 4);
+    const int shots = sc.shots_rev >= 1 ? sc.shots_rev : env_int("SWEEP_B200_EL_SHOTS_PER_CTA", 0);
+    if (!per_shot && shots >= 1) evec::set_group(E, shots);
     pl.gshots = E.group;
     const long long ntl = (long long)G.ntx * G.ntz;
     int gf = per_shot ? 1 : std::min(env_int("SWEEP_B200_EL_SHOTS_PER_CTA_FWD", 4), d->B);
