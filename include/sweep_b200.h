@@ -403,7 +403,7 @@ typedef struct sweep_b200_schedule {
     int32_t shots_fwd;    /* shots per CTA of the forward step kernels (2-D acoustic
                            * fwd_kernel, elastic fwd_vel / fwd_str); 0 = built-in */
     int32_t shots_rev;    /* shots per CTA of the reverse kernels that sum the image
-                           * (2-D acoustic rev_kernel, elastic rev_str); 0 = built-in */
+                           * (2-D acoustic rev_kernel, elastic imaging); 0 = built-in */
     int32_t z_chunks;     /* 3-D acoustic: z chunks each column block is cut into
                            * (grid depth per shot); 0 = built-in */
     int32_t graph_steps;  /* time steps per captured CUDA graph in the step loops

@@ -19,9 +19,9 @@
 // another start address, so a tile is loaded once for all nine taps (the
 // gather of a tile per tap and K step took 9x the loads and shared-memory
 // writes and bound the kernels: 148 us a pass on 16 x 64 x 192 pixels, 64 -> 64
-// channels, 208 us the weight gradient; 49 and 40 us the forward and the data
-// pass and 49 us the weight gradient now; without the loads 41, 32 and 32 us,
-// without the MMAs 43, 31 and 38 us).
+// channels, 208 us the weight gradient; 46 and 38 us the forward and the data
+// pass and 44 us the weight gradient now.  No unit is near its limit: the
+// copies, MMAs and epilogue of one CTA an SM overlap in part).
 //   conv_pass  (forward, data): A = tile, K-major (M = 128 pixels, K = channels),
 //              B = the weights of the CTA's 64 outputs, all nine taps resident;
 //              a CTA walks its tiles, the loads of the next one and the
@@ -45,7 +45,12 @@
 namespace sweep {
 namespace conv {
 
-constexpr int BM = 128, BN = 64, NT = 256;
+constexpr int BM = 128, BN = 64;
+// threads of the tensor-core kernels: the copies and the epilogue are bound by
+// their instructions, at one CTA per SM (256 threads: 49, 40 and 49 us)
+constexpr int NT = 512;
+constexpr int COLS = BN / (NT / 128);        // accumulator columns of a thread
+constexpr int NTC = 256;                     // threads of the cotangent's pass
 
 // ------------------------------------------------------------ tcgen05 path
 namespace umma {
@@ -165,16 +170,16 @@ struct Tile {
 };
 
 // A thread's share of a tile with its halo: one group of 8 channels of every
-// 32nd pixel.
+// ROWS-th pixel.
 struct Halo {
-    static constexpr int N = (umma::PN + 31) / 32;
+    static constexpr int ROWS = NT / 8, N = (umma::PN + ROWS - 1) / ROWS;
     int kc, at[N];                           // row << 8 | column, or -1
     __device__ __forceinline__ Halo()
     {
         kc = threadIdx.x & 7;
 #pragma unroll
         for (int u = 0; u < N; ++u) {
-            const int q = (threadIdx.x >> 3) + 32 * u, r = q / umma::PW;
+            const int q = (threadIdx.x >> 3) + ROWS * u, r = q / umma::PW;
             at[u] = q < umma::PN ? r << 8 | (q - r * umma::PW) : -1;
         }
     }
@@ -190,7 +195,7 @@ struct Halo {
             if (at[u] < 0) continue;
             const int r = at[u] >> 8, w = at[u] & 255;
             const bool in = (unsigned)(hb + r) < (unsigned)S.H && (unsigned)(wb + w) < (unsigned)S.W && c < S.C;
-            umma::copy16(d + u * 512, in ? base + ((long long)r * S.W + w) * S.C : act, in);
+            umma::copy16(d + u * ROWS * 16, in ? base + ((long long)r * S.W + w) * S.C : act, in);
         }
     }
 };
@@ -250,22 +255,26 @@ __global__ void __launch_bounds__(NT) conv_pass(const __nv_bfloat16* __restrict_
                          in ? Bt + ((long long)(n0 + n) * 9 + t) * S.C + c : Bt, in);
         }
     };
+    // this thread's columns of the outputs and their bias
+    const int col = COLS * (warp >> 2), n1 = n0 + col;
+    float bv[COLS];
+#pragma unroll
+    for (int e = 0; e < COLS; ++e) bv[e] = bias && n1 + e < S.Nout ? __ldg(bias + n1 + e) : 0.f;
     auto epilogue = [&](int i) {
         const Tile T(S, t0 + i);
         const int m = 32 * (warp & 3) + lane, h = T.h0 + (m >> 3), w = T.w0 + (m & 7);
-        const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (nch == 1 ? (i & 1) : i) * BN + 32 * (warp >> 2);
-        float v[4][8];
+        const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (nch == 1 ? (i & 1) : i) * BN + col;
+        float v[COLS / 8][8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) umma::ld8(ta + 8 * j, v[j]);
+        for (int j = 0; j < COLS / 8; ++j) umma::ld8(ta + 8 * j, v[j]);
         umma::wait_ld();
         if (h >= S.H || w >= S.W) return;
-        const int n = n0 + 32 * (warp >> 2);
-        Out* o = out + (((long long)T.img * S.H + h) * S.W + w) * S.Nout + n;
+        Out* o = out + (((long long)T.img * S.H + h) * S.W + w) * S.Nout + n1;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (n + 8 * j >= S.Nout) break;
+        for (int j = 0; j < COLS / 8; ++j) {
+            if (n1 + 8 * j >= S.Nout) break;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[j][e] += bias ? __ldg(bias + n + 8 * j + e) : 0.f;
+            for (int e = 0; e < 8; ++e) v[j][e] += bv[8 * j + e];
             put8(o + 8 * j, v[j]);
         }
     };
@@ -364,8 +373,8 @@ __global__ void __launch_bounds__(NT) conv_wgrad(const __nv_bfloat16* __restrict
         halo.load(S, x, T, c0, 1, a + 8 * umma::PS);
         const int n = n0 + 8 * halo.kc;
 #pragma unroll
-        for (int u = 0; u < BM / 32; ++u) {
-            const int q = (tid >> 3) + 32 * u, h = T.h0 + (q >> 3), w = T.w0 + (q & 7);
+        for (int u = 0; u < BM / Halo::ROWS; ++u) {
+            const int q = (tid >> 3) + Halo::ROWS * u, h = T.h0 + (q >> 3), w = T.w0 + (q & 7);
             const bool in = h < S.H && w < S.W && n < S.Nout;
             umma::copy16(d + halo.kc * umma::DS + q * 16,
                          in ? dy + (((long long)T.img * S.H + h) * S.W + w) * S.Nout + n : dy, in);
@@ -403,18 +412,18 @@ __global__ void __launch_bounds__(NT) conv_wgrad(const __nv_bfloat16* __restrict
     }
     ok = ok && tma::mbar_wait(&hd.done[prev], pphase, err, umma::ERR_MMA_WAIT);
     umma::fence_after();
-    const int m = 32 * (warp & 3) + lane, c = c0 + (m & 63), n = n0 + 32 * (warp >> 2);
+    const int m = 32 * (warp & 3) + lane, c = c0 + (m & 63), col = COLS * (warp >> 2), n = n0 + col;
 #pragma unroll 1
     for (int j = 0; j < 6; ++j) {
         const int tap = (j / 2) * 3 + (j & 1 ? 2 : m >> 6);
-        const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + j * BN + 32 * (warp >> 2);
-        float v[4][8];
+        const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + j * BN + col;
+        float v[COLS / 8][8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) umma::ld8(ta + 8 * i, v[i]);
+        for (int i = 0; i < COLS / 8; ++i) umma::ld8(ta + 8 * i, v[i]);
         umma::wait_ld();
         if (!ok || c >= S.C || ((j & 1) && m >= 64)) continue;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < COLS / 8; ++i)
 #pragma unroll
             for (int e = 0; e < 8; ++e)
                 if (n + 8 * i + e < S.Nout) atomicAdd(dw + ((long long)(n + 8 * i + e) * 9 + tap) * S.C + c, v[i][e]);
@@ -428,13 +437,13 @@ __global__ void __launch_bounds__(NT) conv_wgrad(const __nv_bfloat16* __restrict
 // HBM-bound: 75 MB in 14.5 us at 196608 x 64 (a cast and a sum took 12 + 73 us).
 // The output gradient (rows, co) in bf16 and, if part, the sums of its columns
 // over each block's rows: part (gridDim.x, co).  A thread holds 8 channels.
-__global__ void __launch_bounds__(NT) cotangent(const float* __restrict__ g, __nv_bfloat16* __restrict__ out,
+__global__ void __launch_bounds__(NTC) cotangent(const float* __restrict__ g, __nv_bfloat16* __restrict__ out,
                                                 float* __restrict__ part, long long rows, int co)
 {
     extern __shared__ float sums[];
-    const int cg = co / 8, lanes = NT / cg > 0 ? NT / cg : 1;
-    for (int c8 = threadIdx.x % cg; c8 < cg; c8 += NT) {
-        const int r0 = cg > NT ? 0 : threadIdx.x / cg;
+    const int cg = co / 8, lanes = NTC / cg > 0 ? NTC / cg : 1;
+    for (int c8 = threadIdx.x % cg; c8 < cg; c8 += NTC) {
+        const int r0 = cg > NTC ? 0 : threadIdx.x / cg;
         float acc[8] = {};
         if (r0 < lanes) {
             for (long long r = (long long)blockIdx.x * lanes + r0; r < rows; r += (long long)gridDim.x * lanes) {
@@ -450,11 +459,11 @@ __global__ void __launch_bounds__(NT) cotangent(const float* __restrict__ g, __n
 #pragma unroll
                 for (int e = 0; e < 8; ++e) s[8 * c8 + e] = acc[e];
         }
-        if (cg <= NT) break;
+        if (cg <= NTC) break;
     }
     if (!part || lanes == 1) return;
     __syncthreads();
-    for (int c = threadIdx.x; c < co; c += NT) {
+    for (int c = threadIdx.x; c < co; c += NTC) {
         float s = 0.f;
         for (int r = 0; r < lanes; ++r) s += sums[r * co + c];
         part[(long long)blockIdx.x * co + c] = s;
@@ -625,10 +634,10 @@ extern "C" int sweep_b200_conv3x3_backward(const float* gout, const void* x, con
         SWEEP_REQUIRE(k.off <= scratch_bytes, "conv3x3 backward: scratch too small (%lld < %lld bytes)",
                       (long long)scratch_bytes, (long long)k.off);
         cudaStream_t st = static_cast<cudaStream_t>(stream);
-        const int lanes = std::max(1, conv::NT / (co / 8));
+        const int lanes = std::max(1, conv::NTC / (co / 8));
         const int blocks = (int)std::min<long long>((px + lanes - 1) / lanes, conv::kParts);
         const size_t smem = lanes > 1 ? (size_t)lanes * co * 4 : 0;      // 8 KB at most
-        conv::cotangent<<<blocks, conv::NT, smem, st>>>(gout, ws.dy, db ? ws.part : nullptr, px, co);
+        conv::cotangent<<<blocks, conv::NTC, smem, st>>>(gout, ws.dy, db ? ws.part : nullptr, px, co);
         if (db) conv::bias_sum<<<(co + 31) / 32, dim3(32, 8), 0, st>>>(ws.part, blocks, co, db);
         SWEEP_LAUNCH_CHECK();
         if (dx) {
