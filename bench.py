@@ -105,10 +105,11 @@ E_NZ, E_NX, E_NT, E_DT, E_DH, E_ABCN = 400, 1200, 4000, 0.0005, 5.0, 40
 E_NSHOT, E_NREC, E_F0, E_DELAY = 16, 600, 10.0, 0.12
 E_RT = (E_NZ + 2 * E_ABCN + 2 * M, E_NX + 2 * E_ABCN + 2 * M)
 # algorithmic bytes per runtime cell-step: forward velocity 7 floats + stress
-# 8; reverse stress half 15, stress-adjoint 7, velocity-adjoint + velocity
-# reconstruction 17 (one read and one write of every field a kernel touches;
-# CPML memories and the shared, L2-resident models not counted)
-E_BYTES_FWD, E_BYTES_REV = 60, 156
+# 8; reverse transpose into the adjoint velocities 9, stress reconstruction with
+# its image 11, transpose into the adjoint stresses 11, velocity reconstruction
+# 9 (one read and one write of every field a kernel touches; CPML memories,
+# gradient slots and the shared, L2-resident models not counted)
+E_BYTES_FWD, E_BYTES_REV = 60, 160
 
 
 def elastic_survey(seed=SEED):
@@ -135,9 +136,10 @@ def elastic_survey(seed=SEED):
 # with vp, delta = epsilon / 2, rho = 310 vp^0.25; sources on (sH, sV).
 # Algorithmic bytes per runtime cell-step (one read and one write of every
 # field a kernel touches; CPML memories and the models not counted): forward
-# velocity 6 floats + stress 6; reverse stress reconstruction 6, half-step A 4
-# + 6, gradient 8 + 8 slots, half-step B 4 + 6, velocity reconstruction 6.
-V_BYTES_FWD, V_BYTES_REV = 48, 192
+# velocity 6 floats + stress 6; reverse half-step A with the stress
+# reconstruction 12, half-step B with the velocity reconstruction 12, gradient
+# slots (four, each shared by four shots) 2.
+V_BYTES_FWD, V_BYTES_REV = 48, 104
 
 
 def vti_survey(seed=SEED):
@@ -291,7 +293,7 @@ class AcousticC1Workload:
     name = "acoustic2d_c1"
     nt, nshot, rt = C1_NT, 1, C1_RT
     bytes_fwd, bytes_rev = BYTES_FWD, BYTES_REV
-    kernel = "sweep::a2d::rev_kernel (fused adjoint + reconstruction + imaging step)"
+    kernel = "sweep::a2d::rev_small (fused adjoint + reconstruction + imaging step, small grids)"
     cpu_nt = C1_NT
     traffic = None
 
@@ -319,9 +321,10 @@ class AcousticC1Workload:
         return solver, [vp_true], [vp_init], w, src, rec
 
     def launches(self, group):
-        # per gradient: the forward's prep_kernel and one fwd_kernel per step,
-        # the backward's prep_kernel, one rev_kernel per step and finalize_kernel
-        return 2 * self.nt + 3
+        # per gradient: the forward's prep_kernel, two prep_profiles and one
+        # fwd_small per step, the backward's prep_kernel, two prep_profiles, one
+        # rev_small per step and finalize_kernel
+        return 2 * self.nt + 7
 
     def cpu_run(self, nt_sample, shots=1):
         from oracle import oracle as O
@@ -337,8 +340,8 @@ class ElasticWorkload:
     name = "elastic2d"
     nt, nshot, rt = E_NT, E_NSHOT, E_RT
     bytes_fwd, bytes_rev = E_BYTES_FWD, E_BYTES_REV
-    kernel = ("sweep::el2d reverse step (rev_str + rev_sadj + rev_vadj: reconstruction, imaging, "
-              "stress- and velocity-adjoint)")
+    kernel = ("sweep::evec reverse step (rev_a + rev_b: transposes, reconstructions, imaging; events and "
+              "strip restores)")
     cpu_nt = 300
     traffic = None
 
@@ -365,7 +368,9 @@ class ElasticWorkload:
         return solver, m_true, m_init, w, src, rec
 
     def launches(self, group):
-        return 5 * self.nt + 2
+        # forward 2 per step; reverse 5 (events, rev_a, stress restore, rev_b,
+        # velocity restore); prep per pass, prep_profiles and finalize
+        return 2 * self.nt + 5 * (self.nt - 1) + 4
 
     def cpu_run(self, nt_sample, shots=1):
         from oracle import oracle as O
@@ -380,7 +385,7 @@ class ElasticWorkload:
 class VTIWorkload(ElasticWorkload):
     name = "vti2d"
     bytes_fwd, bytes_rev = V_BYTES_FWD, V_BYTES_REV
-    kernel = "sweep::vti reverse step (srev + premA + appA + grad + premB + appB + vrev + band restores)"
+    kernel = "sweep::vtik reverse step (half_a + half_b: transposes, reconstructions, gradient; events and band restores)"
     tunable = False
 
     def config(self, args):
@@ -401,7 +406,10 @@ class VTIWorkload(ElasticWorkload):
         return solver, m_true, m_init, w, src, rec
 
     def launches(self, group):
-        return 5 * self.nt + 11 * (self.nt - 1) + 6
+        # forward 4 per step (velocity, stress, source, bands with the record);
+        # reverse 5 (events, half_a, stress bands, half_b, velocity bands); prep,
+        # two prep_profiles and band_table per pass, finalize
+        return 4 * self.nt + 5 * (self.nt - 1) + 9
 
     def cpu_run(self, nt_sample, shots=1):
         from oracle import oracle as O
@@ -532,11 +540,11 @@ E3_RT = (E3_N + 2 * E3_ABCN + 2 * M,) * 3
 # algorithmic floats per runtime cell-step (one read and one write of every
 # field a kernel touches; models and CPML memories not counted): forward
 # velocity step 6 stresses read + 3 velocities read and written (12), stress
-# step 3 + 6 + 6 (15); reverse: stress reconstruction 15, stress-adjoint
-# prepare 6 + 3 + 3 + 3 read, 3 gradient slots read and written, 9 q written
-# (30), its apply 9 + 6 (15), velocity-adjoint prepare 3 + 9 (12), its apply
-# 9 + 12 (21), carriers 6, velocity reconstruction 12 (111)
-E3_BYTES_FWD, E3_BYTES_REV = 4 * 27, 4 * 111
+# step 3 + 6 + 6 (15); reverse: stress reconstruction with its image 3 + 12 + 6
+# (21), transpose into the adjoint velocities 6 q read, 6, 3 p written (15),
+# into the adjoint stresses 3 + 12 + 6 (21), velocity reconstruction 6 + 6 + 3
+# (15), three gradient slots shared by the shots of a thread 2 (74)
+E3_BYTES_FWD, E3_BYTES_REV = 4 * 27, 4 * 74
 
 
 def elastic3d_survey(seed=SEED):
@@ -575,7 +583,7 @@ class Elastic3DWorkload:
     name = "elastic3d"
     nt, nshot, rt = E3_NT, E3_NSHOT, E3_RT
     bytes_fwd, bytes_rev = E3_BYTES_FWD, E3_BYTES_REV
-    kernel = ("sweep::el3d reverse step (srev3 + sprep3 + sapp3 + vprep3 + vapp3 + cap3 + vrev3 + strip "
+    kernel = ("sweep::el3d reverse step (stress_rev + adj_vel + adj_str + vel_rev + event and strip "
               "kernels)")
     cpu_nt = 24
     traffic = None
@@ -605,11 +613,10 @@ class Elastic3DWorkload:
 
     def launches(self, group):
         # forward 5 per step (velocity, stress, source, strips, record);
-        # reverse 12 (body-force correction only with velocity sources: not
-        # here; residuals, source removal, two reconstructions, two restores,
-        # two prepares, two applies, carriers, receiver rho); prep3 and three
-        # finalize3 per pass
-        return 5 * self.nt + 12 * (self.nt - 1) + 4
+        # reverse 8 (residuals, source removal, stress reconstruction, stress
+        # restore, two transposes, velocity reconstruction, velocity restore);
+        # prep3, prep_profiles3 and band_table per pass, finalize3
+        return 5 * self.nt + 8 * (self.nt - 1) + 7
 
     def cpu_run(self, nt_sample, shots=1):
         from oracle import oracle as O
@@ -628,10 +635,11 @@ class Elastic3DWorkload:
 # on (sH, sV).  Algorithmic floats per runtime cell-step (one read and one
 # write of every field a kernel touches; CPML memories and the models not
 # counted): forward velocity step 2 stresses read + 3 velocities read and
-# written (8), stress step 3 + 4 (7); reverse: stress reconstruction 7,
-# half-step A pre-multiply 2 + 3 and apply 3 + 6, gradient 10 + 8 slots,
-# half-step B 3 + 3 and 3 + 4, velocity reconstruction 8 (60).
-V3_BYTES_FWD, V3_BYTES_REV = 4 * 15, 4 * 60
+# written (8), stress step 3 + 4 (7); reverse: half-step A with the stress
+# reconstruction 3 + 4 + 2 + 6 (15), half-step B with the velocity
+# reconstruction 2 + 6 + 3 + 4 (15), gradient slots (four, each shared by four
+# shots) 2 (32).
+V3_BYTES_FWD, V3_BYTES_REV = 4 * 15, 4 * 32
 
 
 def vti3d_survey(seed=SEED):
@@ -646,7 +654,7 @@ def vti3d_survey(seed=SEED):
 class VTI3DWorkload(Elastic3DWorkload):
     name = "vti3d"
     bytes_fwd, bytes_rev = V3_BYTES_FWD, V3_BYTES_REV
-    kernel = "sweep::vti3 reverse step (srev + premA + appA + grad + premB + appB + vrev + band restores)"
+    kernel = "sweep::vtik reverse step (half_a + half_b: transposes, reconstructions, gradient; events and band restores)"
     cpu_nt = 24
 
     def config(self, args):
@@ -667,11 +675,9 @@ class VTI3DWorkload(Elastic3DWorkload):
         return solver, m_true, m_init, w, src, rec
 
     def launches(self, group):
-        # forward 5 per step (velocity, stress, source, bands, record); reverse
-        # 11 (residuals, source removal, two reconstructions, two band
-        # restores, two pre-multiplies, two applies, gradient); prep per pass
-        # and four finalize
-        return 5 * self.nt + 11 * (self.nt - 1) + 6
+        # forward 4 per step, reverse 5 (as the 2-D workload's); prep, three
+        # prep_profiles and band_table per pass, finalize
+        return 4 * self.nt + 5 * (self.nt - 1) + 11
 
     def cpu_run(self, nt_sample, shots=1):
         from oracle import oracle as O
@@ -1103,9 +1109,9 @@ def main():
     ORDER = int(args.order)
     wl = WORKLOADS[args.workload]()
     if ORDER != 8:
-        # the any-order kernels: one reverse step is adj + recon + strip kernels
-        wl.kernel = (f"sweep::aord reverse step at order {ORDER} (adj{2 if wl.name != 'acoustic3d' else 3} + "
-                     "recon + strip kernels)")
+        if wl.name.startswith("acoustic"):
+            wl.kernel = (f"sweep::aord::rev at order {ORDER} (adjoint, reconstruction, strip restore and imaging "
+                         "step; events)")
         wl.traffic = None
     if args.nt:
         wl.nt = int(args.nt)
