@@ -745,26 +745,32 @@ __global__ void __launch_bounds__(kThreads, kBlocks) vel_rev(const Rev A)
 }
 
 // Velocity strips from a step slot; the rho image of the box's outermost
-// layer is the difference this makes.
+// layer is the difference this makes.  There the thread of a group's first
+// shot walks the group's shots, so that the sum does not depend on timing.
 __global__ void restore_velocity(const Rev A, const void* slot, int fmt)
 {
     const Geo& G = A.G;
     const long long n = (long long)G.B * G.ns;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int b = (int)(e / G.ns), k = (int)(e - (long long)b * G.ns);
+        const int b0 = (int)(e / G.ns), k = (int)(e - (long long)b0 * G.ns);
         const int c = G.cells[k];
         const int ix = c % G.P, r = c / G.P;
         const bool img = A.it > 1 && in_box(G, ix, r % G.ny, r / G.ny);
+        if (img && b0 % G.group) continue;
+        const int b1 = img ? min(b0 + G.group, G.B) : b0 + 1;
         float s = 0.f;
-        for (int fl = VX; fl <= VZ; ++fl) {
-            const long long t = ((long long)b * NFLD + fl) * G.ns + k, i = b * G.S + c;
-            const float v = fmt == SF_F32    ? static_cast<const float*>(slot)[t]
-                            : fmt == SF_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(slot)[t])
-                                             : face_val(G, slot, fl, b, c);
-            if (img) s += A.a[fl][i] * (v - A.f[fl][i]);
-            A.f[fl][i] = v;
+        for (int b = b0; b < b1; ++b) {
+            const long long i = b * G.S + c;
+            for (int fl = VX; fl <= VZ; ++fl) {
+                const long long t = ((long long)b * NFLD + fl) * G.ns + k;
+                const float v = fmt == SF_F32    ? static_cast<const float*>(slot)[t]
+                                : fmt == SF_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(slot)[t])
+                                                 : face_val(G, slot, fl, b, c);
+                if (img) s += A.a[fl][i] * (v - A.f[fl][i]);
+                A.f[fl][i] = v;
+            }
         }
-        if (img) atomicAdd(A.g[2] + b / G.group * G.S + c, s);
+        if (img) A.g[2][b0 / G.group * G.S + c] += s;
     }
 }
 
