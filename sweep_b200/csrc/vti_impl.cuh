@@ -679,9 +679,10 @@ __global__ void finalize(const Geo G, const Slots s, const Models m, const Grads
                 }
                 t[j] *= G.dt;
             }
-            // c11 = c33 (1 + 2 eps), c13 = c33 sqrt(1 + 2 delta), c33 = rho v^2
+            // c11 = c33 (1 + 2 eps), c13 = c33 sqrt(1 + 2 delta), c33 = rho v^2;
+            // in vacuum (v = 0) every stiffness is zero, so t[0] is
             const float v = m.vp[e], rho = m.rho[e], rv2 = rho * (v * v);
-            gv = 2.f * t[0] / v;
+            gv = v != 0.f ? 2.f * t[0] / v : 0.f;
             ge = 2.f * t[1] * rv2;
             gd = t[2] * rv2 / fmaxf(sqrtf(1.f + 2.f * m.dlt[e]), 1e-12f);
             gp = t[3] / rho;

@@ -35,10 +35,12 @@ def _geometry(shape, B, rng):
     return src.astype(np.int64), rec.astype(np.int64)
 
 
-def _check(eq, oracle, names, shape, B, order, free=False):
+def _check(eq, oracle, names, shape, B, order, free=False, vacuum=False):
     from sweep_b200 import PropTorch
     rng = np.random.default_rng(sum(shape) + 7 * order + B)
     ms = _models(names, shape, rng)
+    if vacuum:                                      # a few cells without stiffness
+        ms[0].reshape(-1)[rng.integers(0, ms[0].size, 5)] = 0.0
     src, rec = _geometry(shape, B, rng)
     dh, dt, abcn = 6.0, 0.0006, 5
     t = np.arange(NT) * dt
@@ -76,6 +78,14 @@ def test_vti2d(shape, B, order):
 def test_vti3d(shape, B, order):
     from sweep_b200 import AcousticVTI1st3D
     _check(AcousticVTI1st3D, O.VTI3D, ("vp", "eps", "dlt", "rho"), shape, B, order)
+
+
+@pytest.mark.parametrize("shape,order", [((33, 32), 4), ((17, 15, 34), 4)])
+def test_vti_vacuum_cells(shape, order):
+    """Cells with vp = 0 (and rho > 0) take no part in the misfit by vp."""
+    from sweep_b200 import AcousticVTI1st, AcousticVTI1st3D
+    eq, oracle = (AcousticVTI1st, O.VTI2D) if len(shape) == 2 else (AcousticVTI1st3D, O.VTI3D)
+    _check(eq, oracle, ("vp", "eps", "dlt", "rho"), shape, 2, order, vacuum=True)
 
 
 @pytest.mark.parametrize("shape,B,order", [
