@@ -42,8 +42,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <vector>
 
+#include "bands.cuh"
 #include "common.cuh"
 #include "elastic_orders.cuh"
 #include "elastic_vec.cuh"
@@ -133,7 +133,7 @@ __global__ void prep(const float* __restrict__ vp, const float* __restrict__ vs,
 struct Plan {
     Geo G;
     int nm;                         // model copies
-    std::vector<int> cells;
+    bands::Bands bands;
 };
 
 // staggered first-derivative weights of half-width M (the closed form
@@ -208,24 +208,9 @@ static Plan make_plan(const sweep_elastic_desc* d, int mem_mode)
     for (int k = 0; k < 5; ++k) { G.sf[k] = d->src_fields[k]; G.rf[k] = d->rec_fields[k]; }
     G.src = d->src_loc; G.rec = d->rec_loc; G.wavelet = d->wavelet;
     // the boundary bands (boundary/strip.cuh:46-123: width M + 1 from M cells
-    // outside the box, each band over the box tangentially; a band that would
-    // leave the grid slides back inside)
-    const int w = M + 1, off = -M;
-    auto band_lo = [](int p0, int of, int wd, int n) { int s = p0 + of; if (s + wd > n) s = n - wd; return s < 0 ? 0 : s; };
-    auto band_hi = [](int p1, int of, int wd, int n) { int e = p1 - of; if (e - wd < 0) e = wd; return e > n ? n : e; };
-    const int ts = band_lo(G.z0, off, w, G.nz), be = band_hi(G.z1, off, w, G.nz);
-    const int ls = band_lo(G.x0, off, w, G.nx), re = band_hi(G.x1, off, w, G.nx);
-    // (a cell of two bands once: the x bands leave out what the z bands hold)
-    auto in_zbands = [&](int z, int x) {
-        return x >= G.x0 && x < G.x1 && ((z >= ts && z < ts + w) || (z >= be - w && z < be));
-    };
-    for (int z = ts; z < ts + w; ++z) for (int x = G.x0; x < G.x1; ++x) pl.cells.push_back(z * G.P + x);
-    for (int z = be - w; z < be; ++z) for (int x = G.x0; x < G.x1; ++x) pl.cells.push_back(z * G.P + x);
-    for (int z = G.z0; z < G.z1; ++z)
-        for (int s : {ls, re - w})
-            for (int x = s; x < s + w; ++x)
-                if (!in_zbands(z, x)) pl.cells.push_back(z * G.P + x);
-    G.ns = (int)pl.cells.size();
+    // outside the box, each band over the box tangentially)
+    pl.bands = bands::make<2>(M, G.z0, G.z1, 0, 1, G.x0, G.x1);
+    G.ns = pl.bands.count;
     layout(G, per_shot ? 1 : 4);
     return pl;
 }
@@ -292,9 +277,9 @@ static void setup(const sweep_elastic_desc* d, Plan& pl, const Ws& w, cudaStream
     const int len = xprof_len(G);
     prep_profiles<<<8, 256, 0, st>>>(d->ax, d->bx, d->axh, d->bxh, G.nx, len, w.xprof);
     G.ax = w.xprof + kGuard; G.bx = G.ax + len; G.axh = G.bx + len; G.bxh = G.axh + len;
+    // on the device: a list in host memory would have to outlive a captured call
+    bands::band_table<2><<<std::min(blocks(G.ns), 1024u), 256, 0, st>>>(pl.bands, G.P, G.P, w.cells);
     SWEEP_LAUNCH_CHECK();
-    if (G.ns > 0)
-        SWEEP_CUDA(cudaMemcpyAsync(w.cells, pl.cells.data(), sizeof(int) * G.ns, cudaMemcpyHostToDevice, st));
     SWEEP_CUDA(cudaMemsetAsync(w.zero0, 0, w.zero1 - w.zero0, st));
 }
 
