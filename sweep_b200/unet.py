@@ -48,7 +48,7 @@ class _Conv3x3(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, gout):
-        x, wb = ctx.saved_tensors
+        x, wb = (t.contiguous() for t in ctx.saved_tensors)     # hooks may hand them back in another order
         n, h, wd, c = x.shape
         co = wb.shape[0]
         gout = gout.contiguous()
