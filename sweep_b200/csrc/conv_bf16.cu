@@ -341,6 +341,24 @@ __global__ void __launch_bounds__(NT) conv_pass(const __nv_bfloat16* __restrict_
     if (warp == 0) umma::dealloc(tmem, (uint32_t)cols);
 }
 
+// The sum of a CTA's products of one weight over the pixels inside the image.
+__device__ __noinline__ float inside_sum(const Shape& S, const __nv_bfloat16* __restrict__ x,
+                                         const __nv_bfloat16* __restrict__ dy, int t0, int nt, int tap, int c, int n)
+{
+    float sum = 0.f;
+    for (int t = t0; t < t0 + nt; ++t) {
+        const Tile T(S, t);
+        for (int q = 0; q < BM; ++q) {
+            const int h = T.h0 + (q >> 3), w = T.w0 + (q & 7), hx = h + tap / 3 - 1, wx = w + tap % 3 - 1;
+            if (h >= S.H || w >= S.W || hx < 0 || hx >= S.H || wx < 0 || wx >= S.W) continue;
+            const long long img = (long long)T.img * S.H;
+            sum += __bfloat162float(dy[((img + h) * S.W + w) * S.Nout + n]) *
+                   __bfloat162float(x[((img + hx) * S.W + wx) * S.C + c]);
+        }
+    }
+    return sum;
+}
+
 // dw[co, t, c] += the sum over this CTA's tiles: c in [64 blockIdx.x, + 64), co
 // in [64 blockIdx.y, + 64), tiles [per blockIdx.z, + per).  Accumulator 2 dy holds
 // taps (dy, -1) and (dy, 0), rows 0..63 and 64..127; 2 dy + 1 tap (dy, 1) and
@@ -413,6 +431,7 @@ __global__ void __launch_bounds__(NT) conv_wgrad(const __nv_bfloat16* __restrict
     ok = ok && tma::mbar_wait(&hd.done[prev], pphase, err, umma::ERR_MMA_WAIT);
     umma::fence_after();
     const int m = 32 * (warp & 3) + lane, c = c0 + (m & 63), col = COLS * (warp >> 2), n = n0 + col;
+    const bool over = S.H % umma::BH != 0 || S.W % umma::BW != 0;
 #pragma unroll 1
     for (int j = 0; j < 6; ++j) {
         const int tap = (j / 2) * 3 + (j & 1 ? 2 : m >> 6);
@@ -425,8 +444,14 @@ __global__ void __launch_bounds__(NT) conv_wgrad(const __nv_bfloat16* __restrict
 #pragma unroll
         for (int i = 0; i < COLS / 8; ++i)
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-                if (n + 8 * i + e < S.Nout) atomicAdd(dw + ((long long)(n + 8 * i + e) * 9 + tap) * S.C + c, v[i][e]);
+            for (int e = 0; e < 8; ++e) {
+                const int co = n + 8 * i + e;
+                if (co >= S.Nout) continue;
+                // the zero dy of a tile's pixels outside the image makes a NaN of
+                // an infinite x that only such a pixel's tap reads
+                const float s = over && v[i][e] != v[i][e] ? inside_sum(S, x, dy, t0, nt, tap, c, co) : v[i][e];
+                atomicAdd(dw + ((long long)co * 9 + tap) * S.C + c, s);
+            }
     }
     umma::wait_copies<0>();
     umma::fence_before();

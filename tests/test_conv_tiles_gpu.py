@@ -38,6 +38,31 @@ def test_conv3x3_matches_float64(n, h, w, c, co):
     assert errs[1] < 2.0 ** -8 + 1e-5
 
 
+def test_weight_gradient_keeps_an_infinity_to_its_taps():
+    """Infinite inputs in the last row and column of an image that ends inside a
+    tile: the taps that do not read them keep a finite gradient."""
+    from sweep_b200 import unet
+    gen = torch.Generator().manual_seed(3)
+    x = torch.randn((2, 17, 12, 16), generator=gen).to(torch.bfloat16)
+    x[0, 16, 5, 3], x[1, 4, 11, 9] = float("inf"), float("-inf")
+    g = torch.randn((2, 17, 12, 8), generator=gen).to(torch.bfloat16).float()
+    w = torch.zeros((8, 3, 3, 16), device=DEV, requires_grad=True)
+    y = unet.conv3x3(x.to(DEV), w, torch.zeros(8, device=DEV))
+    y.backward(g.to(DEV))
+    unet.check()
+    want = torch.zeros((8, 3, 3, 16), dtype=torch.float64)
+    for dy in range(3):
+        for dx in range(3):
+            h, v = slice(max(0, 1 - dy), 17 - max(0, dy - 1)), slice(max(0, 1 - dx), 12 - max(0, dx - 1))
+            hx, vx = slice(max(0, dy - 1), 17 - max(0, 1 - dy)), slice(max(0, dx - 1), 12 - max(0, 1 - dx))
+            want[:, dy, dx] = torch.einsum("nhwo,nhwc->oc", g[:, h, v].double(), x[:, hx, vx].double())
+    got = w.grad.double().cpu()
+    assert want[:, 0, :, 3].isfinite().all() and not want[:, 1:, :, 3].isfinite().any()
+    assert want[:, :, 0, 9].isfinite().all() and not want[:, :, 1:, 9].isfinite().any()
+    assert torch.equal(got.isfinite(), want.isfinite())
+    assert rel(got[want.isfinite()], want[want.isfinite()]) < 1e-5
+
+
 def test_saved_tensors_of_another_order():
     """Saved-tensor hooks may hand the operands back in another memory order."""
     from sweep_b200 import unet
