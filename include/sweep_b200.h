@@ -400,17 +400,19 @@ SWEEP_B200_API int sweep_b200_conv3x3_status(void* stream, char* err, int32_t er
  * fastest.  A field left at its "built-in" value keeps the library's default;
  * a per-shot-model problem always runs one shot per CTA. */
 typedef struct sweep_b200_schedule {
-    int32_t shots_fwd;    /* shots per CTA of the forward step kernels (2-D acoustic
-                           * fwd_kernel, elastic fwd_vel / fwd_str); 0 = built-in */
+    int32_t shots_fwd;    /* shots per CTA of the forward step kernels (2-D acoustic,
+                           * elastic fwd_vel / fwd_str); 0 = built-in */
     int32_t shots_rev;    /* shots per CTA of the reverse kernels that sum the image
-                           * (2-D acoustic rev_kernel, elastic imaging); 0 = built-in */
+                           * (2-D acoustic, elastic imaging); 0 = built-in */
     int32_t z_chunks;     /* 3-D acoustic: z chunks each column block is cut into
                            * (grid depth per shot); 0 = built-in */
     int32_t graph_steps;  /* time steps per captured CUDA graph in the step loops
                            * (0: plain stream launches; < 0: built-in); host-tape
                            * loops always use plain launches */
-    int32_t tile_y;       /* 3-D acoustic: rows of the 32-column block a CTA of the
-                           * stencil kernels covers, 8 or 16 (0 = built-in 8) */
+    int32_t tile_y;       /* acoustic: rows of a CTA's tile of the stencil kernels.
+                           * 3-D: 32 columns by 8 or 16 (0 = built-in 8).  2-D: 8
+                           * the kernels of small grids (32 x 8 cells), 32 the tiled
+                           * ones (64 x 32), 0 = by the grid and the shots */
 } sweep_b200_schedule;
 
 #define SWEEP_FAMILY_ACOUSTIC 0   /* desc is a sweep_acoustic_desc (2-D or 3-D) */

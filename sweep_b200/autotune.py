@@ -15,13 +15,15 @@ launch choices the core leaves open for one problem shape:
   into (the grid depth per shot, 3-D acoustic);
 * ``graph_steps`` -- time steps per captured CUDA graph in the step loops
   (0: plain stream launches);
-* ``tile_y`` -- 3-D acoustic: rows of the 32-column block each CTA of the
-  stencil kernels covers, 8 (256 threads, 4 CTAs per SM) or 16 (512 threads,
-  2 CTAs per SM, less halo per cell).
+* ``tile_y`` -- acoustic: rows of the tile each CTA of the stencil kernels
+  covers.  3-D: 32 columns by 8 (256 threads, 4 CTAs per SM) or 16 (512
+  threads, 2 CTAs per SM, less halo per cell).  2-D: 8 the kernels of small
+  grids (32 x 8 cells), 32 the tiled ones (64 x 32), 0 by the grid and the
+  shots; not tuned.
 
-The 2-D and elastic tile shapes are compile-time constants of the kernels
-(they fix the shared-memory staging and register blocking), and there is no
-temporal blocking to choose: every step is one pass over HBM.
+The elastic tile shape is a compile-time constant of the kernels (it fixes the
+shared-memory staging and register blocking), and there is no temporal
+blocking to choose: every step is one pass over HBM.
 
 :func:`tune` times the real forward and backward calls of one shape over a
 truncated time axis, one knob at a time from the built-in defaults

@@ -921,13 +921,15 @@ __global__ void __launch_bounds__(NTH, 2) rev_kernel(const __grid_constant__ Rev
 // four cells per thread (acoustic_vec.cuh), 32 x 8 cells per CTA of 64
 // threads, every load of a step issued at once instead of stage by stage.
 // Such a step is latency, not bandwidth: 96 x 128, one shot, forward 3.9 us
-// and reverse 6.5 us a step (12.3 and 18.5 us on the tiled kernels).
+// and reverse 6.5 us a step (12.3 and 18.5 us on the tiled kernels).  A CTA
+// walks the P.G shots of its group, whose image it sums before it adds it to
+// the group's slot, as the tiled kernels do.
 constexpr int SNTH = SX / 4 * SZ;
 
-__device__ __forceinline__ avec::Cell<2> small_cell(const avec::Geo& G, const Params& P, int tile, int b)
+__device__ __forceinline__ avec::Cell<2> small_cell(const avec::Geo& G, const Params& P, int tile)
 {
     avec::Cell<2> q;
-    q.b = b;
+    q.b = 0;
     q.c[0] = (tile % P.ntx) * SX + 4 * (threadIdx.x & 7);
     q.c[1] = 0;
     q.c[2] = (tile / P.ntx) * SZ + (threadIdx.x >> 3);
@@ -935,156 +937,190 @@ __device__ __forceinline__ avec::Cell<2> small_cell(const avec::Geo& G, const Pa
     return q;
 }
 
-// grid (shot, tile)
+// grid (shot group, tile)
 __global__ void __launch_bounds__(SNTH) fwd_small(const __grid_constant__ avec::Geo G, const __grid_constant__ Params P,
                                                   const __grid_constant__ FwdPtrs F, const float* now,
                                                   const float* prev, const int it)
 {
     __shared__ __align__(16) float out[SX * SZ];
-    const int tile = P.order[blockIdx.y], b = blockIdx.x, key = b * P.ntx * P.ntz + tile;
-    const int s_beg = P.src.off[key], s_end = P.src.off[key + 1], r_beg = P.rec.off[key], r_end = P.rec.off[key + 1];
-    const avec::Cell<2> q = small_cell(G, P, tile, b);
-    const long long k = b * P.S + q.i;
-    avec::F4 un = v4::splat(0.f), u0;
-    if (q.core) {
-        avec::Step A{};
-        A.un = now; A.up = prev;
-        A.ps[0] = F.psix; A.ps[2] = F.psiz; A.psn[0] = F.psixn; A.psn[2] = F.psizn;
-        A.zt[0] = F.zetax; A.zt[2] = F.zetaz;
-        un = avec::step_cells<M, 2>(G, q, A, k, u0);
-        if (F.strips) {
-            const int z = q.c[2];
-            const bool row = z >= P.z0 && z < P.z1;
-            if (row && q.c[0] + 3 >= P.x0 && q.c[0] < P.x1 &&
-                !(z >= P.rz0 && z < P.rz1 && q.c[0] >= P.rx0 && q.c[0] + 3 < P.rx1)) {
+    const int tile = P.order[blockIdx.y];
+    avec::Cell<2> q = small_cell(G, P, tile);
+    const int b1 = min((int)(blockIdx.x + 1) * P.G, P.B);
+    for (int b = blockIdx.x * P.G; b < b1; ++b) {
+        const int key = b * P.ntx * P.ntz + tile;
+        const int s_beg = P.src.off[key], s_end = P.src.off[key + 1], r_beg = P.rec.off[key], r_end = P.rec.off[key + 1];
+        q.b = b;
+        const long long k = b * P.S + q.i;
+        avec::F4 un = v4::splat(0.f), u0;
+        if (q.core) {
+            avec::Step A{};
+            A.un = now; A.up = prev;
+            A.ps[0] = F.psix; A.ps[2] = F.psiz; A.psn[0] = F.psixn; A.psn[2] = F.psizn;
+            A.zt[0] = F.zetax; A.zt[2] = F.zetaz;
+            un = avec::step_cells<M, 2>(G, q, A, k, u0);
+            if (F.strips) {
+                const int z = q.c[2];
+                const bool row = z >= P.z0 && z < P.z1;
+                if (row && q.c[0] + 3 >= P.x0 && q.c[0] < P.x1 &&
+                    !(z >= P.rz0 && z < P.rz1 && q.c[0] >= P.rx0 && q.c[0] + 3 < P.rx1)) {
 #pragma unroll
-                for (int l = 0; l < 4; ++l) {
-                    const int e = strip_index(P, z, q.c[0] + l);
-                    if (e < 0) continue;
-                    const long long o = (long long)b * P.nstrip + e;
-                    if (F.sbf16) static_cast<__nv_bfloat16*>(F.strips)[o] = __float2bfloat16(u0.v[l]);
-                    else static_cast<float*>(F.strips)[o] = u0.v[l];
+                    for (int l = 0; l < 4; ++l) {
+                        const int e = strip_index(P, z, q.c[0] + l);
+                        if (e < 0) continue;
+                        const long long o = (long long)b * P.nstrip + e;
+                        if (F.sbf16) static_cast<__nv_bfloat16*>(F.strips)[o] = __float2bfloat16(u0.v[l]);
+                        else static_cast<float*>(F.strips)[o] = u0.v[l];
+                    }
                 }
             }
         }
-    }
-    if (s_beg != s_end || r_beg != r_end) {
-        v4::st(out + 4 * threadIdx.x, un);
-        __syncthreads();
-        for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
-            const int2 ev = P.src.ev[e];
-            atomicAdd(out + ev.x, __ldg(P.wavelet + (long long)ev.y * P.nt + it));
+        const bool events = s_beg != s_end || r_beg != r_end;
+        if (events) {
+            v4::st(out + 4 * threadIdx.x, un);
+            __syncthreads();
+            for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
+                const int2 ev = P.src.ev[e];
+                atomicAdd(out + ev.x, __ldg(P.wavelet + (long long)ev.y * P.nt + it));
+            }
+            __syncthreads();
+            for (int e = r_beg + threadIdx.x; F.record && e < r_end; e += SNTH) {
+                const int2 ev = P.rec.ev[e];
+                const int rb = ev.y / P.nrec, rr = ev.y - rb * P.nrec;
+                F.record[((long long)rb * P.nt + it) * P.nrec + rr] = out[ev.x];
+            }
+            un = v4::ld(out + 4 * threadIdx.x);
         }
-        __syncthreads();
-        for (int e = r_beg + threadIdx.x; F.record && e < r_end; e += SNTH) {
-            const int2 ev = P.rec.ev[e];
-            const int rb = ev.y / P.nrec, rr = ev.y - rb * P.nrec;
-            F.record[((long long)rb * P.nt + it) * P.nrec + rr] = out[ev.x];
-        }
-        un = v4::ld(out + 4 * threadIdx.x);
+        if (q.core) avec::store_core(G, q, F.u_next + k, un);
+        if (events && b + 1 < b1) __syncthreads();       // the records are read before the next shot's cells arrive
     }
-    if (q.core) avec::store_core(G, q, F.u_next + k, un);
 }
 
-// grid (shot, tile); the step of rev_kernel
+// grid (shot group, tile); the step of rev_kernel
 __global__ void __launch_bounds__(SNTH) rev_small(const __grid_constant__ avec::Geo G, const __grid_constant__ Params P,
                                                   const __grid_constant__ RevPtrs R, const float* lnow,
                                                   const float* lprev, const float* rnow, const float* rprev,
                                                   const int it, const int do_recon)
 {
     __shared__ __align__(16) float lo[SX * SZ], ro[SX * SZ];
-    const int tile = P.order[blockIdx.y], b = blockIdx.x, key = b * P.ntx * P.ntz + tile;
-    const int s_beg = P.src.off[key], s_end = P.src.off[key + 1], r_beg = P.rec.off[key], r_end = P.rec.off[key + 1];
-    const avec::Cell<2> q = small_cell(G, P, tile, b);
-    const long long k = b * P.S + q.i, mi = b * P.ms + q.i;
+    const int tile = P.order[blockIdx.y];
+    avec::Cell<2> q = small_cell(G, P, tile);
     const int z = q.c[2], x = q.c[0];
-    avec::F4 lx = v4::splat(0.f), un = lx, u0 = lx, up = lx;
-    bool phys[4] = {false, false, false, false};
-    if (q.core) {
-        avec::Rev A{};
-        A.ln = lnow; A.lp = lprev;
-        A.ps[0] = R.apx; A.ps[2] = R.apz; A.zt[0] = R.azx; A.zt[2] = R.azz;
-        A.pso[0] = R.apx_o; A.pso[2] = R.apz_o; A.zto[0] = R.azx_o; A.zto[2] = R.azz_o;
-        lx = avec::adj_cells<M, 2>(G, q, A, k, mi);
-        const bool row = z >= P.z0 && z < P.z1;
+    const bool row = q.core && z >= P.z0 && z < P.z1;
+    bool phys[4];
 #pragma unroll
-        for (int l = 0; l < 4; ++l) phys[l] = row && x + l >= P.x0 && x + l < P.x1;
-        if (do_recon && (phys[0] || phys[3] || phys[1] || phys[2])) {
-            u0 = v4::ldg(rnow + k);
-            up = v4::ldg(rprev + k);
-            const bool rrow = z >= P.rz0 && z < P.rz1;
-            if (rrow && x + 3 >= P.rx0 && x < P.rx1) un = avec::recon_cells<M, 2>(G, rnow, k, mi, u0, up);
+    for (int l = 0; l < 4; ++l) phys[l] = row && x + l >= P.x0 && x + l < P.x1;
+    const bool any = phys[0] || phys[1] || phys[2] || phys[3];
+    const float dt2 = P.dt * P.dt;
+    // the group's image so far, loaded beside the first shot's fields
+    const long long slot = blockIdx.x * P.S + q.i;
+    avec::F4 gsum = v4::splat(0.f), is = gsum, ir = gsum, acc = gsum, comp = gsum;
+    if (do_recon && any) {
+        acc = v4::ld(R.gacc + slot);
+        comp = v4::ld(R.gcomp + slot);
+    }
+    const int b1 = min((int)(blockIdx.x + 1) * P.G, P.B);
+    for (int b = blockIdx.x * P.G; b < b1; ++b) {
+        const int key = b * P.ntx * P.ntz + tile;
+        const int s_beg = P.src.off[key], s_end = P.src.off[key + 1], r_beg = P.rec.off[key], r_end = P.rec.off[key + 1];
+        q.b = b;
+        const long long k = b * P.S + q.i, mi = b * P.ms + q.i;
+        avec::F4 lx = v4::splat(0.f), un = lx, u0 = lx, up = lx;
+        if (q.core) {
+            avec::Rev A{};
+            A.ln = lnow; A.lp = lprev;
+            A.ps[0] = R.apx; A.ps[2] = R.apz; A.zt[0] = R.azx; A.zt[2] = R.azz;
+            A.pso[0] = R.apx_o; A.pso[2] = R.apz_o; A.zto[0] = R.azx_o; A.zto[2] = R.azz_o;
+            lx = avec::adj_cells<M, 2>(G, q, A, k, mi);
+            if (do_recon && any) {
+                u0 = v4::ldg(rnow + k);
+                up = v4::ldg(rprev + k);
+                const bool rrow = z >= P.rz0 && z < P.rz1;
+                if (rrow && x + 3 >= P.rx0 && x < P.rx1) un = avec::recon_cells<M, 2>(G, rnow, k, mi, u0, up);
+#pragma unroll
+                for (int l = 0; l < 4; ++l)
+                    if (phys[l] && !(rrow && x + l >= P.rx0 && x + l < P.rx1))
+                        un.v[l] = strip_value(P, R.strips, b, z, x + l);
+            }
+        }
+        const bool events = s_beg != s_end || r_beg != r_end;
+        if (events) {
+            v4::st(lo + 4 * threadIdx.x, lx);
+            v4::st(ro + 4 * threadIdx.x, un);
+            __syncthreads();
+            for (int e = r_beg + threadIdx.x; e < r_end; e += SNTH) {
+                const int2 ev = P.rec.ev[e];
+                const int rb = ev.y / P.nrec, rr = ev.y - rb * P.nrec;
+                atomicAdd(lo + ev.x, __ldg(R.adj + ((long long)rb * P.nt + it) * P.nrec + rr));
+            }
+            if (do_recon) {
+                for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
+                    const int2 ev = P.src.ev[e];
+                    if (strip_index(P, (tile / P.ntx) * SZ + ev.x / SX, (tile % P.ntx) * SX + ev.x % SX) >= 0)
+                        atomicAdd(ro + ev.x, -__ldg(P.wavelet + (long long)ev.y * P.nt + it));
+                }
+            }
+            __syncthreads();
+            if (R.grad_w)
+                for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
+                    const int2 ev = P.src.ev[e];
+                    R.grad_w[(long long)ev.y * P.nt + it] = lo[ev.x];
+                }
+            lx = v4::ld(lo + 4 * threadIdx.x);
+            un = v4::ld(ro + 4 * threadIdx.x);
+        }
+        if (q.core) {
+            avec::store_core(G, q, R.l_next + k, lx);
+            const avec::F4 v = v4::ldg(P.vv + mi);
+#pragma unroll
+            for (int l = 0; l < 4; ++l) {
+                if (!phys[l]) continue;
+                if (do_recon) {
+                    const float utt = (un.v[l] - 2.f * u0.v[l] + up.v[l]) / dt2;
+                    gsum.v[l] += 2.f * P.dt * P.dt * utt * lx.v[l] / v.v[l];
+                    is.v[l] += utt * utt;
+                }
+                ir.v[l] += lx.v[l] * lx.v[l];
+            }
+        }
+        if (events) {
+            __syncthreads();                     // lo and ro are read before they change again
+            if (do_recon) {
+                for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
+                    const int2 ev = P.src.ev[e];
+                    atomicAdd(ro + ev.x, __ldg(P.wavelet + (long long)ev.y * P.nt + it));
+                }
+                __syncthreads();
+                un = v4::ld(ro + 4 * threadIdx.x);
+            }
+        }
+        if (!do_recon) continue;
+        if (phys[0] && phys[3]) {
+            v4::st(R.r_next + k, un);
+        } else {
 #pragma unroll
             for (int l = 0; l < 4; ++l)
-                if (phys[l] && !(rrow && x + l >= P.rx0 && x + l < P.rx1))
-                    un.v[l] = strip_value(P, R.strips, b, z, x + l);
+                if (phys[l]) R.r_next[k + l] = un.v[l];
         }
     }
-    const bool events = s_beg != s_end || r_beg != r_end;
-    if (events) {
-        v4::st(lo + 4 * threadIdx.x, lx);
-        v4::st(ro + 4 * threadIdx.x, un);
-        __syncthreads();
-        for (int e = r_beg + threadIdx.x; e < r_end; e += SNTH) {
-            const int2 ev = P.rec.ev[e];
-            const int rb = ev.y / P.nrec, rr = ev.y - rb * P.nrec;
-            atomicAdd(lo + ev.x, __ldg(R.adj + ((long long)rb * P.nt + it) * P.nrec + rr));
+    if (!any) return;
+    if (do_recon) {
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {            // gsum is zero on the lanes outside the box
+            const float y = gsum.v[l] - comp.v[l];
+            const float t = acc.v[l] + y;
+            comp.v[l] = (t - acc.v[l]) - y;
+            acc.v[l] = t;
         }
-        if (do_recon) {
-            for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
-                const int2 ev = P.src.ev[e];
-                if (strip_index(P, (tile / P.ntx) * SZ + ev.x / SX, (tile % P.ntx) * SX + ev.x % SX) >= 0)
-                    atomicAdd(ro + ev.x, -__ldg(P.wavelet + (long long)ev.y * P.nt + it));
-            }
-        }
-        __syncthreads();
-        if (R.grad_w)
-            for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
-                const int2 ev = P.src.ev[e];
-                R.grad_w[(long long)ev.y * P.nt + it] = lo[ev.x];
-            }
-        lx = v4::ld(lo + 4 * threadIdx.x);
-        un = v4::ld(ro + 4 * threadIdx.x);
+        v4::st(R.gacc + slot, acc);
+        v4::st(R.gcomp + slot, comp);
     }
-    if (q.core) {
-        avec::store_core(G, q, R.l_next + k, lx);
-        const float dt2 = P.dt * P.dt;
-        const avec::F4 v = v4::ldg(P.vv + mi);
+    if (R.illum_s) {
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
             if (!phys[l]) continue;
-            const long long o = k + l;               // the shot's slot
-            float utt = 0.f;
-            if (do_recon) {
-                utt = (un.v[l] - 2.f * u0.v[l] + up.v[l]) / dt2;
-                const float g = 2.f * P.dt * P.dt * utt * lx.v[l] / v.v[l];
-                const float y = g - R.gcomp[o];
-                const float t = R.gacc[o] + y;
-                R.gcomp[o] = (t - R.gacc[o]) - y;
-                R.gacc[o] = t;
-            }
-            if (R.illum_s) {
-                R.illum_s[o] += utt * utt;
-                R.illum_r[o] += lx.v[l] * lx.v[l];
-            }
+            R.illum_s[slot + l] += is.v[l];
+            R.illum_r[slot + l] += ir.v[l];
         }
-    }
-    if (!do_recon) return;
-    if (events) {
-        __syncthreads();
-        for (int e = s_beg + threadIdx.x; e < s_end; e += SNTH) {
-            const int2 ev = P.src.ev[e];
-            atomicAdd(ro + ev.x, __ldg(P.wavelet + (long long)ev.y * P.nt + it));
-        }
-        __syncthreads();
-        un = v4::ld(ro + 4 * threadIdx.x);
-    }
-    if (phys[0] && phys[3]) {
-        v4::st(R.r_next + k, un);
-    } else {
-#pragma unroll
-        for (int l = 0; l < 4; ++l)
-            if (phys[l]) R.r_next[k + l] = un.v[l];
     }
 }
 
@@ -1132,7 +1168,8 @@ __global__ void __launch_bounds__(kQB) quantize_strips(const Params P, const flo
 }
 
 // Model-derived fields, pitched: cf = ((v*v)*dt)*dt (forward, reconstruction),
-// ca = (v*v)*(dt*dt) (adjoint taps), vv = v (imaging); 0 (vv: 1) in the pitch pad.
+// and for a reverse ca = (v*v)*(dt*dt) (adjoint taps), vv = v (imaging); 0 (vv: 1)
+// in the pitch pad.
 __global__ void prep_kernel(const float* __restrict__ vp, int nm, int nz, int nx, int P, float dt,
                             float* __restrict__ cf, float* __restrict__ ca, float* __restrict__ vv)
 {
@@ -1144,10 +1181,13 @@ __global__ void prep_kernel(const float* __restrict__ vp, int nm, int nz, int nx
         if (ix < nx) {
             const float v = vp[row * nx + ix];
             cf[i] = ((v * v) * dt) * dt;
-            ca[i] = (v * v) * dt2;
-            vv[i] = v;
+            if (ca) {
+                ca[i] = (v * v) * dt2;
+                vv[i] = v;
+            }
         } else {
-            cf[i] = 0.f; ca[i] = 0.f; vv[i] = 1.f;
+            cf[i] = 0.f;
+            if (ca) { ca[i] = 0.f; vv[i] = 1.f; }
         }
     }
 }
@@ -1189,7 +1229,9 @@ __global__ void pitch_copy_kernel(const float* __restrict__ src, float* __restri
 }
 
 // ------------------------------------------------------------------- host
-constexpr long long kSmallTiles = 2960;
+// The kernels of a call's forward, and of its reverse (with the replays of the
+// checkpoint modes, whose forward therefore runs the reverse's choice).
+enum Pass { FORWARD, REVERSE };
 
 struct Plan {
     Params P;
@@ -1232,22 +1274,39 @@ static int build_events(const Params& P, const int32_t* loc, int n, int32_t* off
     return off[nkey];
 }
 
-// Shots per CTA: the shape's recorded schedule value if any, else the
-// environment variable `env`, else `preferred` (measured best on B200 for this
-// kernel) capped so the grid still fills the GPU.
-static int choose_group(int ntiles, int B, const char* env, int preferred, int recorded)
+// Shots per CTA: `preferred` (measured best on B200 for the tiled kernel) capped
+// so that its grid of `ntiles` tiles still fills the GPU.
+static int built_in_group(int ntiles, int B, int preferred)
+{
+    int G = std::min({preferred, B, kMaxG});
+    while (G > 1 && (long long)ntiles * ((B + G - 1) / G) < 2LL * 148) --G;
+    return std::max(G, 1);
+}
+
+// The shape's recorded schedule value if any, else the environment variable
+// `env`, else the built-in choice.
+static int choose_group(int built_in, int B, const char* env, int recorded)
 {
     if (recorded >= 1) return std::min({recorded, B, kMaxG});
     if (const char* e = getenv(env)) {
         const int g = atoi(e);
         if (g >= 1) return std::min({g, B, kMaxG});
     }
-    int G = std::min({preferred, B, kMaxG});
-    while (G > 1 && (long long)ntiles * ((B + G - 1) / G) < 2LL * 148) --G;
-    return std::max(G, 1);
+    return built_in;
 }
 
-static Plan make_plan(const sweep_acoustic_desc* d)
+// Few tiles: a step of the tiled kernels lasts as long as one CTA, which
+// walks its shots' tiles through its stages eight cells per thread, so these
+// grids run four cells per thread on 32 x 8 tiles.  The line is where the
+// fields of a step leave the L2, which the tiled kernels' reuse over shots
+// then saves: gradients of 200 steps, small / tiled, 96 x 128 one shot
+// (15 tiles) 2.7 / 6.8 ms, 200 x 400 x 8 shots (512) 8.3 / 11.2,
+// 256 x 768 x 8 (1232) 14.1 / 29.5, x 12 (1848) 22.7 / 34.6, x 16 (2464)
+// 31.0 / 37.3, x 32 (4928) 63 / 51.6, 400 x 1200 x 8 (2480) 33.1 / 36.6.
+constexpr long long kSmallTiles = 2960;     // all shots
+static bool small_kernels(const Params& P, Pass, int ntiles) { return (long long)ntiles * P.B <= kSmallTiles; }
+
+static Plan make_plan(const sweep_acoustic_desc* d, Pass pass)
 {
     SWEEP_REQUIRE(d != nullptr, "null descriptor");
     SWEEP_REQUIRE(d->ndim == 2, "acoustic2d: ndim must be 2 (got %d)", d->ndim);
@@ -1298,33 +1357,29 @@ static Plan make_plan(const sweep_acoustic_desc* d)
     P.tx = TX; P.tz = TZ;
     P.ntx = (d->nx + TX - 1) / TX;
     P.ntz = (d->nz + TZ - 1) / TZ;
-    int ntiles = P.ntx * P.ntz;
+    const int ntiles = P.ntx * P.ntz;
     const sweep_b200_schedule sc = recorded_schedule(d);
-    pl.Gf = P.per_shot ? 1 : choose_group(ntiles, P.B, "SWEEP_B200_SHOTS_PER_CTA_FWD", 2, sc.shots_fwd);
-    pl.Gr = P.per_shot ? 1 : choose_group(ntiles, P.B, "SWEEP_B200_SHOTS_PER_CTA_REV", 8, sc.shots_rev);
+    // a recorded tile height decides instead of the rule; the small kernels'
+    // tiles are blockIdx.y
+    const long long nsmall = (long long)((d->nx + SX - 1) / SX) * ((d->nz + SZ - 1) / SZ);
+    pl.small = nsmall <= 65535 && (sc.tile_y == SZ || (sc.tile_y != TZ && small_kernels(P, pass, ntiles)));
+    // the small kernels' forward keeps no sums over shots, so it has a shot per
+    // CTA; their image has as many slots as the tiled kernels'
+    pl.Gf = P.per_shot ? 1 : choose_group(pl.small ? 1 : built_in_group(ntiles, P.B, 2), P.B,
+                                          "SWEEP_B200_SHOTS_PER_CTA_FWD", sc.shots_fwd);
+    pl.Gr = P.per_shot ? 1 : choose_group(built_in_group(ntiles, P.B, 8), P.B, "SWEEP_B200_SHOTS_PER_CTA_REV",
+                                          sc.shots_rev);
     pl.graph_steps = resolve_graph_steps(sc.graph_steps);
-    // blockIdx.x = shot group (fastest), blockIdx.y = tile slot
-    pl.gridf = dim3((P.B + pl.Gf - 1) / pl.Gf, ntiles);
-    pl.gridr = dim3((P.B + pl.Gr - 1) / pl.Gr, ntiles);
-    pl.nslot = P.per_shot ? P.B : (int)pl.gridr.x;
-    P.G = pl.Gr;
-    // Few tiles: a step of the tiled kernels lasts as long as one CTA, which
-    // walks its shots' tiles through its stages eight cells per thread, so
-    // these grids run four cells per thread on 32 x 8 tiles, one shot per CTA
-    // (the schedule's shots per CTA do not apply).  The line is where the
-    // fields of a step leave the L2, which the tiled kernels' reuse over shots
-    // then saves: gradients of 200 steps, small / tiled, 96 x 128 one shot
-    // (15 tiles) 2.7 / 6.8 ms, 200 x 400 x 8 shots (512) 8.3 / 11.2,
-    // 256 x 768 x 8 (1232) 14.1 / 29.5, x 12 (1848) 22.7 / 34.6, x 16 (2464)
-    // 31.0 / 37.3, x 32 (4928) 63 / 51.6, 400 x 1200 x 8 (2480) 33.1 / 36.6.
-    pl.small = (long long)ntiles * P.B <= kSmallTiles;
     if (pl.small) {
         P.tx = SX; P.tz = SZ;
         P.ntx = (d->nx + SX - 1) / SX;
         P.ntz = (d->nz + SZ - 1) / SZ;
-        pl.gridf = pl.gridr = dim3((unsigned)P.B, (unsigned)(P.ntx * P.ntz));
-        pl.nslot = P.B;
     }
+    // blockIdx.x = shot group (fastest), blockIdx.y = tile slot
+    pl.gridf = dim3((P.B + pl.Gf - 1) / pl.Gf, P.ntx * P.ntz);
+    pl.gridr = dim3((P.B + pl.Gr - 1) / pl.Gr, P.ntx * P.ntz);
+    pl.nslot = P.per_shot ? P.B : (int)pl.gridr.x;
+    P.G = pl.Gr;
     return pl;
 }
 
@@ -1354,13 +1409,16 @@ struct RevWork {
     char* ring;                      // host tape: HostRing::R device strip slots
 };
 
-static Common carve_common(Carve& c, const Plan& pl)
+// rev: with what the adjoint and the imaging read
+static Common carve_common(Carve& c, const Plan& pl, bool rev)
 {
     Common w{};
     const long long nmS = (long long)pl.nm * pl.P.S;
     w.cf = c.take<float>(nmS);
-    w.ca = c.take<float>(nmS);
-    w.vv = c.take<float>(nmS);
+    if (rev) {
+        w.ca = c.take<float>(nmS);
+        w.vv = c.take<float>(nmS);
+    }
     const long long nkey = (long long)pl.P.B * pl.P.ntx * pl.P.ntz + 1;
     w.src_off = c.take<int32_t>(nkey);
     w.rec_off = c.take<int32_t>(nkey);
@@ -1378,7 +1436,7 @@ static Common carve_common(Carve& c, const Plan& pl)
 static FwdWork carve_fwd(Carve& c, const Plan& pl)
 {
     FwdWork w{};
-    w.c = carve_common(c, pl);
+    w.c = carve_common(c, pl, false);
     const long long n = (long long)pl.P.B * pl.P.S;
     for (auto& p : w.u) p = c.take<float>(n);
     w.psix = c.take<float>(n); w.psiz = c.take<float>(n);
@@ -1392,7 +1450,7 @@ static FwdWork carve_fwd(Carve& c, const Plan& pl)
 static RevWork carve_rev(Carve& c, const Plan& pl, bool illum)
 {
     RevWork w{};
-    w.c = carve_common(c, pl);
+    w.c = carve_common(c, pl, true);
     const long long n = (long long)pl.P.B * pl.P.S;
     for (auto& p : w.l) p = c.take<float>(n);
     for (auto& p : w.aux) p = c.take<float>(n);
@@ -1665,10 +1723,12 @@ static void copy_any(void* dst, const void* src, long long bytes, cudaStream_t s
 void sizes(const sweep_acoustic_desc* d, int mem_mode, int ckpt_every, int64_t* ws, int64_t* tape)
 {
     check_mode(mem_mode, ckpt_every);
-    Plan pl = make_plan(d);
+    Plan pl = make_plan(d, REVERSE);
     set_store(pl, mem_mode);
+    Plan plf = mem_mode == SWEEP_MEM_CHECKPOINT ? pl : make_plan(d, FORWARD);
+    set_store(plf, mem_mode);
     Carve cf(nullptr);
-    carve_fwd(cf, pl);
+    carve_fwd(cf, plf);
     Carve cr(nullptr);
     if (mem_mode == SWEEP_MEM_CHECKPOINT) {
         RevWork rw; FwdWork fw; float* chunk;
@@ -1688,17 +1748,17 @@ void sizes(const sweep_acoustic_desc* d, int mem_mode, int ckpt_every, int64_t* 
 
 void schedule_of(const sweep_acoustic_desc* d, sweep_b200_schedule* out)
 {
-    const Plan pl = make_plan(d);
-    out->shots_fwd = pl.Gf;
+    const Plan pf = make_plan(d, FORWARD), pl = make_plan(d, REVERSE);
+    out->shots_fwd = pf.Gf;
     out->shots_rev = pl.Gr;
     out->z_chunks = 0;
     out->graph_steps = pl.graph_steps;
-    out->tile_y = 0;
+    out->tile_y = pf.P.tz == pl.P.tz ? pl.P.tz : 0;      // 0: each pass by its own line
 }
 
 int64_t forward_only_bytes(const sweep_acoustic_desc* d)
 {
-    Plan pl = make_plan(d);
+    Plan pl = make_plan(d, FORWARD);
     Carve c(nullptr);
     carve_fwd(c, pl);
     return c.off;
@@ -1706,7 +1766,7 @@ int64_t forward_only_bytes(const sweep_acoustic_desc* d)
 
 void stage_sizes(const sweep_acoustic_desc* d, int64_t* nkey, int64_t* nev_src, int64_t* nev_rec)
 {
-    Plan pl = make_plan(d);
+    Plan pl = make_plan(d, FORWARD);
     *nkey = (int64_t)pl.P.B * pl.P.ntx * pl.P.ntz + 1;
     *nev_src = (int64_t)d->B * d->nsrc;
     *nev_rec = (int64_t)d->B * d->nrec;
@@ -1781,7 +1841,7 @@ void forward_with(const sweep_acoustic_desc* d, int mem_mode, int ckpt_every, fl
     SWEEP_REQUIRE(record != nullptr || d->nrec == 0, "acoustic2d forward: null record");
     SWEEP_REQUIRE(d->vp != nullptr, "acoustic2d forward: null vp");
     set_attrs();
-    Plan pl = make_plan(d);
+    Plan pl = make_plan(d, ckpt_every > 0 ? REVERSE : FORWARD);
     set_store(pl, ckpt_every > 0 ? SWEEP_MEM_CHECKPOINT : mem_mode);
     Carve c(ws);
     FwdWork w = carve_fwd(c, pl);
@@ -1972,7 +2032,7 @@ void backward_with(const sweep_acoustic_desc* d, int mem_mode, int ckpt_every, c
     SWEEP_REQUIRE(adj != nullptr || d->nrec == 0, "acoustic2d backward: null record cotangent");
     SWEEP_REQUIRE((illum_s == nullptr) == (illum_r == nullptr), "acoustic2d backward: pass both illuminations or neither");
     set_attrs();
-    Plan pl = make_plan(d);
+    Plan pl = make_plan(d, REVERSE);
     set_store(pl, mem_mode);
     Carve c(ws);
     const bool illum = illum_s != nullptr;

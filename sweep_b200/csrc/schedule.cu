@@ -75,15 +75,16 @@ namespace el2d { void schedule_of(const sweep_elastic_desc* d, sweep_b200_schedu
 
 using namespace sweep;
 
-static void check_schedule(const sweep_b200_schedule* s)
+// flat: the shape is a 2-D acoustic one
+static void check_schedule(const sweep_b200_schedule* s, bool flat)
 {
     SWEEP_REQUIRE(s != nullptr, "null schedule");
     SWEEP_REQUIRE(s->shots_fwd >= 0 && s->shots_fwd <= 16, "schedule: shots_fwd must be 0..16 (got %d)", s->shots_fwd);
     SWEEP_REQUIRE(s->shots_rev >= 0 && s->shots_rev <= 16, "schedule: shots_rev must be 0..16 (got %d)", s->shots_rev);
     SWEEP_REQUIRE(s->z_chunks >= 0 && s->z_chunks <= 64, "schedule: z_chunks must be 0..64 (got %d)", s->z_chunks);
     SWEEP_REQUIRE(s->graph_steps <= 4096, "schedule: graph_steps must be <= 4096 (got %d)", s->graph_steps);
-    SWEEP_REQUIRE(s->tile_y == 0 || s->tile_y == 8 || s->tile_y == 16,
-                  "schedule: tile_y must be 0 (built-in), 8 or 16 (got %d)", s->tile_y);
+    SWEEP_REQUIRE(s->tile_y == 0 || s->tile_y == 8 || s->tile_y == 16 || (flat && s->tile_y == 32),
+                  "schedule: tile_y must be 0 (built-in), 8 or 16%s (got %d)", flat ? " or 32" : "", s->tile_y);
 }
 
 extern "C" int sweep_b200_schedule_set(int32_t family, const void* desc, const sweep_b200_schedule* s,
@@ -91,7 +92,8 @@ extern "C" int sweep_b200_schedule_set(int32_t family, const void* desc, const s
 {
     return guarded(err, err_cap, [&] {
         SWEEP_REQUIRE(desc != nullptr, "null descriptor");
-        check_schedule(s);
+        check_schedule(s, family == SWEEP_FAMILY_ACOUSTIC &&
+                              static_cast<const sweep_acoustic_desc*>(desc)->ndim == 2);
         sweep_b200_schedule v = *s;
         if (v.graph_steps < 0) v.graph_steps = -1;
         if (family == SWEEP_FAMILY_ACOUSTIC) {

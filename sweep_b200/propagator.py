@@ -500,7 +500,7 @@ class PropTorch(torch.nn.Module):
     each problem shape (``sweep_b200.autotune.tune``) and records the fastest
     for every later call of that shape; ``schedule={...}`` records the given
     fields instead (``shots_fwd``, ``shots_rev``, ``z_chunks``,
-    ``graph_steps``).  ``tune_report`` holds the tuner's last report."""
+    ``graph_steps``, ``tile_y``).  ``tune_report`` holds the tuner's last report."""
 
     def __init__(self, equation, shape, dh=10.0, dt=0.002, abcn=50, impl="c", memory=None,
                  device=None, dev=None, source_type=None, receiver_type=None,

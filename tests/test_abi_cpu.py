@@ -295,6 +295,24 @@ def test_schedule_table_is_host_only_and_keyed_by_shape():
     assert autotune.get_schedule(_desc(B=8, nz=120, nx=200)) == base
 
 
+def test_acoustic2d_tile_height_is_the_one_that_runs():
+    """The 2-D acoustic kernels of order 8 follow the grid and the shots, or a
+    recorded tile height: 8 rows those of small grids, 32 the tiled ones."""
+    from sweep_b200 import autotune
+    small, large = _desc(B=8, nz=120, nx=200), _desc(B=32, nz=344, nx=856)
+    autotune.clear_schedules()
+    try:
+        assert autotune.get_schedule(small)["tile_y"] == 8
+        assert autotune.get_schedule(large)["tile_y"] == 32
+        for d in (small, large):
+            for rows in (32, 8):
+                autotune.set_schedule(d, {"tile_y": rows, "shots_rev": 3})
+                got = autotune.get_schedule(d)
+                assert got["tile_y"] == rows and got["shots_rev"] == 3
+    finally:
+        autotune.clear_schedules()
+
+
 def test_recursive_checkpoint_options_and_sizes():
     """Ckpt(mode='recursive', count=N) follows the reference's option rules;
     its tape is a token (nothing is kept from the forward) and its workspace
@@ -550,3 +568,34 @@ def test_vti3d_sizes_and_refusals():
         s.forward_runner(torch.zeros(50), src, rec, models)
     with pytest.raises(NotImplementedError, match="orders 2 to 14"):
         PropTorch(AcousticVTI1st3D(spatial_order=16), shape=shape, abcn=3, device="cpu")
+
+
+# Workspace bytes of calls with 20 receivers a shot: equation, order, grid,
+# shots, CPML cells, a model per shot
+WORKSPACES = [
+    ("Acoustic", 8, (256, 768), 16, 40, False, 279406848), ("Acoustic", 8, (200, 400), 8, 20, False, 65335296),
+    ("Acoustic", 8, (400, 1200), 1, 40, False, 53786880),
+]
+
+
+@pytest.mark.parametrize("eq,order,shape,B,abcn,per_shot,limit", WORKSPACES)
+def test_workspace_stays_within_what_it_was(eq, order, shape, B, abcn, per_shot, limit):
+    """A caller near the device's memory is served as it was with the
+    one-cell-per-thread kernels, but for the tables of the sources' and
+    receivers' tiles (at most 256 KB)."""
+    import torch
+    import sweep_b200 as sb
+    from sweep_b200 import _lib
+    nd = len(shape)
+    s = sb.PropTorch(getattr(sb, eq)(spatial_order=order), shape=shape, dh=10.0, dt=5e-4, abcn=abcn, device="cpu")
+    models = {"Acoustic": 1, "Elastic": 3}.get(eq.removesuffix("3D"), 4)
+    src, rec = np.full((B, nd), 3), np.full((B, 20, nd), 4)
+    geo, padded, wb, fields = s._probe(50, src, rec, [torch.ones((1,) * nd).expand(shape)] * models)
+    d = s._desc(geo, padded, wb, fields)
+    if per_shot:
+        setattr(d, "vp_stride" if models == 1 else "model_stride", int(np.prod(s.runtime_shape)))
+    name = {"Acoustic": "acoustic", "Acoustic3D": "acoustic", "Elastic": "elastic", "Elastic3D": "elastic3d",
+            "AcousticVTI1st": "vti", "AcousticVTI1st3D": "vti3d"}[eq]
+    ws, tape = _lib.c_i64(), _lib.c_i64()
+    _lib.call(f"sweep_b200_{name}_sizes", d, _lib.MEM_BOUNDARY, 0, ws, tape)
+    assert ws.value <= limit + 2 ** 18
