@@ -1295,16 +1295,33 @@ static int choose_group(int built_in, int B, const char* env, int recorded)
     return built_in;
 }
 
-// Few tiles: a step of the tiled kernels lasts as long as one CTA, which
-// walks its shots' tiles through its stages eight cells per thread, so these
-// grids run four cells per thread on 32 x 8 tiles.  The line is where the
-// fields of a step leave the L2, which the tiled kernels' reuse over shots
-// then saves: gradients of 200 steps, small / tiled, 96 x 128 one shot
-// (15 tiles) 2.7 / 6.8 ms, 200 x 400 x 8 shots (512) 8.3 / 11.2,
-// 256 x 768 x 8 (1232) 14.1 / 29.5, x 12 (1848) 22.7 / 34.6, x 16 (2464)
-// 31.0 / 37.3, x 32 (4928) 63 / 51.6, 400 x 1200 x 8 (2480) 33.1 / 36.6.
+// Which kernels run a pass.  A step of the tiled kernels lasts as long as a
+// CTA's walk through its shots' tiles and its stages, eight cells per thread,
+// times the waves of the `ctas` CTAs; the small-grid kernels spread the same
+// cells over eight times the CTAs, four cells per thread, and re-read the taps
+// that a tile shares.  So the tiled ones win once they fill several waves.
+// Small / tiled, ms of 200 steps (40 CPML cells a side; tiles: 64 x 32, all shots):
+//   records    256 x 768 x 8 shots 616 CTAs 4.4 / 6.3, x 13 1078 6.5 / 6.8, x 14
+//              1078 7.1 / 7.0, x 15 1232 7.9 / 7.7; 400 x 1200 x 7 1344 7.6 / 7.4;
+//              one shot of 1000 x 1800 1020 3.8 / 3.8, of 1400 x 2800 2162 6.9 / 5.9
+//   gradients  256 x 768 x 8 308 CTAs 14.8 / 30.3, x 16 308 27.9 / 38.0; 600 x 1400 x 3
+//              528 17.7 / 21.1; 700 x 1400 x 4 600 26.3 / 26.3; 800 x 1600 x 2 756
+//              18.2 / 18.4, x 3 756 25.6 / 23.6; 256 x 768 x 32 616 54.5 / 51.4
+// With one shot per CTA the reverse's tiled kernel has no next shot whose loads
+// it could overlap: 900 x 1400 744 CTAs 10.0 / 10.9, 1000 x 1800 1020 14.3 / 13.1,
+// with a model per shot 400 x 1200 x 2 672 8.9 / 11.2, 700 x 1400 x 2 1200 16.7 / 15.8.
+// Where the layers are more than half of the grid, whose cells cost the tiled
+// kernels most, the small ones stay ahead: 60 x 90 x 180 2700 tiles 13.7 / 16.3
+// and 37.0 / 53.5, per-shot 96 x 128 x 60 1440 tiles 5.4 / 7.0 and 19.9 / 25.9.
 constexpr long long kSmallTiles = 2960;     // all shots
-static bool small_kernels(const Params& P, Pass, int ntiles) { return (long long)ntiles * P.B <= kSmallTiles; }
+static bool small_kernels(const Params& P, Pass pass, int ntiles)
+{
+    if ((long long)ntiles * P.B > kSmallTiles) return false;
+    const bool thick = 2LL * (P.z1 - P.z0) * (P.x1 - P.x0) < (long long)P.nz * P.nx;
+    const int g = P.per_shot ? 1 : built_in_group(ntiles, P.B, pass == FORWARD ? 2 : 8);
+    const long long ctas = (long long)ntiles * ((P.B + g - 1) / g);
+    return thick || ctas <= (pass == FORWARD ? 1100 : g == 1 ? 800 : 610);
+}
 
 static Plan make_plan(const sweep_acoustic_desc* d, Pass pass)
 {

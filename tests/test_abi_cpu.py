@@ -313,6 +313,23 @@ def test_acoustic2d_tile_height_is_the_one_that_runs():
         autotune.clear_schedules()
 
 
+@pytest.mark.parametrize("B,nz,nx,pad,per_shot,rows", [
+    (1, 184, 216, 40, False, 8), (8, 344, 856, 40, False, 8), (32, 344, 856, 40, False, 32),
+    (16, 344, 856, 40, False, 0),               # records fill several waves of tiles, the image's shot groups do not
+    (1, 788, 1488, 40, False, 8), (1, 1488, 2888, 40, False, 32), (3, 888, 1688, 40, False, 32),
+    (180, 148, 178, 40, False, 8),              # mostly layers
+    (2, 488, 1288, 40, True, 8), (4, 788, 1488, 40, True, 32)])
+def test_acoustic2d_kernels_follow_the_waves_of_tiles(B, nz, nx, pad, per_shot, rows):
+    """The tile height the schedule resolves to; 0 where the passes differ."""
+    from sweep_b200 import autotune
+    d = _desc(B=B, nz=nz, nx=nx)
+    for f in (0, 1, 4, 5):
+        d.pad[f] = pad
+    d.vp_stride = nz * nx if per_shot else 0
+    autotune.clear_schedules()
+    assert autotune.get_schedule(d)["tile_y"] == rows
+
+
 def test_recursive_checkpoint_options_and_sizes():
     """Ckpt(mode='recursive', count=N) follows the reference's option rules;
     its tape is a token (nothing is kept from the forward) and its workspace
