@@ -85,6 +85,18 @@ struct Carve {
     }
 };
 
+// Rows of `width` floats between two row pitches (in floats): a tape's states
+// hold the grid's cells alone, without their rows' pitch.
+inline void copy_rows(float* dst, long long dst_pitch, const float* src, long long src_pitch, long long width,
+                      long long rows, cudaStream_t st)
+{
+    if (dst_pitch == width && src_pitch == width)
+        SWEEP_CUDA(cudaMemcpyAsync(dst, src, (size_t)(width * rows) * 4, cudaMemcpyDefault, st));
+    else
+        SWEEP_CUDA(cudaMemcpy2DAsync(dst, (size_t)dst_pitch * 4, src, (size_t)src_pitch * 4, (size_t)width * 4,
+                                     (size_t)rows, cudaMemcpyDefault, st));
+}
+
 // Boundary-saving tape in pinned host memory (reference
 // BoundarySaving(storage='cpu'), boundary/runtime.cuh:91-620): the step
 // kernels write a ring of R device slots; a copy stream moves forward slot it

@@ -23,19 +23,19 @@
 // The reverse step is two kernels.  Half-step A needs D- of the forward
 // velocities for the reconstruction and for the stiffness gradient and takes
 // p at its taps straight from lambda_s; half-step B does the same with the
-// stresses, q and the 1 / rho gradient.  Neither p nor q goes through memory
-// (seven kernels and three scratch fields before), so the CPML memories of
-// the adjoint are double-buffered: a cell's neighbours read them while its
-// owner writes the next ones.  The gradient is summed as e = c11 lsH dh + c33
-// lsV dvz + c13 (lsH dvz + lsV dh), lsH dh, lsH dvz + lsV dh and e -
-// lambda_v . grad s / rho (terms that cancel are combined in each step, in
-// one slot); the models' chain rule is applied once, at the end.  Shots that share a model run in groups
-// inside a thread, which reads the stiffness and updates the gradient slots
-// once per group.
+// stresses, q and the 1 / rho gradient, and lambda_v is held as q = lambda_v /
+// rho.  Nothing goes through memory in between (seven kernels and three scratch
+// fields before), so the CPML memories of the adjoint are double-buffered: a
+// cell's neighbours read them while its owner writes the next ones.  The
+// gradient is summed as e = c11 lsH dh + c33 lsV dvz + c13 (lsH dvz + lsV dh),
+// lsH dh, lsH dvz + lsV dh and e - lambda_v . grad s / rho (terms that cancel
+// are combined in each step, in one slot); the models' chain rule is applied
+// once, at the end.  Shots that share a model run in groups inside a thread,
+// which reads the stiffness and updates the gradient slots once per group.
 //
 // Four x cells per thread (vec4.cuh) on pitched rows; a warp covers 32 x 4
-// (x, y) cells in 3-D and 32 x 4 (x, z) cells in 2-D.  A memory is read and
-// written only where its axis has a damping profile (elsewhere it stays zero).
+// (x, y) cells in 3-D and 32 x 4 (x, z) cells in 2-D.  A memory holds the cells
+// where its axis has a damping profile.
 //
 // Bound by field traffic in the forward (velocity step of the 4-shot 128^3
 // survey: 17.6 M cells, 132 us, 289 us with one cell per thread, 100 us of
@@ -78,6 +78,7 @@ struct Geo {
     int P, SY, SZ;                  // row pitch, y stride (= P), z stride
     long long S;                    // shot stride
     int z0, z1, y0, y1, x0, x1;     // physical box
+    int ms0[3], cut[3], wm[3];      // memory slabs by axis: first cell of the high side, cells left out, width
     int nbx;                        // x blocks
     int group, nslot;               // shots per reverse thread, gradient slots
     float dt, ihz, ihy, ihx;
@@ -159,11 +160,28 @@ __device__ __forceinline__ bool band_x(const Geo& G, int x, bool half)
     return x < G.x0 || x + 3 >= G.x1 - (half ? 1 : 0);
 }
 
+// Memories: along x (B, nz, ny, wm[0]) in whole groups of four cells, along y
+// (B, nz, wm[1], P), along z (B, wm[2], ny, P): the layers of the axis and the
+// cells inside them that the taps of a thread near them reach, so that its taps
+// lie beside its own place.  Offset of a group near the layers.
+template <int ND>
+__device__ __forceinline__ long long xmem(const Geo& G, int b, int z, int y, int x)
+{
+    return (((long long)b * G.nz + z) * (ND == 3 ? G.ny : 1) + y) * G.wm[0] + x - (x >= G.ms0[0] ? G.cut[0] : 0);
+}
+__device__ __forceinline__ long long ymem(const Geo& G, int b, int z, int y, int x)
+{
+    return (((long long)b * G.nz + z) * G.wm[1] + y - (y >= G.ms0[1] ? G.cut[1] : 0)) * G.P + x;
+}
+__device__ __forceinline__ long long zmem(const Geo& G, int b, int z, int y, int x)
+{
+    return ((long long)b * G.wm[2] + z - (z >= G.ms0[2] ? G.cut[2] : 0)) * G.SZ + y * G.SY + x;
+}
+
 // the CPML memories of the ND derivatives d[0..ND) (x[, y], z) of a forward
 // step, memories w[m0 ..], profiles at half or integer positions
 template <int ND, bool HALF>
-__device__ __forceinline__ void damp_all(const Geo& G, const Cell<ND>& q, F4 (&d)[ND], const Fields& W, int m0,
-                                         long long k)
+__device__ __forceinline__ void damp_all(const Geo& G, const Cell<ND>& q, F4 (&d)[ND], const Fields& W, int m0)
 {
     const bool rin = q.row_in(G);
     if (rin && q.x >= G.x0 && q.x + 3 < G.x1) return;
@@ -171,13 +189,14 @@ __device__ __forceinline__ void damp_all(const Geo& G, const Cell<ND>& q, F4 (&d
 #pragma unroll
     for (int l = 0; l < 4; ++l) out[l] = q.lane_core(G, l) && !(rin && x_in(G, q.x + l));
     if (band_x(G, q.x, HALF))
-        damp(d[0], W.f[m0] + k, v4::ldg((HALF ? G.ah[0] : G.a[0]) + q.x), v4::ldg((HALF ? G.bh[0] : G.b[0]) + q.x), out);
+        damp(d[0], W.f[m0] + xmem<ND>(G, q.b, q.z, q.y, q.x), v4::ldg((HALF ? G.ah[0] : G.a[0]) + q.x),
+             v4::ldg((HALF ? G.bh[0] : G.b[0]) + q.x), out);
     if (ND == 3 && band(q.y, G.y0, G.y1, HALF))
-        damp(d[1], W.f[m0 + 1] + k, v4::splat(__ldg((HALF ? G.ah[1] : G.a[1]) + q.y)),
+        damp(d[1], W.f[m0 + 1] + ymem(G, q.b, q.z, q.y, q.x), v4::splat(__ldg((HALF ? G.ah[1] : G.a[1]) + q.y)),
              v4::splat(__ldg((HALF ? G.bh[1] : G.b[1]) + q.y)), out);
     if (band(q.z, G.z0, G.z1, HALF))
-        damp(d[ND - 1], W.f[m0 + ND - 1] + k, v4::splat(__ldg((HALF ? G.ah[2] : G.a[2]) + q.z)),
-             v4::splat(__ldg((HALF ? G.bh[2] : G.b[2]) + q.z)), out);
+        damp(d[ND - 1], W.f[m0 + ND - 1] + zmem(G, q.b, q.z, q.y, q.x),
+             v4::splat(__ldg((HALF ? G.ah[2] : G.a[2]) + q.z)), v4::splat(__ldg((HALF ? G.bh[2] : G.b[2]) + q.z)), out);
 }
 
 constexpr int kThreads = 256;
@@ -198,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) vel(const Geo G, const F
     F4 v[ND];
 #pragma unroll
     for (int a = 0; a < ND; ++a) v[a] = v4::ld(F.f[a] + k);
-    damp_all<ND, true>(G, q, d, W, 0, k);
+    damp_all<ND, true>(G, q, d, W, 0);
 #pragma unroll
     for (int a = 0; a < ND; ++a) {
 #pragma unroll
@@ -222,7 +241,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) str(const Geo G, const F
     d[ND - 1] = v4::diff_col<M, false>(F.f[L::VZ] + k, G.SZ, G.c, G.ihz);
     const F4 c11 = v4::ldg(G.cm[C11] + mi), c33 = v4::ldg(G.cm[C33] + mi), c13 = v4::ldg(G.cm[C13] + mi);
     F4 sh = v4::ld(F.f[L::SH] + k), sv = v4::ld(F.f[L::SV] + k);
-    damp_all<ND, false>(G, q, d, W, ND, k);
+    damp_all<ND, false>(G, q, d, W, ND);
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
         if (!q.lane_core(G, l)) continue;
@@ -251,7 +270,8 @@ __device__ __forceinline__ void add(float* p, const F4& a)
 __device__ __forceinline__ float up(float p, float b, float w) { return p + b * (w + p); }
 
 // Reverse half-step A: stress reconstruction (box minus one cell), the
-// stiffness products of the gradient (box), lambda_v += -dt D+ p (core).
+// stiffness products of the gradient (box), lambda_v += -dt D+ p, held as q =
+// lambda_v / rho (core).
 // Wi / Wo: the adjoint memories of the stress step, read / written.
 template <int M, int ND>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) half_a(const Geo G, const Fields F, const Fields A, const Fields Wi,
@@ -306,6 +326,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) half_a(const Geo G, cons
         }
         {
             float p[S::N];
+            const long long m = xmem<ND>(G, b, q.z, q.y, q.x);
 #pragma unroll
             for (int j = -S::LO; j <= S::HI; ++j) {
                 F4 t = ph0;
@@ -316,13 +337,13 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) half_a(const Geo G, cons
                     for (int l = 0; l < 4; ++l) t.v[l] = e.v[l] * h.v[l] + f.v[l] * v.v[l];
                 }
                 if (bx) {
-                    const F4 pb = v4::ldg(G.b[0] + q.x + 4 * j), w = v4::ldg(Wi.f[ND] + k + 4 * j);
+                    const F4 pb = v4::ldg(G.b[0] + q.x + 4 * j), w = v4::ldg(Wi.f[ND] + m + 4 * j);
                     if (j == 0) {
                         const F4 pa = v4::ldg(G.a[0] + q.x);
                         F4 nw;
 #pragma unroll
                         for (int l = 0; l < 4; ++l) nw.v[l] = pa.v[l] * (w.v[l] + t.v[l]);
-                        if (band_x(G, q.x, false)) v4::st(Wo.f[ND] + k, nw);
+                        if (band_x(G, q.x, false)) v4::st(Wo.f[ND] + m, nw);
                     }
 #pragma unroll
                     for (int l = 0; l < 4; ++l)
@@ -336,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) half_a(const Geo G, cons
         // a row tap along an axis: p there, and within the band's reach (`near`)
         // through its memory -- a tap off the band with the profile's zero, so
         // that a thread's loads leave together
-        auto tap = [&](int off, int c, const float* prof, int mem, const float* ca, const float* cb, F4 own,
+        auto tap = [&](int off, int c, const float* prof, const float* mem, const float* ca, const float* cb, F4 own,
                        bool centre, bool near) {
             F4 t = own;
             if (!centre) {
@@ -346,46 +367,52 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) half_a(const Geo G, cons
             }
             if (near) {
                 const float pb = __ldg(prof + c);
-                const F4 w = v4::ldg(Wi.f[mem] + k + off);
+                const F4 w = v4::ldg(mem);
 #pragma unroll
                 for (int l = 0; l < 4; ++l) t.v[l] = up(t.v[l], pb, w.v[l]);
             }
             return t;
         };
-        auto rows = [&](int stride, int c, const float* prof, int mem, const float* ca, const float* cb, const F4& own,
+        auto rows = [&](int stride, int c, const float* prof, auto place, const float* ca, const float* cb, const F4& own,
                         bool near, float inv) {
-            if (near)
+            if (near) {
+                const float* mem = place();
                 return v4::diff<M, true>(
-                    [&](int j) { return tap(j * stride, c + j, prof, mem, ca, cb, own, j == 0, true); }, G.c, inv);
+                    [&](int j) { return tap(j * stride, c + j, prof, mem + j * stride, ca, cb, own, j == 0, true); }, G.c,
+                    inv);
+            }
             return v4::diff<M, true>(
-                [&](int j) { return tap(j * stride, c + j, prof, mem, ca, cb, own, j == 0, false); }, G.c, inv);
+                [&](int j) { return tap(j * stride, c + j, prof, nullptr, ca, cb, own, j == 0, false); }, G.c, inv);
         };
         if (ND == 3) {
-            d[1] = rows(G.SY, q.y, G.b[1], ND + 1, c11, c13, ph0, band(q.y - (M - 1), G.y0, G.y1, false) ||
-                        band(q.y + M, G.y0, G.y1, false), G.ihy);
+            d[1] = rows(G.SY, q.y, G.b[1], [&] { return Wi.f[ND + 1] + ymem(G, b, q.z, q.y, q.x); }, c11, c13, ph0,
+                        band(q.y - (M - 1), G.y0, G.y1, false) || band(q.y + M, G.y0, G.y1, false), G.ihy);
             if (band(q.y, G.y0, G.y1, false)) {
                 const float pa = __ldg(G.a[1] + q.y);
-                F4 w = v4::ldg(Wi.f[ND + 1] + k);
+                const long long o = ymem(G, b, q.z, q.y, q.x);
+                F4 w = v4::ldg(Wi.f[ND + 1] + o);
 #pragma unroll
                 for (int l = 0; l < 4; ++l) w.v[l] = q.lane_core(G, l) ? pa * (w.v[l] + ph0.v[l]) : 0.f;
-                v4::st(Wo.f[ND + 1] + k, w);
+                v4::st(Wo.f[ND + 1] + o, w);
             }
         }
-        d[ND - 1] = rows(G.SZ, q.z, G.b[2], 2 * ND - 1, c13, c33, pv0,
+        d[ND - 1] = rows(G.SZ, q.z, G.b[2], [&] { return Wi.f[2 * ND - 1] + zmem(G, b, q.z, q.y, q.x); }, c13, c33, pv0,
                          band(q.z - (M - 1), G.z0, G.z1, false) || band(q.z + M, G.z0, G.z1, false), G.ihz);
         if (band(q.z, G.z0, G.z1, false)) {
             const float pa = __ldg(G.a[2] + q.z);
-            F4 w = v4::ldg(Wi.f[2 * ND - 1] + k);
+            const long long o = zmem(G, b, q.z, q.y, q.x);
+            F4 w = v4::ldg(Wi.f[2 * ND - 1] + o);
 #pragma unroll
             for (int l = 0; l < 4; ++l) w.v[l] = q.lane_core(G, l) ? pa * (w.v[l] + pv0.v[l]) : 0.f;
-            v4::st(Wo.f[2 * ND - 1] + k, w);
+            v4::st(Wo.f[2 * ND - 1] + o, w);
         }
+        const F4 ir = v4::ldg(G.cm[IRHO] + b * G.ms + q.i);
 #pragma unroll
         for (int a = 0; a < ND; ++a) {
             F4 v = v4::ld(A.f[a] + k);
 #pragma unroll
             for (int l = 0; l < 4; ++l)
-                if (q.lane_core(G, l)) v.v[l] += -G.dt * d[a].v[l];
+                if (q.lane_core(G, l)) v.v[l] += (-G.dt * ir.v[l]) * d[a].v[l];
             v4::st(A.f[a] + k, v);
         }
     }
@@ -416,11 +443,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) half_b(const Geo G, cons
     F4 gr = v4::splat(0.f);
     for (int b = b0; b < b1; ++b) {
         const long long k = b * G.S + q.i;
-        const float* ir = G.cm[IRHO] + b * G.ms + q.i;
-        const F4 r0 = v4::ldg(ir);
-        F4 lv[ND];
+        F4 q0[ND];
 #pragma unroll
-        for (int a = 0; a < ND; ++a) lv[a] = v4::ldg(A.f[a] + k);
+        for (int a = 0; a < ND; ++a) q0[a] = v4::ldg(A.f[a] + k);
         if (img) {
             F4 d[ND];
             d[0] = v4::diff_row<M, true>(F.f[L::SH] + k, G.c, G.ihx);
@@ -429,12 +454,13 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) half_b(const Geo G, cons
 #pragma unroll
             for (int l = 0; l < 4; ++l) {
                 if (!x_in(G, q.x + l)) continue;
-                float s = lv[0].v[l] * d[0].v[l];
+                float s = q0[0].v[l] * d[0].v[l];
 #pragma unroll
-                for (int a = 1; a < ND; ++a) s += lv[a].v[l] * d[a].v[l];
-                gr.v[l] -= r0.v[l] * s;
+                for (int a = 1; a < ND; ++a) s += q0[a].v[l] * d[a].v[l];
+                gr.v[l] -= s;
             }
             if (rrev) {
+                const F4 r0 = v4::ldg(G.cm[IRHO] + b * G.ms + q.i);
 #pragma unroll
                 for (int a = 0; a < ND; ++a) {
                     F4 v = v4::ld(F.f[a] + k);
@@ -445,30 +471,22 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) half_b(const Geo G, cons
                 }
             }
         }
-        F4 d[ND], q0[ND];
-#pragma unroll
-        for (int a = 0; a < ND; ++a)
-#pragma unroll
-            for (int l = 0; l < 4; ++l) q0[a].v[l] = r0.v[l] * lv[a].v[l];
+        F4 d[ND];
         {
             float p[S::N];
+            const long long m = xmem<ND>(G, b, q.z, q.y, q.x);
 #pragma unroll
             for (int j = -S::LO; j <= S::HI; ++j) {
-                F4 t = q0[0];
-                if (j != 0) {
-                    const F4 r = v4::ldg(ir + 4 * j), v = v4::ldg(A.f[0] + k + 4 * j);
-#pragma unroll
-                    for (int l = 0; l < 4; ++l) t.v[l] = r.v[l] * v.v[l];
-                }
+                F4 t = j == 0 ? q0[0] : v4::ldg(A.f[0] + k + 4 * j);
                 if (bx) {
-                    const F4 pb = v4::ldg(G.bh[0] + q.x + 4 * j), w = v4::ldg(Wi.f[0] + k + 4 * j);
+                    const F4 pb = v4::ldg(G.bh[0] + q.x + 4 * j), w = v4::ldg(Wi.f[0] + m + 4 * j);
                     if (j == 0 && band_x(G, q.x, true)) {
                         const F4 pa = v4::ldg(G.ah[0] + q.x);
                         F4 nw;
 #pragma unroll
                         for (int l = 0; l < 4; ++l)
                             nw.v[l] = rin && x_in(G, q.x + l) ? 0.f : pa.v[l] * (w.v[l] + t.v[l]);
-                        v4::st(Wo.f[0] + k, nw);
+                        v4::st(Wo.f[0] + m, nw);
                     }
 #pragma unroll
                     for (int l = 0; l < 4; ++l)
@@ -481,43 +499,38 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) half_b(const Geo G, cons
         }
         // a row tap along y or z (see half_a); in: the row at c + j and the other
         // of y and z lie in the box, where the memory runs outside it along x only
-        auto rows = [&](int stride, int c, int c0, int c1, bool oin, const float* prof, int mem, const float* lam,
+        auto rows = [&](int stride, int c, int c0, int c1, bool oin, const float* prof, auto place, const float* lam,
                         const F4& own, float inv) {
-            auto value = [&](int j) {
-                F4 t = own;
-                if (j != 0) {
-                    const F4 r = v4::ldg(ir + j * stride), v = v4::ldg(lam + j * stride);
-#pragma unroll
-                    for (int l = 0; l < 4; ++l) t.v[l] = r.v[l] * v.v[l];
-                }
-                return t;
-            };
+            auto value = [&](int j) { return j == 0 ? own : v4::ldg(lam + j * stride); };
             if (!band(c - M, c0, c1, true) && !band(c + M - 1, c0, c1, true)) return v4::diff<M, false>(value, G.c, inv);
+            const float* mem = place();
             return v4::diff<M, false>(
                 [&](int j) {
                     F4 t = value(j);
                     const bool in = oin && c + j >= c0 && c + j < c1;
                     const float pb = __ldg(prof + c + j);
-                    const F4 w = v4::ldg(Wi.f[mem] + k + j * stride);
+                    const F4 w = v4::ldg(mem + j * stride);
 #pragma unroll
                     for (int l = 0; l < 4; ++l) t.v[l] = up(t.v[l], in && x_in(G, q.x + l) ? 0.f : pb, w.v[l]);
                     return t;
                 },
                 G.c, inv);
         };
-        auto keep = [&](int mem, float pa, const F4& own) {
-            F4 w = v4::ldg(Wi.f[mem] + k);
+        auto keep = [&](int mem, long long o, float pa, const F4& own) {
+            F4 w = v4::ldg(Wi.f[mem] + o);
 #pragma unroll
             for (int l = 0; l < 4; ++l)
                 w.v[l] = q.lane_core(G, l) && !(rin && x_in(G, q.x + l)) ? pa * (w.v[l] + own.v[l]) : 0.f;
-            v4::st(Wo.f[mem] + k, w);
+            v4::st(Wo.f[mem] + o, w);
         };
         if (ND == 3) {
-            d[1] = rows(G.SY, q.y, G.y0, G.y1, zin, G.bh[1], 1, A.f[1] + k, q0[1], G.ihy);
-            if (band(q.y, G.y0, G.y1, true)) keep(1, __ldg(G.ah[1] + q.y), q0[1]);
+            d[1] = rows(G.SY, q.y, G.y0, G.y1, zin, G.bh[1], [&] { return Wi.f[1] + ymem(G, b, q.z, q.y, q.x); },
+                        A.f[1] + k, q0[1], G.ihy);
+            if (band(q.y, G.y0, G.y1, true)) keep(1, ymem(G, b, q.z, q.y, q.x), __ldg(G.ah[1] + q.y), q0[1]);
         }
-        d[ND - 1] = rows(G.SZ, q.z, G.z0, G.z1, yin, G.bh[2], ND - 1, A.f[L::VZ] + k, q0[ND - 1], G.ihz);
-        if (band(q.z, G.z0, G.z1, true)) keep(ND - 1, __ldg(G.ah[2] + q.z), q0[ND - 1]);
+        d[ND - 1] = rows(G.SZ, q.z, G.z0, G.z1, yin, G.bh[2],
+                         [&] { return Wi.f[ND - 1] + zmem(G, b, q.z, q.y, q.x); }, A.f[L::VZ] + k, q0[ND - 1], G.ihz);
+        if (band(q.z, G.z0, G.z1, true)) keep(ND - 1, zmem(G, b, q.z, q.y, q.x), __ldg(G.ah[2] + q.z), q0[ND - 1]);
         F4 sh = v4::ld(A.f[L::SH] + k), sv = v4::ld(A.f[L::SV] + k);
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
@@ -562,7 +575,7 @@ __global__ void inject(const Geo G, const Fields F, int it)
 }
 
 // reverse: the source of step it taken out of F, the residuals (unsigned)
-// into the adjoint fields
+// into the adjoint fields (the velocities' as q)
 template <int ND>
 __global__ void events(const Geo G, const Fields F, const Fields A, const float* __restrict__ adj, int it)
 {
@@ -574,7 +587,10 @@ __global__ void events(const Geo G, const Fields F, const Fields A, const float*
     const int c = loc<ND>(G, G.rec + (long long)ND * e);
     if (c < 0) return;
     const float* res = adj + (((long long)b * G.nt + it) * G.nrec + r) * G.nrf;
-    for (int k = 0; k < G.nrf; ++k) atomicAdd(A.f[G.rf[k]] + b * G.S + c, res[k]);
+    for (int k = 0; k < G.nrf; ++k) {
+        const int f = G.rf[k];
+        atomicAdd(A.f[f] + b * G.S + c, f < Lay<ND>::SH ? G.cm[IRHO][b * G.ms + c] * res[k] : res[k]);
+    }
 }
 
 // forward: record[b, it, r, k] = field rf[k] at receiver r (slot and record
@@ -779,6 +795,17 @@ Plan make_plan(const Desc& d, int mem_mode, const char* name)
     G.nsrc = d.nsrc; G.nrec = d.nrec; G.nsf = d.nsf; G.nrf = d.nrf;
     for (int k = 0; k < NF; ++k) { G.sf[k] = d.sf[k]; G.rf[k] = d.rf[k]; }
     G.src = d.src; G.rec = d.rec; G.wavelet = d.wavelet;
+    // a thread within M cells of the layers reads memories up to M cells (along
+    // x: the groups of those) further in
+    auto slab = [&](int a, int c0, int c1, int n, int reach, int unit) {
+        const int low = (c0 + reach + unit - 1) / unit * unit, high = std::max(0, c1 - 1 - reach) / unit * unit;
+        G.ms0[a] = high;
+        G.cut[a] = std::max(0, high - low);
+        G.wm[a] = (n + unit - 1) / unit * unit - G.cut[a];
+    };
+    slab(0, G.x0, G.x1, G.nx, M + 4 * v4::groups(M) + 4, 4);
+    slab(1, G.y0, G.y1, G.ny, 2 * M, 1);
+    slab(2, G.z0, G.z1, G.nz, 2 * M, 1);
     G.nbx = (G.nx + 31) / 32;
     // shots per reverse thread: as many as still leave four blocks per SM;
     // one for per-shot models
@@ -803,6 +830,16 @@ struct Ws {
     char *zero0, *zero1;
 };
 
+// memory k: x[, y], z of the stress derivatives, then of the velocities'
+template <int ND>
+long long mem_floats(const Geo& G, int k)
+{
+    const int a = k % ND;
+    return a == 0        ? (long long)G.B * G.nz * G.ny * G.wm[0]
+           : a == ND - 1 ? (long long)G.B * G.wm[2] * G.SZ
+                         : (long long)G.B * G.nz * G.wm[1] * G.P;
+}
+
 template <int ND>
 void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
 {
@@ -818,7 +855,7 @@ void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
     w.zero0 = c.base ? c.base + c.off : nullptr;
     for (int k = 0; k < L::NF; ++k) w.f[k] = c.take<float>(n);
     for (int s = 0; s < (rev ? 2 : 1); ++s)
-        for (int k = 0; k < L::NMEM; ++k) w.m[s][k] = c.take<float>(n);
+        for (int k = 0; k < L::NMEM; ++k) w.m[s][k] = c.take<float>(mem_floats<ND>(G, k));
     if (rev) {
         for (int k = 0; k < L::NF; ++k) w.a[k] = c.take<float>(n);
         for (float*& p : w.g) p = c.take<float>(G.nslot * G.S);
@@ -830,6 +867,9 @@ void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
 template <int ND>
 long long slot_floats(const Plan& pl) { return (long long)pl.G.B * Lay<ND>::NF * pl.G.ns; }
 
+// rows of a field of every shot
+inline long long rows_of(const Geo& G) { return (long long)G.B * G.nz * G.ny; }
+
 template <int ND>
 void sizes(const Plan& pl, int64_t* ws_bytes, int64_t* tape_bytes)
 {
@@ -838,7 +878,7 @@ void sizes(const Plan& pl, int64_t* ws_bytes, int64_t* tape_bytes)
     carve<ND>(f, pl, false, w);
     carve<ND>(r, pl, true, w);
     *ws_bytes = std::max(f.off, r.off);
-    *tape_bytes = ((long long)pl.G.nt * slot_floats<ND>(pl) + (long long)Lay<ND>::NF * pl.G.B * pl.G.S) * 4;
+    *tape_bytes = ((long long)pl.G.nt * slot_floats<ND>(pl) + Lay<ND>::NF * rows_of(pl.G) * pl.G.nx) * 4;
 }
 
 inline unsigned blocks(long long n) { return (unsigned)std::max<long long>((n + 255) / 256, 1); }
@@ -909,9 +949,7 @@ void forward(const Desc& d, Plan& pl, float* record, void* tape, void* ws, int64
     sg.flush();
     if (tp) {
         float* last = tp + (long long)G.nt * slot_floats<ND>(pl);
-        const long long n = (long long)G.B * G.S;
-        for (int f = 0; f < L::NF; ++f)
-            SWEEP_CUDA(cudaMemcpyAsync(last + f * n, w.f[f], sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+        for (int f = 0; f < L::NF; ++f) copy_rows(last + f * rows_of(G) * G.nx, G.nx, w.f[f], G.P, G.nx, rows_of(G), st);
     }
 }
 
@@ -930,9 +968,7 @@ void backward(const Desc& d, Plan& pl, const float* adj, const void* tape, const
     const Geo& G = pl.G;
     const float* tp = static_cast<const float*>(tape);
     const float* last = tp + (long long)G.nt * slot_floats<ND>(pl);
-    const long long n = (long long)G.B * G.S;
-    for (int f = 0; f < L::NF; ++f)
-        SWEEP_CUDA(cudaMemcpyAsync(w.f[f], last + f * n, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+    for (int f = 0; f < L::NF; ++f) copy_rows(w.f[f], G.P, last + f * rows_of(G) * G.nx, G.nx, G.nx, rows_of(G), st);
     Fields F{}, A{}, W[2]{};
     for (int k = 0; k < L::NF; ++k) { F.f[k] = w.f[k]; A.f[k] = w.a[k]; }
     for (int k = 0; k < L::NMEM; ++k) { W[0].f[k] = w.m[0][k]; W[1].f[k] = w.m[1][k]; }

@@ -587,16 +587,21 @@ def test_vti3d_sizes_and_refusals():
         PropTorch(AcousticVTI1st3D(spatial_order=16), shape=shape, abcn=3, device="cpu")
 
 
-# Workspace bytes of calls with 20 receivers a shot: equation, order, grid,
-# shots, CPML cells, a model per shot
+# Workspace and tape bytes of calls of 50 steps with 20 receivers a shot:
+# equation, order, grid, shots, CPML cells, a model per shot
 WORKSPACES = [
-    ("Acoustic", 8, (256, 768), 16, 40, False, 279406848), ("Acoustic", 8, (200, 400), 8, 20, False, 65335296),
-    ("Acoustic", 8, (400, 1200), 1, 40, False, 53786880),
+    ("Acoustic", 8, (256, 768), 16, 40, False, 279406848, 70491648),
+    ("Acoustic", 8, (200, 400), 8, 20, False, 65335296, 16557056),
+    ("Acoustic", 8, (400, 1200), 1, 40, False, 53786880, 8309248),
+    ("AcousticVTI1st", 4, (400, 1200), 16, 40, True, 875048448, 281972736),
+    ("AcousticVTI1st", 8, (400, 1200), 16, 40, False, 734203392, 365707264),
+    ("AcousticVTI1st3D", 4, (128, 128, 128), 1, 16, False, 477555712, 381602880),
+    ("AcousticVTI1st3D", 4, (128, 128, 128), 4, 16, True, 1906701568, 1526411520),
 ]
 
 
-@pytest.mark.parametrize("eq,order,shape,B,abcn,per_shot,limit", WORKSPACES)
-def test_workspace_stays_within_what_it_was(eq, order, shape, B, abcn, per_shot, limit):
+@pytest.mark.parametrize("eq,order,shape,B,abcn,per_shot,limit,tape_limit", WORKSPACES)
+def test_workspace_stays_within_what_it_was(eq, order, shape, B, abcn, per_shot, limit, tape_limit):
     """A caller near the device's memory is served as it was with the
     one-cell-per-thread kernels, but for the tables of the sources' and
     receivers' tiles (at most 256 KB)."""
@@ -616,3 +621,4 @@ def test_workspace_stays_within_what_it_was(eq, order, shape, B, abcn, per_shot,
     ws, tape = _lib.c_i64(), _lib.c_i64()
     _lib.call(f"sweep_b200_{name}_sizes", d, _lib.MEM_BOUNDARY, 0, ws, tape)
     assert ws.value <= limit + 2 ** 18
+    assert tape.value <= tape_limit
