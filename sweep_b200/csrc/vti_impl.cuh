@@ -28,10 +28,11 @@
 // fields before), so the CPML memories of the adjoint are double-buffered: a
 // cell's neighbours read them while its owner writes the next ones.  The
 // gradient is summed as e = c11 lsH dh + c33 lsV dvz + c13 (lsH dvz + lsV dh),
-// lsH dh, lsH dvz + lsV dh and e - lambda_v . grad s / rho (terms that cancel
-// are combined in each step, in one slot); the models' chain rule is applied
-// once, at the end.  Shots that share a model run in groups inside a thread,
-// which reads the stiffness and updates the gradient slots once per group.
+// lsH dh, lsH dvz + lsV dh and e - lambda_v . grad s / rho (half A leaves a
+// step's e for half B: the two parts cancel, so the slot takes their difference,
+// not one after the other); the models' chain rule is applied once, at the end.
+// Shots that share a model run in groups inside a thread, which reads the
+// stiffness and updates the gradient slots once per group.
 //
 // Four x cells per thread (vec4.cuh) on pitched rows; a warp covers 32 x 4
 // (x, y) cells in 3-D and 32 x 4 (x, z) cells in 2-D.  A memory holds the cells
@@ -255,6 +256,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) str(const Geo G, const F
 
 struct Slots {
     float* g[4];                    // sums over time and a shot group: e, lsH dh, lsH dvz + lsV dh, e - lv . grad s / rho
+    float* e;                       // e of the step at hand
 };
 
 __device__ __forceinline__ void add(float* p, const F4& a)
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) half_a(const Geo G, cons
         add(g.g[0] + s, ge);
         add(g.g[1] + s, g11);
         add(g.g[2] + s, g13);
-        add(g.g[3] + s, ge);
+        v4::st(g.e + s, ge);
     }
 }
 
@@ -543,6 +545,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) half_b(const Geo G, cons
     }
     if (img) {
         const long long s = q.b * G.S + q.i;
+        const F4 e = v4::ld(g.e + s);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) gr.v[l] += e.v[l];
         add(g.g[3] + s, gr);
     }
 }
@@ -827,6 +832,7 @@ struct Ws {
     float* m[2][6];                 // forward: [0]; reverse: the adjoint's, double-buffered
     float* a[5];
     float* g[4];
+    float* e;
     char *zero0, *zero1;
 };
 
@@ -862,6 +868,7 @@ void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
     }
     c.take<char>(0);
     w.zero1 = c.base ? c.base + c.off : nullptr;
+    if (rev) w.e = c.take<float>(G.nslot * G.S);
 }
 
 template <int ND>
@@ -972,7 +979,7 @@ void backward(const Desc& d, Plan& pl, const float* adj, const void* tape, const
     Fields F{}, A{}, W[2]{};
     for (int k = 0; k < L::NF; ++k) { F.f[k] = w.f[k]; A.f[k] = w.a[k]; }
     for (int k = 0; k < L::NMEM; ++k) { W[0].f[k] = w.m[0][k]; W[1].f[k] = w.m[1][k]; }
-    const Slots g{{w.g[0], w.g[1], w.g[2], w.g[3]}};
+    const Slots g{{w.g[0], w.g[1], w.g[2], w.g[3]}, w.e};
     const dim3 grid = grid_of<ND>(G, G.nslot), block = block_of<ND>();
     const long long ne = (long long)G.B * G.nsrc + (long long)G.B * G.nrec;
     const unsigned bb = blocks((long long)G.B * G.ns);
