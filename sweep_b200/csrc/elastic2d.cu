@@ -760,7 +760,7 @@ __global__ void restore(const Geo G, const evec::Geo E, const evec::Rev R, const
         const long long i = b * G.S + c;
         for (int f = VX; f <= VZ; ++f) {
             const float v = strip_val(G, slot, b, f, iz, ix, si);
-            sum += R.a.f[f][i] * (v - R.f.f[f][i]);
+            sum += R.p[f][i] / E.kv[b * E.ms + c] * (v - R.f.f[f][i]);
             R.f.f[f][i] = v;
         }
     }
@@ -993,7 +993,7 @@ struct RevWs {
     Common cm;
     float* f[5];
     float* xprof;
-    float* a[5];
+    float* a[2];
     float* q[3];
     float* p[2];
     float* m[2][evec::NMEM];
@@ -1014,12 +1014,12 @@ static void carve_rev(Carve& c, const Plan& pl, RevWs& w)
     w.zero0 = c.base ? c.base + c.off : nullptr;
     for (float*& p : w.a) p = c.take<float>((long long)G.B * G.S);
     for (float*& p : w.q) p = c.take<float>((long long)G.B * G.S);
+    for (float*& p : w.p) p = c.take<float>((long long)G.B * G.S);
     for (auto& m : w.m)
         for (int k = 0; k < evec::NMEM; ++k) m[k] = c.take<float>(evec::mem_floats(pl.E, k));
     for (float*& p : w.g) p = c.take<float>((long long)pl.E.nslot * G.S);
     c.take<char>(0);
     w.zero1 = c.base ? c.base + c.off : nullptr;
-    for (float*& p : w.p) p = c.take<float>((long long)G.B * G.S);
     w.xprof = c.take<float>(4LL * evec::xprof_len(pl.E));
     if (pl.host_tape) w.ring = c.take<char>((long long)HostRing::R * G.st.step);
 }
@@ -1426,9 +1426,9 @@ static void backward_with(const sweep_elastic_desc* d, int mem_mode, int ckpt_ev
     SWEEP_LAUNCH_CHECK();
     E.ax = w.xprof + evec::kGuard; E.bx = E.ax + plen; E.axh = E.bx + plen; E.bxh = E.axh + plen;
     evec::Rev R{};
-    for (int k = 0; k < 5; ++k) { R.f.f[k] = w.f[k]; R.a.f[k] = w.a[k]; }
+    for (int k = 0; k < 5; ++k) R.f.f[k] = w.f[k];
     for (int k = 0; k < 3; ++k) { R.q[k] = w.q[k]; R.g[k] = w.g[k]; }
-    for (int k = 0; k < 2; ++k) R.p[k] = w.p[k];
+    for (int k = 0; k < 2; ++k) { R.a[k] = w.a[k]; R.p[k] = w.p[k]; }
     R.adj = adj;
     const long long ne = (long long)G.B * G.nsrc + (long long)G.B * G.nrec;
     const unsigned rblocks = (unsigned)(((long long)G.B * G.nstrip + 255) / 256);

@@ -103,7 +103,7 @@ __global__ void restore(const Geo G, const Rev R, const float* __restrict__ slot
         const long long i = b * G.S + c;
         for (int f = VX; f <= VZ; ++f) {
             const float v = __ldg(slot + (b * 5LL + f) * G.ns + n);
-            s += R.a.f[f][i] * (v - R.f.f[f][i]);
+            s += R.p[f][i] / G.kv[b * G.ms + c] * (v - R.f.f[f][i]);
             R.f.f[f][i] = v;
         }
     }
@@ -221,7 +221,7 @@ struct Ws {
     int* cells;
     float* f[5];
     float* m[2][NMEM];              // forward memories ([0]) / adjoint memories, double-buffered
-    float* a[5];
+    float* a[2];
     float* q[3];
     float* p[2];
     float* g[3];
@@ -244,12 +244,11 @@ static void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
     if (rev) {
         for (float*& p : w.a) p = c.take<float>(n);
         for (float*& p : w.q) p = c.take<float>(n);
+        for (float*& p : w.p) p = c.take<float>(n);
         for (float*& p : w.g) p = c.take<float>(G.nslot * G.S);
     }
     c.take<char>(0);
     w.zero1 = c.base ? c.base + c.off : nullptr;
-    if (rev)
-        for (float*& p : w.p) p = c.take<float>(n);
 }
 
 static long long slot_floats(const Plan& pl) { return (long long)pl.G.B * 5 * pl.G.ns; }
@@ -262,7 +261,7 @@ void sizes(const sweep_elastic_desc* d, int mem_mode, int, int64_t* ws_bytes, in
     carve(f, pl, false, w);
     carve(r, pl, true, w);
     *ws_bytes = std::max(f.off, r.off);
-    *tape_bytes = ((long long)pl.G.nt * slot_floats(pl) + 5LL * pl.G.B * pl.G.S) * 4;
+    *tape_bytes = ((long long)pl.G.nt * slot_floats(pl) + 5LL * pl.G.B * pl.G.nz * pl.G.nx) * 4;
 }
 
 static unsigned blocks(long long n) { return (unsigned)std::max<long long>((n + 255) / 256, 1); }
@@ -315,11 +314,10 @@ static void forward_m(const sweep_elastic_desc* d, Plan& pl, float* record, void
     }
     sg.flush();
     if (tp) {
-        // the final state, (5, B, S)
+        // the final state, (5, B, nz, nx)
         float* last = tp + (long long)G.nt * slot_floats(pl);
-        const long long n = (long long)G.B * G.S;
-        for (int f = 0; f < 5; ++f)
-            SWEEP_CUDA(cudaMemcpyAsync(last + f * n, w.f[f], sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+        const long long rows = (long long)G.B * G.nz;
+        for (int f = 0; f < 5; ++f) copy_rows(last + f * rows * G.nx, G.nx, w.f[f], G.P, G.nx, rows, st);
     }
 }
 
@@ -337,13 +335,12 @@ static void backward_m(const sweep_elastic_desc* d, Plan& pl, const float* adj, 
     const Geo& G = pl.G;
     const float* tp = static_cast<const float*>(tape);
     const float* last = tp + (long long)G.nt * slot_floats(pl);
-    const long long n = (long long)G.B * G.S;
-    for (int f = 0; f < 5; ++f)
-        SWEEP_CUDA(cudaMemcpyAsync(w.f[f], last + f * n, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+    const long long rows = (long long)G.B * G.nz;
+    for (int f = 0; f < 5; ++f) copy_rows(w.f[f], G.P, last + f * rows * G.nx, G.nx, G.nx, rows, st);
     Rev R{};
-    for (int k = 0; k < 5; ++k) { R.f.f[k] = w.f[k]; R.a.f[k] = w.a[k]; }
+    for (int k = 0; k < 5; ++k) R.f.f[k] = w.f[k];
     for (int k = 0; k < 3; ++k) { R.q[k] = w.q[k]; R.g[k] = w.g[k]; }
-    for (int k = 0; k < 2; ++k) R.p[k] = w.p[k];
+    for (int k = 0; k < 2; ++k) { R.a[k] = w.a[k]; R.p[k] = w.p[k]; }
     R.adj = adj;
     const long long ne = (long long)G.B * G.nsrc + (long long)G.B * G.nrec;
     const unsigned bb = blocks((long long)G.B * G.ns);

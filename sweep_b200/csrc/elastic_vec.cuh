@@ -348,12 +348,16 @@ __device__ __forceinline__ void inject_at(const Geo& G, const Fields& F, int e, 
     for (int k = 0; k < G.nsf; ++k) atomicAdd(F.f[G.sf[k]] + e / G.nsrc * G.S + c, w);
 }
 // ---------------------------------------------------------------- reverse
+// The adjoint velocities are held as p = kv lambda_v and the adjoint shear
+// stress as qxz = dt mu lambda_xz alone: the transposes read these, and where
+// mu = 0 lambda_xz reaches no result.
 struct Rev {
-    Fields f, a;                    // reconstructed forward fields, adjoint fields
-    Mems ai, ao;                    // adjoint CPML memories: read, written
+    Fields f;                       // reconstructed forward fields
+    float* a[2];                    // adjoint sxx, szz
     float* q[3];                    // dt C lambda_s: xx, zz, xz
     float* p[2];                    // kv lambda_v
-    float* g[3];                    // slots of a shot group: gl, gm - 2 gl, the rho image (times rho)
+    Mems ai, ao;                    // adjoint CPML memories: read, written
+    float* g[3];                    // slots of a shot group: gl, dt mu (gm - 2 gl), the rho image (times rho)
     const float* adj;               // (B, nt, nrec, nrf)
     int it;
 };
@@ -373,8 +377,8 @@ __device__ __forceinline__ void stiff(float dt, float lam, float mu, float sxx, 
     }
 }
 
-// signed residuals into the adjoint fields (stress -1, velocity +1) and what
-// they add to q; the source of step it out of the forward fields
+// signed residuals (stress -1, velocity +1) into the adjoint stresses, q and
+// p; the source of step it out of the forward fields
 __global__ static void events(const Geo G, const Rev R)
 {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -390,8 +394,8 @@ __global__ static void events(const Geo G, const Rev R)
     for (int k = 0; k < G.nrf; ++k) {
         const int f = G.rf[k];
         const float v = f >= SXX ? -res[k] : res[k];
-        atomicAdd(R.a.f[f] + i, v);
-        if (f < SXX) continue;
+        if (f < SXX) { atomicAdd(R.p[f] + i, G.kv[mi] * v); continue; }
+        if (f != SXZ) atomicAdd(R.a[f - SXX] + i, v);
         if (f == SXZ) {
             if (!fs_zero_shear(G, l[0], l[1])) atomicAdd(R.q[2] + i, (G.dt * G.mu[mi]) * v);
             continue;
@@ -416,7 +420,8 @@ __device__ __forceinline__ void add4(float* p, const F4& a)
 // with gl, gm the derivatives of the misfit by lambda and mu (up to -dt), grad
 // vp = -2 rho vp dt gl, grad vs = -2 rho vs dt (gm - 2 gl), and the stiffness
 // part of rho times grad rho, -dt (gl (lam + 2 mu) + (gm - 2 gl) mu)
-// (reference kernels.cuh:365-535, 601-663).
+// (reference kernels.cuh:365-535, 601-663).  The shear part of dt mu gm is
+// qxz (dvx/dz + dvz/dx); qxz is zero where a face zeroes the shear.
 template <int M, bool FS, bool GRP>
 __device__ __forceinline__ void stress_rev(const Geo& G, const Rev& R, const Cell& q)
 {
@@ -428,7 +433,7 @@ __device__ __forceinline__ void stress_rev(const Geo& G, const Rev& R, const Cel
         const long long k = b * G.S + q.i, mi = b * G.ms + q.i;
         const Four d = velocity_diffs<M, FS>(G, R.f, q, k);
         const F4 lam = v4::ldg(G.lam + mi), mu = v4::ldg(G.mu + mi);
-        const F4 bxx = v4::ldg(R.a.f[SXX] + k), bzz = v4::ldg(R.a.f[SZZ] + k), bxz = v4::ldg(R.a.f[SXZ] + k);
+        const F4 bxx = v4::ldg(R.a[0] + k), bzz = v4::ldg(R.a[1] + k), qxz = v4::ldg(R.q[2] + k);
         F4 sxx = v4::ld(R.f.f[SXX] + k), szz = v4::ld(R.f.f[SZZ] + k), sxz = v4::ld(R.f.f[SXZ] + k);
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
@@ -446,11 +451,10 @@ __device__ __forceinline__ void stress_rev(const Geo& G, const Rev& R, const Cel
                 gl = (bxx.v[l] + bzz.v[l]) * (vxx + vzz);
                 gm = 2.f * (bxx.v[l] * vxx + bzz.v[l] * vzz);
             }
-            if (!(FS && fs_zero_shear(G, x, q.z))) gm = gm + bxz.v[l] * (d.xz.v[l] + d.zx.v[l]);
-            const float gm2 = gm - 2.f * gl;
+            const float gs = (G.dt * m) * (gm - 2.f * gl) + qxz.v[l] * (d.xz.v[l] + d.zx.v[l]);
             sl.v[l] += gl;
-            sm.v[l] += gm2;
-            sr.v[l] -= G.dt * (gl * l2m + gm2 * m);
+            sm.v[l] += gs;
+            sr.v[l] -= (G.dt * gl) * l2m + gs;
             if (rrow && x >= G.rx0 && x < G.rx1) {
                 sxx.v[l] = sxx.v[l] - G.dt * (l2m * vxx + L * vzz);
                 szz.v[l] = szz.v[l] - G.dt * (l2m * vzz + L * vxx);
@@ -477,15 +481,15 @@ __device__ __forceinline__ void vel_rev(const Geo& G, const Rev& R, const Cell& 
     for (int b = b0; b < b1; ++b) {
         const long long k = b * G.S + q.i;
         const Four d = stress_diffs<M, FS>(G, R.f, q, k);
-        const F4 kv = v4::ldg(G.kv + b * G.ms + q.i), lx = v4::ldg(R.a.f[VX] + k), lz = v4::ldg(R.a.f[VZ] + k);
+        const F4 kv = v4::ldg(G.kv + b * G.ms + q.i), px = v4::ldg(R.p[0] + k), pz = v4::ldg(R.p[1] + k);
         F4 vx = v4::ld(R.f.f[VX] + k), vz = v4::ld(R.f.f[VZ] + k);
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
             if (q.x + l < G.rx0 || q.x + l >= G.rx1) continue;
-            const float ux = kv.v[l] * (d.xx.v[l] + d.xz.v[l]), uz = kv.v[l] * (d.zx.v[l] + d.zz.v[l]);
-            vx.v[l] = vx.v[l] - ux;
-            vz.v[l] = vz.v[l] - uz;
-            sr.v[l] -= lx.v[l] * ux + lz.v[l] * uz;
+            const float gx = d.xx.v[l] + d.xz.v[l], gz = d.zx.v[l] + d.zz.v[l];
+            vx.v[l] = vx.v[l] - kv.v[l] * gx;
+            vz.v[l] = vz.v[l] - kv.v[l] * gz;
+            sr.v[l] -= px.v[l] * gx + pz.v[l] * gz;
         }
         v4::st(R.f.f[VX] + k, vx);
         v4::st(R.f.f[VZ] + k, vz);
@@ -578,8 +582,8 @@ __device__ __forceinline__ void keep(const float* wi, float* wo, const F4& a, co
     v4::st(wo, t);
 }
 
-// the stress step's transpose (reference kernels.cuh:664-837): lambda_v on the
-// core, then p = kv lambda_v
+// the stress step's transpose (reference kernels.cuh:664-837): lambda_v, as p,
+// on the core
 template <int M, bool FS>
 __device__ __forceinline__ void adj_vel(const Geo& G, const Rev& R, const Cell& q)
 {
@@ -600,33 +604,25 @@ __device__ __forceinline__ void adj_vel(const Geo& G, const Rev& R, const Cell& 
         keep(R.ai.m[M_VZZ] + mz, R.ao.m[M_VZZ] + mz, v4::splat(__ldg(G.az + q.z)), v4::ldg(qzz), on);
         keep(R.ai.m[M_VXZ] + mz, R.ao.m[M_VXZ] + mz, v4::splat(__ldg(G.azh + q.z)), v4::ldg(qxz), on);
     }
-    F4 dvx = v4::splat(0.f), dvz = dvx;
-    if (q.core) {
-        const F4 a = adj_x<M, FS, false>(G, q, qxx, R.ai.m[M_VXX], G.bx, true, true);
-        const F4 b = adj_z<M, FS, true>(G, q, qxz, R.ai.m[M_VXZ], G.bzh, false, false);
-        const F4 c = adj_x<M, FS, true>(G, q, qxz, R.ai.m[M_VZX], G.bxh, false, false);
-        const F4 d = adj_z<M, FS, false>(G, q, qzz, R.ai.m[M_VZZ], G.bz, true, true);
-#pragma unroll
-        for (int l = 0; l < 4; ++l)
-            if (q.lane(G, l)) { dvx.v[l] = a.v[l] + b.v[l]; dvz.v[l] = c.v[l] + d.v[l]; }
-    }
+    if (!q.core) return;
+    const F4 a = adj_x<M, FS, false>(G, q, qxx, R.ai.m[M_VXX], G.bx, true, true);
+    const F4 b = adj_z<M, FS, true>(G, q, qxz, R.ai.m[M_VXZ], G.bzh, false, false);
+    const F4 c = adj_x<M, FS, true>(G, q, qxz, R.ai.m[M_VZX], G.bxh, false, false);
+    const F4 d = adj_z<M, FS, false>(G, q, qzz, R.ai.m[M_VZZ], G.bz, true, true);
     const F4 kv = v4::ldg(G.kv + q.b * G.ms + q.i);
-    F4 vx = v4::ld(R.a.f[VX] + k), vz = v4::ld(R.a.f[VZ] + k), px, pz;
+    F4 px = v4::ld(R.p[0] + k), pz = v4::ld(R.p[1] + k);
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
-        vx.v[l] = vx.v[l] + dvx.v[l];
-        vz.v[l] = vz.v[l] + dvz.v[l];
-        px.v[l] = kv.v[l] * vx.v[l];
-        pz.v[l] = kv.v[l] * vz.v[l];
+        if (!q.lane(G, l)) continue;
+        px.v[l] = px.v[l] + kv.v[l] * (a.v[l] + b.v[l]);
+        pz.v[l] = pz.v[l] + kv.v[l] * (c.v[l] + d.v[l]);
     }
-    v4::st(R.a.f[VX] + k, vx);
-    v4::st(R.a.f[VZ] + k, vz);
     v4::st(R.p[0] + k, px);
     v4::st(R.p[1] + k, pz);
 }
 
 // the velocity step's transpose (reference kernels.cuh:873-1019): lambda_s on
-// the core, then q = dt C lambda_s
+// the core, and q = dt C lambda_s
 template <int M, bool FS>
 __device__ __forceinline__ void adj_str(const Geo& G, const Rev& R, const Cell& q)
 {
@@ -647,32 +643,26 @@ __device__ __forceinline__ void adj_str(const Geo& G, const Rev& R, const Cell& 
         keep(R.ai.m[M_SXZZ] + mz, R.ao.m[M_SXZZ] + mz, v4::splat(__ldg(G.az + q.z)), v4::ldg(px), on);
         keep(R.ai.m[M_SZZZ] + mz, R.ao.m[M_SZZZ] + mz, v4::splat(__ldg(G.azh + q.z)), v4::ldg(pz), on);
     }
-    F4 dxx = v4::splat(0.f), dzz = dxx, dxz = dxx;
-    if (q.core) {
-        const F4 a = adj_x<M, FS, true>(G, q, px, R.ai.m[M_SXXX], G.bxh, true, false);
-        const F4 b = adj_z<M, FS, true>(G, q, pz, R.ai.m[M_SZZZ], G.bzh, true, false);
-        const F4 c = adj_z<M, FS, false>(G, q, px, R.ai.m[M_SXZZ], G.bz, true, true);
-        const F4 d = adj_x<M, FS, false>(G, q, pz, R.ai.m[M_SXZX], G.bx, true, true);
-#pragma unroll
-        for (int l = 0; l < 4; ++l)
-            if (q.lane(G, l)) { dxx.v[l] = a.v[l]; dzz.v[l] = b.v[l]; dxz.v[l] = c.v[l] + d.v[l]; }
-    }
+    if (!q.core) return;
+    const F4 a = adj_x<M, FS, true>(G, q, px, R.ai.m[M_SXXX], G.bxh, true, false);
+    const F4 b = adj_z<M, FS, true>(G, q, pz, R.ai.m[M_SZZZ], G.bzh, true, false);
+    const F4 c = adj_z<M, FS, false>(G, q, px, R.ai.m[M_SXZZ], G.bz, true, true);
+    const F4 d = adj_x<M, FS, false>(G, q, pz, R.ai.m[M_SXZX], G.bx, true, true);
     const F4 lam = v4::ldg(G.lam + mi), mu = v4::ldg(G.mu + mi);
-    F4 sxx = v4::ld(R.a.f[SXX] + k), szz = v4::ld(R.a.f[SZZ] + k), sxz = v4::ld(R.a.f[SXZ] + k), qxx, qzz, qxz;
+    F4 sxx = v4::ld(R.a[0] + k), szz = v4::ld(R.a[1] + k), qxx, qzz, qxz = v4::ld(R.q[2] + k);
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
+        const bool on_core = q.lane(G, l);
         const bool zs = FS && fs_zrow(G, q.z), xs = FS && fs_xcol(G, q.x + l);
         const bool sh = FS && fs_zero_shear(G, q.x + l, q.z);
         // what the surfaces zero starts the step at zero (kernels.cuh:592-600)
-        sxx.v[l] = (xs ? 0.f : sxx.v[l]) + dxx.v[l];
-        szz.v[l] = (zs ? 0.f : szz.v[l]) + dzz.v[l];
-        sxz.v[l] = (sh ? 0.f : sxz.v[l]) + dxz.v[l];
+        sxx.v[l] = (xs ? 0.f : sxx.v[l]) + (on_core ? a.v[l] : 0.f);
+        szz.v[l] = (zs ? 0.f : szz.v[l]) + (on_core ? b.v[l] : 0.f);
         stiff(G.dt, lam.v[l], mu.v[l], sxx.v[l], szz.v[l], zs, xs, qxx.v[l], qzz.v[l]);
-        qxz.v[l] = sh ? 0.f : (G.dt * mu.v[l]) * sxz.v[l];
+        qxz.v[l] = sh ? 0.f : on_core ? qxz.v[l] + (G.dt * mu.v[l]) * (c.v[l] + d.v[l]) : qxz.v[l];
     }
-    v4::st(R.a.f[SXX] + k, sxx);
-    v4::st(R.a.f[SZZ] + k, szz);
-    v4::st(R.a.f[SXZ] + k, sxz);
+    v4::st(R.a[0] + k, sxx);
+    v4::st(R.a[1] + k, szz);
     v4::st(R.q[0] + k, qxx);
     v4::st(R.q[1] + k, qzz);
     v4::st(R.q[2] + k, qxz);
@@ -726,7 +716,7 @@ __global__ static void finalize(const Geo G, const Rev R, const Out o)
             }
             const float rho = o.rho[e];
             t[0] = -2.f * rho * o.vp[e] * t[0] * G.dt;
-            t[1] = -2.f * rho * o.vs[e] * t[1] * G.dt;
+            t[1] = o.vs[e] != 0.f ? -2.f * t[1] / o.vs[e] : 0.f;     // mu = rho vs^2
             t[2] = t[2] / rho;
         }
         for (int j = 0; j < 3; ++j) o.g[j][e] = t[j];

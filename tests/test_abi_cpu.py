@@ -593,6 +593,9 @@ WORKSPACES = [
     ("Acoustic", 8, (256, 768), 16, 40, False, 279406848, 70491648),
     ("Acoustic", 8, (200, 400), 8, 20, False, 65335296, 16557056),
     ("Acoustic", 8, (400, 1200), 1, 40, False, 53786880, 8309248),
+    ("Elastic", 8, (400, 1200), 16, 40, False, 620846848, 460817920),
+    ("Elastic", 8, (400, 1200), 1, 40, False, 58973440, 28805120),
+    ("Elastic", 4, (400, 1200), 16, 40, True, 1193233920, 352465920),
     ("AcousticVTI1st", 4, (400, 1200), 16, 40, True, 875048448, 281972736),
     ("AcousticVTI1st", 8, (400, 1200), 16, 40, False, 734203392, 365707264),
     ("AcousticVTI1st3D", 4, (128, 128, 128), 1, 16, False, 477555712, 381602880),

@@ -35,12 +35,14 @@ def _geometry(shape, B, rng):
     return src.astype(np.int64), rec.astype(np.int64)
 
 
-def _check(eq, oracle, names, shape, B, order, free=False, vacuum=False):
+def _check(eq, oracle, names, shape, B, order, free=False, vacuum=False, fluid=False):
     from sweep_b200 import PropTorch
     rng = np.random.default_rng(sum(shape) + 7 * order + B)
     ms = _models(names, shape, rng)
     if vacuum:                                      # a few cells without stiffness
         ms[0].reshape(-1)[rng.integers(0, ms[0].size, 5)] = 0.0
+    if fluid:                                       # water above solid
+        ms[1][:shape[0] // 3] = 0.0
     src, rec = _geometry(shape, B, rng)
     dh, dt, abcn = 6.0, 0.0006, 5
     t = np.arange(NT) * dt
@@ -132,3 +134,11 @@ def test_elastic2d_order8(shape, B, free):
     """The last one sums the images of several shots per thread."""
     from sweep_b200 import Elastic
     _check(Elastic, O.Elastic2D, ("vp", "vs", "rho"), shape, B, 8, free)
+
+
+@pytest.mark.parametrize("shape,order,free", [((33, 45), 4, False), ((33, 45), 8, True), ((17, 15, 34), 4, False)])
+def test_elastic_water_layer(shape, order, free):
+    """Cells with vs = 0, whose adjoint shear stress reaches no result."""
+    from sweep_b200 import Elastic, Elastic3D
+    eq, oracle = (Elastic, O.Elastic2D) if len(shape) == 2 else (Elastic3D, O.Elastic3D)
+    _check(eq, oracle, ("vp", "vs", "rho"), shape, 2, order, free, fluid=True)
