@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(kQB) quant3(const Geo G, const Fields F, void*
 // the adjoint stresses), `vel_rev` (velocity reconstruction and the rho
 // image), the velocity strips.  `adj_str` leaves q = dt C lambda_s beside the
 // adjoint stresses it writes (six fields; the reference's nine differ by the
-// CPML memory alone) and `adj_vel` p = kv lambda_v beside the velocities, so
+// CPML memory alone), and the adjoint velocities are held as p = kv lambda_v, so
 // no pass of its own prepares them and the stencils read one field per tap; a
 // band's taps add the adjoint memory, which is therefore double-buffered.
 // (q and p formed at every tap from lambda, the stiffness and 1 / rho instead:
@@ -594,11 +594,11 @@ struct Rev {
     Geo G;
     Models m;
     float* f[NFLD];      // reconstructed forward fields
-    float* a[NFLD];      // adjoint fields
+    float* a[3];         // adjoint sxx, syy, szz
     float* q[6];         // dt C lambda_s: xx, yy, zz, xy, xz, yz
     float* p[3];         // kv lambda_v
     Slabs ai, ao;        // adjoint memories: read, written
-    float* g[3];         // slots of a shot group: gl, gm - 2 gl and the rho image (times rho)
+    float* g[3];         // slots of a shot group: gl, dt mu (gm - 2 gl) and the rho image (times rho)
     const float* adj;    // (B, nt, nrec, nrf)
     int it;
 };
@@ -632,11 +632,11 @@ __global__ void res3(Rev A)
         for (int k = 0; k < G.nrf; ++k) {
             const int fl = G.rf[k];
             const float v = fl >= SXX ? -res[k] : res[k];
-            atomicAdd(A.a[fl] + i, v);
-            if (fl < SXX) continue;
-            // and what it adds to q
+            if (fl < SXX) { atomicAdd(A.p[fl] + i, A.m.kv[b * G.ms + i - b * G.S] * v); continue; }
             const float lam = A.m.lam[b * G.ms + i - b * G.S], mu = A.m.mu[b * G.ms + i - b * G.S];
             if (fl >= SXY) { atomicAdd(A.q[fl - SXX] + i, G.dt * mu * v); continue; }
+            atomicAdd(A.a[fl - SXX] + i, v);
+            // and what it adds to q
             const float x = fl == SXX ? v : 0.f, y = fl == SYY ? v : 0.f, z = fl == SZZ ? v : 0.f;
             float q3[3];
             stiff(G.dt, lam, mu, x, y, z, G.fst && l[2] == G.z0, q3);
@@ -658,6 +658,7 @@ __device__ __forceinline__ void add4(float* p, const F4& a)
 // with gl, gm the derivatives of the misfit by lambda and mu (up to -dt),
 // grad vp = -2 rho vp dt gl, grad vs = -2 rho vs dt (gm - 2 gl), and the
 // stiffness part of rho times grad rho, -dt (gl (lam + 2 mu) + (gm - 2 gl) mu).
+// The shear part of dt mu gm is the shears of q times their strains.
 template <bool FS>
 __global__ void __launch_bounds__(kThreads, kBlocks) stress_rev(const Rev A)
 {
@@ -677,13 +678,13 @@ __global__ void __launch_bounds__(kThreads, kBlocks) stress_rev(const Rev A)
         const long long k = b * G.S + q.i, mi = b * G.ms + q.i;
         const Nine d = velocity_diffs<FS>(G, A.f, k, q.z);
         const F4 lam = v4::ldg(A.m.lam + mi), mu = v4::ldg(A.m.mu + mi);
-        const F4 bxx = v4::ldg(A.a[SXX] + k), byy = v4::ldg(A.a[SYY] + k), bzz = v4::ldg(A.a[SZZ] + k);
-        const F4 bxy = v4::ldg(A.a[SXY] + k), bxz = v4::ldg(A.a[SXZ] + k), byz = v4::ldg(A.a[SYZ] + k);
+        const F4 bxx = v4::ldg(A.a[0] + k), byy = v4::ldg(A.a[1] + k), bzz = v4::ldg(A.a[2] + k);
+        const F4 qxy = v4::ldg(A.q[3] + k), qxz = v4::ldg(A.q[4] + k), qyz = v4::ldg(A.q[5] + k);
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
             if (!box[l]) continue;
-            const float shear = bxz.v[l] * (d.xz.v[l] + d.zx.v[l]) + bxy.v[l] * (d.xy.v[l] + d.yx.v[l]) +
-                                byz.v[l] * (d.yz.v[l] + d.zy.v[l]);
+            const float shear = qxz.v[l] * (d.xz.v[l] + d.zx.v[l]) + qxy.v[l] * (d.xy.v[l] + d.yx.v[l]) +
+                                qyz.v[l] * (d.yz.v[l] + d.zy.v[l]);
             const float l2m = lam.v[l] + 2.f * mu.v[l];
             float gl, gm;
             if (surf) {
@@ -692,15 +693,15 @@ __global__ void __launch_bounds__(kThreads, kBlocks) stress_rev(const Rev A)
                 const float dcl = 4.f * r * r, dcm = 4.f * (1.f - 2.f * r + 2.f * r * r), dc2m = 2.f * w * w;
                 gl = dcl * (bxx.v[l] + byy.v[l]) * (d.xx.v[l] + d.yy.v[l]);
                 gm = bxx.v[l] * (dcm * d.xx.v[l] + dc2m * d.yy.v[l]) +
-                     byy.v[l] * (dc2m * d.xx.v[l] + dcm * d.yy.v[l]) + shear;
+                     byy.v[l] * (dc2m * d.xx.v[l] + dcm * d.yy.v[l]);
             } else {
                 gl = (bxx.v[l] + byy.v[l] + bzz.v[l]) * (d.xx.v[l] + d.yy.v[l] + d.zz.v[l]);
-                gm = 2.f * (bxx.v[l] * d.xx.v[l] + byy.v[l] * d.yy.v[l] + bzz.v[l] * d.zz.v[l]) + shear;
+                gm = 2.f * (bxx.v[l] * d.xx.v[l] + byy.v[l] * d.yy.v[l] + bzz.v[l] * d.zz.v[l]);
             }
-            const float gm2 = gm - 2.f * gl;
+            const float gs = (G.dt * mu.v[l]) * (gm - 2.f * gl) + shear;
             sl.v[l] += gl;
-            sm.v[l] += gm2;
-            sr.v[l] -= G.dt * (gl * l2m + gm2 * mu.v[l]);
+            sm.v[l] += gs;
+            sr.v[l] -= (G.dt * gl) * l2m + gs;
         }
         if (inner) stress_update(G, A.f, k, d, lam, mu, -G.dt, on, false);
     }
@@ -724,18 +725,18 @@ __global__ void __launch_bounds__(kThreads, kBlocks) vel_rev(const Rev A)
         const long long k = b * G.S + q.i;
         const Nine d = stress_diffs<FS>(G, A.f, k, q.z);
         const F4 kv = v4::ldg(A.m.kv + b * G.ms + q.i);
-        const F4 lx = v4::ldg(A.a[VX] + k), ly = v4::ldg(A.a[VY] + k), lz = v4::ldg(A.a[VZ] + k);
+        const F4 px = v4::ldg(A.p[VX] + k), py = v4::ldg(A.p[VY] + k), pz = v4::ldg(A.p[VZ] + k);
         F4 vx = v4::ld(A.f[VX] + k), vy = v4::ld(A.f[VY] + k), vz = v4::ld(A.f[VZ] + k);
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
             if (!(q.x + l > G.x0 && q.x + l < G.x1 - 1)) continue;
-            const float ux = kv.v[l] * (d.xx.v[l] + d.xy.v[l] + d.xz.v[l]);
-            const float uy = kv.v[l] * (d.yx.v[l] + d.yy.v[l] + d.yz.v[l]);
-            const float uz = kv.v[l] * (d.zx.v[l] + d.zy.v[l] + d.zz.v[l]);
-            vx.v[l] -= ux;
-            vy.v[l] -= uy;
-            vz.v[l] -= uz;
-            sr.v[l] -= lx.v[l] * ux + ly.v[l] * uy + lz.v[l] * uz;
+            const float gx = d.xx.v[l] + d.xy.v[l] + d.xz.v[l];
+            const float gy = d.yx.v[l] + d.yy.v[l] + d.yz.v[l];
+            const float gz = d.zx.v[l] + d.zy.v[l] + d.zz.v[l];
+            vx.v[l] -= kv.v[l] * gx;
+            vy.v[l] -= kv.v[l] * gy;
+            vz.v[l] -= kv.v[l] * gz;
+            sr.v[l] -= px.v[l] * gx + py.v[l] * gy + pz.v[l] * gz;
         }
         v4::st(A.f[VX] + k, vx);
         v4::st(A.f[VY] + k, vy);
@@ -766,7 +767,7 @@ __global__ void restore_velocity(const Rev A, const void* slot, int fmt)
                 const float v = fmt == SF_F32    ? static_cast<const float*>(slot)[t]
                                 : fmt == SF_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(slot)[t])
                                                  : face_val(G, slot, fl, b, c);
-                if (img) s += A.a[fl][i] * (v - A.f[fl][i]);
+                if (img) s += A.p[fl][i] / A.m.kv[b * G.ms + c] * (v - A.f[fl][i]);
                 A.f[fl][i] = v;
             }
         }
@@ -848,8 +849,8 @@ __device__ __forceinline__ F4 adj_z(const Geo& G, const Cell& q, const float* u,
         q.z, odd, half);
 }
 
-// The stress step's transpose: lambda_v += D(q) on the core, q through the
-// memories of the velocities' derivatives; then p = kv lambda_v.
+// The stress step's transpose: lambda_v += D(q), held as p, on the core, q
+// through the memories of the velocities' derivatives.
 template <bool FS>
 __global__ void __launch_bounds__(kThreads, kBlocks) adj_vel(const Rev A)
 {
@@ -878,22 +879,15 @@ __global__ void __launch_bounds__(kThreads, kBlocks) adj_vel(const Rev A)
         keep(A.ai.z[MZ_VY] + o, A.ao.z[MZ_VY] + o, a, v4::ldg(qyz));
         keep(A.ai.z[MZ_VZ] + o, A.ao.z[MZ_VZ] + o, v4::splat(__ldg(G.az + q.z)), v4::ldg(qzz));
     }
+    if (!q.core) return;
     const F4 kv = v4::ldg(A.m.kv + q.b * G.ms + q.i);
     auto put = [&](int fl, const F4& a, const F4& b, const F4& c) {
-        F4 v = v4::ld(A.a[fl] + k), p;
+        F4 p = v4::ld(A.p[fl] + k);
 #pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            if (q.core && q.lane(G, l)) v.v[l] += a.v[l] + b.v[l] + c.v[l];
-            p.v[l] = kv.v[l] * v.v[l];
-        }
-        v4::st(A.a[fl] + k, v);
+        for (int l = 0; l < 4; ++l)
+            if (q.lane(G, l)) p.v[l] += kv.v[l] * (a.v[l] + b.v[l] + c.v[l]);
         v4::st(A.p[fl] + k, p);
     };
-    if (!q.core) {
-        const F4 z = v4::splat(0.f);
-        for (int fl = VX; fl <= VZ; ++fl) put(fl, z, z, z);
-        return;
-    }
     put(VX, adj_x<true>(G, q, qxx, A.ai.x[MX_VX], G.bx), adj_y<false>(G, q, qxy, A.ai.y[MY_VX], G.byh),
         adj_z<FS, true>(G, q, qxz, A.ai.z[MZ_VX], G.bzh, false, false));
     put(VY, adj_x<false>(G, q, qxy, A.ai.x[MX_VY], G.bxh), adj_y<true>(G, q, qyy, A.ai.y[MY_VY], G.by),
@@ -903,7 +897,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) adj_vel(const Rev A)
 }
 
 // The velocity step's transpose: lambda_s += D(p) on the core, p through the
-// memories of the stresses' derivatives; then q = dt C lambda_s.
+// memories of the stresses' derivatives, and q = dt C lambda_s; of the shears
+// q alone is kept (where mu = 0 they reach no result).
 template <bool FS>
 __global__ void __launch_bounds__(kThreads, kBlocks) adj_str(const Rev A)
 {
@@ -938,23 +933,26 @@ __global__ void __launch_bounds__(kThreads, kBlocks) adj_str(const Rev A)
         for (int l = 0; l < 4; ++l) t.v[l] = a.v[l] + b.v[l];
         return t;
     };
+    const bool c = q.core;
     auto put = [&](int fl, const F4& d, bool clear) {
-        F4 v = v4::ld(A.a[fl] + k);
+        F4 v = v4::ld(A.a[fl - SXX] + k);
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
             if (clear) v.v[l] = 0.f;
-            if (q.core && q.lane(G, l)) v.v[l] += d.v[l];
+            if (c && q.lane(G, l)) v.v[l] += d.v[l];
         }
-        v4::st(A.a[fl] + k, v);
+        v4::st(A.a[fl - SXX] + k, v);
         return v;
     };
     auto shear = [&](int fl, const F4& d) {
-        F4 v = put(fl, d, false);
+        F4 v = v4::ld(A.q[fl - SXX] + k);
 #pragma unroll
-        for (int l = 0; l < 4; ++l) v.v[l] = G.dt * mu.v[l] * v.v[l];
+        for (int l = 0; l < 4; ++l)
+            if (c && q.lane(G, l)) v.v[l] += (G.dt * mu.v[l]) * d.v[l];
         v4::st(A.q[fl - SXX] + k, v);
     };
-    const bool c = q.core;
+    // (the test before each stencil keeps its loads apart from the next one's:
+    // without it the kernel spills 448 bytes instead of 24)
     shear(SXY, c ? sum(adj_y<true>(G, q, px, A.ai.y[MY_SXY], G.by), adj_x<true>(G, q, py, A.ai.x[MX_SXY], G.bx)) : zero);
     shear(SXZ, c ? sum(adj_z<FS, false>(G, q, px, A.ai.z[MZ_SXZ], G.bz, true, true),
                        adj_x<true>(G, q, pz, A.ai.x[MX_SXZ], G.bx)) : zero);
@@ -1028,7 +1026,7 @@ __global__ void finalize3(const Rev A, const Out o)
             }
             const float rho = o.rho[e];
             t[0] = -2.f * rho * o.vp[e] * t[0] * G.dt;
-            t[1] = -2.f * rho * o.vs[e] * t[1] * G.dt;
+            t[1] = o.vs[e] != 0.f ? -2.f * t[1] / o.vs[e] : 0.f;     // mu = rho vs^2
             t[2] = t[2] / rho;
         }
         for (int j = 0; j < 3; ++j) o.g[j][e] = t[j];
@@ -1224,7 +1222,7 @@ static void carve_fwd(Carve& c, const Plan& pl, FwdWs& w)
 struct RevWs {
     Common cm;
     float* f[NFLD];
-    float* a[NFLD];
+    float* a[3];
     float* q[6];
     float* p[3];
     Slabs am[2];                 // adjoint memories, double-buffered
@@ -1240,10 +1238,10 @@ static void carve_rev(Carve& c, const Plan& pl, RevWs& w)
     carve_common(c, pl, w.cm);
     const Geo& G = pl.G;
     const long long n = (long long)G.B * G.S;
-    for (int k = 0; k < NFLD; ++k) w.f[k] = c.take<float>(n);
     c.take<char>(0);
     w.zero0 = c.base ? c.base + c.off : nullptr;
-    for (int k = 0; k < NFLD; ++k) w.a[k] = c.take<float>(n);
+    for (int k = 0; k < NFLD; ++k) w.f[k] = c.take<float>(n);
+    for (float*& p : w.a) p = c.take<float>(n);
     for (float*& p : w.q) p = c.take<float>(n);
     for (float*& p : w.p) p = c.take<float>(n);
     for (Slabs& s : w.am) carve_slabs(c, G, s);
@@ -1262,11 +1260,14 @@ static void carve_rev_ckpt(Carve& c, const Plan& pl, int k, RevWs& w)
     w.chunk = c.take<float>((long long)(k + 1) * chunk_floats(pl));
 }
 
+// rows of a field of every shot
+static long long rows_of(const Geo& G) { return (long long)G.B * G.nz * G.ny; }
+
 // Boundary-saving tape: one strip slot per step (G.st.step bytes), then the
 // final nine-field state (9, B, nz, ny, nx).
 static int64_t tape_bytes_of(const Plan& pl)
 {
-    return (int64_t)pl.G.nt * pl.G.st.step + (int64_t)NFLD * pl.G.B * pl.G.S * 4;
+    return (int64_t)pl.G.nt * pl.G.st.step + (int64_t)NFLD * rows_of(pl.G) * pl.G.nx * 4;
 }
 
 static void* tape_slot(const void* tape, const Plan& pl, int it)
@@ -1458,7 +1459,7 @@ void forward(const sweep_elastic3d_desc* d, int mem_mode, int ckpt_every, float*
         if (tape) {
             float* last = tape_last(tape, pl);
             for (int k = 0; k < NFLD; ++k)
-                SWEEP_CUDA(cudaMemcpyAsync(last + k * n, w.f[k], sizeof(float) * n, cudaMemcpyDefault, st));
+                copy_rows(last + k * rows_of(G) * G.nx, G.nx, w.f[k], G.P, G.nx, rows_of(G), st);
         }
         return;
     }
@@ -1506,9 +1507,9 @@ void backward(const sweep_elastic3d_desc* d, int mem_mode, int ckpt_every, const
     Rev A{};
     A.G = G;
     A.m = models_of(w.cm);
-    for (int k = 0; k < NFLD; ++k) { A.f[k] = w.f[k]; A.a[k] = w.a[k]; }
+    for (int k = 0; k < NFLD; ++k) A.f[k] = w.f[k];
     for (int k = 0; k < 6; ++k) A.q[k] = w.q[k];
-    for (int k = 0; k < 3; ++k) { A.p[k] = w.p[k]; A.g[k] = w.g[k]; }
+    for (int k = 0; k < 3; ++k) { A.a[k] = w.a[k]; A.p[k] = w.p[k]; A.g[k] = w.g[k]; }
     A.adj = adj;
     Fields F{};
     for (int k = 0; k < NFLD; ++k) F.f[k] = w.f[k];
@@ -1621,7 +1622,7 @@ void backward(const sweep_elastic3d_desc* d, int mem_mode, int ckpt_every, const
     } else if (!ckpt) {
         const float* last = tape_last(tape, pl);
         for (int k = 0; k < NFLD; ++k)
-            SWEEP_CUDA(cudaMemcpyAsync(w.f[k], last + k * n, sizeof(float) * n, cudaMemcpyDefault, st));
+            copy_rows(w.f[k], G.P, last + k * rows_of(G) * G.nx, G.nx, G.nx, rows_of(G), st);
         if (host) {
             hr.open(w.ring, const_cast<void*>(tape), G.st.step, st);
             for (int t = G.nt - 2; t >= 0 && t > G.nt - 2 - HostRing::R; --t) hr.fetch(t, false);

@@ -596,6 +596,8 @@ WORKSPACES = [
     ("Elastic", 8, (400, 1200), 16, 40, False, 620846848, 460817920),
     ("Elastic", 8, (400, 1200), 1, 40, False, 58973440, 28805120),
     ("Elastic", 4, (400, 1200), 16, 40, True, 1193233920, 352465920),
+    ("Elastic3D", 8, (128, 128, 128), 4, 16, False, 2903838976, 4210743808),
+    ("Elastic3D", 4, (101, 119, 141), 2, 20, True, 1438300928, 1239298200),
     ("AcousticVTI1st", 4, (400, 1200), 16, 40, True, 875048448, 281972736),
     ("AcousticVTI1st", 8, (400, 1200), 16, 40, False, 734203392, 365707264),
     ("AcousticVTI1st3D", 4, (128, 128, 128), 1, 16, False, 477555712, 381602880),
