@@ -244,8 +244,8 @@ __global__ void finalize(const Geo G, const float* __restrict__ slots, int image
     }
 }
 
-// model fields of the steps, pitched
-__global__ void prep(const Geo G, long long rows, float* __restrict__ cf, float* __restrict__ ca)
+// v^2 dt^2, pitched
+__global__ void prep(const Geo G, long long rows, float* __restrict__ cf)
 {
     const long long n = rows * G.P;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
@@ -253,7 +253,6 @@ __global__ void prep(const Geo G, long long rows, float* __restrict__ cf, float*
         const int x = (int)(k - row * G.P);
         const float v = x < G.nx ? G.vp[row * G.nx + x] : 0.f;
         cf[k] = ((v * v) * G.dt) * G.dt;
-        ca[k] = (v * v) * (G.dt * G.dt);
     }
 }
 
@@ -323,10 +322,10 @@ static Plan make_plan(const sweep_acoustic_desc* d, int mem_mode)
 }
 
 struct Ws {
-    float *cf, *ca;
+    float* cf;
     float* prof[3];
     float* u[3];                    // forward: u_prev, u, u_next; backward: reconstruction
-    float* l[3];                    // backward: adjoint
+    float* l[2];                    // backward: adjoint, two times of which the older is written over
     float* ps[2][3];                // CPML psi (forward) / adjoint psi, double-buffered
     float* zt[2][3];                // zeta (forward: [0] only) / adjoint zeta, double-buffered
     float *g, *is, *ir;             // backward: per-shot image, illumination slots
@@ -339,7 +338,6 @@ static void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
     const long long n = (long long)G.B * G.S;
     w = Ws{};
     w.cf = c.take<float>(pl.nm * G.S);
-    w.ca = c.take<float>(pl.nm * G.S);
     const int len[3] = {G.P + 2 * kGuard, G.ny + 2 * kGuard, G.nz + 2 * kGuard};
     for (int a = 0; a < 3; ++a) w.prof[a] = c.take<float>(4LL * len[a]);
     c.take<char>(0);
@@ -352,7 +350,7 @@ static void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
         for (int a = 0; a < 3; ++a)
             if (a != 1 || G.nd == 3) w.zt[s][a] = c.take<float>(n);
     if (rev) {
-        for (int k = 0; k < 3; ++k) w.l[k] = c.take<float>(n);
+        for (float*& p : w.l) p = c.take<float>(n);
         w.g = c.take<float>(n);
         w.is = c.take<float>(n);
         w.ir = c.take<float>(n);
@@ -363,13 +361,12 @@ static void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
 
 static long long slot_floats(const Plan& pl) { return (long long)pl.G.B * pl.G.ns; }
 
-// The tape's states hold the grid's cells alone, without the rows' pitch.
+// cells of the state of a tape
 static long long state_floats(const Geo& G) { return (long long)G.B * G.nz * G.ny * G.nx; }
 
 static void copy_state(const Geo& G, float* dst, int dst_pitch, const float* src, int src_pitch, cudaStream_t st)
 {
-    SWEEP_CUDA(cudaMemcpy2DAsync(dst, (size_t)dst_pitch * 4, src, (size_t)src_pitch * 4, (size_t)G.nx * 4,
-                                 (size_t)G.B * G.nz * G.ny, cudaMemcpyDeviceToDevice, st));
+    copy_rows(dst, dst_pitch, src, src_pitch, G.nx, (long long)G.B * G.nz * G.ny, st);
 }
 
 void sizes(const sweep_acoustic_desc* d, int mem_mode, int, int64_t* ws_bytes, int64_t* tape_bytes)
@@ -407,9 +404,9 @@ static unsigned blocks_of(long long n, int per)
 static void setup(const sweep_acoustic_desc* d, Plan& pl, const Ws& w, cudaStream_t st)
 {
     Geo& G = pl.G;
-    G.cf = w.cf; G.ca = w.ca;
+    G.cf = G.ca = w.cf;
     const long long rows = (long long)pl.nm * G.nz * G.ny;
-    prep<<<blocks_of(rows * G.P, 256), 256, 0, st>>>(G, rows, w.cf, w.ca);
+    prep<<<blocks_of(rows * G.P, 256), 256, 0, st>>>(G, rows, w.cf);
     const float* in[3][3] = {{d->ax, d->bx, d->dbx}, {d->ay, d->by, d->dby}, {d->az, d->bz, d->dbz}};
     const int n[3] = {G.nx, G.ny, G.nz};
     for (int a = 0; a < 3; ++a) {
@@ -500,7 +497,7 @@ static void backward_m(const sweep_acoustic_desc* d, Plan& pl, const float* adj,
     const float* tail = tp + (long long)G.nt * slot_floats(pl);
     copy_state(G, rp, G.P, tail + state_floats(G), G.nx, st);
     copy_state(G, rn, G.P, tail, G.nx, st);
-    float *lp = w.l[0], *ln = w.l[1], *lx = w.l[2];
+    float *lp = w.l[0], *ln = w.l[1];
     int cur = 0;
     const dim3 grid = cell_grid(G), block = cell_block(G);
     const unsigned cb = blocks_of(n, 256), srcb = (unsigned)(G.B * G.nsrc + 127) / 128;
@@ -510,7 +507,7 @@ static void backward_m(const sweep_acoustic_desc* d, Plan& pl, const float* adj,
         cudaStream_t s = sg.stream();
         const bool recon = it > 0;
         Rev A{};
-        A.ln = ln; A.lp = lp; A.lx = lx;
+        A.ln = ln; A.lp = A.lx = lp;
         for (int a = 0; a < 3; ++a) {
             A.ps[a] = w.ps[cur][a]; A.zt[a] = w.zt[cur][a];
             A.pso[a] = w.ps[cur ^ 1][a]; A.zto[a] = w.zt[cur ^ 1][a];
@@ -519,7 +516,7 @@ static void backward_m(const sweep_acoustic_desc* d, Plan& pl, const float* adj,
         A.slot = recon ? tp + (long long)(it - 1) * slot_floats(pl) : nullptr;
         A.g = w.g;
         rev<M, ND><<<grid, block, 0, s>>>(G, A);
-        const RevEv E{lx, recon ? rx : nullptr, rn, rp, adj, w.g, grad_wavelet, il ? 0 : 1};
+        const RevEv E{lp, recon ? rx : nullptr, rn, rp, adj, w.g, grad_wavelet, il ? 0 : 1};
         if (parts && one_launch(G)) {
             rev_events<<<dim3(1, G.B), kEventBlock, 0, s>>>(G, E, it, parts);
         } else {
@@ -530,7 +527,7 @@ static void backward_m(const sweep_acoustic_desc* d, Plan& pl, const float* adj,
             // u_tt without the source: out of the restored strips for the
             // illumination's read, then back everywhere
             if (recon && G.nsrc > 0) add_src<<<srcb, 128, 0, s>>>(G, rx, it, -1.f, 1);
-            illum<<<cb, 256, 0, s>>>(G, rx, rn, rp, lx, recon ? w.is : nullptr, w.ir);
+            illum<<<cb, 256, 0, s>>>(G, rx, rn, rp, lp, recon ? w.is : nullptr, w.ir);
             if (recon && G.nsrc > 0) {
                 add_src<<<srcb, 128, 0, s>>>(G, rx, it, 1.f, 1);
                 add_src<<<srcb, 128, 0, s>>>(G, rx, it, 1.f, 0);
@@ -538,7 +535,7 @@ static void backward_m(const sweep_acoustic_desc* d, Plan& pl, const float* adj,
         }
         SWEEP_LAUNCH_CHECK();
         sg.step_done();
-        { float* t = lp; lp = ln; ln = lx; lx = t; }
+        std::swap(lp, ln);
         { float* t = rp; rp = rn; rn = rx; rx = t; }
         cur ^= 1;
     }

@@ -32,7 +32,7 @@ struct Geo {
     // profiles by axis: a, b, d b, d a (centred difference of a), packed; the x
     // ones may be read kGuard floats past their ends
     const float *a[3], *b[3], *db[3], *da[3];
-    const float *cf, *ca;           // ((v v) dt) dt and (v v) (dt dt), pitched, per model copy
+    const float *cf, *ca;           // v^2 dt^2 of the forward and of the adjoint, pitched, per model copy
     const float* vp;                // the caller's models
     long long ms;                   // stride between model copies (0: one for every shot)
     int nsrc, nrec;
@@ -317,7 +317,7 @@ __device__ __forceinline__ void store_core(const Geo& G, const Cell<ND>& q, floa
 // ----------------------------------------------------------- reverse step
 struct Rev {
     const float *ln, *lp;           // lambda(it + 1), lambda(it + 2)
-    float* lx;                      // lambda(it)
+    float* lx;                      // lambda(it); may be lp's buffer, which a thread reads at its own cells alone
     const float *ps[3], *zt[3];     // adjoint CPML memories (read)
     float *pso[3], *zto[3];         // (written)
     const float *rn, *rp;           // u(it), u(it + 1)
@@ -410,7 +410,7 @@ __device__ __forceinline__ F4 axis_adj(const Geo& G, const Cell<ND>& q, const Re
 template <int M, int ND>
 __device__ __forceinline__ F4 adj_cells(const Geo& G, const Cell<ND>& q, const Rev& A, long long k, long long mi)
 {
-    const F4 l0 = v4::ldg(A.ln + k), lp = v4::ldg(A.lp + k);
+    const F4 l0 = v4::ldg(A.ln + k), lp = v4::ld(A.lp + k);
     F4 w = axis_adj<M, ND, 0>(G, q, A, k, mi);
     if constexpr (ND == 3) {
         const F4 t = axis_adj<M, ND, 1>(G, q, A, k, mi);

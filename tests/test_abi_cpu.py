@@ -593,6 +593,9 @@ WORKSPACES = [
     ("Acoustic", 8, (256, 768), 16, 40, False, 279406848, 70491648),
     ("Acoustic", 8, (200, 400), 8, 20, False, 65335296, 16557056),
     ("Acoustic", 8, (400, 1200), 1, 40, False, 53786880, 8309248),
+    ("Acoustic", 4, (256, 768), 16, 40, False, 315196416, 56624640),
+    ("Acoustic3D", 4, (101, 119, 141), 2, 20, False, 770538456, 168141200),
+    ("Acoustic3D", 4, (128, 128, 128), 4, 16, True, 1553777664, 366193408),
     ("Elastic", 8, (400, 1200), 16, 40, False, 620846848, 460817920),
     ("Elastic", 8, (400, 1200), 1, 40, False, 58973440, 28805120),
     ("Elastic", 4, (400, 1200), 16, 40, True, 1193233920, 352465920),
