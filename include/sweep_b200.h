@@ -37,7 +37,7 @@
 extern "C" {
 #endif
 
-#define SWEEP_B200_ABI_VERSION 8
+#define SWEEP_B200_ABI_VERSION 9
 
 #if defined(__GNUC__)
 #define SWEEP_B200_API __attribute__((visibility("default")))

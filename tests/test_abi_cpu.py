@@ -2,7 +2,10 @@
 declares, reports the right ABI version, and the host-side size query and
 argument checks work (no device work is issued)."""
 import ctypes
+import os
 import re
+import subprocess
+import sys
 from pathlib import Path
 
 import numpy as np
@@ -28,6 +31,17 @@ def test_library_exports_every_declared_symbol():
     for name in _declared():
         assert hasattr(lib, name), name
     assert lib.sweep_b200_abi_version() == _lib.ABI_VERSION
+
+
+def test_a_library_without_the_newest_entries_is_refused(tmp_path):
+    """The version before the convolution's backward entries: the loader asks for
+    a rebuild instead of failing on a missing symbol."""
+    src, lib = tmp_path / "old.c", tmp_path / "old.so"
+    src.write_text("int sweep_b200_abi_version(void) { return 8; }\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
+    run = subprocess.run([sys.executable, "-c", "from sweep_b200 import _lib; _lib.load()"], cwd=ROOT,
+                         env=dict(os.environ, SWEEP_B200_LIB=str(lib)), capture_output=True, text=True)
+    assert run.returncode and "rebuild it" in run.stderr
 
 
 def _desc(B=2, nz=40, nx=60, nt=10, nsrc=1, nrec=3, M=4):
