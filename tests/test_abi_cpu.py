@@ -33,11 +33,11 @@ def test_library_exports_every_declared_symbol():
     assert lib.sweep_b200_abi_version() == _lib.ABI_VERSION
 
 
-def test_a_library_without_the_newest_entries_is_refused(tmp_path):
-    """The version before the convolution's backward entries: the loader asks for
-    a rebuild instead of failing on a missing symbol."""
+def test_a_library_of_the_version_before_is_refused(tmp_path):
+    """Version 8 did not have the convolution's backward entries; its number
+    alone asks for a rebuild."""
     src, lib = tmp_path / "old.c", tmp_path / "old.so"
-    src.write_text("int sweep_b200_abi_version(void) { return 8; }\n")
+    src.write_text("".join(f"int {name}(void) {{ return 8; }}\n" for name in _declared()))
     subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
     run = subprocess.run([sys.executable, "-c", "from sweep_b200 import _lib; _lib.load()"], cwd=ROOT,
                          env=dict(os.environ, SWEEP_B200_LIB=str(lib)), capture_output=True, text=True)
