@@ -268,6 +268,7 @@ static Plan make_plan(const sweep_acoustic_desc* d, int mem_mode)
     SWEEP_REQUIRE(d->ndim == 2 || d->ndim == 3, "acoustic: ndim %d is not built", d->ndim);
     SWEEP_REQUIRE(d->M >= 1 && d->M <= MAXM, "acoustic: spatial orders 2 to %d are built (got order %d)", 2 * MAXM,
                   2 * d->M);
+    SWEEP_REQUIRE(d->M != 4, "acoustic: order 8 runs on kernels of its own");
     SWEEP_REQUIRE(mem_mode == SWEEP_MEM_BOUNDARY,
                   "acoustic order %d: boundary saving with fp32 strips in device memory is built for orders other "
                   "than 8 (mem_mode %d; checkpoints, reduced strip formats and the host tape run at order 8)",
@@ -551,7 +552,6 @@ static void backward_m(const sweep_acoustic_desc* d, Plan& pl, const float* adj,
     case 1: CALL(1); break;                                                        \
     case 2: CALL(2); break;                                                        \
     case 3: CALL(3); break;                                                        \
-    case 4: CALL(4); break;                                                        \
     case 5: CALL(5); break;                                                        \
     case 6: CALL(6); break;                                                        \
     default: CALL(7); break;                                                       \

@@ -136,29 +136,12 @@ struct Plan {
     bands::Bands bands;
 };
 
-// staggered first-derivative weights of half-width M (the closed form
-// a_m = (-1)^(m+1) / (2m - 1) prod_{n != m} |(2n-1)^2 / ((2n-1)^2 - (2m-1)^2)|,
-// reference operators/staggered.cuh), each rounded from the exact ratio
-static void staggered_weights(int M, float* c)
-{
-    for (int m = 1; m <= M; ++m) {
-        long long num = 1, den = 2 * m - 1;
-        for (int n = 1; n <= M; ++n) {
-            if (n == m) continue;
-            const long long a = (long long)(2 * n - 1) * (2 * n - 1), q = (long long)(2 * m - 1) * (2 * m - 1);
-            num *= a;
-            den *= a > q ? a - q : q - a;
-        }
-        const double v = (double)num / (double)den;
-        c[m] = (float)((m % 2 == 1) ? v : -v);
-    }
-}
-
 static Plan make_plan(const sweep_elastic_desc* d, int mem_mode)
 {
     SWEEP_REQUIRE(d != nullptr, "null descriptor");
     SWEEP_REQUIRE(d->M >= 1 && d->M <= MAXM, "elastic: spatial orders 2 to %d are built (got order %d)", 2 * MAXM,
                   2 * d->M);
+    SWEEP_REQUIRE(d->M != 4, "elastic: order 8 runs on kernels of its own");
     SWEEP_REQUIRE(mem_mode == SWEEP_MEM_BOUNDARY,
                   "elastic order %d: boundary saving with fp32 strips in device memory is built for orders other "
                   "than 8 (mem_mode %d; checkpoints, reduced strip formats and the host tape run at order 8)",
@@ -198,7 +181,7 @@ static Plan make_plan(const sweep_elastic_desc* d, int mem_mode)
     SWEEP_REQUIRE(G.z1 - G.z0 >= 2 && G.x1 - G.x0 >= 2, "elastic: the physical box must be at least 2 cells per axis");
     G.dt = d->dt; G.ihz = 1.f / d->dz; G.ihx = 1.f / d->dx;
     for (int k = 0; k <= MAXM; ++k) G.c[k] = 0.f;
-    staggered_weights(M, G.c);
+    v4::staggered_weights(M, G.c);
     G.az = d->az; G.bz = d->bz; G.azh = d->azh; G.bzh = d->bzh;
     const bool per_shot = d->model_stride != 0;
     SWEEP_REQUIRE(!per_shot || d->model_stride == cells, "elastic: model_stride must be 0 or nz * nx");
@@ -370,7 +353,6 @@ static void backward_m(const sweep_elastic_desc* d, Plan& pl, const float* adj, 
     case 1: CALL(1); break;           \
     case 2: CALL(2); break;           \
     case 3: CALL(3); break;           \
-    case 4: CALL(4); break;           \
     case 5: CALL(5); break;           \
     case 6: CALL(6); break;           \
     default: CALL(7); break;          \

@@ -104,5 +104,23 @@ __device__ __forceinline__ F4 diff_col(const float* p, int stride, const float* 
     return diff<M, PLUS>([&](int k) { return ldg(p + k * stride); }, c, inv);
 }
 
+// staggered first-derivative weights of half-width M (the closed form
+// a_m = (-1)^(m+1) / (2m - 1) prod_{n != m} |(2n-1)^2 / ((2n-1)^2 - (2m-1)^2)|,
+// reference operators/staggered.cuh), each rounded from the exact ratio
+inline void staggered_weights(int M, float* c)
+{
+    for (int m = 1; m <= M; ++m) {
+        long long num = 1, den = 2 * m - 1;
+        for (int n = 1; n <= M; ++n) {
+            if (n == m) continue;
+            const long long a = (long long)(2 * n - 1) * (2 * n - 1), q = (long long)(2 * m - 1) * (2 * m - 1);
+            num *= a;
+            den *= a > q ? a - q : q - a;
+        }
+        const double v = (double)num / (double)den;
+        c[m] = (float)((m % 2 == 1) ? v : -v);
+    }
+}
+
 }  // namespace v4
 }  // namespace sweep

@@ -737,24 +737,6 @@ struct Plan {
     const char* name;
 };
 
-// staggered first-derivative weights of half-width M (the closed form
-// a_m = (-1)^(m+1) / (2m - 1) prod_{n != m} |(2n-1)^2 / ((2n-1)^2 - (2m-1)^2)|,
-// reference operators/staggered.cuh), each rounded from the exact ratio
-inline void staggered_weights(int M, float* c)
-{
-    for (int m = 1; m <= M; ++m) {
-        long long num = 1, den = 2 * m - 1;
-        for (int n = 1; n <= M; ++n) {
-            if (n == m) continue;
-            const long long a = (long long)(2 * n - 1) * (2 * n - 1), q = (long long)(2 * m - 1) * (2 * m - 1);
-            num *= a;
-            den *= a > q ? a - q : q - a;
-        }
-        const double v = (double)num / (double)den;
-        c[m] = (float)((m % 2 == 1) ? v : -v);
-    }
-}
-
 template <int ND>
 Plan make_plan(const Desc& d, int mem_mode, const char* name)
 {
@@ -792,7 +774,7 @@ Plan make_plan(const Desc& d, int mem_mode, const char* name)
     SWEEP_REQUIRE(G.z1 - G.z0 >= 2 && (ND == 2 || G.y1 - G.y0 >= 2) && G.x1 - G.x0 >= 2,
                   "%s: the physical box must be at least 2 cells per axis", name);
     G.dt = d.dt; G.ihz = 1.f / d.dz; G.ihy = 1.f / d.dy; G.ihx = 1.f / d.dx;
-    staggered_weights(M, G.c);
+    v4::staggered_weights(M, G.c);
     const bool per_shot = d.model_stride != 0;
     SWEEP_REQUIRE(!per_shot || d.model_stride == cells, "%s: model_stride must be 0 or the cells of a shot", name);
     G.ms = per_shot ? G.S : 0;
