@@ -1742,7 +1742,8 @@ void sizes(const sweep_acoustic_desc* d, int mem_mode, int ckpt_every, int64_t* 
     check_mode(mem_mode, ckpt_every);
     Plan pl = make_plan(d, REVERSE);
     set_store(pl, mem_mode);
-    Plan plf = mem_mode == SWEEP_MEM_CHECKPOINT ? pl : make_plan(d, FORWARD);
+    const bool replays = mem_mode == SWEEP_MEM_CHECKPOINT || mem_mode == SWEEP_MEM_RECURSIVE;
+    Plan plf = replays ? pl : make_plan(d, FORWARD);
     set_store(plf, mem_mode);
     Carve cf(nullptr);
     carve_fwd(cf, plf);
@@ -1858,7 +1859,7 @@ void forward_with(const sweep_acoustic_desc* d, int mem_mode, int ckpt_every, fl
     SWEEP_REQUIRE(record != nullptr || d->nrec == 0, "acoustic2d forward: null record");
     SWEEP_REQUIRE(d->vp != nullptr, "acoustic2d forward: null vp");
     set_attrs();
-    Plan pl = make_plan(d, ckpt_every > 0 ? REVERSE : FORWARD);
+    Plan pl = make_plan(d, ckpt_every > 0 || mem_mode == SWEEP_MEM_RECURSIVE ? REVERSE : FORWARD);
     set_store(pl, ckpt_every > 0 ? SWEEP_MEM_CHECKPOINT : mem_mode);
     Carve c(ws);
     FwdWork w = carve_fwd(c, pl);
@@ -1941,8 +1942,7 @@ void forward(const sweep_acoustic_desc* d, int mem_mode, int ckpt_every, float* 
                   (long long)ws_bytes, (long long)need_ws);
     // recursive checkpointing keeps nothing from the forward: the backward
     // replays from the initial state
-    forward_with(d, mem_mode == SWEEP_MEM_RECURSIVE ? SWEEP_MEM_BOUNDARY : mem_mode,
-                 mem_mode == SWEEP_MEM_CHECKPOINT ? ckpt_every : 0, record,
+    forward_with(d, mem_mode, mem_mode == SWEEP_MEM_CHECKPOINT ? ckpt_every : 0, record,
                  mem_mode == SWEEP_MEM_RECURSIVE ? nullptr : tape, ws, ws_bytes, st, nullptr, nullptr, 0, 0);
 }
 

@@ -178,3 +178,26 @@ def test_elastic3d_recursive_checkpointing(count):
     for name, a, b in zip(("vp", "vs", "rho"), g_rc, g_ck):
         assert np.array_equal(a, b)
         assert rel(a, d["grad_" + name]) < GRAD_TOL
+
+
+def test_recursive_equals_chunks_where_the_passes_run_other_kernels():
+    """493 shots of 65 x 65: the forward of a plain call runs the tiled kernels,
+    the reverse those of small grids, and both checkpoint modes the reverse's."""
+    from sweep_b200 import Acoustic, Ckpt, PropTorch
+    rng = np.random.default_rng(2)
+    B, shape, nt = 493, (65, 65), 80
+    src, rec = rng.integers(5, 60, (B, 2)), rng.integers(0, 65, (B, 3, 2))
+    w = torch.tensor(rng.standard_normal(nt), dtype=torch.float32, device=DEV)
+    vp = torch.tensor(2500 + 100 * rng.standard_normal(shape), dtype=torch.float32, device=DEV)
+    out = []
+    for memory in (Ckpt(chunks=64), Ckpt(mode="recursive", count=1), None):
+        s = PropTorch(Acoustic(spatial_order=8, device=DEV), shape=shape, dh=10.0, dt=1e-3, abcn=5, device=DEV,
+                      memory=memory)
+        v = vp.clone().requires_grad_(True)
+        pred = s(w, src, rec, models=[v])
+        assert s.launch_schedule(nt, src, rec, [vp])["tile_y"] == 0
+        pred.square().sum().backward()
+        out.append((pred.detach(), v.grad))
+    (ra, ga), (rb, gb), (rc, gc) = out
+    assert torch.equal(ra, rb) and torch.equal(ga, gb)
+    assert rel(rc.cpu(), ra.cpu()) < 1e-5 and rel(gc.cpu(), ga.cpu()) < 1e-4
