@@ -1035,7 +1035,7 @@ __global__ void __launch_bounds__(SNTH) rev_small(const __grid_constant__ avec::
                 u0 = v4::ldg(rnow + k);
                 up = v4::ldg(rprev + k);
                 const bool rrow = z >= P.rz0 && z < P.rz1;
-                if (rrow && x + 3 >= P.rx0 && x < P.rx1) un = avec::recon_cells<M, 2>(G, rnow, k, mi, u0, up);
+                if (rrow && x + 3 >= P.rx0 && x < P.rx1) un = avec::recon_cells<M, 2>(G, rnow, k, v4::ldg(G.cf + mi), u0, up);
 #pragma unroll
                 for (int l = 0; l < 4; ++l)
                     if (phys[l] && !(rrow && x + l >= P.rx0 && x + l < P.rx1))

@@ -32,8 +32,8 @@
 // 52 us reverse (31 and 66 + 31 + 14 us in nine launches with one cell per
 // thread; 8.5 and 26 us of field traffic at the copy rate), a 101 x 119 x 141
 // grid's with two shots 70 and 124 us (123 and 296 us; 20 and 50 us).  Bound
-// by latency at 64 registers a thread and, in the layers, by the memories'
-// taps.
+// by latency at 64 registers a thread (`rev` spills 84 bytes in 2-D and 136 in
+// 3-D for them) and, in the layers, by the memories' taps.
 // Memory: boundary saving with fp32 strips in device memory (SWEEP_MEM_BOUNDARY).
 #include <cuda_runtime.h>
 
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kThreads, blocks_for(M)) rev(const Geo G, cons
     if (!any) return;
     const F4 u0 = v4::ldg(A.rn + k), up = v4::ldg(A.rp + k);
     F4 un = u0;
-    if (rec[0] || rec[1] || rec[2] || rec[3]) un = recon_cells<M, ND>(G, A.rn, k, mi, u0, up);
+    if (rec[0] || rec[1] || rec[2] || rec[3]) un = recon_cells<M, ND>(G, A.rn, k, coef<ND>(G, q), u0, up);
     const float* slot = A.slot + (long long)q.b * G.ns;
     F4 g = v4::ld(A.g + k);
     bool all = true;
@@ -244,15 +244,16 @@ __global__ void finalize(const Geo G, const float* __restrict__ slots, int image
     }
 }
 
-// v^2 dt^2, pitched
-__global__ void prep(const Geo G, long long rows, float* __restrict__ cf)
+// the model field of a pass, pitched: cf of the forward, ca of the reverse (whose
+// reconstruction takes cf from the caller's models: a field less per model)
+__global__ void prep(const Geo G, long long rows, int rev, float* __restrict__ c)
 {
     const long long n = rows * G.P;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
         const long long row = k / G.P;
         const int x = (int)(k - row * G.P);
         const float v = x < G.nx ? G.vp[row * G.nx + x] : 0.f;
-        cf[k] = ((v * v) * G.dt) * G.dt;
+        c[k] = rev ? (v * v) * (G.dt * G.dt) : ((v * v) * G.dt) * G.dt;
     }
 }
 
@@ -323,7 +324,7 @@ static Plan make_plan(const sweep_acoustic_desc* d, int mem_mode)
 }
 
 struct Ws {
-    float* cf;
+    float* model;
     float* prof[3];
     float* u[3];                    // forward: u_prev, u, u_next; backward: reconstruction
     float* l[2];                    // backward: adjoint, two times of which the older is written over
@@ -338,7 +339,7 @@ static void carve(Carve& c, const Plan& pl, bool rev, Ws& w)
     const Geo& G = pl.G;
     const long long n = (long long)G.B * G.S;
     w = Ws{};
-    w.cf = c.take<float>(pl.nm * G.S);
+    w.model = c.take<float>(pl.nm * G.S);
     const int len[3] = {G.P + 2 * kGuard, G.ny + 2 * kGuard, G.nz + 2 * kGuard};
     for (int a = 0; a < 3; ++a) w.prof[a] = c.take<float>(4LL * len[a]);
     c.take<char>(0);
@@ -381,8 +382,8 @@ void sizes(const sweep_acoustic_desc* d, int mem_mode, int, int64_t* ws_bytes, i
     *tape_bytes = ((long long)pl.G.nt * slot_floats(pl) + 2 * state_floats(pl.G)) * 4;
 }
 
-// Rows of a 2-D block: 32, or 8 where that leaves the GPU with less than a
-// block per SM (a small grid's step is one round of memory latency, and lasts
+// Rows of a 2-D block: 32, or 8 where that leaves the GPU with less than two
+// blocks per SM (a small grid's step is one round of memory latency, and lasts
 // as long as its fullest SM).
 static int rows_of(const Geo& G)
 {
@@ -402,12 +403,12 @@ static unsigned blocks_of(long long n, int per)
     return (unsigned)std::max<long long>(std::min<long long>((n + per - 1) / per, 8192), 1);
 }
 
-static void setup(const sweep_acoustic_desc* d, Plan& pl, const Ws& w, cudaStream_t st)
+static void setup(const sweep_acoustic_desc* d, Plan& pl, const Ws& w, bool rev, cudaStream_t st)
 {
     Geo& G = pl.G;
-    G.cf = G.ca = w.cf;
+    (rev ? G.ca : G.cf) = w.model;
     const long long rows = (long long)pl.nm * G.nz * G.ny;
-    prep<<<blocks_of(rows * G.P, 256), 256, 0, st>>>(G, rows, w.cf);
+    prep<<<blocks_of(rows * G.P, 256), 256, 0, st>>>(G, rows, rev, w.model);
     const float* in[3][3] = {{d->ax, d->bx, d->dbx}, {d->ay, d->by, d->dby}, {d->az, d->bz, d->dbz}};
     const int n[3] = {G.nx, G.ny, G.nz};
     for (int a = 0; a < 3; ++a) {
@@ -439,7 +440,7 @@ static void forward_m(const sweep_acoustic_desc* d, Plan& pl, float* record, voi
     carve(c, pl, false, w);
     SWEEP_REQUIRE(ws != nullptr && c.off <= ws_bytes, "acoustic forward: workspace too small (%lld < %lld bytes)",
                   (long long)ws_bytes, (long long)c.off);
-    setup(d, pl, w, st);
+    setup(d, pl, w, false, st);
     const Geo& G = pl.G;
     if (G.nrec == 0) record = nullptr;
     if (record) SWEEP_CUDA(cudaMemsetAsync(record, 0, sizeof(float) * (size_t)G.B * G.nt * G.nrec, st));
@@ -486,7 +487,7 @@ static void backward_m(const sweep_acoustic_desc* d, Plan& pl, const float* adj,
     SWEEP_REQUIRE(ws != nullptr && c.off <= ws_bytes, "acoustic backward: workspace too small (%lld < %lld bytes)",
                   (long long)ws_bytes, (long long)c.off);
     SWEEP_REQUIRE(tape != nullptr, "acoustic backward: the forward's tape is required");
-    setup(d, pl, w, st);
+    setup(d, pl, w, true, st);
     const Geo& G = pl.G;
     if (G.nsrc == 0) grad_wavelet = nullptr;
     if (grad_wavelet)

@@ -32,7 +32,7 @@ struct Geo {
     // profiles by axis: a, b, d b, d a (centred difference of a), packed; the x
     // ones may be read kGuard floats past their ends
     const float *a[3], *b[3], *db[3], *da[3];
-    const float *cf, *ca;           // v^2 dt^2 of the forward and of the adjoint, pitched, per model copy
+    const float *cf, *ca;           // ((v v) dt) dt and (v v) (dt dt), pitched, per model copy
     const float* vp;                // the caller's models
     long long ms;                   // stride between model copies (0: one for every shot)
     int nsrc, nrec;
@@ -424,9 +424,24 @@ __device__ __forceinline__ F4 adj_cells(const Geo& G, const Cell<ND>& q, const R
     return lx;
 }
 
-// (2 u(it) - u(it+1)) + v^2 dt^2 Lap u(it) of a group
+// the forward's coefficient of a group from the caller's models, which are not
+// pitched (a reverse that keeps one pitched model field keeps the adjoint's)
+template <int ND>
+__device__ __forceinline__ F4 coef(const Geo& G, const Cell<ND>& q)
+{
+    const long long row = ((G.ms ? (long long)q.b * G.nz : 0) + q.c[2]) * G.ny + q.c[1];
+    F4 c;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        const float v = __ldg(G.vp + row * G.nx + min(q.c[0] + l, G.nx - 1));
+        c.v[l] = ((v * v) * G.dt) * G.dt;
+    }
+    return c;
+}
+
+// (2 u(it) - u(it+1)) + cf Lap u(it) of a group
 template <int M, int ND>
-__device__ __forceinline__ F4 recon_cells(const Geo& G, const float* rn, long long k, long long mi, const F4& u0,
+__device__ __forceinline__ F4 recon_cells(const Geo& G, const float* rn, long long k, const F4& cf, const F4& u0,
                                           const F4& up)
 {
     Line<M, 0> x;
@@ -441,7 +456,7 @@ __device__ __forceinline__ F4 recon_cells(const Geo& G, const float* rn, long lo
 #pragma unroll
         for (int l = 0; l < 4; ++l) w.v[l] += t.v[l];
     }
-    const F4 t = lap<M, 2>(z, G), cf = v4::ldg(G.cf + mi);
+    const F4 t = lap<M, 2>(z, G);
     F4 un;
 #pragma unroll
     for (int l = 0; l < 4; ++l) un.v[l] = (2.f * u0.v[l] - up.v[l]) + cf.v[l] * (w.v[l] + t.v[l]);
