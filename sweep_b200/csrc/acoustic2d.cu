@@ -1806,7 +1806,7 @@ static FwdMaps fwd_maps(const FwdWork& w, const Params& P)
     return maps;
 }
 
-// Forward steps [it0, it1): one fwd_kernel launch per step; `strips_of(it)`
+// Forward steps [it0, it1): one launch per step; `strips_of(it)`
 // is the strip slot step `it` writes (null: none), `record` may be null.
 template <class StripsOf>
 static void forward_steps(const Plan& pl, const FwdMaps& maps, const FwdWork& w, float* record, FwdState& S,
@@ -1861,6 +1861,7 @@ void forward_with(const sweep_acoustic_desc* d, int mem_mode, int ckpt_every, fl
     set_attrs();
     Plan pl = make_plan(d, ckpt_every > 0 || mem_mode == SWEEP_MEM_RECURSIVE ? REVERSE : FORWARD);
     set_store(pl, ckpt_every > 0 ? SWEEP_MEM_CHECKPOINT : mem_mode);
+    if (stepped) same_layout(*seg, a == 0, 2 * pl.nslot + pl.small);
     Carve c(ws);
     FwdWork w = carve_fwd(c, pl);
     SWEEP_REQUIRE(ws != nullptr && ws_bytes >= c.off, "acoustic2d forward: workspace too small (%lld < %lld)",
@@ -2057,6 +2058,7 @@ void backward_with(const sweep_acoustic_desc* d, int mem_mode, int ckpt_every, c
     const bool recursive = mem_mode == SWEEP_MEM_RECURSIVE;
     SWEEP_REQUIRE(!stepped || (!ckpt && !recursive), "acoustic2d stepped backward: boundary saving only");
     const bool first = top == d->nt;
+    if (stepped) same_layout(*seg, first, 2 * pl.nslot + pl.small);
     RevWork w;
     FwdWork fw{};
     float* chunk = nullptr;

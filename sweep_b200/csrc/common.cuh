@@ -262,9 +262,18 @@ private:
 struct StepState {
     int next = 0;            // forward: next step; backward: the step above the next segment
     bool begun = false;      // the first segment has run (fields set up)
+    int layout = 0;          // what the first segment's schedule made of the workspace
     int idx[8] = {};
     void* ptr[8] = {};
 };
+
+// A schedule recorded between two segments of a stepped run must not lay the
+// workspace out anew: the kernels' tables and the image slots size it.
+inline void same_layout(StepState& seg, bool first, int layout)
+{
+    if (first) seg.layout = layout;
+    SWEEP_REQUIRE(seg.layout == layout, "runner: the launch schedule changed between the segments of a run");
+}
 
 // Source / receiver events grouped by (shot, tile): a CSR table so that the
 // CTA owning a tile finds its point sources and receivers without scanning the

@@ -1404,6 +1404,7 @@ static void backward_with(const sweep_elastic_desc* d, int mem_mode, int ckpt_ev
     const bool recursive = mem_mode == SWEEP_MEM_RECURSIVE;
     SWEEP_REQUIRE(!stepped || (!ckpt && !recursive), "elastic2d stepped backward: boundary saving only");
     Plan pl = make_plan(d);
+    if (stepped) same_layout(*seg, first, pl.gshots);
     set_store(pl, mem_mode);
     Carve c(ws);
     RevWs w{};

@@ -144,3 +144,29 @@ def test_refusals():
     with pytest.raises(ValueError, match="boundary saving"):
         _solver(d, Ckpt(chunks=20)).forward_runner(torch.tensor(d["wavelet"], device=DEV), d["src"], d["rec"],
                                                    models=_models(d))
+
+
+@pytest.mark.parametrize("name, schedule", [("acoustic2d_multi", {"tile_y": 32}), ("elastic2d", {"shots_rev": 2})])
+def test_a_schedule_change_between_segments_is_refused(name, schedule):
+    """These schedules lay the workspace out in fewer bytes than the built-in
+    choice, so that it would be large enough: with the fields and the image
+    slots elsewhere."""
+    from sweep_b200 import autotune
+    d = load(name)
+    s = _solver(d)
+    autotune.clear_schedules()
+    try:
+        r = s.forward_runner(torch.tensor(d["wavelet"], device=DEV), d["src"], d["rec"], models=_models(d))
+        r.run(0, r.nt)
+        br = r.backward_runner(torch.ones_like(r.record))
+        br.run(r.nt, r.nt - 10)
+        autotune.set_schedule(r.desc, schedule)
+        with pytest.raises(RuntimeError, match="schedule changed"):
+            br.run(r.nt - 10, 0)
+        autotune.clear_schedules()
+        br.run(r.nt - 10, 0)
+        assert float(br.gradients()[0].abs().max()) > 0
+        r.close()
+        br.close()
+    finally:
+        autotune.clear_schedules()
