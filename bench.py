@@ -105,11 +105,13 @@ E_NZ, E_NX, E_NT, E_DT, E_DH, E_ABCN = 400, 1200, 4000, 0.0005, 5.0, 40
 E_NSHOT, E_NREC, E_F0, E_DELAY = 16, 600, 10.0, 0.12
 E_RT = (E_NZ + 2 * E_ABCN + 2 * M, E_NX + 2 * E_ABCN + 2 * M)
 # algorithmic bytes per runtime cell-step: forward velocity 7 floats + stress
-# 8; reverse transpose into the adjoint velocities 9, stress reconstruction with
-# its image 11, transpose into the adjoint stresses 11, velocity reconstruction
-# 9 (one read and one write of every field a kernel touches; CPML memories,
-# gradient slots and the shared, L2-resident models not counted)
-E_BYTES_FWD, E_BYTES_REV = 60, 160
+# 8; reverse transpose into the adjoint velocities 3 q read, 2 p read and written
+# (7), stress reconstruction with its image 2 + 6 + 3 (11), transpose into the
+# adjoint stresses 2 p read, 2 stresses and the shear's q read and written, 2 q
+# written (10), velocity reconstruction 3 + 4 + 2 (9) (one read and one write of
+# every field a kernel touches; CPML memories, gradient slots and the shared,
+# L2-resident models not counted)
+E_BYTES_FWD, E_BYTES_REV = 60, 148
 
 
 def elastic_survey(seed=SEED):
@@ -138,8 +140,8 @@ def elastic_survey(seed=SEED):
 # field a kernel touches; CPML memories and the models not counted): forward
 # velocity 6 floats + stress 6; reverse half-step A with the stress
 # reconstruction 12, half-step B with the velocity reconstruction 12, gradient
-# slots (four, each shared by four shots) 2.
-V_BYTES_FWD, V_BYTES_REV = 48, 104
+# slots and the step's e (ten accesses, shared by four shots) 2.5.
+V_BYTES_FWD, V_BYTES_REV = 48, 106
 
 
 def vti_survey(seed=SEED):
@@ -541,10 +543,11 @@ E3_RT = (E3_N + 2 * E3_ABCN + 2 * M,) * 3
 # field a kernel touches; models and CPML memories not counted): forward
 # velocity step 6 stresses read + 3 velocities read and written (12), stress
 # step 3 + 6 + 6 (15); reverse: stress reconstruction with its image 3 + 12 + 6
-# (21), transpose into the adjoint velocities 6 q read, 6, 3 p written (15),
-# into the adjoint stresses 3 + 12 + 6 (21), velocity reconstruction 6 + 6 + 3
-# (15), three gradient slots shared by the shots of a thread 2 (74)
-E3_BYTES_FWD, E3_BYTES_REV = 4 * 27, 4 * 74
+# (21), transpose into the adjoint velocities 6 q read, 3 p read and written
+# (12), into the adjoint stresses 3 p read, 3 stresses and 3 shears of q read and
+# written, 3 q written (18), velocity reconstruction 6 + 6 + 3 (15), three
+# gradient slots shared by the shots of a thread 2 (68)
+E3_BYTES_FWD, E3_BYTES_REV = 4 * 27, 4 * 68
 
 
 def elastic3d_survey(seed=SEED):
@@ -637,9 +640,9 @@ class Elastic3DWorkload:
 # counted): forward velocity step 2 stresses read + 3 velocities read and
 # written (8), stress step 3 + 4 (7); reverse: half-step A with the stress
 # reconstruction 3 + 4 + 2 + 6 (15), half-step B with the velocity
-# reconstruction 2 + 6 + 3 + 4 (15), gradient slots (four, each shared by four
-# shots) 2 (32).
-V3_BYTES_FWD, V3_BYTES_REV = 4 * 15, 4 * 32
+# reconstruction 2 + 6 + 3 + 4 (15), gradient slots and the step's e (ten
+# accesses, shared by four shots) 2.5 (32.5).
+V3_BYTES_FWD, V3_BYTES_REV = 4 * 15, 130
 
 
 def vti3d_survey(seed=SEED):

@@ -920,8 +920,8 @@ __global__ void __launch_bounds__(NTH, 2) rev_kernel(const __grid_constant__ Rev
 // The same steps on grids that fill no GPU with 64 x 32 tiles: one group of
 // four cells per thread (acoustic_vec.cuh), 32 x 8 cells per CTA of 64
 // threads, every load of a step issued at once instead of stage by stage.
-// Such a step is latency, not bandwidth: 96 x 128, one shot, forward 3.9 us
-// and reverse 6.5 us a step (12.3 and 18.5 us on the tiled kernels).  A CTA
+// Such a step is latency, not bandwidth: 96 x 128, one shot, forward 4.0 us
+// and reverse 6.7 us a step (12.3 and 18.5 us on the tiled kernels).  A CTA
 // walks the P.G shots of its group, whose image it sums before it adds it to
 // the group's slot, as the tiled kernels do.
 constexpr int SNTH = SX / 4 * SZ;

@@ -29,9 +29,9 @@
 // and written, only where its profile reaches.
 //
 // Measured, order 4: the 16-shot 256 x 768 survey's steps 24 us forward and
-// 52 us reverse (31 and 66 + 31 + 14 us in nine launches with one cell per
+// 48 us reverse (31 and 66 + 31 + 14 us in nine launches with one cell per
 // thread; 8.5 and 26 us of field traffic at the copy rate), a 101 x 119 x 141
-// grid's with two shots 70 and 124 us (123 and 296 us; 20 and 50 us).  Bound
+// grid's with two shots 71 and 123 us (123 and 296 us; 20 and 50 us).  Bound
 // by latency at 64 registers a thread (`rev` spills 84 bytes in 2-D and 136 in
 // 3-D for them) and, in the layers, by the memories' taps.
 // Memory: boundary saving with fp32 strips in device memory (SWEEP_MEM_BOUNDARY).

@@ -585,11 +585,14 @@ __global__ void __launch_bounds__(kQB) quant3(const Geo G, const Fields F, void*
 // no pass of its own prepares them and the stencils read one field per tap; a
 // band's taps add the adjoint memory, which is therefore double-buffered.
 // (q and p formed at every tap from lambda, the stiffness and 1 / rho instead:
-// 666 + 556 us a step against 366 + 301 on the 2-shot 128^3 survey at order 8.)  The rho image of step `it` is
-// lambda_v . (v(it - 1) - v(it)): inside, minus kv lambda_v . div s (what the
-// reconstruction takes back), on the box's outermost layer the difference of
-// the restored strips (`restore_velocity`).  The image of the update of step
-// 1 is left out, as by the reference's staggered reverse.
+// 666 + 556 us a step against 337 + 283 on the 2-shot 128^3 survey at order 8.)
+// The rho image of step `it` is lambda_v . (v(it - 1) - v(it)): inside, minus
+// kv lambda_v . div s (what the reconstruction takes back), on the box's
+// outermost layer the difference of the restored strips (`restore_velocity`).
+// The image of the update of step 1 is left out, as by the reference's
+// staggered reverse.  All four kernels wait for loads (DRAM at 28 to 45 %); the
+// bound of 64 registers makes adj_vel spill 428 bytes, stress_rev 368 and
+// vel_rev 160, a quarter to two fifths of their L1 traffic.
 struct Rev {
     Geo G;
     Models m;
@@ -1113,8 +1116,8 @@ static Plan make_plan(const sweep_elastic3d_desc* d)
     G.ms = per_shot ? G.S : 0;
     pl.nm = per_shot ? d->B : 1;
     G.nbx = (G.nx + 31) / 32;
-    // shots per imaging thread: as many as still leave four blocks per SM; one
-    // for per-shot models
+    // shots per imaging thread: as many as still leave each SM four pairs of
+    // blocks along y, which is all it holds; one for per-shot models
     const long long blocks = (long long)G.nbx * ((G.ny + 7) / 8) * ((G.nz + 3) / 4);
     G.group = 1;
     if (!per_shot)

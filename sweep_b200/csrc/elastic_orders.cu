@@ -1,8 +1,9 @@
 // elastic_orders.cu -- the 2-D isotropic elastic forward and boundary-saving
 // adjoint at every spatial order but 8 (M = 1..7: orders 2, 4, 6, 10, 12,
-// 14), for sm_100a.  Order 8 runs the tiled kernels of elastic2d.cu; the
-// reference's Elastic defaults to order 4, so a drop-in caller lands here
-// unless it asks for order 8.
+// 14), for sm_100a.  Order 8 runs through elastic2d.cu: its forward on tiled
+// kernels, its reverse on those of elastic_vec.cuh as here.  The reference's
+// Elastic defaults to order 4, so a drop-in caller lands here unless it asks
+// for order 8.
 //
 // Restates the reference's templated elastic2d path (src/sweep/csrc/cuda/
 // equations/elastic2d/kernels.cuh, common/sg_driver.cuh step order,
@@ -34,10 +35,9 @@
 // by the reference's staggered reverse.
 //
 // Measured at order 4: 8 shots of 187 x 331 with a free top face, 300 steps,
-// 18.9 ms a gradient (51 ms on fourteen launches of one cell per thread a
-// reverse step): 14 + 13 us the two reverse kernels, 7 + 9 us the forward's;
-// 16 shots of 400 x 1200: 187 + 170 and 68 + 77 us.  The small grid is bound
-// by latency and launches, the large one by latency at 64 registers.
+// 18.5 ms a gradient (51 ms on fourteen launches of one cell per thread a
+// reverse step): 14 + 12 us the two reverse kernels, 7 + 9 us the forward's.
+// The small grid is bound by latency and launches.
 // Memory: boundary saving with fp32 bands in device memory (SWEEP_MEM_BOUNDARY).
 #include <cuda_runtime.h>
 

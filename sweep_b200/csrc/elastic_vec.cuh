@@ -4,13 +4,16 @@
 // faces (FS) by the image method.  Shared by the orders other than 8
 // (elastic_orders.cu) and by the reverse of order 8 (elastic2d.cu).
 //
-// Measured at order 8 on 16 shots of 400 x 1200: 219 us rev_a, 208 us
-// rev_b and 34 us the restores and events, where 32 x 32 tiles of one cell per
+// Measured at order 8 on 16 shots of 400 x 1200: 205 us rev_a, 194 us
+// rev_b and 45 us the restores and events, where 32 x 32 tiles of one cell per
 // thread and row, with q and p rebuilt in shared memory for tile and halo, took
-// 652 us a step.  A reverse kernel moves 80 bytes a cell: 123 us at the copy
-// rate; the rest is load latency at 64 registers a thread, 1024 threads an SM.
+// 652 us a step.  A reverse kernel moves 68 bytes a cell: 105 us at the copy
+// rate; its warps wait for loads (long scoreboard 12 to 13 an issue, DRAM at 42
+// and 47 %) at 64 registers a thread, 1024 threads an SM, a bound that spills
+// 192 and 80 bytes at order 8, a fifth and a tenth of the L1 traffic.
 // The image of up to four shots is summed by a thread (layout): 187 + 170 us
-// against 198 + 175 us with a slot per shot, at order 4 on the same grid.
+// against 198 + 175 us with a slot per shot, at order 4 on the same grid (both
+// with the adjoint velocities beside p, 80 bytes a cell).
 #pragma once
 
 #include <algorithm>

@@ -30,7 +30,9 @@
 // gradient is summed as e = c11 lsH dh + c33 lsV dvz + c13 (lsH dvz + lsV dh),
 // lsH dh, lsH dvz + lsV dh and e - lambda_v . grad s / rho (half A leaves a
 // step's e for half B: the two parts cancel, so the slot takes their difference,
-// not one after the other); the models' chain rule is applied once, at the end.
+// not one after the other, which put the density gradient 1.07 and 1.09 times
+// as far from 64 bits over 24 seeds of a 90 x 121 grid and 16 of a 40 x 36 x 44
+// one); the models' chain rule is applied once, at the end.
 // Shots that share a model run in groups inside a thread, which reads the
 // stiffness and updates the gradient slots once per group.
 //
@@ -38,10 +40,11 @@
 // (x, y) cells in 3-D and 32 x 4 (x, z) cells in 2-D.  A memory holds the cells
 // where its axis has a damping profile.
 //
-// Bound by field traffic in the forward (velocity step of the 4-shot 128^3
-// survey: 17.6 M cells, 132 us, 289 us with one cell per thread, 100 us of
-// traffic at the copy rate) and by latency at 64 registers in the reverse (a
-// step 612 us, 1110 us before; 390 us of traffic).
+// 4-shot 128^3 survey at order 4 (17.6 M cells): velocity step 130 us (289 us
+// with one cell per thread; 87 us of field traffic at the copy rate), a reverse
+// step 604 us and its bands 58 us (1110 us before; 345 us of traffic).  The
+// reverse waits for loads (long scoreboard 18 to 21 an issue, DRAM at 40 and 47 %)
+// at 64 registers, for which half_a spills 196 bytes, a fifth of its L1 traffic.
 #pragma once
 
 #include <algorithm>

@@ -679,13 +679,14 @@ class PropTorch(torch.nn.Module):
         geo, padded, wb, fields = self._probe(wavelet_len, sources, receivers, models)
         desc = self._desc(geo, padded, wb, fields)
         if isinstance(desc, _lib.Elastic3DDesc):
-            return {"fixed": "one thread per cell, 32 x 4 x 2 cell blocks, two z planes of a shot per grid row"}
+            return {"fixed": "four x cells per thread, 32 x 4 x 4 cell blocks per shot"}
         if isinstance(desc, _lib.VTIDesc):
-            return {"fixed": "one thread per cell, 32 x 8 cell tiles per shot"}
+            return {"fixed": "four x cells per thread, 32 x 32 cell blocks per shot"}
         if isinstance(desc, _lib.VTI3DDesc):
-            return {"fixed": "one thread per cell, 32 x 4 x 2 cell blocks, two z planes of a shot per grid row"}
+            return {"fixed": "four x cells per thread, 32 x 8 x 4 cell blocks per shot"}
         if desc.M != 4:
-            return {"fixed": f"order {2 * desc.M}: one thread per cell, 32 x 8 cell tiles per plane and shot"}
+            blocks = "32 x 8 x 4" if geo.ndim == 3 else "32 x 32 (32 x 8 on small grids)"
+            return {"fixed": f"order {2 * desc.M}: four x cells per thread, {blocks} cell blocks per shot"}
         return autotune.get_schedule(desc)
 
     def tape_bytes(self, wavelet_len, sources, receivers, models):

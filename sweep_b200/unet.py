@@ -2,8 +2,8 @@
 
 The network maps ``[gradient, source illumination, current vp]`` (each
 standardised) to a vp update.  Every 3x3 convolution runs on the tensor cores
-through ``sweep_b200_conv3x3_gemm`` / ``sweep_b200_conv3x3_wgrad``: BF16
-activations and weights, FP32 accumulation; master weights, biases and the
+through ``sweep_b200_conv3x3_gemm`` forward and ``sweep_b200_conv3x3_backward``:
+BF16 activations and weights, FP32 accumulation; master weights, biases and the
 optimiser state stay FP32.  Pooling, upsampling, concatenation and GELU are
 plain tensor operations around them.  The reference has no learned
 component; the convolutions are checked against PyTorch's float32 ``conv2d``.

@@ -158,7 +158,7 @@ def test_elastic_sizes_and_errors():
     ws, tape = _lib.c_i64(), _lib.c_i64()
     _lib.call("sweep_b200_elastic_sizes", d, _lib.MEM_BOUNDARY, 0, ws, tape)
     n = 2 * 40 * 64                                  # pitched to 64 columns
-    assert ws.value >= 17 * n * 4                    # 5 forward + 2 carriers + 5 adjoint + 3 x 2 gradient slots
+    assert ws.value >= 17 * n * 4                    # 5 forward + 7 adjoint + 3 gradient slots a shot, memories
     pz, px = 40 - 18, 60 - 18
     nstrip = 2 * 4 * px + 2 * (px + 8) + (pz - 2) * 10
     assert tape.value >= (10 * 2 * 5 * nstrip + 5 * n) * 4
@@ -537,7 +537,7 @@ def test_vti_sizes_and_refusals():
     ws, tape = _lib.c_i64(), _lib.c_i64()
     _lib.call("sweep_b200_vti_sizes", d, _lib.MEM_BOUNDARY, 0, ws, tape)
     assert tape.value > 50 * 4 * 4 and ws.value > 0
-    assert s.launch_schedule(50, src, rec, models) == {"fixed": "one thread per cell, 32 x 8 cell tiles per shot"}
+    assert s.launch_schedule(50, src, rec, models) == {"fixed": "four x cells per thread, 32 x 32 cell blocks per shot"}
     for mode in (_lib.MEM_CHECKPOINT, _lib.MEM_BOUNDARY_FP16, _lib.MEM_BOUNDARY | _lib.MEM_HOST_TAPE):
         with pytest.raises(RuntimeError, match="boundary saving with fp32 strips"):
             _lib.call("sweep_b200_vti_sizes", d, mode, 10, ws, tape)
@@ -583,7 +583,7 @@ def test_vti3d_sizes_and_refusals():
         box[z0:z0 + 10, y0:y0 + 12, lo:hi] = True
     assert tape.value == 4 * (50 * 5 * int(box.sum()) + 5 * 20 * 22 * 24)
     assert s.launch_schedule(50, src, rec, models) == {
-        "fixed": "one thread per cell, 32 x 4 x 2 cell blocks, two z planes of a shot per grid row"}
+        "fixed": "four x cells per thread, 32 x 8 x 4 cell blocks per shot"}
     for mode in (_lib.MEM_CHECKPOINT, _lib.MEM_BOUNDARY_FP16):
         with pytest.raises(RuntimeError, match="boundary saving with fp32 strips"):
             _lib.call("sweep_b200_vti3d_sizes", d, mode, 10, ws, tape)
