@@ -105,13 +105,14 @@ E_NZ, E_NX, E_NT, E_DT, E_DH, E_ABCN = 400, 1200, 4000, 0.0005, 5.0, 40
 E_NSHOT, E_NREC, E_F0, E_DELAY = 16, 600, 10.0, 0.12
 E_RT = (E_NZ + 2 * E_ABCN + 2 * M, E_NX + 2 * E_ABCN + 2 * M)
 # algorithmic bytes per runtime cell-step: forward velocity 7 floats + stress
-# 8; reverse transpose into the adjoint velocities 3 q read, 2 p read and written
-# (7), stress reconstruction with its image 2 + 6 + 3 (11), transpose into the
-# adjoint stresses 2 p read, 2 stresses and the shear's q read and written, 2 q
-# written (10), velocity reconstruction 3 + 4 + 2 (9) (one read and one write of
-# every field a kernel touches; CPML memories, gradient slots and the shared,
-# L2-resident models not counted)
-E_BYTES_FWD, E_BYTES_REV = 60, 148
+# 8; reverse first kernel 17: 3 q read, 2 p read and written, and for the stress
+# reconstruction with its image 2 velocities and 2 adjoint stresses read, 3
+# stresses read and written; second kernel 17: 2 p read, 2 adjoint stresses and
+# the shear's q read and written, 2 q written, and for the velocity
+# reconstruction with its image 3 stresses read, 2 velocities read and written
+# (one read and one write of every field a kernel touches; CPML memories,
+# gradient slots and the shared, L2-resident models not counted)
+E_BYTES_FWD, E_BYTES_REV = 60, 136
 
 
 def elastic_survey(seed=SEED):
